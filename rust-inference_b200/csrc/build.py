@@ -44,6 +44,7 @@ SOURCES: Dict[str, Tuple[str, ...]] = {
     "pair_embedding": ("pair_embedding.cu", "common.cuh"),
     "delta_rule": ("delta_rule.cu", "common.cuh"),
     "moe": ("moe.cu", "common.cuh", "mma_helpers.cuh"),
+    "moe_tc": ("moe_tc.cu", "common.cuh", "mma_helpers.cuh"),
     "sampling": ("sampling.cu", "common.cuh"),
     "attention_decode": ("attention_decode.cu", "common.cuh", "mma_helpers.cuh", "softcap.cuh", "distance_bias.cuh", "pair_heads.cuh"),
     "attention_prefill": ("attention_prefill.cu", "common.cuh", "mma_helpers.cuh", "softcap.cuh", "distance_bias.cuh"),

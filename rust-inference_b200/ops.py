@@ -46,6 +46,9 @@ _SIGNATURES = {
     ("moe", "ri_moe_route"): [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     ("moe", "ri_moe_plan"): [_P, _P, _P, _P, _I, _I, _I, _I, _P],
     ("moe", "ri_moe_grouped_linear"): [_P, _L, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+    ("moe", "ri_moe_grouped_gated"): [_P, _L, _P, _P, _L, _P, _P, _P] + [_I] * 6 + [_F, _F, _P],
+    ("moe_tc", "ri_moe_tc"): [_P, _L, _L, _P, _P, _L, _P, _P, _P] + [_I] * 7 + [_F, _F, _P, _P],
+    ("moe_tc", "ri_moe_gather"): [_P, _L, _P, _P, _P, _I, _I, _I, _P],
     ("moe", "ri_moe_combine"): [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     ("rope_kv", "ri_qk_norm_rope_append_pairs"): [_P] * 10 + [_F, _P, _I, _I] + [_I] * 10 + [_P, _P],
     ("latent_attention", "ri_latent_prep"): [_P, _L, _I, _I] + [_P] * 8 + [_F, _P] + [_I] * 12 + [_P, _P],
@@ -1429,14 +1432,14 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, correction: Optional[torch.
     return idx, weight
 
 
-MOE_TILE_ROWS, MOE_TILE_ROWS_WIDE = 32, 64
+MOE_TILE_ROWS, MOE_TILE_ROWS_WIDE = 32, 256
 
 
 def moe_plan(idx: torch.Tensor, experts: int, wide: bool = False):
     """The step's (token, choice) pairs grouped by expert for the grouped products: (perm int32 [pairs], tiles int32
     [max_tiles, 3] of (expert, first row, rows), meta int32 [2] = (tiles, rows), rows per tile); choices >= ``experts``
-    are left out.  ``wide``: tiles of 64 rows instead of 32 (many pairs per expert; bfloat16 products whose rows are whole
-    16-byte pieces).  Everything stays on the device."""
+    are left out.  ``wide``: tiles of 256 rows instead of 32, for the tcgen05 products (many pairs per expert; bfloat16
+    products whose rows are whole 16-byte pieces).  Everything stays on the device."""
     _need(idx, "idx", torch.int32)
     pairs = idx.numel()
     bm = MOE_TILE_ROWS_WIDE if wide else MOE_TILE_ROWS
@@ -1483,9 +1486,57 @@ def moe_grouped_linear(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, ga
     if out_dtype not in (a.dtype, torch.float32):
         raise KernelError("moe_grouped_linear: the result is float32 or the compute dtype")
     y = torch.empty((rows_out, N), dtype=out_dtype, device=a.device)
+    if bm == MOE_TILE_ROWS_WIDE:
+        if gather_div > 0:
+            a = _moe_gather(a, plan, rows_out, gather_div)
+        _call("moe_tc", "ri_moe_tc", a.data_ptr(), a.shape[0], a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
+              tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], E, N, K, 1 if scatter else 0,
+              1 if out_dtype == torch.float32 else 0, 0, 0.0, 0.0, error_flag(a.device).data_ptr(), _stream())
+        return y
     _call("moe", "ri_moe_grouped_linear", a.data_ptr(), a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
           tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], int(bm), N, K, int(gather_div), 1 if scatter else 0,
           1 if out_dtype == torch.float32 else 0, _code(a.dtype), _stream())
+    return y
+
+
+def _moe_gather(x: torch.Tensor, plan, pairs: int, div: int) -> torch.Tensor:
+    """[pairs, K]: row r is x[perm[r] // div] for the plan's rows (bfloat16 rows of whole 16-byte pieces)."""
+    perm, _, meta, _ = plan
+    out = torch.empty((pairs, x.shape[1]), dtype=x.dtype, device=x.device)
+    _call("moe_tc", "ri_moe_gather", x.data_ptr(), x.stride(0), out.data_ptr(), perm.data_ptr(), meta.data_ptr(), perm.numel(), int(div),
+          x.shape[1], _stream())
+    return out
+
+
+def moe_grouped_gated(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, kind: str, limit: float = 0.0, alpha: float = 1.0,
+                      gather_div: int = 0) -> torch.Tensor:
+    """y[r] = f(gate) * up' with (gate, up) the two halves of w[e] a[in(r)] for every row r of the plan's tiles: the first
+    product of gated experts, ``w`` [E, 2 N, K] with an expert's gate rows in front of its up rows (``kind``, ``limit``,
+    ``alpha`` as for ``gated_act``; in(r) as for ``moe_grouped_linear``).  bfloat16: the products' epilogues apply the gate
+    to the float32 sums; float32: the product and ``gated_act`` one after the other."""
+    perm, tiles, meta, bm = plan
+    if kind not in GATES:
+        raise KernelError(f"gate {kind!r} is not built (known: {', '.join(sorted(GATES))})")
+    if a.dtype != torch.bfloat16:
+        return gated_act(moe_grouped_linear(a, w, plan, rows_out, gather_div=gather_div), kind, None, limit, alpha)
+    _need(a, "a")
+    _need(w, "w", a.dtype)
+    E, two, K = w.shape
+    if a.dim() != 2 or a.shape[1] != K or two % 2:
+        raise KernelError(f"moe_grouped_gated: a {tuple(a.shape)} and w {tuple(w.shape)} do not fit")
+    N = two // 2
+    if bm != MOE_TILE_ROWS_WIDE:
+        y = torch.empty((rows_out, N), dtype=a.dtype, device=a.device)
+        _call("moe", "ri_moe_grouped_gated", a.data_ptr(), a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
+              tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], int(bm), N, K, int(gather_div), GATES[kind] + 1, float(limit),
+              float(alpha), _stream())
+        return y
+    if gather_div > 0:
+        a = _moe_gather(a, plan, rows_out, gather_div)
+    y = torch.empty((rows_out, N), dtype=a.dtype, device=a.device)
+    _call("moe_tc", "ri_moe_tc", a.data_ptr(), a.shape[0], a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
+          tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], E, N, K, 0, 0, GATES[kind] + 1, float(limit),
+          float(alpha), error_flag(a.device).data_ptr(), _stream())
     return y
 
 

@@ -13,8 +13,8 @@ gated feed-forwards of one record (``parts/mlp.py``'s "gated" kind gives the for
 [experts, ...] at load.  ``shared`` is a feed-forward part of its own that every token takes.
 
 Order of work: router and choice (``ops.moe_route``); the step's (token, choice) pairs grouped by expert, on the device
-(``ops.moe_plan``); gate and up of every pair as one grouped product over the experts' tiles, the gate function, the down
-product scattered back to the pairs' places (``ops.moe_grouped_linear``, ``ops.gated_act``); the weighted sum over a
+(``ops.moe_plan``); gate and up of every pair as one grouped product over the experts' tiles with the gate function
+(``ops.moe_grouped_gated``), the down product scattered back to the pairs' places (``ops.moe_grouped_linear``); the weighted sum over a
 token's choices with the identity experts and the shared output (``ops.moe_combine``).  Nothing comes back to the host,
 so one-token steps replay from a graph.
 """
@@ -94,7 +94,7 @@ class MixtureOfExperts(FeedForward):
         s, ex = self.spec, self.spec.expert
         T = x.shape[0]
         with section("moe router"):
-            # many pairs per expert (a prompt): tiles of 64 rows, where the bfloat16 kernel for them takes the sizes
+            # many pairs per expert (a prompt): tiles of 256 rows, where the tcgen05 kernel for them takes the sizes
             wide = (x.dtype == torch.bfloat16 and T * s.top >= 48 * s.experts and s.hidden_size % 8 == 0
                     and ex.intermediate_size % 8 == 0)
             if self.by_table:
@@ -106,8 +106,7 @@ class MixtureOfExperts(FeedForward):
                                             getattr(s, "route_scale", 1.0), getattr(s, "renormalize", True), bias=self.router_bias)
                 plan = ops.moe_plan(idx, s.experts, wide)
         with section("moe experts"):
-            gu = ops.moe_grouped_linear(x, self.gate_up, plan, T * s.top, gather_div=s.top)
-            act = ops.gated_act(gu, ex.gate, None, ex.limit, ex.alpha)
+            act = ops.moe_grouped_gated(x, self.gate_up, plan, T * s.top, ex.gate, ex.limit, ex.alpha, gather_div=s.top)
             if weight is None and s.top == 1 and self.shared is None:
                 # one expert of weight 1: its output is the token's
                 return ops.moe_grouped_linear(act, self.down, plan, T, scatter=True)
