@@ -6,10 +6,10 @@
 // then per head  y_t = o_t / sqrt(mean_j(o_t[j]^2) + eps) * gain * silu(g_t)   (`gla_head_norm_gate`).
 //
 // `gla_recurrent`: a block owns one (sequence, head, tile of value columns j) and walks the sequence's new
-// tokens in order; a thread owns one column of the state (in registers for heads of up to 128 key channels, else in
-// shared memory), loaded from / stored to the sequence's slot of the state tensor at the ends.  The decay is computed as
-// exp(log_sigmoid(z) / tau) with float32 functions; q, k, v and z come from bfloat16 or float32 projections and
-// are widened once.  A token's result depends on the tokens before it only through the state, so prompts,
+// tokens in order with its part of the state in registers (heads of up to 128 key channels) or in shared memory, loaded
+// from / stored to the sequence's slot of the state tensor at the ends.  The decay is computed as
+// exp(log_sigmoid(z) / tau) with float32 functions (for prompts by `gla_decay`, once for all blocks of a head); q, k, v and z
+// come from bfloat16 or float32 projections and are widened once.  A token's result depends on the tokens before it only through the state, so prompts,
 // pieces of prompts and single tokens give the same bits.
 //
 // The same kernels run a second form (`gates` given): one decay per token and head instead of one per key channel, and
@@ -25,7 +25,6 @@
 #include "common.cuh"
 
 #define GLA_TILE 64
-#define GLA_COLS 256            // threads per block of the register kernel
 
 __device__ __forceinline__ float gla_decay(float z, float inv_tau) {
     // log(sigmoid(z)) = min(z, 0) - log1p(exp(-|z|))
@@ -33,184 +32,417 @@ __device__ __forceinline__ float gla_decay(float z, float inv_tau) {
     return expf(ls * inv_tau);
 }
 
-// The kernel for heads of up to 128 key channels.  A block of 256 threads owns 16 value columns of the state, and
-// sixteen threads share a column: each keeps a sixteenth of the column's key channels in registers (DIMC / 16 of
-// them, DIMC the head's key channels rounded up to 64 or 128; channels past `dim` hold zeros and stay zero).  The
-// sixteen are four neighbouring lanes in each of four warps (part p = 4 (warp % 4) + lane % 4 has channels
-// 64 c + 4 p .. + 3 for c = 0, 1, ..; warps 4 i .. 4 i + 3 own columns 8 i .. 8 i + 7), so that a warp's loads and
-// stores of the state cover 8 neighbouring columns, and what the block stages per token serves 16 columns.
-// Many small threads instead of few large ones: the recurrence has little to do in parallel (heads x columns), and
-// this way a prompt of one sequence still puts some warps on every SM.
-// The block stages the decay, key and scaled query of GROUP tokens in shared memory (two buffers): the loads of the
-// next group are on their way while the current group is computed, and the decay's exponentials are taken when a
-// group is stored.  A group that the sequence does not fill is padded with tokens of decay 1 and key 0, which leave
-// the state as it is, bit for bit.  A thread walks its channels in the outer loop and the group's tokens in the
-// inner one,
-//     S[d] = a_g[d] S[d] + k_g[d] v_g;  acc_g += S[d] q_g[d]            g = 0 .. GROUP-1
-// so that neighbouring instructions belong to different accumulators; at the end of the group the partial sums are
-// added: the four lanes of a warp by shuffles (pairs first, then the pairs), the four warps through shared memory in
-// warp order.  Every token's sum thus has one order that depends on the head's size only: prompts, pieces of
-// prompts and single tokens give the same bits (GROUP = 1, for steps in which every sequence brings one token,
-// walks the same order).
-#define GLA_SPLIT 4             // lanes of a warp that share a column
-#define GLA_WARPS 4             // ... and warps
-#define GLA_BCOLS (GLA_COLS / GLA_SPLIT / GLA_WARPS)
-template <typename T, int DIMC, int GROUP>
-__global__ void __launch_bounds__(GLA_COLS)
-gla_recurrent_reg_kernel(const T* __restrict__ proj, long long ld, int q_col, int k_col, int v_col,
-                         const T* __restrict__ z, const float* __restrict__ bias, float inv_tau, float qscale,
-                         float* __restrict__ state, float* __restrict__ o, const int* __restrict__ seq_slot,
-                         const int* __restrict__ seq_start, int H, int dim, int vdim_in, const float* __restrict__ gates,
-                         int gate_pitch, int ones) {
-    const int vdim = vdim_in + ones;                                         // columns of the state and of the output
-    constexpr int PARTS = GLA_SPLIT * GLA_WARPS;
-    constexpr int CH = DIMC / PARTS;                                         // channels per thread
-    constexpr int BCOLS = GLA_BCOLS;                                         // columns per block
-    static_assert(CH % 4 == 0 && GLA_COLS % (32 * GLA_WARPS) == 0, "whole float4s per thread; sets of four warps");
-    extern __shared__ __align__(16) float gla_dyn[];
-    float (*stage)[GROUP][3][DIMC] = reinterpret_cast<float (*)[GROUP][3][DIMC]>(gla_dyn);                 // [2]
-    float (*stage_v)[GROUP][BCOLS] = reinterpret_cast<float (*)[GROUP][BCOLS]>(gla_dyn + 2 * GROUP * 3 * DIMC);   // [2]
-    float (*partial)[GROUP][BCOLS][GLA_WARPS] =
-        reinterpret_cast<float (*)[GROUP][BCOLS][GLA_WARPS]>(gla_dyn + 2 * GROUP * 3 * DIMC + 2 * GROUP * BCOLS);  // [2]
-    constexpr int PER = (GROUP * DIMC + GLA_COLS - 1) / GLA_COLS;            // staged elements per thread and array
-    constexpr int VPER = (GROUP * BCOLS + GLA_COLS - 1) / GLA_COLS;          // staged values per thread
+// two float32 multiply-adds (products) per instruction, each rounded as fmaf (a product) rounds it
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 gla_fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 gla_mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 gla_pack2(float x, float y) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ void gla_unpack2(f32x2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+
+// eight neighbouring elements as they come from memory, widened (and cleared where they are not the token's own) only when they
+// are stored into a buffer.  VEC: on 16 bytes.
+template <typename T, bool VEC>
+struct GlaPiece {
+    alignas(16) T v[8];
+    __device__ __forceinline__ void load(const T* p, int valid) {            // valid: elements that may be read, at least 1
+        if (VEC) {
+#pragma unroll
+            for (int i = 0; i < (int)(sizeof(T) / 2); i++) reinterpret_cast<uint4*>(v)[i] = reinterpret_cast<const uint4*>(p)[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = p[min(i, valid - 1)];
+        }
+    }
+};
+
+// exp(log_sigmoid(z + bias) / tau) of a prompt's tokens: float32 [tokens, HD], HD = heads x key channels
+template <typename T>
+__global__ void __launch_bounds__(256)
+gla_decay_kernel(const T* z, const float* __restrict__ bias, float inv_tau, float* __restrict__ decay, int HD) {
     pdl_trigger();
-    const int b = blockIdx.z, h = blockIdx.y;
+    const int d = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const float b0 = d < HD ? bias[d] : 0.0f, b1 = d + 1 < HD ? bias[d + 1] : 0.0f;
+    pdl_wait();
+    const size_t at = (size_t)blockIdx.y * HD + d;
+    if (d < HD) decay[at] = gla_decay(ld_f(z + at) + b0, inv_tau);
+    if (d + 1 < HD) decay[at + 1] = gla_decay(ld_f(z + at + 1) + b1, inv_tau);
+}
+
+// BYTES from global to shared memory without a register in between
+template <int BYTES>
+__device__ __forceinline__ void gla_copy(void* dst, const void* src) {
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// Barriers between the computing and the staging warps of a block: `arrive` goes on, `sync` waits for everybody
+__device__ __forceinline__ void gla_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void gla_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// The kernel for heads of up to 128 key channels (DIMC: that rounded up to 64 or 128; channels past `dim` hold zeros and stay
+// zero).  What bounds it: reading a token's vectors from shared memory, 32 words a cycle for an SM whether the lanes of a warp
+// want the same words or not, and the multiply-adds, three per element of the state and token.  A thread keeps four key channels
+// of four neighbouring columns in registers, LP = DIMC / 4 lanes share the columns: per token 16 words for 24
+// instructions of two multiply-adds (eight channels of one column: 26 words for 12, 243 cycles of shared memory a token and SM
+// where this takes some 80).  A block's four computing warps, one for each scheduler of an SM, own 512 / LP columns; a
+// head of 64 x 128 is four blocks.
+// Four more warps of the block stage GROUP tokens at a time into a ring of GLA_RING buffers and write the outputs of the groups
+// that have been computed, so that nothing of a group's trip to memory, its conversions and its outputs stands between the
+// tokens.  The copies of GLA_AHEAD groups are on their way together (cp.async into slots of the thread's own, widened from there:
+// with the next group's loads in registers every group of 16 tokens took a trip to memory, 2.5 us).  A group that the sequence
+// does not fill is padded with tokens of decay 1 and key 0, which leave the state as it is, bit for bit.
+//     S[d, j] = a[d] S[d, j] + k[d] v[j];  acc_j += S[d, j] q[d]
+// A thread's sum of a column runs over its channels in order (even and odd ones apart, then added); the LP lanes' sums go
+// down a tree (neighbours first), for four tokens and columns side by side: every step halves the number of sums a lane still
+// holds, so that each lane ends with one.  Every token's sum thus has one order that depends on the head's size only: prompts,
+// pieces of prompts and single tokens give the same bits (GROUP = 1, for steps in which every sequence brings one token,
+// takes the decay from z itself and walks the same order).
+// 2,048 tokens of 32 heads of 64 x 128, with the decays' kernel: 607 -> 217 us (106 ns a token); three sequences of 2,302 tokens in
+// all 645 -> 203 us; 16 heads of 128 x 129 with one decay 443 -> 280 us.  (Before: one column and four channels a thread, the
+// tokens staged and the decays taken by the same warps of every block.)
+#define GLA_CT 128              // computing threads
+#define GLA_ST 128              // staging threads
+#define GLA_RING 3
+#define GLA_AHEAD 3
+template <typename T, int DIMC, int GROUP, bool VEC>
+__global__ void __launch_bounds__(GROUP == 1 ? GLA_CT : GLA_CT + GLA_ST)
+gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, const T* z, const float* __restrict__ bias,
+                float inv_tau, float qscale, const float* decay, float* state, float* __restrict__ o,
+                const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int H, int dim, int vdim_in, const float* gates,
+                int gate_pitch, int ones) {
+    constexpr bool SINGLE = GROUP == 1;
+    constexpr int LP = DIMC / 4;                                             // lanes that share four columns
+    constexpr int WCOLS = 4 * (32 / LP), BCOLS = 4 * (GLA_CT / LP);          // columns per warp and per block
+    constexpr int KP = DIMC / 8, VP = BCOLS / 8;                             // staged pieces of eight per token
+    constexpr int PER = (GROUP * KP + GLA_ST - 1) / GLA_ST;                  // ... and per thread
+    static_assert(GROUP * VP <= GLA_ST && (SINGLE || GROUP % 4 == 0), "a piece of values per thread; tokens in fours");
+    constexpr int ROW = 3 * DIMC + BCOLS;                                    // a staged token: decay, key, query, values
+    constexpr int ALL = GLA_CT + GLA_ST;
+    extern __shared__ __align__(16) float gla_dyn[];                         // [ring][GROUP][ROW], outputs [ring][GROUP][BCOLS]
+    const int vdim = vdim_in + ones;                                         // columns of the state and of the output
+    const int b = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * BCOLS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wpart = warp % GLA_WARPS;                                      // this warp's share of the channels
-    const int col = (warp / GLA_WARPS) * (32 / GLA_SPLIT) + lane / GLA_SPLIT, part = wpart * GLA_SPLIT + lane % GLA_SPLIT;
-    const int j = blockIdx.x * BCOLS + col;
-    const bool mine = j < vdim;
+    if (SINGLE) pdl_trigger();
     const int t0 = seq_start[b], t1 = seq_start[b + 1];
     const int slot = seq_slot[b];
-    float bs[PER];
-#pragma unroll
-    for (int e = 0; e < PER; e++) {
-        const int d = (threadIdx.x + e * GLA_COLS) % DIMC;
-        bs[e] = (d < dim && !gates) ? bias[h * dim + d] : 0.0f;
-    }
     pdl_wait();
-    float* st = state + ((size_t)slot * H + h) * dim * vdim;
-    float S[CH];
-#pragma unroll
-    for (int i = 0; i < CH; i++) {
-        const int d = (i / 4) * 4 * PARTS + 4 * part + (i & 3);
-        S[i] = (mine && d < dim) ? st[(size_t)d * vdim + j] : 0.0f;
-    }
-    // as they come from memory (widened only when they are stored into a buffer, so that nothing waits for a load
-    // before the group at hand has been computed)
-    T rz[PER], rk[PER], rq[PER], rv[VPER];
-    float ra[PER], rb[PER];                   // the second form's decay and key factor of the element's token
+    if (t0 >= t1) return;                     // (a sequence without tokens keeps its state; the whole block leaves)
+
+    const int st_id = SINGLE ? threadIdx.x : threadIdx.x - GLA_CT;           // among the staging threads
+    GlaPiece<T, VEC> rk[PER], rq[PER], rz[SINGLE ? PER : 1], rv;
+    GlaPiece<float, VEC> ra[SINGLE ? 1 : PER];
+    float ga[PER], gb[PER];
+    // Loads are never under a condition (a load that is gets waited for where it stands): past the group, the sequence or the
+    // head something that exists is read and left out by `store`.
     auto fetch = [&](int base) {              // the raw values of tokens base .. base + GROUP - 1 into registers
 #pragma unroll
         for (int e = 0; e < PER; e++) {
-            const int idx = threadIdx.x + e * GLA_COLS;
-            const int g = idx / DIMC, d = idx % DIMC, t = base + g;
-            rz[e] = rk[e] = rq[e] = T(0.0f);
-            ra[e] = rb[e] = 1.0f;
-            if (g < GROUP && t < t1 && d < dim) {
-                const T* row = proj + (size_t)t * ld;
-                if (gates) {
-                    ra[e] = gates[((size_t)t * H + h) * gate_pitch];
-                    rb[e] = gates[((size_t)t * H + h) * gate_pitch + 1];
-                } else {
-                    rz[e] = z[((size_t)t * H + h) * dim + d];
-                }
-                rk[e] = row[k_col + h * dim + d];
-                rq[e] = row[q_col + h * dim + d];
+            const int idx = st_id + e * GLA_ST;
+            const int t = min(base + idx / KP, t1 - 1), d = (idx % KP) * 8 < dim ? (idx % KP) * 8 : 0;
+            const T* row = proj + (size_t)t * ld + h * dim + d;
+            rk[e].load(row + k_col, dim - d);
+            rq[e].load(row + q_col, dim - d);
+            if (gates) {
+                ga[e] = gates[((size_t)t * H + h) * gate_pitch];
+                gb[e] = gates[((size_t)t * H + h) * gate_pitch + 1];
+            } else if (SINGLE) {
+                rz[e].load(z + ((size_t)t * H + h) * dim + d, dim - d);
+            } else {
+                ra[e].load(decay + ((size_t)t * H + h) * dim + d, dim - d);
             }
         }
-        // the values: thread i takes token i / BCOLS of the group, column i % BCOLS (and so on, GLA_COLS further)
-#pragma unroll
-        for (int e = 0; e < VPER; e++) {
-            const int idx = threadIdx.x + e * GLA_COLS;
-            const int g = idx / BCOLS, jj = blockIdx.x * BCOLS + idx % BCOLS;
-            rv[e] = T(0.0f);
-            if (g < GROUP && base + g < t1 && jj < vdim_in) rv[e] = proj[(size_t)(base + g) * ld + v_col + h * vdim_in + jj];
-            else if (g < GROUP && base + g < t1 && jj < vdim) rv[e] = T(1.0f);          // the column of ones
-        }
+        const int t = min(base + st_id / VP, t1 - 1), jj = min(j0 + (st_id % VP) * 8, (vdim_in - 1) & ~7);
+        rv.load(proj + (size_t)t * ld + v_col + h * vdim_in + jj, vdim_in - jj);
     };
     auto store = [&](int buf, int base) {     // ... and from there into a buffer
+        float* to = gla_dyn + buf * GROUP * ROW;
 #pragma unroll
         for (int e = 0; e < PER; e++) {
-            const int idx = threadIdx.x + e * GLA_COLS;
-            const int g = idx / DIMC, d = idx % DIMC;
+            const int idx = st_id + e * GLA_ST;
+            const int g = idx / KP, d = (idx % KP) * 8;
             if (g < GROUP) {
                 // a token past the sequence's end: decay 1, key 0 (the state stays); a channel past dim: all zero
                 const bool live = base + g < t1;
-                stage[buf][g][0][d] = d < dim ? (live ? (gates ? ra[e] : gla_decay(ld_f(&rz[e]) + bs[e], inv_tau)) : 1.0f) : 0.0f;
-                stage[buf][g][1][d] = gates ? ld_f(&rk[e]) * rb[e] : ld_f(&rk[e]);
-                stage[buf][g][2][d] = ld_f(&rq[e]) * qscale;
+                float a[8], k[8], q[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const bool own = d + i < dim;
+                    k[i] = !(live && own) ? 0.0f : gates ? ld_f(&rk[e].v[i]) * gb[e] : ld_f(&rk[e].v[i]);
+                    q[i] = !(live && own) ? 0.0f : ld_f(&rq[e].v[i]) * qscale;
+                    if (gates) a[i] = ga[e];
+                    else if (SINGLE) a[i] = gla_decay(ld_f(&rz[e].v[i]) + (own ? bias[h * dim + d + i] : 0.0f), inv_tau);
+                    else a[i] = ra[e].v[i];
+                    a[i] = !own ? 0.0f : live ? a[i] : 1.0f;
+                }
+                float* row = to + g * ROW + d;
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) {
+                    *reinterpret_cast<float4*>(row + i) = make_float4(a[i], a[i + 1], a[i + 2], a[i + 3]);
+                    *reinterpret_cast<float4*>(row + DIMC + i) = make_float4(k[i], k[i + 1], k[i + 2], k[i + 3]);
+                    *reinterpret_cast<float4*>(row + 2 * DIMC + i) = make_float4(q[i], q[i + 1], q[i + 2], q[i + 3]);
+                }
             }
         }
+        if (st_id < GROUP * VP) {
+            const int jj = j0 + (st_id % VP) * 8;
+            float* row = to + (st_id / VP) * ROW + 3 * DIMC + (st_id % VP) * 8;
+            float x[8];
 #pragma unroll
-        for (int e = 0; e < VPER; e++) {
-            const int idx = threadIdx.x + e * GLA_COLS;
-            if (idx < GROUP * BCOLS) stage_v[buf][idx / BCOLS][idx % BCOLS] = ld_f(&rv[e]);
+            for (int i = 0; i < 8; i++) x[i] = jj + i < vdim_in ? ld_f(&rv.v[i]) : jj + i < vdim ? 1.0f : 0.0f;      // the column of ones
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(row + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
         }
     };
-    auto reduce = [&](int buf, int base) {    // a group's outputs: the four warps' sums in warp order
+    float* outs = gla_dyn + GLA_RING * GROUP * ROW;
+    if (!SINGLE && threadIdx.x >= GLA_CT) {
+        // ---- the staging warps.  Barriers 1 + buf: the buffer is full; 1 + GLA_RING + buf: it was read, its outputs are there ----------
+        // VEC: this thread's pieces of the groups on their way, [GLA_AHEAD][16 bytes of a piece][staging thread]
+        constexpr int PT = sizeof(T) / 2;                                    // 16-byte pieces of eight elements
+        constexpr int EACH = 2 * PT + 2, SLOT = PER * EACH + PT;
+        uint4* raw = reinterpret_cast<uint4*>(outs + GLA_RING * GROUP * BCOLS);
+        auto piece16 = [&](int slot_, int i) -> uint4& { return raw[(slot_ * SLOT + i) * GLA_ST + st_id]; };
+        auto issue = [&](int slot_, int base) {
 #pragma unroll
-        for (int e = 0; e < VPER; e++) {
-            const int idx = threadIdx.x + e * GLA_COLS;
-            if (idx < GROUP * BCOLS) {
-                const int g = idx / BCOLS, c = idx % BCOLS, jj = blockIdx.x * BCOLS + c;
-                float acc = partial[buf][g][c][0];
+            for (int e = 0; e < PER; e++) {
+                const int idx = st_id + e * GLA_ST;
+                const int t = min(base + idx / KP, t1 - 1), d = (idx % KP) * 8 < dim ? (idx % KP) * 8 : 0;
+                const T* row = proj + (size_t)t * ld + h * dim + d;
 #pragma unroll
-                for (int w = 1; w < GLA_WARPS; w++) acc += partial[buf][g][c][w];
-                if (jj < vdim && base + g < t1) o[((size_t)(base + g) * H + h) * vdim + jj] = acc;
+                for (int i = 0; i < PT; i++) {
+                    gla_copy<16>(&piece16(slot_, e * EACH + i), reinterpret_cast<const uint4*>(row + k_col) + i);
+                    gla_copy<16>(&piece16(slot_, e * EACH + PT + i), reinterpret_cast<const uint4*>(row + q_col) + i);
+                }
+                if (!gates) {
+                    const float* dec = decay + ((size_t)t * H + h) * dim + d;
+                    gla_copy<16>(&piece16(slot_, e * EACH + 2 * PT), dec);
+                    gla_copy<16>(&piece16(slot_, e * EACH + 2 * PT + 1), dec + 4);
+                } else {
+                    const float* two = gates + ((size_t)t * H + h) * gate_pitch;
+                    gla_copy<4>(&piece16(slot_, e * EACH + 2 * PT).x, two);
+                    gla_copy<4>(&piece16(slot_, e * EACH + 2 * PT).y, two + 1);
+                }
             }
+            const int t = min(base + st_id / VP, t1 - 1), jj = min(j0 + (st_id % VP) * 8, (vdim_in - 1) & ~7);
+#pragma unroll
+            for (int i = 0; i < PT; i++)
+                gla_copy<16>(&piece16(slot_, PER * EACH + i), reinterpret_cast<const uint4*>(proj + (size_t)t * ld + v_col + h * vdim_in + jj) + i);
+        };
+        auto take = [&](int slot_) {          // a slot's pieces into the registers that `store` widens
+#pragma unroll
+            for (int e = 0; e < PER; e++) {
+#pragma unroll
+                for (int i = 0; i < PT; i++) {
+                    reinterpret_cast<uint4*>(rk[e].v)[i] = piece16(slot_, e * EACH + i);
+                    reinterpret_cast<uint4*>(rq[e].v)[i] = piece16(slot_, e * EACH + PT + i);
+                }
+                const uint4 lo = piece16(slot_, e * EACH + 2 * PT);
+                if (gates) {
+                    ga[e] = __uint_as_float(lo.x);
+                    gb[e] = __uint_as_float(lo.y);
+                } else if (!SINGLE) {
+                    reinterpret_cast<uint4*>(ra[e].v)[0] = lo;
+                    reinterpret_cast<uint4*>(ra[e].v)[1] = piece16(slot_, e * EACH + 2 * PT + 1);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < PT; i++) reinterpret_cast<uint4*>(rv.v)[i] = piece16(slot_, PER * EACH + i);
+        };
+        auto write_out = [&](int buf, int base) {
+            for (int i = st_id; i < GROUP * BCOLS; i += GLA_ST) {
+                const int g = i / BCOLS, c = i % BCOLS;
+                if (base + g < t1 && j0 + c < vdim) o[((size_t)(base + g) * H + h) * vdim + j0 + c] = outs[(buf * GROUP + g) * BCOLS + c];
+            }
+        };
+        if (VEC) {
+            for (int i = 0; i < GLA_AHEAD; i++) {
+                if (t0 + i * GROUP < t1) issue(i, t0 + i * GROUP);
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+            }
+        } else {
+            fetch(t0);
+        }
+        int n = 0;
+        for (int base = t0; base < t1; base += GROUP, n++) {
+            const int buf = n % GLA_RING;
+            if (VEC) {
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(GLA_AHEAD - 1) : "memory");
+                take(n % GLA_AHEAD);
+                if (base + GLA_AHEAD * GROUP < t1) issue(n % GLA_AHEAD, base + GLA_AHEAD * GROUP);
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+            }
+            if (n >= GLA_RING) {
+                gla_bar_sync(1 + GLA_RING + buf, ALL);
+                write_out(buf, base - GLA_RING * GROUP);
+            }
+            store(buf, base);
+            gla_bar_arrive(1 + buf, ALL);
+            if (!VEC && base + GROUP < t1) fetch(base + GROUP);
+        }
+        for (int m = n > GLA_RING ? n - GLA_RING : 0; m < n; m++) {
+            gla_bar_sync(1 + GLA_RING + m % GLA_RING, ALL);
+            write_out(m % GLA_RING, t0 + m * GROUP);
+        }
+        return;
+    }
+    // ---- the computing warps ----------------------------------------------------------------------------------------------------
+    const int part = lane % LP, col = warp * WCOLS + 4 * (lane / LP);        // this thread's channels 4 part .. and columns col ..
+    const int j = j0 + col, d0 = 4 * part;
+    float* st = state + ((size_t)slot * H + h) * dim * vdim;
+    f32x2 S[4][2];                            // [column][pair of channels]
+    const bool whole = vdim % 4 == 0 && ((uintptr_t)state & 15) == 0;        // the state's rows start on 16 bytes, columns come in fours
+    float4 x4[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float* row = st + (size_t)(d0 + i) * vdim + j;
+        x4[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (d0 + i < dim) {
+            if (whole) {
+                if (j < vdim) x4[i] = *reinterpret_cast<const float4*>(row);
+            } else {
+                if (j < vdim) x4[i].x = row[0];
+                if (j + 1 < vdim) x4[i].y = row[1];
+                if (j + 2 < vdim) x4[i].z = row[2];
+                if (j + 3 < vdim) x4[i].w = row[3];
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        S[0][i] = gla_pack2(x4[2 * i].x, x4[2 * i + 1].x);
+        S[1][i] = gla_pack2(x4[2 * i].y, x4[2 * i + 1].y);
+        S[2][i] = gla_pack2(x4[2 * i].z, x4[2 * i + 1].z);
+        S[3][i] = gla_pack2(x4[2 * i].w, x4[2 * i + 1].w);
+    }
+    struct Token {                            // a token's decay, key and query (this thread's channels) and its four values
+        ulonglong2 a, k, q;
+        float4 v;
+    };
+    auto load = [&](Token& x, const float* row) {
+        x.a = *reinterpret_cast<const ulonglong2*>(row + d0);
+        x.k = *reinterpret_cast<const ulonglong2*>(row + DIMC + d0);
+        x.q = *reinterpret_cast<const ulonglong2*>(row + 2 * DIMC + d0);
+        x.v = *reinterpret_cast<const float4*>(row + 3 * DIMC + col);
+    };
+    auto token = [&](const Token& x, float* out) {
+        const float v[4] = {x.v.x, x.v.y, x.v.z, x.v.w};
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const f32x2 vv = gla_pack2(v[c], v[c]);
+            S[c][0] = gla_fma2(x.a.x, S[c][0], gla_mul2(x.k.x, vv));
+            S[c][1] = gla_fma2(x.a.y, S[c][1], gla_mul2(x.k.y, vv));
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            float lo, hi;
+            gla_unpack2(gla_fma2(S[c][1], x.q.y, gla_mul2(S[c][0], x.q.x)), lo, hi);
+            out[c] = lo + hi;
         }
     };
-    fetch(t0);
-    store(0, t0);
-    __syncthreads();
-    int buf = 0;
-    for (int base = t0; base < t1; base += GROUP) {
-        const bool more = base + GROUP < t1;
-        if (more) fetch(base + GROUP);
-        float acc[GROUP], vv[GROUP];
+    if (SINGLE) {
+        fetch(t0);
+        store(0, t0);
+        __syncthreads();
+        Token x;
+        load(x, gla_dyn);
+        float v[4];
+        token(x, v);
 #pragma unroll
-        for (int g = 0; g < GROUP; g++) {
-            acc[g] = 0.0f;
-            vv[g] = stage_v[buf][g][col];
+        for (int m = 1; m < LP; m <<= 1)
+#pragma unroll
+            for (int c = 0; c < 4; c++) v[c] += __shfl_xor_sync(0xffffffffu, v[c], m);
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (part == c && j + c < vdim) o[((size_t)t0 * H + h) * vdim + j + c] = v[c];
+    } else {
+        // the token of four and the column of four whose output this lane ends with (lanes 16 .. of 32 hold copies)
+        const int my_t = 2 * (part & 1) + ((part >> 1) & 1), my_c = 2 * ((part >> 2) & 1) + ((part >> 3) & 1);
+        int n = 0;
+        for (int base = t0; base < t1; base += GROUP, n++) {
+            const int buf = n % GLA_RING;
+            gla_bar_sync(1 + buf, ALL);
+            const float* rows = gla_dyn + buf * GROUP * ROW;
+            Token x[2];                       // the token at hand and the next one, on its way from shared memory
+            load(x[0], rows);
+#pragma unroll
+            for (int g = 0; g < GROUP; g += 4) {
+                float v[16];
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    if (g + t + 1 < GROUP) load(x[(t + 1) & 1], rows + (g + t + 1) * ROW);
+                    token(x[t & 1], v + 4 * t);
+                }
+#pragma unroll
+                for (int m = 1, k = 8; m < 16; m <<= 1, k >>= 1) {
+                    const bool upper = (lane & m) != 0;
+#pragma unroll
+                    for (int i = 0; i < k; i++) {
+                        const float give = upper ? v[i] : v[i + k], keep = upper ? v[i + k] : v[i];
+                        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+                    }
+                }
+                if (LP == 32) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+                if (part < 16) outs[(buf * GROUP + g + my_t) * BCOLS + col + my_c] = v[0];
+            }
+            gla_bar_arrive(1 + GLA_RING + buf, ALL);
         }
+        pdl_trigger();                        // the next kernel may come in once the walk is over
+    }
 #pragma unroll
-        for (int c = 0; c < CH / 4; c++) {
+    for (int i = 0; i < 4; i++) {
+        float x[4], y[4];
 #pragma unroll
-            for (int g = 0; g < GROUP; g++) {
-                const int at = (c * PARTS + part) * 4;
-                const float4 a = *reinterpret_cast<const float4*>(&stage[buf][g][0][at]);
-                const float4 k = *reinterpret_cast<const float4*>(&stage[buf][g][1][at]);
-                const float4 q = *reinterpret_cast<const float4*>(&stage[buf][g][2][at]);
-                S[4 * c] = fmaf(a.x, S[4 * c], k.x * vv[g]);
-                acc[g] = fmaf(S[4 * c], q.x, acc[g]);
-                S[4 * c + 1] = fmaf(a.y, S[4 * c + 1], k.y * vv[g]);
-                acc[g] = fmaf(S[4 * c + 1], q.y, acc[g]);
-                S[4 * c + 2] = fmaf(a.z, S[4 * c + 2], k.z * vv[g]);
-                acc[g] = fmaf(S[4 * c + 2], q.z, acc[g]);
-                S[4 * c + 3] = fmaf(a.w, S[4 * c + 3], k.w * vv[g]);
-                acc[g] = fmaf(S[4 * c + 3], q.w, acc[g]);
+        for (int c = 0; c < 4; c++) gla_unpack2(S[c][i / 2], x[c], y[c]);
+        const float4 w = i & 1 ? make_float4(y[0], y[1], y[2], y[3]) : make_float4(x[0], x[1], x[2], x[3]);
+        float* row = st + (size_t)(d0 + i) * vdim + j;
+        if (d0 + i < dim) {
+            if (whole) {
+                if (j < vdim) *reinterpret_cast<float4*>(row) = w;
+            } else {
+                if (j < vdim) row[0] = w.x;
+                if (j + 1 < vdim) row[1] = w.y;
+                if (j + 2 < vdim) row[2] = w.z;
+                if (j + 3 < vdim) row[3] = w.w;
             }
         }
-#pragma unroll
-        for (int g = 0; g < GROUP; g++) {
-            acc[g] += __shfl_xor_sync(0xffffffffu, acc[g], 1);
-            acc[g] += __shfl_xor_sync(0xffffffffu, acc[g], 2);
-            if (lane % GLA_SPLIT == 0) partial[buf][g][col][wpart] = acc[g];
-        }
-        if (more) store(buf ^ 1, base + GROUP);
-        __syncthreads();              // the next group is staged, this one's partial sums are written
-        reduce(buf, base);            // (the next group writes the other buffer of partial sums)
-        buf ^= 1;
     }
-    if (mine) {
-#pragma unroll
-        for (int i = 0; i < CH; i++) {
-            const int d = (i / 4) * 4 * PARTS + 4 * part + (i & 3);
-            if (d < dim) st[(size_t)d * vdim + j] = S[i];
-        }
+}
+
+template <typename T, int DIMC, int GROUP, bool VEC>
+static int gla_walk_go(const void* proj, long long ld, int q_col, int k_col, int v_col, const void* z, const float* bias, float tau,
+                       float qscale, const float* decay, float* state, float* o, const int* seq_slot, const int* seq_start, int seqs,
+                       int H, int dim, int vdim_in, const float* gates, int gate_pitch, int ones, cudaStream_t stream) {
+    constexpr int BCOLS = GLA_CT * 16 / DIMC, PER = (GROUP * (DIMC / 8) + GLA_ST - 1) / GLA_ST, PT = sizeof(T) / 2;
+    constexpr size_t RAW = GROUP > 1 && VEC ? (size_t)GLA_AHEAD * (PER * (2 * PT + 2) + PT) * GLA_ST * 16 : 0;      // the slots of pieces
+    constexpr size_t sm = (GROUP == 1 ? (size_t)(3 * DIMC + BCOLS) : (size_t)GLA_RING * GROUP * (3 * DIMC + 2 * BCOLS)) * sizeof(float) + RAW;
+    const dim3 grid((vdim_in + ones + BCOLS - 1) / BCOLS, H, seqs);
+    if (sm > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(gla_walk_kernel<T, DIMC, GROUP, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e != cudaSuccess) RI_FAIL((int)e, "gla_recurrent: %s", cudaGetErrorString(e));
     }
+    // A prompt's kernel is launched the ordinary way, not as a dependent launch: its long-lived blocks must spread over the
+    // SMs, and blocks that come in while the kernel before still holds most SMs pile up on the first that get free.
+    if (GROUP == 1)
+        ri_launch_pdl(gla_walk_kernel<T, DIMC, GROUP, VEC>, grid, dim3(GLA_CT), sm, stream, (const T*)proj, ld, q_col, k_col, v_col,
+                      (const T*)z, bias, 1.0f / tau, qscale, decay, state, o, seq_slot, seq_start, H, dim, vdim_in, gates, gate_pitch, ones);
+    else
+        gla_walk_kernel<T, DIMC, GROUP, VEC><<<grid, dim3(GLA_CT + GLA_ST), sm, stream>>>((const T*)proj, ld, q_col, k_col, v_col, (const T*)z,
+                      bias, 1.0f / tau, qscale, decay, state, o, seq_slot, seq_start, H, dim, vdim_in, gates, gate_pitch, ones);
+    RI_CHECK_LAUNCH("gla_recurrent");
+    return 0;
 }
 
 // Any number of key channels: the state tile [dim][GLA_TILE] lives in shared memory.
@@ -258,10 +490,10 @@ gla_recurrent_kernel(const T* __restrict__ proj, long long ld, int q_col, int k_
 }
 
 static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col, int v_col, const void* z,
-                            const float* bias, float tau, float qscale, float* state, float* o, const int* seq_slot,
-                            const int* seq_start, int seqs, int H, int dim, int vdim_in, int single, int dtype,
+                            const float* bias, float tau, float qscale, float* decay, float* state, float* o, const int* seq_slot,
+                            const int* seq_start, int tokens, int seqs, int H, int dim, int vdim_in, int single, int dtype,
                             const float* gates, int gate_pitch, int ones, cudaStream_t stream) {
-    // single: every sequence brings one token (a smaller staging group; the same results)
+    // single: every sequence brings one token (no staging of groups; the same results)
     if (seqs == 0) return 0;
     const int vdim = vdim_in + ones;                 // what the grid covers
     RI_REQUIRE(seqs > 0 && H > 0 && dim > 0 && vdim_in > 0 && tau > 0.0f, "gla_recurrent: bad sizes");
@@ -269,37 +501,36 @@ static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col
     RI_REQUIRE(seqs <= 65535 && H <= 65535, "gla_recurrent: %d sequences, %d heads: too many for one launch", seqs, H);
     RI_REQUIRE(dtype == RI_DTYPE_F32 || dtype == RI_DTYPE_BF16, "gla_recurrent: unknown dtype %d", dtype);
     if (dim <= 128) {
-        const int threads = GLA_COLS;             // all of them stage the tokens, whatever the number of columns
-        const dim3 grid((vdim + GLA_BCOLS - 1) / GLA_BCOLS, H, seqs);
-#define GLA_REG1(T, DIMC, GROUP)                                                                                           \
-        do {                                                                                                               \
-            const size_t sm = (size_t)(2 * GROUP * 3 * DIMC + 2 * GROUP * GLA_BCOLS * (1 + GLA_WARPS)) * sizeof(float);    \
-            cudaError_t e = sm > 48 * 1024 ? cudaFuncSetAttribute(gla_recurrent_reg_kernel<T, DIMC, GROUP>,                \
-                                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)   \
-                                           : cudaSuccess;                                                                  \
-            if (e != cudaSuccess) RI_FAIL((int)e, "gla_recurrent: %s", cudaGetErrorString(e));                             \
-            ri_launch_pdl(gla_recurrent_reg_kernel<T, DIMC, GROUP>, grid, dim3(threads), sm, stream, (const T*)proj, ld,   \
-                          q_col, k_col, v_col, (const T*)z, bias, 1.0f / tau, qscale, state, o, seq_slot, seq_start, H,    \
-                          dim, vdim_in, gates, gate_pitch, ones);                                                          \
+        if (!gates && !single) {
+            RI_REQUIRE(decay || tokens == 0, "gla_recurrent: a prompt needs room for its decays");
+            const int HD = H * dim;
+            for (int t = 0; t < tokens; t += 65535) {        // (a grid's second dimension)
+                const dim3 g((HD + 511) / 512, tokens - t < 65535 ? tokens - t : 65535);
+                const size_t at = (size_t)t * HD;
+                if (dtype == RI_DTYPE_F32)
+                    ri_launch_pdl(gla_decay_kernel<float>, g, dim3(256), 0, stream, (const float*)z + at, bias, 1.0f / tau, decay + at, HD);
+                else
+                    ri_launch_pdl(gla_decay_kernel<__nv_bfloat16>, g, dim3(256), 0, stream, (const __nv_bfloat16*)z + at, bias, 1.0f / tau,
+                                  decay + at, HD);
+                RI_CHECK_LAUNCH("gla_decay");
+            }
+        }
+        const bool vec = dim % 8 == 0 && vdim_in % 8 == 0 && ld % 8 == 0 && q_col % 8 == 0 && k_col % 8 == 0 && v_col % 8 == 0 &&
+                         (((uintptr_t)proj | (uintptr_t)z | (uintptr_t)decay) & 15) == 0;
+#define GLA_GO3(T, DIMC, GROUP, VEC)                                                                                           \
+        return gla_walk_go<T, DIMC, GROUP, VEC>(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, decay, state, o, seq_slot, \
+                                                seq_start, seqs, H, dim, vdim_in, gates, gate_pitch, ones, stream)
+#define GLA_GO2(T, DIMC)                                                                                                       \
+        do {                                                                                                                   \
+            if (single) { if (vec) GLA_GO3(T, DIMC, 1, true); else GLA_GO3(T, DIMC, 1, false); }                               \
+            else { if (vec) GLA_GO3(T, DIMC, 16, true); else GLA_GO3(T, DIMC, 16, false); }                                    \
         } while (0)
-    // tokens staged together: many, so that a trip to memory is paid once per 32 (16) tokens
-#define GLA_REG(T, DIMC)                                                                                                   \
-        do {                                                                                                               \
-            if (single) GLA_REG1(T, DIMC, 1);                                                                              \
-            else GLA_REG1(T, DIMC, (DIMC > 64 ? 16 : 32));                                                                 \
-        } while (0)
-#define GLA_BY_DIM(T)                                                                                                      \
-        do {                                                                                                               \
-            if (dim <= 64) GLA_REG(T, 64);                                                                                 \
-            else GLA_REG(T, 128);                                                                                          \
-        } while (0)
-        if (dtype == RI_DTYPE_F32) GLA_BY_DIM(float);
-        else GLA_BY_DIM(__nv_bfloat16);
-#undef GLA_BY_DIM
-#undef GLA_REG
-#undef GLA_REG1
-        RI_CHECK_LAUNCH("gla_recurrent");
-        return 0;
+#define GLA_GO1(T) do { if (dim <= 64) GLA_GO2(T, 64); else GLA_GO2(T, 128); } while (0)
+        if (dtype == RI_DTYPE_F32) GLA_GO1(float);
+        else GLA_GO1(__nv_bfloat16);
+#undef GLA_GO1
+#undef GLA_GO2
+#undef GLA_GO3
     }
     const size_t smem = ((size_t)dim * GLA_TILE + 6 * (size_t)dim) * sizeof(float);
     RI_REQUIRE(smem <= 200 * 1024, "gla_recurrent: %d key channels per head do not fit in shared memory", dim);
@@ -320,12 +551,13 @@ static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col
     return 0;
 }
 
+// decay: float32 scratch [tokens, H, dim] that a call for prompts (not `single`) with up to 128 key channels fills
 extern "C" int ri_gla_recurrent(const void* proj, long long ld, int q_col, int k_col, int v_col, const void* z,
-                                const float* bias, float tau, float qscale, float* state, float* o, const int* seq_slot,
-                                const int* seq_start, int seqs, int H, int dim, int vdim, int single, int dtype,
+                                const float* bias, float tau, float qscale, float* decay, float* state, float* o, const int* seq_slot,
+                                const int* seq_start, int tokens, int seqs, int H, int dim, int vdim, int single, int dtype,
                                 cudaStream_t stream) {
-    return gla_recurrent_go(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, state, o, seq_slot, seq_start, seqs, H, dim,
-                            vdim, single, dtype, nullptr, 0, 0, stream);
+    return gla_recurrent_go(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, decay, state, o, seq_slot, seq_start, tokens, seqs, H,
+                            dim, vdim, single, dtype, nullptr, 0, 0, stream);
 }
 
 // The second form: gates [tokens, H, gate_pitch] float32 with the decay at [0] and the key's factor at [1]; ones: the
@@ -335,8 +567,8 @@ extern "C" int ri_gla_recurrent_scalar(const void* proj, long long ld, int q_col
                                        const int* seq_start, int seqs, int H, int dim, int vdim, int single, int dtype,
                                        cudaStream_t stream) {
     RI_REQUIRE(gates != nullptr && (ones == 0 || ones == 1), "gla_recurrent_scalar: gates are needed");
-    return gla_recurrent_go(proj, ld, q_col, k_col, v_col, nullptr, nullptr, 1.0f, qscale, state, o, seq_slot, seq_start, seqs,
-                            H, dim, vdim, single, dtype, gates, gate_pitch, ones, stream);
+    return gla_recurrent_go(proj, ld, q_col, k_col, v_col, nullptr, nullptr, 1.0f, qscale, nullptr, state, o, seq_slot, seq_start, 0,
+                            seqs, H, dim, vdim, single, dtype, gates, gate_pitch, ones, stream);
 }
 
 // y[t, h, j] = T( o[t, h, j] / sqrt(mean_j o[t, h, :]^2 + eps) * gain[j] * f(g[t, h vdim + j]) ),  f: silu (fn 1) or

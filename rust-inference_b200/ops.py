@@ -52,7 +52,7 @@ _SIGNATURES = {
     ("moe", "ri_moe_combine"): [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     ("rope_kv", "ri_qk_norm_rope_append_pairs"): [_P] * 10 + [_F, _P, _I, _I] + [_I] * 10 + [_P, _P],
     ("latent_attention", "ri_latent_prep"): [_P, _L, _I, _I] + [_P] * 8 + [_F, _P] + [_I] * 12 + [_P, _P],
-    ("gla", "ri_gla_recurrent"): [_P, _L, _I, _I, _I, _P, _P, _F, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    ("gla", "ri_gla_recurrent"): [_P, _L, _I, _I, _I, _P, _P, _F, _F, _P, _P, _P, _P, _P] + [_I] * 7 + [_P],
     ("gla", "ri_gla_head_norm_gate"): [_P, _P, _F, _P, _L, _P, _I, _I, _I, _I, _I, _P],
     ("linear_f32", "ri_linear_heads_f32"): [_P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _L, _P],
     ("elementwise", "ri_rmsnorm"): [_P, _P, _P, _P, _P, _I, _I, _F, _I, _I, _P, _I, _I, _P],
@@ -416,9 +416,14 @@ def gla_recurrent(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, z: tor
     if max(q_col, k_col) + heads * dim > ld or v_col + heads * vdim > ld:
         raise KernelError("gla_recurrent: the projection is narrower than its columns")
     o = torch.empty((tokens, heads, vdim), dtype=torch.float32, device=proj.device)
+    alone = single and tokens == seqs
+    # the decays of a prompt's tokens, which every block of a head reads
+    decay = None if alone or dim > 128 else torch.empty((tokens, heads * dim), dtype=torch.float32, device=proj.device)
     _call("gla", "ri_gla_recurrent", proj.data_ptr(), ld, int(q_col), int(k_col), int(v_col), z.data_ptr(), bias.data_ptr(),
-          float(tau), float(qscale), state.data_ptr(), o.data_ptr(), seq_slot.data_ptr(), seq_start.data_ptr(), seqs, heads,
-          dim, vdim, 1 if single and tokens == seqs else 0, _code(proj.dtype), _stream())
+          float(tau), float(qscale), _ptr(decay), state.data_ptr(), o.data_ptr(), seq_slot.data_ptr(), seq_start.data_ptr(), tokens,
+          seqs, heads, dim, vdim, 1 if alone else 0, _code(proj.dtype), _stream())
+    if decay is not None:
+        add_launches(1)
     return o
 
 
