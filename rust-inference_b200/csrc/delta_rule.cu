@@ -204,150 +204,305 @@ delta_prep_kernel(float* __restrict__ qkv, int C, int q_col, int k_col, const T*
 }
 
 // ---- the recurrence -------------------------------------------------------------------------------------------------
-#ifndef DR_THREADS
-#define DR_THREADS 128
+#define DR_CT 128               // computing threads
+#define DR_ST 128               // staging threads
+#ifndef DR_C
+#define DR_C 2
 #endif
+#define DR_RING 6               // buffers of staged tokens
+#define DR_AHEAD 4              // of which so many are being filled
 
-// SPLIT: neighbouring lanes that share a value column (a block owns DR_THREADS / SPLIT columns); CH: key channels per
-// lane (dim <= SPLIT CH; lane `part` of a column has channels 4 SPLIT i + 4 part .. + 3, so that the lanes of a column
-// read neighbouring 16-byte pieces of a staged vector); GROUP: tokens staged at a time.  The recurrence is a chain from
-// token to token, so a warp's time per token is what counts: many lanes per column keep the chain short (a handful of
-// channels per lane, then log2(SPLIT) shuffles), and the many small blocks put warps on every SM even for one sequence.
-// The next group's values are loaded into registers before the group at hand is computed and stored into the other of
-// two buffers afterwards: one barrier per group, and memory works while the arithmetic runs.  A sum over d is taken in
-// four partial sums per lane (channels 4 i + j into sum j), added as (s0 + s1) + (s2 + s3), then over the lanes.
-// The read-out after the write, o = (S' + k u^T)^T q with S' the decayed state, is taken as S'^T q + u (k . q): both
-// sums over d then run over the same S' side by side (their shuffles travel together), and the write S' + k u^T is
-// off the chain to the next token's sums by one multiply-add.
+// two float32 multiply-adds (products) per instruction, each rounded as fmaf (a product) rounds it
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 dr_fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 dr_mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 dr_pack2(float x, float y) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ void dr_unpack2(f32x2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ float dr_sum2(f32x2 v) {
+    float x, y;
+    dr_unpack2(v, x, y);
+    return x + y;
+}
+
+// BYTES from global to shared memory without a register in between; `valid` false: zeros, nothing is read
+template <int BYTES>
+__device__ __forceinline__ void dr_copy(void* dst, const void* src, bool valid) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+
+// Barriers between the computing and the staging warps of a block: `arrive` goes on, `sync` waits for everybody
+__device__ __forceinline__ void dr_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void dr_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// SPLIT: neighbouring lanes that share COLS (one or two) neighbouring value columns (a block owns COLS DR_CT / SPLIT columns); R:
+// key channels per lane (dim <= SPLIT R; lane `part` has channels 4 SPLIT i + 4 part .. + 3, so that the lanes of a column
+// read neighbouring 16-byte pieces of a staged vector); GROUP: tokens staged at a time.
+// What bounds it: the chain from token to token, S' = g S, p = S'^T k, u = beta (v - p), S = S' + k u^T (a multiply-add takes six
+// cycles, a shuffle 24), and beside it reading a token's vectors from shared memory, 32 words a cycle for an SM whether the
+// lanes of a warp want the same words or not.  The read-out after the write, o = S^T q, is taken as S'^T q + u (k . q): both sums
+// run over the same S' side by side (their shuffles travel together), and the next token's vectors are in registers before
+// this token's sums are taken.  With two columns the first shuffle of a sum leaves the even lanes with the first column and the
+// odd ones with the second, and one more brings the other's u.  A sum over d is taken in four partial sums per lane (two pairs
+// of channels by turns), then over the lanes, neighbours first: the same bits with one column per lane as with two.
+// Four more warps of the block copy the tokens into a ring of DR_RING buffers, DR_AHEAD groups on their way together, and write
+// the outputs of the groups that have been computed, so that neither a group's trip to memory nor its outputs stand
+// between the tokens (with one group's loads in registers every group took a trip to memory, 2.5 us).
 // SCALAR (one decay per head): the sums run over the undecayed state and are multiplied by the decay afterwards,
-// S'^T k = g (S^T k), so that the decay itself, S' = g S, is off the chain; only its one number per token is staged.
-template <int CH, int SPLIT, int GROUP, bool SCALAR>
-__global__ void __launch_bounds__(DR_THREADS)
-delta_rule_kernel(const float* __restrict__ qkv, int C, int q_col, int k_col, int v_col, const float* __restrict__ decay,
-                  const float* __restrict__ beta, float* __restrict__ state, float* __restrict__ o,
-                  const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int H, int G, int dim, int vdim) {
-    constexpr int DIMC = CH * SPLIT;
-    constexpr int DR_BCOLS = DR_THREADS / SPLIT;
-    constexpr int PER = (GROUP * DIMC + DR_THREADS - 1) / DR_THREADS;      // staged elements per thread and array
-    constexpr int VPER = (GROUP * DR_BCOLS + DR_THREADS - 1) / DR_THREADS;
-    __shared__ __align__(16) float s_g[2][GROUP][SCALAR ? 4 : DIMC], s_k[2][GROUP][DIMC], s_q[2][GROUP][DIMC];
-    __shared__ float s_v[2][GROUP][DR_BCOLS], s_beta[2][GROUP], s_kq[2][GROUP];
-    static_assert(3 * GROUP <= DR_THREADS, "a thread per staged beta, product and decay");
+// S'^T k = g (S^T k); only its one number per token is staged.
+// DR_FIGURES
+template <int R, int SPLIT, int COLS, int GROUP, bool SCALAR, bool VEC>
+__global__ void __launch_bounds__(GROUP == 1 ? DR_CT : DR_CT + DR_ST)
+delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, const float* decay, const float* beta, float* state,
+                  float* __restrict__ o, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int H, int G, int dim,
+                  int vdim) {
+    constexpr bool SINGLE = GROUP == 1;                                    // every sequence brings one token
+    constexpr int DIMC = R * SPLIT;
+    constexpr int BCOLS = COLS * DR_CT / SPLIT;
+    constexpr int RING = SINGLE ? 1 : DR_RING;
+    constexpr int KP = DIMC / 4;                                           // staged pieces of four channels per token
+    constexpr int PER = (GROUP * KP + DR_ST - 1) / DR_ST;                  // ... and per thread
+    constexpr int VPER = (GROUP * BCOLS + DR_ST - 1) / DR_ST;
+    constexpr int VECS = SCALAR ? 2 : 3;                                   // k, q, and the decays g
+    constexpr bool AHEAD = !SINGLE && R <= 16;                             // the next token's vectors in registers
+    constexpr int ALL = DR_CT + DR_ST;
+    extern __shared__ __align__(16) float dr_dyn[];
+    float (*s_x)[GROUP][VECS][DIMC] = reinterpret_cast<float (*)[GROUP][VECS][DIMC]>(dr_dyn);                             // [RING]
+    float (*s_c)[GROUP][4] = reinterpret_cast<float (*)[GROUP][4]>(dr_dyn + RING * GROUP * VECS * DIMC);                  // beta, k . q, the decay (SCALAR)
+    float (*s_v)[GROUP][BCOLS] = reinterpret_cast<float (*)[GROUP][BCOLS]>(dr_dyn + RING * GROUP * (VECS * DIMC + 4));
+    float (*s_o)[GROUP][BCOLS] = reinterpret_cast<float (*)[GROUP][BCOLS]>(dr_dyn + RING * GROUP * (VECS * DIMC + 4 + BCOLS));
+    static_assert(3 * GROUP <= DR_ST, "a thread per staged beta, product and decay");
     // (the kernel after this one is let in only when the walk is over, see below)
-    const int b = blockIdx.z, h = blockIdx.y;
+    const int b = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * BCOLS;
     const int kvh = h / (H / G);
-    const int part = threadIdx.x % SPLIT, col = threadIdx.x / SPLIT;
-    const int j = blockIdx.x * DR_BCOLS + col;
-    const bool mine = j < vdim;
     pdl_wait();
     const int t0 = seq_start[b], t1 = seq_start[b + 1];
-    float* st = state + ((size_t)seq_slot[b] * H + h) * dim * vdim;
-    float S[CH];
+    if (t0 >= t1) return;                     // a sequence without tokens keeps its state (the whole block leaves)
+    const int st_id = SINGLE ? threadIdx.x : threadIdx.x - DR_CT;          // among the staging threads
+    // Copies of a group of tokens into its buffer (VEC: 16 bytes, else words): past the sequence's tokens and the columns
+    // something that exists is copied and not used, past the head's channels zeros are written (the state is zero there).
+    auto copy = [&](int buf, int base) {
 #pragma unroll
-    for (int i = 0; i < CH; i++) {
-        const int d = 4 * SPLIT * (i / 4) + 4 * part + (i & 3);
-        S[i] = (mine && d < dim) ? st[(size_t)d * vdim + j] : 0.0f;
+        for (int e = 0; e < PER; e++) {
+            const int idx = st_id + e * DR_ST;
+            const int g = idx / KP, d = (idx % KP) * 4, t = min(base + g, t1 - 1);
+            if (g < GROUP) {
+                const float* src[3] = {qkv + (size_t)t * C + k_col + kvh * dim + d, qkv + (size_t)t * C + q_col + kvh * dim + d,
+                                       decay + (SCALAR ? 0 : ((size_t)t * H + h) * dim + d)};
+#pragma unroll
+                for (int w = 0; w < VECS; w++) {
+                    if (VEC) {
+                        dr_copy<16>(&s_x[buf][g][w][d], d < dim ? src[w] : qkv, d < dim);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) dr_copy<4>(&s_x[buf][g][w][d + i], d + i < dim ? src[w] + i : qkv, d + i < dim);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < VPER; e++) {
+            const int idx = st_id + e * DR_ST;
+            if (idx < GROUP * BCOLS)
+                dr_copy<4>(&(&s_v[buf][0][0])[idx], qkv + (size_t)min(base + idx / BCOLS, t1 - 1) * C + v_col + h * vdim + min(j0 + idx % BCOLS, vdim - 1), true);
+        }
+        if (st_id < (SCALAR ? 3 : 2) * GROUP) {      // betas, products k . q, decays
+            const int g = st_id % GROUP, which = st_id / GROUP, t = min(base + g, t1 - 1);
+            dr_copy<4>(&s_c[buf][g][which], which < 2 ? beta + (size_t)t * (H + G) + (which == 0 ? h : H + kvh) : decay + (size_t)t * H + h, true);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    if (!SINGLE && threadIdx.x >= DR_CT) {
+        // ---- the staging warps.  Barriers 1 + buf: the buffer is full; 1 + RING + buf: it was read, its outputs are there ----------------
+        auto write_out = [&](int buf, int base) {
+            for (int i = st_id; i < GROUP * BCOLS; i += DR_ST) {
+                const int g = i / BCOLS, c = i % BCOLS;
+                if (base + g < t1 && j0 + c < vdim) o[((size_t)(base + g) * H + h) * vdim + j0 + c] = s_o[buf][g][c];
+            }
+        };
+        const int groups = (t1 - t0 + GROUP - 1) / GROUP;
+        for (int i = 0; i < DR_AHEAD; i++) {
+            if (i < groups) copy(i, t0 + i * GROUP);
+            else asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+        for (int n = 0; n < groups; n++) {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(DR_AHEAD - 1) : "memory");
+            dr_bar_arrive(1 + n % RING, ALL);
+            const int m = n + DR_AHEAD, buf = m % RING;                    // the group whose copies start now
+            if (m >= RING) {                                               // (m - RING < groups: DR_AHEAD < RING)
+                dr_bar_sync(1 + RING + buf, ALL);
+                write_out(buf, t0 + (m - RING) * GROUP);
+            }
+            if (m < groups) copy(buf, t0 + m * GROUP);
+            else asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+        for (int m = groups + DR_AHEAD > RING ? groups + DR_AHEAD - RING : 0; m < groups; m++) {      // the groups that the loop has not written
+            dr_bar_sync(1 + RING + m % RING, ALL);
+            write_out(m % RING, t0 + m * GROUP);
+        }
+        return;
     }
-    float rg[PER], rk[PER], rq[PER], rv[VPER], rb = 0.0f;
-    auto fetch = [&](int base) {
+    // ---- the computing warps ----------------------------------------------------------------------------------------------------
+    const int part = threadIdx.x % SPLIT, first = COLS * (threadIdx.x / SPLIT);   // this lane's channels; its first column
+    const int odd = COLS == 2 ? part & 1 : 0, col = first + odd;           // the column whose sums this lane ends with
+    const int j = j0 + first;
+    float* st = state + ((size_t)seq_slot[b] * H + h) * dim * vdim;
+    const bool whole = COLS == 2 && vdim % 2 == 0 && ((uintptr_t)state & 7) == 0;     // the state's rows start on 8 bytes
+    f32x2 S[COLS][R / 2];
 #pragma unroll
-        for (int e = 0; e < PER; e++) {
-            const int idx = threadIdx.x + e * DR_THREADS;
-            const int g = idx / DIMC, d = idx % DIMC, t = base + g;
-            rg[e] = rk[e] = rq[e] = 0.0f;
-            if (g < GROUP && t < t1 && d < dim) {
-                if (!SCALAR) rg[e] = decay[((size_t)t * H + h) * dim + d];
-                rk[e] = qkv[(size_t)t * C + k_col + kvh * dim + d];
-                rq[e] = qkv[(size_t)t * C + q_col + kvh * dim + d];
-            }
-        }
+    for (int i = 0; i < R; i += 2) {
+        const int d = 4 * SPLIT * (i / 4) + 4 * part + (i & 3);
+        if (whole) {
+            const float2 x = j < vdim && d < dim ? *reinterpret_cast<const float2*>(st + (size_t)d * vdim + j) : make_float2(0.0f, 0.0f);
+            const float2 y = j < vdim && d + 1 < dim ? *reinterpret_cast<const float2*>(st + (size_t)(d + 1) * vdim + j) : make_float2(0.0f, 0.0f);
+            S[0][i / 2] = dr_pack2(x.x, y.x);
+            S[COLS - 1][i / 2] = dr_pack2(COLS == 2 ? x.y : x.x, COLS == 2 ? y.y : y.x);
+        } else {
 #pragma unroll
-        for (int e = 0; e < VPER; e++) {
-            const int idx = threadIdx.x + e * DR_THREADS;
-            const int g = idx / DR_BCOLS, jj = blockIdx.x * DR_BCOLS + idx % DR_BCOLS;
-            rv[e] = (g < GROUP && base + g < t1 && jj < vdim) ? qkv[(size_t)(base + g) * C + v_col + h * vdim + jj] : 0.0f;
+            for (int c = 0; c < COLS; c++)
+                S[c][i / 2] = dr_pack2(j + c < vdim && d < dim ? st[(size_t)d * vdim + j + c] : 0.0f,
+                                       j + c < vdim && d + 1 < dim ? st[(size_t)(d + 1) * vdim + j + c] : 0.0f);
         }
-        if (threadIdx.x < 2 * GROUP) {
-            const int g = threadIdx.x % GROUP;
-            rb = base + g < t1 ? beta[(size_t)(base + g) * (H + G) + (threadIdx.x < GROUP ? h : H + kvh)] : 0.0f;
-        } else if (SCALAR && threadIdx.x < 3 * GROUP) {
-            const int g = threadIdx.x - 2 * GROUP;
-            rb = base + g < t1 ? decay[(size_t)(base + g) * H + h] : 0.0f;
-        }
+    }
+    struct Token {                                                         // a token's vectors in registers
+        f32x2 x[VECS][R / 2];
+        float v, beta, kq, g;
     };
-    auto store = [&](int buf) {
+    auto load = [&](Token& t, int buf, int g) {
 #pragma unroll
-        for (int e = 0; e < PER; e++) {
-            const int idx = threadIdx.x + e * DR_THREADS;
-            if (idx < GROUP * DIMC) {
-                if (!SCALAR) (&s_g[buf][0][0])[idx] = rg[e];
-                (&s_k[buf][0][0])[idx] = rk[e];
-                (&s_q[buf][0][0])[idx] = rq[e];
+        for (int w = 0; w < VECS; w++)
+#pragma unroll
+            for (int i = 0; i < R; i += 4) {
+                const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(&s_x[buf][g][w][4 * SPLIT * (i / 4) + 4 * part]);
+                t.x[w][i / 2] = p.x;
+                t.x[w][i / 2 + 1] = p.y;
             }
-        }
-#pragma unroll
-        for (int e = 0; e < VPER; e++) {
-            const int idx = threadIdx.x + e * DR_THREADS;
-            if (idx < GROUP * DR_BCOLS) (&s_v[buf][0][0])[idx] = rv[e];
-        }
-        if (threadIdx.x < GROUP) s_beta[buf][threadIdx.x] = rb;
-        else if (threadIdx.x < 2 * GROUP) s_kq[buf][threadIdx.x - GROUP] = rb;
-        else if (SCALAR && threadIdx.x < 3 * GROUP) s_g[buf][threadIdx.x - 2 * GROUP][0] = rb;
+        t.v = s_v[buf][g][col];
+        t.beta = s_c[buf][g][0];
+        t.kq = s_c[buf][g][1];
+        if (SCALAR) t.g = s_c[buf][g][2];
     };
-    fetch(t0);
-    int buf = 0;
-    for (int base = t0; base < t1; base += GROUP) {
-        store(buf);
-        __syncthreads();             // this group is staged (the other buffer was last read before the barrier before)
-        if (base + GROUP < t1) fetch(base + GROUP);
-        const int n = min(GROUP, t1 - base);
-        for (int g = 0; g < n; g++) {
-            float p[4] = {0.0f, 0.0f, 0.0f, 0.0f}, a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            float4 kr[CH / 4];
+    auto partial = [&](const f32x2* s, const f32x2* x) {                   // this lane's share of a column's sum
+        f32x2 p0 = dr_mul2(s[0], x[0]), p1 = dr_mul2(s[1], x[1]);
 #pragma unroll
-            for (int i = 0; i < CH; i += 4) {
-                const int at = 4 * SPLIT * (i / 4) + 4 * part;
-                const float4 gg = SCALAR ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : *reinterpret_cast<const float4*>(&s_g[buf][g][SCALAR ? 0 : at]);
-                const float4 kk = *reinterpret_cast<const float4*>(&s_k[buf][g][at]);
-                const float4 qq = *reinterpret_cast<const float4*>(&s_q[buf][g][at]);
-                kr[i / 4] = kk;
-                if (!SCALAR) S[i] *= gg.x;     p[0] = fmaf(S[i], kk.x, p[0]);     a[0] = fmaf(S[i], qq.x, a[0]);
-                if (!SCALAR) S[i + 1] *= gg.y; p[1] = fmaf(S[i + 1], kk.y, p[1]); a[1] = fmaf(S[i + 1], qq.y, a[1]);
-                if (!SCALAR) S[i + 2] *= gg.z; p[2] = fmaf(S[i + 2], kk.z, p[2]); a[2] = fmaf(S[i + 2], qq.z, a[2]);
-                if (!SCALAR) S[i + 3] *= gg.w; p[3] = fmaf(S[i + 3], kk.w, p[3]); a[3] = fmaf(S[i + 3], qq.w, a[3]);
-            }
-            float pred = (p[0] + p[1]) + (p[2] + p[3]);
-            float acc = (a[0] + a[1]) + (a[2] + a[3]);
-#pragma unroll
-            for (int sh = 1; sh < SPLIT; sh <<= 1) {
-                pred += __shfl_xor_sync(0xffffffffu, pred, sh);
-                acc += __shfl_xor_sync(0xffffffffu, acc, sh);
-            }
-            const float gs = SCALAR ? s_g[buf][g][0] : 1.0f;
-            const float u = s_beta[buf][g] * (SCALAR ? fmaf(-gs, pred, s_v[buf][g][col]) : s_v[buf][g][col] - pred);
-            if (SCALAR) {
-                acc *= gs;
-#pragma unroll
-                for (int i = 0; i < CH; i++) S[i] *= gs;
-            }
-#pragma unroll
-            for (int i = 0; i < CH; i += 4) {
-                S[i] = fmaf(kr[i / 4].x, u, S[i]);
-                S[i + 1] = fmaf(kr[i / 4].y, u, S[i + 1]);
-                S[i + 2] = fmaf(kr[i / 4].z, u, S[i + 2]);
-                S[i + 3] = fmaf(kr[i / 4].w, u, S[i + 3]);
-            }
-            acc = fmaf(u, s_kq[buf][g], acc);
-            if (part == 0 && mine) o[((size_t)(base + g) * H + h) * vdim + j] = acc;
+        for (int i = 2; i < R / 2; i += 2) {
+            p0 = dr_fma2(s[i], x[i], p0);
+            p1 = dr_fma2(s[i + 1], x[i + 1], p1);
         }
-        buf ^= 1;
+        return dr_sum2(p0) + dr_sum2(p1);
+    };
+    auto step = [&](const Token& t, int buf, int g) {
+        const f32x2 *k = t.x[0], *q = t.x[1];
+        if (!SCALAR) {
+#pragma unroll
+            for (int i = 0; i < R / 2; i++)
+#pragma unroll
+                for (int c = 0; c < COLS; c++) S[c][i] = dr_mul2(t.x[VECS - 1][i], S[c][i]);
+        }
+        float p[COLS], a[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; c++) p[c] = partial(S[c], k);
+#pragma unroll
+        for (int c = 0; c < COLS; c++) a[c] = partial(S[c], q);
+        float pred = p[0], acc = a[0];
+        if (COLS == 2) {
+            pred = (odd ? p[COLS - 1] : p[0]) + __shfl_xor_sync(0xffffffffu, odd ? p[0] : p[COLS - 1], 1);
+            acc = (odd ? a[COLS - 1] : a[0]) + __shfl_xor_sync(0xffffffffu, odd ? a[0] : a[COLS - 1], 1);
+        }
+#pragma unroll
+        for (int sh = COLS; sh < SPLIT; sh <<= 1) {
+            const float x = __shfl_xor_sync(0xffffffffu, pred, sh), y = __shfl_xor_sync(0xffffffffu, acc, sh);
+            pred += x;
+            acc += y;
+        }
+        if (SCALAR) {
+            const f32x2 gs = dr_pack2(t.g, t.g);
+#pragma unroll
+            for (int i = 0; i < R / 2; i++)
+#pragma unroll
+                for (int c = 0; c < COLS; c++) S[c][i] = dr_mul2(gs, S[c][i]);
+            acc *= t.g;
+        }
+        const float u = t.beta * (SCALAR ? fmaf(-t.g, pred, t.v) : t.v - pred);
+        float ub[COLS];
+        ub[0] = u;
+        if (COLS == 2) {
+            const float other = __shfl_xor_sync(0xffffffffu, u, 1);
+            ub[0] = odd ? other : u;
+            ub[COLS - 1] = odd ? u : other;
+        }
+#pragma unroll
+        for (int c = 0; c < COLS; c++) {
+            const f32x2 uu = dr_pack2(ub[c], ub[c]);
+#pragma unroll
+            for (int i = 0; i < R / 2; i++) S[c][i] = dr_fma2(k[i], uu, S[c][i]);
+        }
+        acc = fmaf(u, t.kq, acc);
+        if (part < COLS) s_o[buf][g][col] = acc;
+    };
+    if (SINGLE) {
+        copy(0, t0);
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        Token one;
+        load(one, 0, 0);
+        step(one, 0, 0);
+        if (part < COLS && j0 + col < vdim) o[((size_t)t0 * H + h) * vdim + j0 + col] = s_o[0][0][col];
+    } else {
+        int nth = 0;
+        for (int base = t0; base < t1; base += GROUP, nth++) {
+            const int buf = nth % RING, n = min(GROUP, t1 - base);
+            dr_bar_sync(1 + buf, ALL);
+            if (AHEAD) {
+                Token one, two;
+                load(one, buf, 0);
+#pragma unroll 1
+                for (int g = 0; g < n; g += 2) {
+                    load(two, buf, g + 1);
+                    step(one, buf, g);
+                    if (g + 2 < GROUP) load(one, buf, g + 2);
+                    if (g + 1 < n) step(two, buf, g + 1);
+                }
+            } else {
+#pragma unroll 1
+                for (int g = 0; g < n; g++) {
+                    Token one;
+                    load(one, buf, g);
+                    step(one, buf, g);
+                }
+            }
+            dr_bar_arrive(1 + RING + buf, ALL);
+        }
     }
     pdl_trigger();               // the next kernel may come in once the walk is over
-    if (mine) {
 #pragma unroll
-        for (int i = 0; i < CH; i++) {
-            const int d = 4 * SPLIT * (i / 4) + 4 * part + (i & 3);
-            if (d < dim) st[(size_t)d * vdim + j] = S[i];
+    for (int i = 0; i < R; i += 2) {
+        const int d = 4 * SPLIT * (i / 4) + 4 * part + (i & 3);
+        float x[COLS], y[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; c++) dr_unpack2(S[c][i / 2], x[c], y[c]);
+        if (whole) {
+            if (j < vdim && d < dim) *reinterpret_cast<float2*>(st + (size_t)d * vdim + j) = make_float2(x[0], x[COLS - 1]);
+            if (j < vdim && d + 1 < dim) *reinterpret_cast<float2*>(st + (size_t)(d + 1) * vdim + j) = make_float2(y[0], y[COLS - 1]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < COLS; c++) {
+                if (j + c < vdim && d < dim) st[(size_t)d * vdim + j + c] = x[c];
+                if (j + c < vdim && d + 1 < dim) st[(size_t)(d + 1) * vdim + j + c] = y[c];
+            }
         }
     }
 }
@@ -383,31 +538,43 @@ extern "C" int ri_delta_rule_recurrent(float* qkv, int C, int q_col, int k_col, 
     // dependent instructions, one warp per scheduler) must spread one per SM, and blocks that come in while the kernel
     // before still holds most SMs pile up on the first SMs that get free and stay there (2,048 tokens of 8 heads of
     // 128 x 128: 0.97 ms as a dependent launch, 0.59 ms as an ordinary one).
-#define DR_GO(CH, SPLIT, GROUP, SC)                                                                                        \
+    // 16-byte copies of four channels where every row of q, k and the decays starts on 16 bytes
+    const bool vec = dim % 4 == 0 && C % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && (((uintptr_t)qkv | (uintptr_t)decay) & 15) == 0;
+#define DR_GO(R, SPLIT, GROUP, SC, VEC)                                                                                    \
     do {                                                                                                                 \
-        const int bcols = DR_THREADS / SPLIT;                                                                            \
+        constexpr int bcols = DR_C * DR_CT / SPLIT;                                                                      \
+        constexpr size_t sm = (size_t)(GROUP == 1 ? 1 : DR_RING) * GROUP * ((SC ? 2 : 3) * R * SPLIT + 4 + 2 * bcols) * sizeof(float); \
         const dim3 grid((vdim + bcols - 1) / bcols, H, seqs);                                                            \
-        delta_rule_kernel<CH, SPLIT, GROUP, SC><<<grid, dim3(DR_THREADS), 0, stream>>>(                                       \
+        cudaError_t e = sm > 48 * 1024 ? cudaFuncSetAttribute(delta_rule_kernel<R, SPLIT, DR_C, GROUP, SC, VEC>,          \
+                                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) : cudaSuccess; \
+        if (e != cudaSuccess) RI_FAIL((int)e, "delta_rule_recurrent: %s", cudaGetErrorString(e));                        \
+        delta_rule_kernel<R, SPLIT, DR_C, GROUP, SC, VEC><<<grid, dim3(GROUP == 1 ? DR_CT : DR_CT + DR_ST), sm, stream>>>( \
             (const float*)qkv, C, q_col, k_col, v_col, (const float*)decay, (const float*)beta, state, o, seq_slot,      \
             seq_start, H, G, dim, vdim);                                                                                 \
     } while (0)
-#define DR_BY_GROUP(CH, SPLIT, GROUP)                                                                                    \
+#define DR_BY_VEC(R, SPLIT, GROUP, SC)                                                                                   \
+    do {                                                                                                                 \
+        if (vec) DR_GO(R, SPLIT, GROUP, SC, true);                                                                       \
+        else DR_GO(R, SPLIT, GROUP, SC, false);                                                                          \
+    } while (0)
+#define DR_BY_GROUP(R, SPLIT, GROUP)                                                                                     \
     do {                                                                                                                 \
         if (ddim == 1 && dim > 1) {                                                                                      \
-            if (single) DR_GO(CH, SPLIT, 1, true);                                                                       \
-            else DR_GO(CH, SPLIT, GROUP, true);                                                                          \
+            if (single) DR_BY_VEC(R, SPLIT, 1, true);                                                                    \
+            else DR_BY_VEC(R, SPLIT, GROUP, true);                                                                       \
         } else {                                                                                                         \
-            if (single) DR_GO(CH, SPLIT, 1, false);                                                                      \
-            else DR_GO(CH, SPLIT, GROUP, false);                                                                         \
+            if (single) DR_BY_VEC(R, SPLIT, 1, false);                                                                   \
+            else DR_BY_VEC(R, SPLIT, GROUP, false);                                                                      \
         }                                                                                                                \
     } while (0)
     if (dim <= 16) DR_BY_GROUP(4, 4, 16);
     else if (dim <= 32) DR_BY_GROUP(4, 8, 16);
-    else if (dim <= 64) DR_BY_GROUP(4, 16, 16);
+    else if (dim <= 64) DR_BY_GROUP(8, 8, 16);
     else if (dim <= 128) DR_BY_GROUP(8, 16, 8);
     else if (dim <= 256) DR_BY_GROUP(16, 16, 4);
     else DR_BY_GROUP(32, 16, 2);
 #undef DR_BY_GROUP
+#undef DR_BY_VEC
 #undef DR_GO
     RI_CHECK_LAUNCH("delta_rule_recurrent");
     return 0;
