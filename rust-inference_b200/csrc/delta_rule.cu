@@ -206,9 +206,6 @@ delta_prep_kernel(float* __restrict__ qkv, int C, int q_col, int k_col, const T*
 // ---- the recurrence -------------------------------------------------------------------------------------------------
 #define DR_CT 128               // computing threads
 #define DR_ST 128               // staging threads
-#ifndef DR_C
-#define DR_C 2
-#endif
 #define DR_RING 6               // buffers of staged tokens
 #define DR_AHEAD 4              // of which so many are being filled
 
@@ -263,7 +260,10 @@ __device__ __forceinline__ void dr_bar_arrive(int id, int threads) { asm volatil
 // between the tokens (with one group's loads in registers every group took a trip to memory, 2.5 us).
 // SCALAR (one decay per head): the sums run over the undecayed state and are multiplied by the decay afterwards,
 // S'^T k = g (S^T k); only its one number per token is staged.
-// DR_FIGURES
+// 2,048 tokens with the preparation: 16 heads of 128 x 128 744 -> 435 us, 8 heads 592 -> 395 us, 8 of 64 x 64 453 -> 335 us, 16 of 128 x
+// 128 with one decay per head 586 -> 455 us; four sequences of 512 tokens and 16 heads 503 -> 314 us.  (Before: 16 lanes a column,
+// one multiply-add an instruction, the tokens staged by the warps that compute.)  What is left is some 370 cycles a token: the
+// chain of about 210 and the instructions that do not fit beside it, one warp to a scheduler.
 template <int R, int SPLIT, int COLS, int GROUP, bool SCALAR, bool VEC>
 __global__ void __launch_bounds__(GROUP == 1 ? DR_CT : DR_CT + DR_ST)
 delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, const float* decay, const float* beta, float* state,
@@ -417,6 +417,13 @@ delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, cons
         for (int c = 0; c < COLS; c++) p[c] = partial(S[c], k);
 #pragma unroll
         for (int c = 0; c < COLS; c++) a[c] = partial(S[c], q);
+        if (SCALAR) {
+            const f32x2 gs = dr_pack2(t.g, t.g);
+#pragma unroll
+            for (int i = 0; i < R / 2; i++)
+#pragma unroll
+                for (int c = 0; c < COLS; c++) S[c][i] = dr_mul2(gs, S[c][i]);
+        }
         float pred = p[0], acc = a[0];
         if (COLS == 2) {
             pred = (odd ? p[COLS - 1] : p[0]) + __shfl_xor_sync(0xffffffffu, odd ? p[0] : p[COLS - 1], 1);
@@ -428,14 +435,7 @@ delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, cons
             pred += x;
             acc += y;
         }
-        if (SCALAR) {
-            const f32x2 gs = dr_pack2(t.g, t.g);
-#pragma unroll
-            for (int i = 0; i < R / 2; i++)
-#pragma unroll
-                for (int c = 0; c < COLS; c++) S[c][i] = dr_mul2(gs, S[c][i]);
-            acc *= t.g;
-        }
+        if (SCALAR) acc *= t.g;
         const float u = t.beta * (SCALAR ? fmaf(-t.g, pred, t.v) : t.v - pred);
         float ub[COLS];
         ub[0] = u;
@@ -540,40 +540,63 @@ extern "C" int ri_delta_rule_recurrent(float* qkv, int C, int q_col, int k_col, 
     // 128 x 128: 0.97 ms as a dependent launch, 0.59 ms as an ordinary one).
     // 16-byte copies of four channels where every row of q, k and the decays starts on 16 bytes
     const bool vec = dim % 4 == 0 && C % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && (((uintptr_t)qkv | (uintptr_t)decay) & 15) == 0;
-#define DR_GO(R, SPLIT, GROUP, SC, VEC)                                                                                    \
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        sms = n > 0 ? n : 148;
+    }
+    // One column a lane where all blocks of a prompt's step then still have an SM to themselves, two otherwise (one a lane / two;
+    // 2,048 tokens: 8 heads of 128 x 128 395 / 418 us, 8 of 64 x 64 335 / 357, 16 of 128 x 128 516 / 435, four sequences
+    // of 512 tokens and 16 heads 490 / 314).  With one decay per head half as many channels a lane (16 heads of 128 x 128: 455
+    // us, with eight channels 516): there is a third less to read.
+#define DR_GO(R, SPLIT, COLS, GROUP, SC, VEC)                                                                              \
     do {                                                                                                                 \
-        constexpr int bcols = DR_C * DR_CT / SPLIT;                                                                      \
+        constexpr int bcols = COLS * DR_CT / SPLIT;                                                                      \
         constexpr size_t sm = (size_t)(GROUP == 1 ? 1 : DR_RING) * GROUP * ((SC ? 2 : 3) * R * SPLIT + 4 + 2 * bcols) * sizeof(float); \
         const dim3 grid((vdim + bcols - 1) / bcols, H, seqs);                                                            \
-        cudaError_t e = sm > 48 * 1024 ? cudaFuncSetAttribute(delta_rule_kernel<R, SPLIT, DR_C, GROUP, SC, VEC>,          \
+        cudaError_t e = sm > 48 * 1024 ? cudaFuncSetAttribute(delta_rule_kernel<R, SPLIT, COLS, GROUP, SC, VEC>,          \
                                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) : cudaSuccess; \
         if (e != cudaSuccess) RI_FAIL((int)e, "delta_rule_recurrent: %s", cudaGetErrorString(e));                        \
-        delta_rule_kernel<R, SPLIT, DR_C, GROUP, SC, VEC><<<grid, dim3(GROUP == 1 ? DR_CT : DR_CT + DR_ST), sm, stream>>>( \
+        delta_rule_kernel<R, SPLIT, COLS, GROUP, SC, VEC><<<grid, dim3(GROUP == 1 ? DR_CT : DR_CT + DR_ST), sm, stream>>>( \
             (const float*)qkv, C, q_col, k_col, v_col, (const float*)decay, (const float*)beta, state, o, seq_slot,      \
             seq_start, H, G, dim, vdim);                                                                                 \
     } while (0)
-#define DR_BY_VEC(R, SPLIT, GROUP, SC)                                                                                   \
+#define DR_BY_VEC(R, SPLIT, COLS, GROUP, SC)                                                                             \
     do {                                                                                                                 \
-        if (vec) DR_GO(R, SPLIT, GROUP, SC, true);                                                                       \
-        else DR_GO(R, SPLIT, GROUP, SC, false);                                                                          \
+        if (vec) DR_GO(R, SPLIT, COLS, GROUP, SC, true);                                                                 \
+        else DR_GO(R, SPLIT, COLS, GROUP, SC, false);                                                                    \
     } while (0)
-#define DR_BY_GROUP(R, SPLIT, GROUP)                                                                                     \
+#define DR_CHANNEL(R, SPLIT, GROUP)                                                                                      \
     do {                                                                                                                 \
-        if (ddim == 1 && dim > 1) {                                                                                      \
-            if (single) DR_BY_VEC(R, SPLIT, 1, true);                                                                    \
-            else DR_BY_VEC(R, SPLIT, GROUP, true);                                                                       \
-        } else {                                                                                                         \
-            if (single) DR_BY_VEC(R, SPLIT, 1, false);                                                                   \
-            else DR_BY_VEC(R, SPLIT, GROUP, false);                                                                      \
-        }                                                                                                                \
+        const long long blocks = (long long)((vdim + DR_CT / SPLIT - 1) / (DR_CT / SPLIT)) * H * seqs;                   \
+        if (single) DR_BY_VEC(R, SPLIT, 2, 1, false);                                                                    \
+        else if (blocks <= sms) DR_BY_VEC(R, SPLIT, 1, GROUP, false);                                                    \
+        else DR_BY_VEC(R, SPLIT, 2, GROUP, false);                                                                       \
     } while (0)
-    if (dim <= 16) DR_BY_GROUP(4, 4, 16);
-    else if (dim <= 32) DR_BY_GROUP(4, 8, 16);
-    else if (dim <= 64) DR_BY_GROUP(8, 8, 16);
-    else if (dim <= 128) DR_BY_GROUP(8, 16, 8);
-    else if (dim <= 256) DR_BY_GROUP(16, 16, 4);
-    else DR_BY_GROUP(32, 16, 2);
-#undef DR_BY_GROUP
+#define DR_HEAD(R, SPLIT, GROUP)                                                                                         \
+    do {                                                                                                                 \
+        if (single) DR_BY_VEC(R, SPLIT, 2, 1, true);                                                                     \
+        else DR_BY_VEC(R, SPLIT, 2, GROUP, true);                                                                        \
+    } while (0)
+    if (ddim == 1 && dim > 1) {
+        if (dim <= 16) DR_HEAD(4, 4, 16);
+        else if (dim <= 32) DR_HEAD(4, 8, 16);
+        else if (dim <= 64) DR_HEAD(4, 16, 16);
+        else if (dim <= 128) DR_HEAD(4, 32, 8);
+        else if (dim <= 256) DR_HEAD(16, 16, 4);
+        else DR_HEAD(32, 16, 2);
+    } else {
+        if (dim <= 16) DR_CHANNEL(4, 4, 16);
+        else if (dim <= 32) DR_CHANNEL(4, 8, 16);
+        else if (dim <= 64) DR_CHANNEL(8, 8, 16);
+        else if (dim <= 128) DR_CHANNEL(8, 16, 8);
+        else if (dim <= 256) DR_CHANNEL(16, 16, 4);
+        else DR_CHANNEL(32, 16, 2);
+    }
+#undef DR_HEAD
+#undef DR_CHANNEL
 #undef DR_BY_VEC
 #undef DR_GO
     RI_CHECK_LAUNCH("delta_rule_recurrent");

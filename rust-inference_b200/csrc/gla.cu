@@ -111,8 +111,8 @@ __device__ __forceinline__ void gla_bar_arrive(int id, int threads) { asm volati
 // holds, so that each lane ends with one.  Every token's sum thus has one order that depends on the head's size only: prompts,
 // pieces of prompts and single tokens give the same bits (GROUP = 1, for steps in which every sequence brings one token,
 // takes the decay from z itself and walks the same order).
-// 2,048 tokens of 32 heads of 64 x 128, with the decays' kernel: 607 -> 217 us (106 ns a token); three sequences of 2,302 tokens in
-// all 645 -> 203 us; 16 heads of 128 x 129 with one decay 443 -> 280 us.  (Before: one column and four channels a thread, the
+// 2,048 tokens of 32 heads of 64 x 128, with the decays' kernel: 608 -> 203 us (99 ns a token); three sequences of 2,302 tokens in
+// all 645 -> 207 us; 16 heads of 128 x 129 with one decay 445 -> 278 us; 64 single tokens of 32 heads 73 -> 69 us.  (Before: one column and four channels a thread, the
 // tokens staged and the decays taken by the same warps of every block.)
 #define GLA_CT 128              // computing threads
 #define GLA_ST 128              // staging threads
@@ -304,6 +304,17 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
     float* st = state + ((size_t)slot * H + h) * dim * vdim;
     f32x2 S[4][2];                            // [column][pair of channels]
     const bool whole = vdim % 4 == 0 && ((uintptr_t)state & 15) == 0;        // the state's rows start on 16 bytes, columns come in fours
+    // A single token is bound by its state's trip to memory: rows that do not start on 16 bytes go through shared memory, whole
+    // rows of the block's columns at a time.
+    float* tile = gla_dyn + ROW;              // [DIMC][BCOLS + 1]
+    if (SINGLE && !whole) {
+#pragma unroll 16
+        for (int i = threadIdx.x; i < DIMC * BCOLS; i += GLA_CT) {
+            const int d = i / BCOLS, c = i % BCOLS;
+            tile[d * (BCOLS + 1) + c] = d < dim && j0 + c < vdim ? st[(size_t)d * vdim + j0 + c] : 0.0f;
+        }
+        __syncthreads();
+    }
     float4 x4[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -312,6 +323,9 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
         if (d0 + i < dim) {
             if (whole) {
                 if (j < vdim) x4[i] = *reinterpret_cast<const float4*>(row);
+            } else if (SINGLE) {
+                const float* sr = tile + (d0 + i) * (BCOLS + 1) + col;
+                x4[i] = make_float4(sr[0], sr[1], sr[2], sr[3]);
             } else {
                 if (j < vdim) x4[i].x = row[0];
                 if (j + 1 < vdim) x4[i].y = row[1];
@@ -411,12 +425,22 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
         if (d0 + i < dim) {
             if (whole) {
                 if (j < vdim) *reinterpret_cast<float4*>(row) = w;
+            } else if (SINGLE) {
+                float* sr = tile + (d0 + i) * (BCOLS + 1) + col;
+                sr[0] = w.x; sr[1] = w.y; sr[2] = w.z; sr[3] = w.w;
             } else {
                 if (j < vdim) row[0] = w.x;
                 if (j + 1 < vdim) row[1] = w.y;
                 if (j + 2 < vdim) row[2] = w.z;
                 if (j + 3 < vdim) row[3] = w.w;
             }
+        }
+    }
+    if (SINGLE && !whole) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < DIMC * BCOLS; i += GLA_CT) {
+            const int d = i / BCOLS, c = i % BCOLS;
+            if (d < dim && j0 + c < vdim) st[(size_t)d * vdim + j0 + c] = tile[d * (BCOLS + 1) + c];
         }
     }
 }
@@ -427,7 +451,7 @@ static int gla_walk_go(const void* proj, long long ld, int q_col, int k_col, int
                        int H, int dim, int vdim_in, const float* gates, int gate_pitch, int ones, cudaStream_t stream) {
     constexpr int BCOLS = GLA_CT * 16 / DIMC, PER = (GROUP * (DIMC / 8) + GLA_ST - 1) / GLA_ST, PT = sizeof(T) / 2;
     constexpr size_t RAW = GROUP > 1 && VEC ? (size_t)GLA_AHEAD * (PER * (2 * PT + 2) + PT) * GLA_ST * 16 : 0;      // the slots of pieces
-    constexpr size_t sm = (GROUP == 1 ? (size_t)(3 * DIMC + BCOLS) : (size_t)GLA_RING * GROUP * (3 * DIMC + 2 * BCOLS)) * sizeof(float) + RAW;
+    constexpr size_t sm = (GROUP == 1 ? (size_t)(3 * DIMC + BCOLS + DIMC * (BCOLS + 1)) : (size_t)GLA_RING * GROUP * (3 * DIMC + 2 * BCOLS)) * sizeof(float) + RAW;
     const dim3 grid((vdim_in + ones + BCOLS - 1) / BCOLS, H, seqs);
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(gla_walk_kernel<T, DIMC, GROUP, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
