@@ -79,10 +79,12 @@ _SIGNATURES = {
     ("linear_stream_tc", "ri_linear_stream_tc"): [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     ("linear_stream_tc", "ri_linear_stream_tc_gate"): [_P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P, _P],
     ("attention_prefill_tc", "ri_attention_prefill_tc"): [_P] * 8 + [_I] * 9 + [_F, _I, _P, _F, _P, _I, _I] + [_I, _I, _I, _F, _F, _F] + [_P, _P],
+    ("attention_latent_tc", "ri_attention_latent_tc"): [_P] * 7 + [_I] * 8 + [_F, _I, _P, _I, _P, _P],
     ("attention_prefill", "ri_attention_prefill"): [_P] * 8 + [_I] * 8 + [_F, _I, _P, _I, _F, _P, _I, _I, _I, _P, _P],
 }
 DECODE_CHUNK = 128          # keys per partial result of the decode attention kernel
 MAX_FAST_HEAD_DIM = 256
+LATENT_TC_ROW, LATENT_TC_VALUES = 256, 192     # rows (and leading value elements) of the tcgen05 kernel for latent attention
 TCGEN05_HEAD_DIMS = (64, 128)   # head sizes the tcgen05 prefill attention kernel is built for
 _NO_TCGEN05 = os.environ.get("RUST_INFERENCE_B200_NO_TCGEN05") == "1"   # for comparisons
 # the skinny linear applies the SiLU gate in its epilogue (one kernel less per layer: 2 % faster at batch 1 of
@@ -1154,6 +1156,15 @@ def attention_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
               q.shape[0], seqs, int(max_new), H, KV, Dh, page_table.shape[1], page_size, pages, float(scale),
               _mask(window, chunk), _sink(sink, H), _cap(softcap), *_bias(dist_bias, H), int(keep), int(width), int(vdim), int(pair_dim),
               float(lam), float(eps), float(gain), error_flag(q.device).data_ptr(), _stream(), defines={"RI_HEAD_DIM": Dh})
+        return out
+    if (Dh == LATENT_TC_ROW and 0 < v_dims <= LATENT_TC_VALUES and v_pool.data_ptr() == k_pool.data_ptr() and pair is None
+            and dist_bias is None and not softcap and (keep == 0 or window <= 0) and not _NO_TCGEN05):
+        # latent rows whose first elements are the values: the tcgen05 kernel that reads a tile once for both
+        out = torch.empty_like(q)
+        _call("attention_latent_tc", "ri_attention_latent_tc", q.data_ptr(), k_pool.data_ptr(), out.data_ptr(),
+              page_table.data_ptr(), seq_slot.data_ptr(), seq_start.data_ptr(), seq_len.data_ptr(), tokens, seqs, int(max_new), H,
+              KV, page_table.shape[1], page_size, pages, float(scale), _mask(window, chunk), _sink(sink, H), int(v_dims),
+              error_flag(q.device).data_ptr(), _stream())
         return out
     out = torch.empty(q.shape, dtype=q.dtype if pair is None else torch.float32, device=q.device)
     _call("attention_prefill", "ri_attention_prefill", q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),
