@@ -78,7 +78,8 @@ linear_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, floa
 // (fma.rn.f32x2 rounds each as fmaf does), the next 16 k on their way in registers and two buffers in shared memory.  What
 // bounds it: the multiply-adds (one instruction of two takes two cycles of a scheduler) and, at half their rate, the words that a
 // thread reads from shared memory for them: 16 for 64 with TN = 8, where the kernel above reads 8 for 16.  Every output is the
-// same chain of multiply-adds over ascending k: the same bits.  512 tokens of width 4,096 and 6,144 outputs: LF_FIGURES
+// same chain of multiply-adds over ascending k: the same bits.  512 tokens of width 4,096 and 6,144 outputs:
+// 643 us, 40 TFLOP/s, where the kernel above takes 893 us; 2,048 tokens 2,140 (48 TFLOP/s) and 2,961 us.
 #define LW_BM 128
 #define LW_THREADS 256
 template <int TN>
@@ -178,8 +179,11 @@ linear_f32_wide_kernel(const float* __restrict__ x, const float* __restrict__ w,
     }
 }
 
-// Which kernel: the one whose busiest SM has the least to do, in outputs times what one costs there (measured: the wide kernel 1
-// with TN = 8, 1.08 with 6, 1.3 with 4; the first kernel 2).
+// Which kernel: the one whose busiest SM has the least to do, in outputs times what one costs there.  Measured at K = 4,096: a
+// block of the wide kernel 430 us with TN = 8, 334 with 6, 250 with 4 (26 to 30 ns an output, with one or more blocks on
+// the SM alike); one of the first kernel 146 us among several (36 ns an output) and 334 us alone, so it is left for few rows
+// of more outputs than the SMs take at once.  64 rows of 4,096 outputs: 250 us with TN = 4, 334 with the first; 512 rows of 4,096:
+// 455 with TN = 8, 479 with 4, 586 with the first.
 static int lf_launch(const float* x, const float* w, float* y, int M, int N, int K, int heads, int vec_ok, long long ldx, long long ldy,
                      long long x_head, long long w_head, long long y_head, cudaStream_t stream) {
     static int sms = 0;
@@ -193,13 +197,11 @@ static int lf_launch(const float* x, const float* w, float* y, int M, int N, int
         const long long blocks = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) * heads;
         return (double)((blocks + sms - 1) / sms) * bm * bn * each;
     };
-    const double c[4] = {cost(LF_BM, LF_BN, 2.0), cost(LW_BM, 64, 1.3), cost(LW_BM, 96, 1.08), cost(LW_BM, 128, 1.0)};
+    const double alone = 2.3 * LF_BM * LF_BN * 1.36, first = cost(LF_BM, LF_BN, 1.36);
+    const double c[4] = {first < alone ? alone : first, cost(LW_BM, 64, 1.17), cost(LW_BM, 96, 1.06), cost(LW_BM, 128, 1.0)};
     int best = 0;
     for (int i = 1; i < 4; i++)
         if (c[i] < c[best]) best = i;
-#ifdef LF_FORCE
-    best = LF_FORCE;
-#endif
     const int bm = best ? LW_BM : LF_BM, bn = best == 0 ? LF_BN : best == 1 ? 64 : best == 2 ? 96 : 128;
     const dim3 grid((N + bn - 1) / bn, (M + bm - 1) / bm, heads);
 #define LW_GO(TN) linear_f32_wide_kernel<TN><<<grid, LW_THREADS, 0, stream>>>(x, w, y, M, N, K, vec_ok, ldx, ldy, x_head, w_head, y_head)

@@ -546,15 +546,26 @@ __global__ void sp_select_end_kernel(SpArgs a, int mode, int rows) {
 // them hold the same floor, prefix and remaining weight in registers and nobody waits for a leader.  The row's
 // histogram has three copies that take turns: while a pass adds to one, the blocks clear the next, and the one
 // before may still be read by a block that is late.  Sums are the same integers as in the other forms, so the
-// token is the same bit for bit.  A pass costs about five trips to the L2 cache; a draw at a temperature is seven
-// passes, a top-k or a top-p six more each.  Every wait is bounded by time (error 5, and the block returns).
+// token is the same bit for bit.  Every wait is bounded by time (error 5, and the block returns).
+//
+// A pass over the vocabulary costs about five trips to the L2 cache and a barrier, 6 to 8 us, and a search over five digits
+// has five of them; so only the top digit is searched that way.  What it leaves, the tokens of one bin (a top-k: of that bin
+// and those above it, all that the rest of the work can choose from), goes into a list of 2,048 keys in memory, from which a
+// block ends the search by itself, the same digits and sums over eight keys a thread (the L1 cache has them).  Three barriers with a top-k or a plain
+// draw, four with a top-p, where each search had five and each total one.  A list that does not fit (flat rows, a top-k of
+// thousands) leaves the lower digits to passes over the vocabulary as before.  8 rows of 151,936 logits, top-k 50 and top-p
+// 0.9: SP_FIGURES
 //
 // Scratch memory per row (SpFusedRow): zero at the start for `arrive` and `totals`: the launcher clears them.
 // ---------------------------------------------------------------------------
 #define SPF_TOTALS 4
+#define SPF_TOP ((SP_PASSES - 1) * SP_DIGIT)     // the shift of a key's top digit
+#define SPF_LIST 2048                       // keys of a list: eight per thread
+static_assert(2 * SPF_LIST <= SP_BINS, "the lists lie in the histogram that the kernels of one pass each use");
 struct __align__(16) SpFusedRow {
     unsigned arrive;
-    unsigned pad[3];
+    unsigned listed[2];      // keys in the row's two lists
+    unsigned pad;
     u64 totals[SPF_TOTALS];
 };
 
@@ -562,6 +573,7 @@ struct SpFusedArgs {
     SpArgs a;
     SpFusedRow* rows;        // [rows]
     u64* hist3;              // [rows][3][SP_BINS]
+    u64* lists;              // [rows][2][SPF_LIST]
     int* err;
 };
 
@@ -688,43 +700,114 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         ti++;
         return true;
     };
-    // The radix search (see radix_select): the largest key K such that the tokens with floor_key <= key and key >= K
-    // weigh `target` or more.  `last`: nobody but slice 0 needs the result of the last digit.
-    auto select = [&](u64 target, int counting, bool last, u64* K, int* found_out) -> bool {
-        u64 prefix = 0, remaining = target;
+    // w added to a bin: a 64-bit addition to shared memory is a compare-and-swap loop that crawls when many threads want
+    // one address, so the low word is added with the old value coming back (which tells whether this addition carried) and
+    // the high word takes the carry along.
+    unsigned* bins32 = reinterpret_cast<unsigned*>(bins);
+    auto add_bin = [&](unsigned bin, u64 w) {
+        const unsigned w_lo = (unsigned)w, w_hi = (unsigned)(w >> 32);
+        const unsigned old = atomicAdd(&bins32[2 * bin], w_lo);
+        const unsigned carry = old + w_lo < old ? 1u : 0u;
+        if (w_hi + carry) atomicAdd(&bins32[2 * bin + 1], w_hi + carry);
+    };
+    auto clear_bins = [&]() {
+        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) bins[b] = 0;
+        __syncthreads();
+    };
+    // this slice's part of the top digit's histogram (sign, exponent, three bits of the mantissa: the tokens crowd into a few
+    // bins), collected in shared memory
+    auto top_sweep = [&](int counting, u64* hist) {
+        __syncthreads();
+        clear_bins();
+#pragma unroll 4
+        for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
+            float zi = r.z(i);
+            u64 k = r.key(i, zi);
+            if (k < floor_key) continue;
+            const u64 w = weight_of(zi, zmax, counting);
+            if (w) add_bin((unsigned)(k >> SPF_TOP) & (SP_BINS - 1), w);
+        }
+        __syncthreads();
+        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) {
+            const u64 v = bins[b];
+            if (v) atomicAdd(&hist[b], v);
+        }
+    };
+    auto read_hist = [&](const u64* hist) {
+        __syncthreads();
+#pragma unroll 8
+        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) bins[b] = __ldcg(hist + b);
+        __syncthreads();
+    };
+    // The bin, from the top one down, at which the bins' running sum reaches `remaining`: its digit goes into prefix, what is
+    // above it comes off remaining; found 0 when all bins together stay below.
+    auto pick = [&](int shift, u64& prefix, u64& remaining, int& found) {
+        // sums of the 32 groups of 128 bins: a warp takes four groups, its lanes stride through a group
+        // (neighbouring lanes, neighbouring bins: no two lanes on one bank)
+        {
+            const int per = SP_BINS / 32;
+#pragma unroll
+            for (int q = 0; q < 32 / (SPW_THREADS / 32); q++) {
+                const int g = warp * (32 / (SPW_THREADS / 32)) + q;
+                u64 t = 0;
+#pragma unroll
+                for (int j = 0; j < per / 32; j++) t += bins[g * per + j * 32 + lane];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0) s_group[g] = t;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            // lane l stands for group l; from the top group down
+            const int per = SP_BINS / 32;
+            const u64 mine = s_group[lane];
+            const u64 above = spf_sum_above(mine, lane);
+            const int owner = (above < remaining && above + mine >= remaining) ? 1 : 0;
+            const unsigned ballot = __ballot_sync(0xffffffffu, owner);
+            if (ballot == 0) {
+                if (lane == 0) s_found = 0;
+            } else {
+                // inside the owning group the same once more: lane l holds bins 4 l .. 4 l + 3 of it
+                const int g = __ffs(ballot) - 1;
+                const u64 g_above = __shfl_sync(0xffffffffu, above, g);
+                u64 b4[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) b4[j] = bins[g * per + 4 * lane + j];
+                const u64 mine4 = (b4[0] + b4[1]) + (b4[2] + b4[3]);
+                const u64 above4 = g_above + spf_sum_above(mine4, lane);
+                if (above4 < remaining && above4 + mine4 >= remaining) {
+                    u64 acc = above4;
+                    int chosen = g * per + 4 * lane;
+#pragma unroll
+                    for (int j = 3; j >= 0; j--) {
+                        if (acc + b4[j] >= remaining) { chosen = g * per + 4 * lane + j; break; }
+                        acc += b4[j];
+                    }
+                    s_prefix = prefix | ((u64)chosen << shift);
+                    s_remaining = remaining - acc;
+                    s_found = 1;
+                }
+            }
+        }
+        __syncthreads();
+        found = s_found;
+        if (found) { prefix = s_prefix; remaining = s_remaining; }
+        __syncthreads();
+    };
+    // The radix search over the vocabulary (see radix_select): the largest key K such that the tokens with floor_key <= key and
+    // key >= K weigh `target` or more, from digit `pass` on (prefix: the digits above it).  `last`: nobody but slice 0 needs
+    // the result of the last digit.
+    auto select = [&](int pass, u64 prefix, u64 remaining, int counting, bool last, u64* K, int* found_out) -> bool {
         int found = 1;
-        for (int pass = SP_PASSES - 1; pass >= 0; pass--, hp++) {
+        for (; pass >= 0; pass--, hp++) {
             const int shift = pass * SP_DIGIT;
             u64* hist = hist3 + (size_t)(hp % 3) * SP_BINS;
             if (found && pass == SP_PASSES - 1) {
-                // The top digit (sign, exponent, three bits of the mantissa): the tokens crowd into a few bins.  A
-                // 64-bit addition to shared memory is a compare-and-swap loop that crawls when many threads want
-                // one address, so a bin is kept as two 32-bit words: the low word is added with the old value
-                // coming back (which tells whether this addition carried), the high word takes the carry along.
-                unsigned* lo32 = reinterpret_cast<unsigned*>(bins);
-                unsigned* hi32 = lo32 + SP_BINS;
-                for (int b = threadIdx.x; b < 2 * SP_BINS; b += SPW_THREADS) lo32[b] = 0;
-                __syncthreads();
-                for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
-                    float zi = r.z(i);
-                    u64 k = r.key(i, zi);
-                    if (k < floor_key) continue;
-                    const u64 w = weight_of(zi, zmax, counting);
-                    if (!w) continue;
-                    const unsigned bin = (unsigned)(k >> shift) & (SP_BINS - 1);
-                    const unsigned w_lo = (unsigned)w, w_hi = (unsigned)(w >> 32);
-                    const unsigned old = atomicAdd(&lo32[bin], w_lo);
-                    const unsigned carry = old + w_lo < old ? 1u : 0u;
-                    if (w_hi + carry) atomicAdd(&hi32[bin], w_hi + carry);
-                }
-                __syncthreads();
-                for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) {
-                    const u64 v = ((u64)hi32[b] << 32) + lo32[b];
-                    if (v) atomicAdd(&hist[b], v);
-                }
+                top_sweep(counting, hist);
             } else if (found) {
-                // a lower digit: only the tokens that share the digits found so far count, a handful as a rule;
-                // they are added to the row's histogram directly
+                // a lower digit: only the tokens that share the digits found so far count; they are added to the row's
+                // histogram directly
                 for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
                     float zi = r.z(i);
                     u64 k = r.key(i, zi);
@@ -739,60 +822,8 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, waits, f.err)) return false;
             if (!waits) return true;                   // the last digit of the draw: slice 0 finishes alone
             if (found) {
-                for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) bins[b] = __ldcg(hist + b);
-                __syncthreads();
-                // sums of the 32 groups of 128 bins: a warp takes four groups, its lanes stride through a group
-                // (neighbouring lanes, neighbouring bins: no two lanes on one bank)
-                {
-                    const int per = SP_BINS / 32;
-#pragma unroll
-                    for (int q = 0; q < 32 / (SPW_THREADS / 32); q++) {
-                        const int g = warp * (32 / (SPW_THREADS / 32)) + q;
-                        u64 t = 0;
-#pragma unroll
-                        for (int j = 0; j < per / 32; j++) t += bins[g * per + j * 32 + lane];
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-                        if (lane == 0) s_group[g] = t;
-                    }
-                }
-                __syncthreads();
-                if (threadIdx.x < 32) {
-                    // lane l stands for group l; from the top group down
-                    const int per = SP_BINS / 32;
-                    const u64 mine = s_group[lane];
-                    const u64 above = spf_sum_above(mine, lane);
-                    const int owner = (above < remaining && above + mine >= remaining) ? 1 : 0;
-                    const unsigned ballot = __ballot_sync(0xffffffffu, owner);
-                    if (ballot == 0) {
-                        if (lane == 0) s_found = 0;
-                    } else {
-                        // inside the owning group the same once more: lane l holds bins 4 l .. 4 l + 3 of it
-                        const int g = __ffs(ballot) - 1;
-                        const u64 g_above = __shfl_sync(0xffffffffu, above, g);
-                        u64 b4[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) b4[j] = bins[g * per + 4 * lane + j];
-                        const u64 mine4 = (b4[0] + b4[1]) + (b4[2] + b4[3]);
-                        const u64 above4 = g_above + spf_sum_above(mine4, lane);
-                        if (above4 < remaining && above4 + mine4 >= remaining) {
-                            u64 acc = above4;
-                            int chosen = g * per + 4 * lane;
-#pragma unroll
-                            for (int j = 3; j >= 0; j--) {
-                                if (acc + b4[j] >= remaining) { chosen = g * per + 4 * lane + j; break; }
-                                acc += b4[j];
-                            }
-                            s_prefix = prefix | ((u64)chosen << shift);
-                            s_remaining = remaining - acc;
-                            s_found = 1;
-                        }
-                    }
-                }
-                __syncthreads();
-                found = s_found;
-                if (found) { prefix = s_prefix; remaining = s_remaining; }
-                __syncthreads();
+                read_hist(hist);
+                pick(shift, prefix, remaining, found);
             }
         }
         *K = prefix;
@@ -800,33 +831,222 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         return true;
     };
 
-    u64 K;
-    int found;
-    const int k = (use_top_k && a.top_k) ? a.top_k[row] : 0;
-    if (k > 0 && k < a.vocab) {
-        if (!select((u64)k, 1, false, &K, &found)) return;
-        if (found) floor_key = K;
-    }
-    if (!sum_total()) return;
+    // ---- lists: the keys of a few bins, from which a block ends a search by itself ---------------------------------
+    // the keys of this slice whose top digit lies in [first, last], into list `which` of the row (what does not fit is counted
+    // only); true when the wait ended
+    u64* lists = f.lists + (size_t)row * 2 * SPF_LIST;
+    auto gather = [&](unsigned first, unsigned last, int which, bool wait) -> bool {
+        int mine = 0;
+#pragma unroll 4
+        for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
+            const unsigned top = (unsigned)(r.key(i, r.z(i)) >> SPF_TOP);
+            mine += top >= first && top <= last;
+        }
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const int all = __shfl_sync(0xffffffffu, upto, 31);
+        if (all) {
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&shared_row->listed[which], (unsigned)all);
+            at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)(upto - mine);
+            if (mine)
+                for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
+                    const u64 k = r.key(i, r.z(i));
+                    const unsigned top = (unsigned)(k >> SPF_TOP);
+                    if (top < first || top > last) continue;
+                    if (at < SPF_LIST) lists[which * SPF_LIST + at] = k;
+                    at++;
+                }
+        }
+        return spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, wait, f.err);
+    };
+    // Key q of this thread (~0: none; it is above every floor and no prefix has it).  An ordinary load: nobody reads a list
+    // before the barrier that ends its writing, and from then on the L1 cache may keep it.
+    const u64* list = lists;
+    unsigned listed = 0;
+    auto key_at = [&](int q) {
+        const unsigned i = threadIdx.x + q * SPW_THREADS;
+        return i < listed ? list[i] : ~0ull;
+    };
+    // exp(z - zmax) of a key, with z from the key: the same bits as from the logit
+    auto key_weight = [&](u64 k) {
+        const unsigned u = (unsigned)(k >> SP_IDX_BITS);
+        const float zi = u == 0u ? __uint_as_float(0x7fffffffu) : __uint_as_float((u & 0x80000000u) ? u ^ 0x80000000u : ~u);
+        return weight_of(zi, zmax, 0);
+    };
+    auto list_sum = [&](u64 from) {
+        u64 part = 0;
+#pragma unroll
+        for (int q = 0; q < SPF_LIST / SPW_THREADS; q++) {
+            const u64 k = key_at(q);
+            if (k != ~0ull && k >= from) part += key_weight(k);
+        }
+        return block_sum_u64(part, red);
+    };
+    // the same search over the list's keys, with the same digits and sums; when one key is left, that is the one
+    auto select_list = [&](int pass, u64 prefix, u64 remaining, int counting, u64* K) -> int {
+        int found = 1;
+        for (; pass >= 0 && found; pass--) {
+            const int shift = pass * SP_DIGIT;
+            int mine = 0;
+            u64 key = 0;
+            unsigned alive = 0;
+#pragma unroll
+            for (int q = 0; q < SPF_LIST / SPW_THREADS; q++) {
+                const u64 k = key_at(q);
+                const bool in = k != ~0ull && k >= floor_key && (k >> (shift + SP_DIGIT)) == (prefix >> (shift + SP_DIGIT)) &&
+                                (counting || key_weight(k));
+                if (in) { mine++; key = k; alive |= 1u << q; }
+            }
+            const int several = __syncthreads_or(mine > 1);
+            if (__syncthreads_count(mine == 1) == 1 && !several) {
+                if (mine) s_prefix = key;
+                __syncthreads();
+                prefix = s_prefix;
+                __syncthreads();
+                break;
+            }
+            clear_bins();
+#pragma unroll
+            for (int q = 0; q < SPF_LIST / SPW_THREADS; q++)
+                if (alive >> q & 1) {
+                    const u64 k = key_at(q);
+                    add_bin((unsigned)(k >> shift) & (SP_BINS - 1), counting ? 1ull : key_weight(k));
+                }
+            __syncthreads();
+            pick(shift, prefix, remaining, found);
+        }
+        *K = prefix;
+        return found;
+    };
+    auto finish = [&](int found, u64 K) {
+        if (s == 0 && threadIdx.x == 0) {
+            int tok = bi;                                 // cannot happen for total > 0; stay in range
+            if (found && total != 0) tok = (int)(((1u << SP_IDX_BITS) - 1u) - (unsigned)(K & ((1u << SP_IDX_BITS) - 1u)));
+            a.out[row] = tok;
+        }
+    };
+
     const float tp = (use_top_p && a.top_p) ? a.top_p[row] : 1.0f;
-    if (tp < 1.0f) {
+    auto top_p_target = [&]() {
         const double want = (double)tp * (double)total;
         u64 target = (u64)want;
         if ((double)target < want) target += 1;           // ceil
-        if (target < 1) target = 1;
-        if (!select(target, 0, false, &K, &found)) return;
+        return target < 1 ? (u64)1 : target;
+    };
+    auto draw_target = [&]() {
+        const double ru = (double)a.uniform[row] * (double)total;
+        const u64 target = (u64)ru + 1;                   // running sum > u * total
+        return target > total ? total : target;
+    };
+    u64 K;
+    int found;
+    const int k = (use_top_k && a.top_k) ? a.top_k[row] : 0;
+    const bool top_k = k > 0 && k < a.vocab;
+    // the top digit of the first search: the count for a top-k, else the weight
+    top_sweep(top_k, hist3);
+    clear_share(1);
+    if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, true, f.err)) return;
+    read_hist(hist3);
+    hp = 1;
+    bool narrowed = false;                                // the vocabulary is down to floor_key and `total` is its weight
+    if (top_k) {
+        u64 prefix = 0, remaining = (u64)k;
+        pick(SPF_TOP, prefix, remaining, found);
+        const unsigned first = (unsigned)(prefix >> SPF_TOP);
+        const u64 n = (u64)k - remaining + bins[first];   // tokens in that bin and above
+        if (found && n <= SPF_LIST) {
+            // all that the rest can choose from fits a list: slice 0 ends the work alone
+            if (!gather(first, SP_BINS - 1, 0, s == 0) || s != 0) return;
+            listed = (unsigned)n;
+            if (select_list(SP_PASSES - 2, prefix, remaining, 1, &K)) floor_key = K;
+            total = list_sum(floor_key);
+            if (tp < 1.0f && select_list(SP_PASSES - 1, 0, top_p_target(), 0, &K)) {
+                floor_key = K;
+                total = list_sum(floor_key);
+            }
+            found = select_list(SP_PASSES - 1, 0, draw_target(), 0, &K);
+            finish(found, K);
+            return;
+        }
+        if (found && !select(SP_PASSES - 2, prefix, remaining, 1, false, &K, &found)) return;
         if (found) floor_key = K;
         if (!sum_total()) return;
+        if (tp < 1.0f) {
+            if (!select(SP_PASSES - 1, 0, top_p_target(), 0, false, &K, &found)) return;
+            if (found) floor_key = K;
+            if (!sum_total()) return;
+        }
+        narrowed = true;
+    } else {
+        u64 part = 0;
+        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) part += bins[b];
+        total = block_sum_u64(part, red);
+        unsigned floor_bin = 0;                           // bins below it are out; list 0 has its keys when floor_listed
+        bool floor_listed = false;
+        if (tp < 1.0f) {
+            const u64 target = top_p_target();
+            u64 prefix = 0, remaining = target;
+            pick(SPF_TOP, prefix, remaining, found);
+            if (found) {
+                const u64 above = target - remaining;
+                floor_bin = (unsigned)(prefix >> SPF_TOP);
+                if (!gather(floor_bin, floor_bin, 0, true)) return;
+                const unsigned n = __ldcg(&shared_row->listed[0]);
+                if (n <= SPF_LIST) {
+                    listed = n;
+                    floor_listed = select_list(SP_PASSES - 2, prefix, remaining, 0, &K) != 0;
+                    u64 inside = 0;
+                    if (floor_listed) {
+                        floor_key = K;
+                        inside = list_sum(K);
+                        total = above + inside;
+                    }
+                    read_hist(hist3);
+                    if (floor_listed) {
+                        for (int b = threadIdx.x; b <= (int)floor_bin; b += SPW_THREADS) bins[b] = b == (int)floor_bin ? inside : 0;
+                        __syncthreads();
+                    }
+                } else {
+                    if (!select(SP_PASSES - 2, prefix, remaining, 0, false, &K, &found)) return;
+                    if (found) floor_key = K;
+                    if (!sum_total()) return;
+                    narrowed = true;
+                }
+            }
+        }
+        if (!narrowed) {
+            u64 prefix = 0, remaining = draw_target();
+            pick(SPF_TOP, prefix, remaining, found);
+            if (!found) {
+                finish(0, 0);
+                return;
+            }
+            const unsigned bin = (unsigned)(prefix >> SPF_TOP);
+            if (!(floor_listed && bin == floor_bin)) {
+                if (!gather(bin, bin, 1, true)) return;
+                const unsigned n = __ldcg(&shared_row->listed[1]);
+                if (n > SPF_LIST) {
+                    if (!select(SP_PASSES - 2, prefix, remaining, 0, true, &K, &found)) return;
+                    finish(found, K);
+                    return;
+                }
+                if (s != 0) return;
+                list = lists + SPF_LIST;
+                listed = n;
+            }
+            if (s != 0) return;
+            found = select_list(SP_PASSES - 2, prefix, remaining, 0, &K);
+            finish(found, K);
+            return;
+        }
     }
-    const double ru = (double)a.uniform[row] * (double)total;
-    u64 target = (u64)ru + 1;                             // running sum > u * total
-    if (target > total) target = total;
-    if (!select(target, 0, true, &K, &found)) return;
-    if (s == 0 && threadIdx.x == 0) {
-        int tok = bi;                                     // cannot happen for total > 0; stay in range
-        if (found && total != 0) tok = (int)(((1u << SP_IDX_BITS) - 1u) - (unsigned)(K & ((1u << SP_IDX_BITS) - 1u)));
-        a.out[row] = tok;
-    }
+    if (!select(SP_PASSES - 1, 0, draw_target(), 0, true, &K, &found)) return;
+    finish(found, K);
 }
 
 static size_t spw_align(size_t n) { return (n + 255) & ~(size_t)255; }
@@ -886,6 +1106,7 @@ static int launch_sample_wide(SpArgs a, int rows, void* work, int use_top_k, int
         f.a = a;
         f.rows = fused_rows;
         f.hist3 = hist3;
+        f.lists = a.hist;
         f.err = err_flag;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(a.slices, rows);

@@ -1,0 +1,53 @@
+"""The one-kernel sampler ends a search over a list of at most 2,048 keys: the same tokens, bit for bit, as the form that passes
+over the vocabulary for every digit (whole-number sums, so there is nothing to tolerate)."""
+import pytest
+import torch
+
+from rust_inference_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+KINDS = ["normal", "flat", "narrow", "wide", "masked", "nan", "inf", "equal_pairs"]
+
+
+def _logits(kind, rows, vocab, g):
+    x = torch.randn((rows, vocab), generator=g, device="cuda")
+    if kind == "flat":
+        return torch.full_like(x, 0.75)
+    if kind == "narrow":
+        return 3.0 + 1e-3 * x
+    if kind == "wide":
+        return 40.0 * x
+    x = 2.5 * x
+    if kind == "masked":
+        x[:, 37:] = -float("inf")
+    if kind == "nan":
+        x[:, 5::7] = float("nan")
+        x[0] = float("nan")
+    if kind == "inf":
+        x[:, 11::4099] = float("inf")
+    if kind == "equal_pairs":
+        x = (x * 8).round() / 8
+    return x
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rows,vocab", [(1, 32000), (9, 151936), (37, 50257)])
+def test_lists_choose_what_the_passes_choose(kind, rows, vocab, monkeypatch):
+    g = torch.Generator(device="cuda").manual_seed(rows * 1000 + len(kind))
+    logits = _logits(kind, rows, vocab, g)
+    temperature = torch.rand(rows, generator=g, device="cuda") * 1.5 + 0.2
+    temperature[rows // 2] = 0.0 if rows > 1 else 1.0
+    # edges of a list: exactly full, one too many, nothing, all
+    ks = torch.tensor([0, 1, 50, 1500, 2047, 2048, 2049, 6000, vocab], dtype=torch.int32, device="cuda")
+    ps = torch.tensor([1.0, 0.9, 1e-7, 0.5, 0.9999, 0.0, 0.05], device="cuda")
+    for shift in range(3):
+        top_k = ks[(torch.arange(rows, device="cuda") + 3 * shift) % len(ks)].contiguous()
+        top_p = ps[(torch.arange(rows, device="cuda") + shift) % len(ps)].contiguous()
+        u = torch.rand(rows, generator=g, device="cuda")
+        for k, p in ((top_k, top_p), (top_k, None), (None, top_p), (None, None)):
+            monkeypatch.setattr(ops, "SAMPLE_ONE_KERNEL", True)
+            got = ops.sample(logits, temperature, u, top_k=k, top_p=p)
+            monkeypatch.setattr(ops, "SAMPLE_ONE_KERNEL", False)
+            want = ops.sample(logits, temperature, u, top_k=k, top_p=p)
+            assert torch.equal(got, want), (shift, k is not None, p is not None)
