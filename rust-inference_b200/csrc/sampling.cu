@@ -616,12 +616,13 @@ __device__ __forceinline__ u64 spf_sum_above(u64 mine, int lane) {
 }
 
 __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, int use_top_k, int use_top_p) {
-    __shared__ u64 bins[SP_BINS];
+    __shared__ __align__(16) u64 bins[SP_BINS];
     __shared__ u64 red[33];
     __shared__ float fred[SPW_THREADS / 32];
     __shared__ int ired[SPW_THREADS / 32];
     __shared__ u64 s_prefix, s_remaining, s_group[32];
     __shared__ int s_found;
+    __shared__ unsigned s_base;
     const SpArgs& a = f.a;
     const int row = blockIdx.y, s = blockIdx.x, slices = a.slices;
     SpFusedRow* shared_row = f.rows + row;
@@ -726,7 +727,9 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             u64 k = r.key(i, zi);
             if (k < floor_key) continue;
             const u64 w = weight_of(zi, zmax, counting);
-            if (w) add_bin((unsigned)(k >> SPF_TOP) & (SP_BINS - 1), w);
+            const unsigned bin = (unsigned)(k >> SPF_TOP) & (SP_BINS - 1);
+            if (counting) atomicAdd(&bins32[2 * bin], 1u);        // a vocabulary's count fits the low word
+            else if (w) add_bin(bin, w);
         }
         __syncthreads();
         for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) {
@@ -837,11 +840,14 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
     // only); true when the wait ended
     u64* lists = f.lists + (size_t)row * 2 * SPF_LIST;
     auto gather = [&](unsigned first, unsigned last, int which, bool wait) -> bool {
-        int mine = 0;
+        int mine = 0, j = 0;
+        unsigned hits = 0;                                // which of this thread's first 32 tokens
 #pragma unroll 4
-        for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
+        for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS, j++) {
             const unsigned top = (unsigned)(r.key(i, r.z(i)) >> SPF_TOP);
-            mine += top >= first && top <= last;
+            const bool in = top >= first && top <= last;
+            mine += in;
+            if (in && j < 32) hits |= 1u << j;
         }
         int upto = mine;
 #pragma unroll
@@ -849,19 +855,29 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             const int v = __shfl_up_sync(0xffffffffu, upto, o);
             if (lane >= o) upto += v;
         }
-        const int all = __shfl_sync(0xffffffffu, upto, 31);
-        if (all) {
-            unsigned at = 0;
-            if (lane == 0) at = atomicAdd(&shared_row->listed[which], (unsigned)all);
-            at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)(upto - mine);
-            if (mine)
-                for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
-                    const u64 k = r.key(i, r.z(i));
-                    const unsigned top = (unsigned)(k >> SPF_TOP);
-                    if (top < first || top > last) continue;
-                    if (at < SPF_LIST) lists[which * SPF_LIST + at] = k;
-                    at++;
-                }
+        if (lane == 31) ired[warp] = upto;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int all = 0;
+            for (int w = 0; w < SPW_THREADS / 32; w++) {
+                const int t = ired[w];
+                ired[w] = all;
+                all += t;
+            }
+            s_base = all ? atomicAdd(&shared_row->listed[which], (unsigned)all) : 0u;
+        }
+        __syncthreads();
+        if (mine) {
+            unsigned at = s_base + (unsigned)(ired[warp] + upto - mine);
+            j = 0;
+            for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS, j++) {
+                if (j < 32 && !(hits >> j & 1)) continue;
+                const u64 k = r.key(i, r.z(i));
+                const unsigned top = (unsigned)(k >> SPF_TOP);
+                if (top < first || top > last) continue;
+                if (at < SPF_LIST) lists[which * SPF_LIST + at] = k;
+                at++;
+            }
         }
         return spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, wait, f.err);
     };
@@ -944,6 +960,51 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         const u64 target = (u64)ru + 1;                   // running sum > u * total
         return target > total ? total : target;
     };
+    // The end of a top-k of at most a thread's key each: the k keys and their weights side by side in shared memory, each
+    // thread's running sum over all of them (keys are unique), and from it the top-p's key, what it leaves, and the draw's.  False
+    // when a weight is none of a finite number: such sums wrap around, which only the digits' order repeats.
+    auto few_left = [&](int n) -> bool {
+        __syncthreads();
+        if (threadIdx.x == 0) s_base = 0;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < SPF_LIST / SPW_THREADS; q++) {
+            const u64 k = key_at(q);
+            if (k != ~0ull && k >= floor_key) bins[2 * atomicAdd(&s_base, 1u)] = k;
+        }
+        __syncthreads();
+        const u64 key = (int)threadIdx.x < n ? bins[2 * threadIdx.x] : 0;
+        const u64 w = (int)threadIdx.x < n ? key_weight(key) : 0;
+        if (__syncthreads_or(w > (1ull << 40))) return false;
+        if ((int)threadIdx.x < n) bins[2 * threadIdx.x + 1] = w;
+        __syncthreads();
+        u64 sum = 0, all = 0;
+        if (warp * 32 < n)
+            for (int j = 0; j < n; j++) {
+                const ulonglong2 other = *reinterpret_cast<const ulonglong2*>(&bins[2 * j]);
+                all += other.y;
+                if (other.x >= key) sum += other.y;
+            }
+        if (threadIdx.x == 0) { s_remaining = all; s_prefix = 0; }
+        __syncthreads();
+        total = s_remaining;
+        if (tp < 1.0f) {
+            const u64 target = top_p_target();
+            __syncthreads();
+            if (w && sum >= target && sum - w < target) { s_prefix = key; s_remaining = sum; }
+            __syncthreads();
+            floor_key = s_prefix;
+            total = s_remaining;
+        }
+        const u64 target = draw_target();
+        if (threadIdx.x == 0) s_found = 0;
+        __syncthreads();
+        if (w && sum >= target && sum - w < target) { s_prefix = key; s_found = 1; }
+        __syncthreads();
+        finish(s_found, s_prefix);
+        return true;
+    };
+
     u64 K;
     int found;
     const int k = (use_top_k && a.top_k) ? a.top_k[row] : 0;
@@ -964,7 +1025,10 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             // all that the rest can choose from fits a list: slice 0 ends the work alone
             if (!gather(first, SP_BINS - 1, 0, s == 0) || s != 0) return;
             listed = (unsigned)n;
-            if (select_list(SP_PASSES - 2, prefix, remaining, 1, &K)) floor_key = K;
+            if (select_list(SP_PASSES - 2, prefix, remaining, 1, &K)) {
+                floor_key = K;                            // k keys are left
+                if (k <= SPW_THREADS && few_left(k)) return;
+            }
             total = list_sum(floor_key);
             if (tp < 1.0f && select_list(SP_PASSES - 1, 0, top_p_target(), 0, &K)) {
                 floor_key = K;
