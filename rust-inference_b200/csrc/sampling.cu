@@ -81,7 +81,11 @@ __device__ u64 block_sum_u64(u64 v, u64* red) {
 // weight of token i: 1 when counting, exp(z - zmax) * 2^40 as an integer otherwise
 __device__ __forceinline__ u64 weight_of(float zi, float zmax, int counting) {
     if (counting) return 1ull;
-    return (u64)(expf(zi - zmax) * 1099511627776.0f);      // 2^40: exact scaling, sums stay below 2^64
+    // 2^40: exact scaling, sums stay below 2^64.  The conversion by its instruction: what a cast makes of a NaN is the compiler's choice, and
+    // has to be one and the same (2^63) everywhere
+    u64 w;
+    asm("cvt.rzi.u64.f32 %0, %1;" : "=l"(w) : "f"(expf(zi - zmax) * 1099511627776.0f));
+    return w;
 }
 
 // The largest key K (among tokens with key >= floor_key) such that the weight of
@@ -780,7 +784,11 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                 for (int j = 0; j < 4; j++) b4[j] = bins[g * per + 4 * lane + j];
                 const u64 mine4 = (b4[0] + b4[1]) + (b4[2] + b4[3]);
                 const u64 above4 = g_above + spf_sum_above(mine4, lane);
-                if (above4 < remaining && above4 + mine4 >= remaining) {
+                // one lane, unless NaN or +inf among the logits made the sums wrap around: then the topmost
+                const unsigned owners = __ballot_sync(0xffffffffu, above4 < remaining && above4 + mine4 >= remaining);
+                if (owners == 0) {
+                    if (lane == 0) s_found = 0;
+                } else if (lane == 31 - __clz(owners)) {
                     u64 acc = above4;
                     int chosen = g * per + 4 * lane;
 #pragma unroll
