@@ -84,7 +84,10 @@ _SIGNATURES = {
 }
 DECODE_CHUNK = 128          # keys per partial result of the decode attention kernel
 MAX_FAST_HEAD_DIM = 256
-LATENT_TC_ROW, LATENT_TC_VALUES = 256, 192     # rows (and leading value elements) of the tcgen05 kernel for latent attention
+# Rows (and leading value elements) of the tcgen05 kernel for latent attention; it is the faster one at every length, mma.sync
+# kernel behind it (us, 32 heads): 2 new tokens alone 12.3 / 14.3, 64 alone 13.1 / 16.3, 3 behind 2,000 61.4 / 235.5, 8 x 64
+# behind 1,000 75.8 / 148.3, 2,048 alone 100 / 576.
+LATENT_TC_ROW, LATENT_TC_VALUES = 256, 192
 TCGEN05_HEAD_DIMS = (64, 128)   # head sizes the tcgen05 prefill attention kernel is built for
 _NO_TCGEN05 = os.environ.get("RUST_INFERENCE_B200_NO_TCGEN05") == "1"   # for comparisons
 # the skinny linear applies the SiLU gate in its epilogue (one kernel less per layer: 2 % faster at batch 1 of
