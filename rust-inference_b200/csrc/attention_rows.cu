@@ -16,8 +16,8 @@
 // Work is shared between rows, not split inside one: a block takes up to `tile_q` consecutive new tokens
 // of one sequence and up to `group_chunk` query heads of one kv head, stages each strip of keys and
 // values once in shared memory (as float32) for all of them, and every warp then takes the rows
-// w, w + 8, ... two at a time (two query heads of one token: what is read of a key or a value from shared memory
-// serves both): a row belongs to one warp from start to end, its running maximum, sum and output live in shared
+// w, w + 8, ... four or two at a time (query heads of one token: what is read of a key or a value from shared memory
+// serves them all): a row belongs to one warp from start to end, its running maximum, sum and output live in shared
 // memory between strips.  Keys and values are thus read from memory once per
 // (tile, kv head) where one block per (token, head) would read them tile_q x group size times.
 //
@@ -55,7 +55,7 @@ template <> struct ArVec<__nv_bfloat16> {
 
 __host__ __device__ inline int ar_key_pitch(int Dh, bool vec4) { return vec4 ? Dh + 4 : Dh + 1; }    // floats per staged key
 
-// One strip of keys for R (1 or 2) rows that follow each other in shared memory and see the same keys j_lo .. j_hi of
+// One strip of keys for R (1, 2 or 4) rows that follow each other in shared memory and see the same keys j_lo .. j_hi of
 // the strip, except hole_lo .. hole_hi - 1 (between the kept first keys and the window; a key in the hole has weight 0):
 // scores (lane j = key j), the online-softmax update of each row's maximum and sum, and the rows' outputs
 // (a lane owns head elements lane, lane + 32, ...; the keys are added in rising order).
@@ -230,11 +230,13 @@ attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, con
             }
         }
         __syncthreads();
-        // a warp takes two query heads of one token at a time (they see the same keys): a key or a value read from
-        // shared memory then serves both rows; each row's own arithmetic and its order are what they would be alone
-        const int pairs = (ng + 1) >> 1;
-        for (int unit = warp; unit < nq * pairs; unit += AR_WARPS) {
-            const int i = unit / pairs, g_first = 2 * (unit - i * pairs);
+        // A warp takes four query heads of one token at a time (they see the same keys), or two where fours would leave warps idle:
+        // a key or a value read from shared memory then serves all of them; each row's own arithmetic and its order are
+        // what they would be alone
+        const int per_unit = nq * ((ng + 3) >> 2) >= AR_WARPS ? 4 : 2;
+        const int units = (ng + per_unit - 1) / per_unit;
+        for (int unit = warp; unit < nq * units; unit += AR_WARPS) {
+            const int i = unit / units, g_first = per_unit * (unit - i * units);
             const int pos = pos0 + i;
             const int first = ri_first_visible(pos, window);
             // the token's keys in this strip: from the window's first one (or, where kept keys are, from the strip's start)
@@ -244,15 +246,20 @@ attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, con
             int j_hi = min(pos - key0, width - 1);
             if (hole_hi > j_hi) j_hi = min(j_hi, hole_lo - 1);
             if (j_lo > j_hi) continue;                                // none: the rows' state stays as it is
-            const int row_a = i * ng + g_first;
-            const float* bias_row = bias.table ? ri_bias_row(bias, kvh * G + g0 + g_first) : nullptr;
             const int distance = pos - key0 - lane;
-            if (g_first + 1 < ng)
-                ar_strip<VEC4, 2>(qs, accs, ms, ls, ks, vs, row_a, Dh, kpitch, j_lo, j_hi, hole_lo, hole_hi, scale, softcap, lane, bias_row,
-                                  bias.len, distance);
-            else
-                ar_strip<VEC4, 1>(qs, accs, ms, ls, ks, vs, row_a, Dh, kpitch, j_lo, j_hi, hole_lo, hole_hi, scale, softcap, lane, bias_row,
-                                  bias.len, distance);
+            const int g_end = min(g_first + per_unit, ng);
+            for (int g = g_first; g < g_end;) {
+                const int row_a = i * ng + g;
+                const float* bias_row = bias.table ? ri_bias_row(bias, kvh * G + g0 + g) : nullptr;
+#define AR_STRIP_GO(R) \
+    ar_strip<VEC4, R>(qs, accs, ms, ls, ks, vs, row_a, Dh, kpitch, j_lo, j_hi, hole_lo, hole_hi, scale, softcap, lane, bias_row, \
+                      bias.len, distance); \
+    g += R
+                if (g + 3 < g_end) { AR_STRIP_GO(4); }
+                else if (g + 1 < g_end) { AR_STRIP_GO(2); }
+                else { AR_STRIP_GO(1); }
+#undef AR_STRIP_GO
+            }
         }
         key0 += width;
     }
