@@ -1504,6 +1504,8 @@ def moe_grouped_linear(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, ga
     out_dtype = out_dtype or a.dtype
     if out_dtype not in (a.dtype, torch.float32):
         raise KernelError("moe_grouped_linear: the result is float32 or the compute dtype")
+    if bm == MOE_TILE_ROWS_WIDE and a.dtype != torch.bfloat16:
+        raise KernelError(f"moe_grouped_linear: a plan with tiles of {bm} rows is for bfloat16 products, not {a.dtype}")
     y = torch.empty((rows_out, N), dtype=out_dtype, device=a.device)
     if bm == MOE_TILE_ROWS_WIDE:
         if gather_div > 0:
@@ -1521,6 +1523,7 @@ def moe_grouped_linear(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, ga
 def _moe_gather(x: torch.Tensor, plan, pairs: int, div: int) -> torch.Tensor:
     """[pairs, K]: row r is x[perm[r] // div] for the plan's rows (bfloat16 rows of whole 16-byte pieces)."""
     perm, _, meta, _ = plan
+    _need(x, "x", torch.bfloat16)
     out = torch.empty((pairs, x.shape[1]), dtype=x.dtype, device=x.device)
     _call("moe_tc", "ri_moe_gather", x.data_ptr(), x.stride(0), out.data_ptr(), perm.data_ptr(), meta.data_ptr(), perm.numel(), int(div),
           x.shape[1], _stream())
