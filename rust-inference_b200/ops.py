@@ -88,6 +88,8 @@ MAX_FAST_HEAD_DIM = 256
 # kernel behind it (us, 32 heads): 2 new tokens alone 12.3 / 14.3, 64 alone 13.1 / 16.3, 3 behind 2,000 61.4 / 235.5, 8 x 64
 # behind 1,000 75.8 / 148.3, 2,048 alone 100 / 576.
 LATENT_TC_ROW, LATENT_TC_VALUES = 256, 192
+# ... which masks a score before it is scaled: -FLT_MAX times the scale has to lie far below every score that counts
+LATENT_TC_SCALE = 1e-30
 TCGEN05_HEAD_DIMS = (64, 128)   # head sizes the tcgen05 prefill attention kernel is built for
 _NO_TCGEN05 = os.environ.get("RUST_INFERENCE_B200_NO_TCGEN05") == "1"   # for comparisons
 # the skinny linear applies the SiLU gate in its epilogue (one kernel less per layer: 2 % faster at batch 1 of
@@ -1161,13 +1163,14 @@ def attention_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
               float(lam), float(eps), float(gain), error_flag(q.device).data_ptr(), _stream(), defines={"RI_HEAD_DIM": Dh})
         return out
     if (Dh == LATENT_TC_ROW and 0 < v_dims <= LATENT_TC_VALUES and v_pool.data_ptr() == k_pool.data_ptr() and pair is None
-            and dist_bias is None and not softcap and (keep == 0 or window <= 0) and not _NO_TCGEN05):
+            and dist_bias is None and not softcap and (keep == 0 or (keep > 0 and not window and not chunk))
+            and scale >= LATENT_TC_SCALE and pages * KV * page_size < 1 << 31 and not _NO_TCGEN05):
         # latent rows whose first elements are the values: the tcgen05 kernel that reads a tile once for both
         out = torch.empty_like(q)
         _call("attention_latent_tc", "ri_attention_latent_tc", q.data_ptr(), k_pool.data_ptr(), out.data_ptr(),
-              page_table.data_ptr(), seq_slot.data_ptr(), seq_start.data_ptr(), seq_len.data_ptr(), tokens, seqs, int(max_new), H,
-              KV, page_table.shape[1], page_size, pages, float(scale), _mask(window, chunk), _sink(sink, H), int(v_dims),
-              error_flag(q.device).data_ptr(), _stream())
+              page_table.data_ptr(), seq_slot.data_ptr(), seq_start.data_ptr(), seq_len.data_ptr(), tokens, seqs,
+              min(int(max_new), tokens), H, KV, page_table.shape[1], page_size, pages, float(scale), _mask(window, chunk),
+              _sink(sink, H), int(v_dims), error_flag(q.device).data_ptr(), _stream())
         return out
     out = torch.empty(q.shape, dtype=q.dtype if pair is None else torch.float32, device=q.device)
     _call("attention_prefill", "ri_attention_prefill", q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),

@@ -40,3 +40,25 @@ def test_plans_of_wide_tiles_are_for_bfloat16(launches, dtype, gather):
     ops.moe_grouped_linear(a, w, plan, 8, gather_div=gather)
     ops.moe_grouped_gated(a, w, plan, 8, "silu", gather_div=gather)
     assert [fn for _, fn, _ in launches] == (["ri_moe_gather"] if gather else []) + ["ri_moe_tc"] + (["ri_moe_gather"] if gather else []) + ["ri_moe_tc"]
+
+
+# latent rows (keys of 256 elements whose first ones are the values): what the tcgen05 kernel does not do stays with the mma.sync kernel
+TCGEN05, MMA = "ri_attention_latent_tc", "ri_attention_prefill"
+
+
+@pytest.mark.parametrize("form, want", [
+    ({}, TCGEN05), (dict(window=40), TCGEN05), (dict(chunk=64), TCGEN05), (dict(keep=3), TCGEN05), (dict(v_dims=190), TCGEN05),
+    (dict(max_new=64), TCGEN05),                                     # an upper bound of what a sequence brings
+    (dict(window=40, keep=3), MMA), (dict(chunk=64, keep=3), MMA), (dict(keep=-1), MMA),
+    (dict(scale=0.0), MMA), (dict(scale=-0.1), MMA), (dict(scale=1e-38), MMA), (dict(scale=float("nan")), MMA),
+    (dict(v_dims=0), MMA), (dict(v_dims=256), MMA), (dict(softcap=20.0), MMA)])
+def test_forms_of_latent_prompts(launches, monkeypatch, form, want):
+    monkeypatch.setattr(ops, "_NO_TCGEN05", False)
+    q, pool = torch.zeros((5, 2, 256), dtype=torch.bfloat16), torch.zeros((2, 1, 32, 256), dtype=torch.bfloat16)
+    one = torch.zeros(1, dtype=torch.int32)
+    args = {**dict(max_new=5, scale=0.1, window=0, v_dims=192), **form}
+    ops.attention_prefill(q, pool, pool, torch.zeros((1, 1), dtype=torch.int32), one, torch.zeros(2, dtype=torch.int32), one, **args)
+    (_, fn, sent), = launches
+    assert fn == want
+    if want == TCGEN05:
+        assert sent[7] == 5 and sent[9] == 5                        # tokens; the most of one sequence is no more than that

@@ -58,3 +58,26 @@ def test_latent_rows_against_plain_attention(lens, H, KV, v_dims, window, sink):
             # weights rounded to 8 bits (their sum is not), the result once more: 2^-8 of the weighted magnitudes, twice
             assert (diff <= 2.0 ** -7 * (p @ k[:, :v_dims].abs()) + 1e-5).all(), (b, h)
     assert torch.isfinite(got[..., :v_dims].float()).all()
+
+
+# forms that the kernel above does not take, and more tokens announced than there are
+@pytest.mark.parametrize("form", [dict(chunk=50, keep=3), dict(window=33, keep=40), dict(scale=0.0), dict(scale=-0.05), dict(max_new=500)])
+def test_other_forms_against_plain_attention(form):
+    from rust_inference_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(7)
+    n, H, v_dims = 170, 3, 192
+    row = (torch.randn((n, 256), generator=g, device=DEV) * 0.7).to(torch.bfloat16)
+    pool = torch.zeros((6, 1, 32, 256), dtype=torch.bfloat16, device=DEV)
+    pool.view(192, 256)[:n] = row
+    q = torch.randn((n, H, 256), generator=g, device=DEV).to(torch.bfloat16)
+    args = {**dict(max_new=n, scale=0.08, window=0, v_dims=v_dims), **form}
+    got = ops.attention_prefill(q, pool, pool, _i32([list(range(6))]), _i32([0]), _i32([0, n]), _i32([n]), **args)
+    assert int(ops.error_flag(DEV).item()) == 0
+    i, j = torch.arange(n, device=DEV)[:, None], torch.arange(n, device=DEV)[None, :]
+    inside = i - j < form["window"] if "window" in form else i // form["chunk"] == j // form["chunk"] if "chunk" in form else j >= 0
+    seen = (j <= i) & (inside | (j < form.get("keep", 0)))
+    k = row.double()
+    for h in range(H):
+        p = torch.softmax((q[:, h].double() @ k.t() * args["scale"]).masked_fill(~seen, -math.inf), dim=1)
+        diff = (got[:, h, :v_dims].double() - p @ k[:, :v_dims]).abs()
+        assert (diff <= 2.0 ** -7 * (p @ k[:, :v_dims].abs()) + 1e-5).all(), h      # the bound of the test above
