@@ -1163,7 +1163,7 @@ def attention_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
               float(lam), float(eps), float(gain), error_flag(q.device).data_ptr(), _stream(), defines={"RI_HEAD_DIM": Dh})
         return out
     if (Dh == LATENT_TC_ROW and 0 < v_dims <= LATENT_TC_VALUES and v_pool.data_ptr() == k_pool.data_ptr() and pair is None
-            and dist_bias is None and not softcap and (keep == 0 or (keep > 0 and not window and not chunk))
+            and dist_bias is None and not softcap and keep >= 0 and not (keep and window)
             and scale >= LATENT_TC_SCALE and pages * KV * page_size < 1 << 31 and not _NO_TCGEN05):
         # latent rows whose first elements are the values: the tcgen05 kernel that reads a tile once for both
         out = torch.empty_like(q)

@@ -49,7 +49,8 @@ TCGEN05, MMA = "ri_attention_latent_tc", "ri_attention_prefill"
 @pytest.mark.parametrize("form, want", [
     ({}, TCGEN05), (dict(window=40), TCGEN05), (dict(chunk=64), TCGEN05), (dict(keep=3), TCGEN05), (dict(v_dims=190), TCGEN05),
     (dict(max_new=64), TCGEN05),                                     # an upper bound of what a sequence brings
-    (dict(window=40, keep=3), MMA), (dict(chunk=64, keep=3), MMA), (dict(keep=-1), MMA),
+    (dict(chunk=64, keep=3), TCGEN05),                               # kept keys count beside a window only
+    (dict(window=40, keep=3), MMA), (dict(keep=-1), MMA),
     (dict(scale=0.0), MMA), (dict(scale=-0.1), MMA), (dict(scale=1e-38), MMA), (dict(scale=float("nan")), MMA),
     (dict(v_dims=0), MMA), (dict(v_dims=256), MMA), (dict(softcap=20.0), MMA)])
 def test_forms_of_latent_prompts(launches, monkeypatch, form, want):

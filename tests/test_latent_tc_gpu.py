@@ -60,8 +60,8 @@ def test_latent_rows_against_plain_attention(lens, H, KV, v_dims, window, sink):
     assert torch.isfinite(got[..., :v_dims].float()).all()
 
 
-# forms that the kernel above does not take, and more tokens announced than there are
-@pytest.mark.parametrize("form", [dict(chunk=50, keep=3), dict(window=33, keep=40), dict(scale=0.0), dict(scale=-0.05), dict(max_new=500)])
+# forms that the kernel above does not take; kept keys, which count beside a window only; more tokens announced than there are
+@pytest.mark.parametrize("form", [dict(window=33, keep=40), dict(chunk=50, keep=3), dict(scale=0.0), dict(scale=-0.05), dict(max_new=500)])
 def test_other_forms_against_plain_attention(form):
     from rust_inference_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(7)
@@ -75,7 +75,7 @@ def test_other_forms_against_plain_attention(form):
     assert int(ops.error_flag(DEV).item()) == 0
     i, j = torch.arange(n, device=DEV)[:, None], torch.arange(n, device=DEV)[None, :]
     inside = i - j < form["window"] if "window" in form else i // form["chunk"] == j // form["chunk"] if "chunk" in form else j >= 0
-    seen = (j <= i) & (inside | (j < form.get("keep", 0)))
+    seen = (j <= i) & (inside | (j < form.get("keep", 0) if "window" in form else inside))
     k = row.double()
     for h in range(H):
         p = torch.softmax((q[:, h].double() @ k.t() * args["scale"]).masked_fill(~seen, -math.inf), dim=1)
