@@ -104,7 +104,7 @@ __device__ __forceinline__ void gla_bar_arrive(int id, int threads) { asm volati
 // that have been computed, so that nothing of a group's trip to memory, its conversions and its outputs stands between the
 // tokens.  The copies of GLA_AHEAD groups are on their way together (cp.async into slots of the thread's own, widened from there:
 // with the next group's loads in registers every group of 16 tokens took a trip to memory, 2.5 us).  A group that the sequence
-// does not fill is padded with tokens of decay 1 and key 0, which leave the state as it is, bit for bit.
+// does not fill is padded with tokens of decay 1, key 0 and value 0, which leave the state as it is.
 //     S[d, j] = a[d] S[d, j] + k[d] v[j];  acc_j += S[d, j] q[d]
 // A thread's sum of a column runs over its channels in order (even and odd ones apart, then added); the LP lanes' sums go
 // down a tree (neighbours first), for four tokens and columns side by side: every step halves the number of sums a lane still
@@ -200,9 +200,10 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
         if (st_id < GROUP * VP) {
             const int jj = j0 + (st_id % VP) * 8;
             float* row = to + (st_id / VP) * ROW + 3 * DIMC + (st_id % VP) * 8;
+            const bool live = base + st_id / VP < t1;      // (a value of a token past the end may be infinite, and 0 times that a NaN)
             float x[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) x[i] = jj + i < vdim_in ? ld_f(&rv.v[i]) : jj + i < vdim ? 1.0f : 0.0f;      // the column of ones
+            for (int i = 0; i < 8; i++) x[i] = !live ? 0.0f : jj + i < vdim_in ? ld_f(&rv.v[i]) : jj + i < vdim ? 1.0f : 0.0f;      // the column of ones
 #pragma unroll
             for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(row + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
         }
