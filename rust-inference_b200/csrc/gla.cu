@@ -109,42 +109,39 @@ __device__ __forceinline__ void gla_bar_arrive(int id, int threads) { asm volati
 // A thread's sum of a column runs over its channels in order (even and odd ones apart, then added); the LP lanes' sums go
 // down a tree (neighbours first), for four tokens and columns side by side: every step halves the number of sums a lane still
 // holds, so that each lane ends with one.  Every token's sum thus has one order that depends on the head's size only: prompts,
-// pieces of prompts and single tokens give the same bits (GROUP = 1, for steps in which every sequence brings one token,
-// takes the decay from z itself and walks the same order).
+// pieces of prompts and single tokens (`gla_single`, below) give the same bits.
 // 2,048 tokens of 32 heads of 64 x 128, with the decays' kernel: 608 -> 203 us (99 ns a token); three sequences of 2,302 tokens in
-// all 645 -> 207 us; 16 heads of 128 x 129 with one decay 445 -> 278 us; 64 single tokens of 32 heads 73 -> 69 us.  (Before: one column and four channels a thread, the
+// all 645 -> 207 us; 16 heads of 128 x 129 with one decay 445 -> 278 us.  (Before: one column and four channels a thread, the
 // tokens staged and the decays taken by the same warps of every block.)
 #define GLA_CT 128              // computing threads
 #define GLA_ST 128              // staging threads
 #define GLA_RING 3
 #define GLA_AHEAD 3
 template <typename T, int DIMC, int GROUP, bool VEC>
-__global__ void __launch_bounds__(GROUP == 1 ? GLA_CT : GLA_CT + GLA_ST)
+__global__ void __launch_bounds__(GLA_CT + GLA_ST)
 gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, const T* z, const float* __restrict__ bias,
                 float inv_tau, float qscale, const float* decay, float* state, float* __restrict__ o,
                 const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int H, int dim, int vdim_in, const float* gates,
                 int gate_pitch, int ones) {
-    constexpr bool SINGLE = GROUP == 1;
     constexpr int LP = DIMC / 4;                                             // lanes that share four columns
     constexpr int WCOLS = 4 * (32 / LP), BCOLS = 4 * (GLA_CT / LP);          // columns per warp and per block
     constexpr int KP = DIMC / 8, VP = BCOLS / 8;                             // staged pieces of eight per token
     constexpr int PER = (GROUP * KP + GLA_ST - 1) / GLA_ST;                  // ... and per thread
-    static_assert(GROUP * VP <= GLA_ST && (SINGLE || GROUP % 4 == 0), "a piece of values per thread; tokens in fours");
+    static_assert(GROUP * VP <= GLA_ST && GROUP % 4 == 0, "a piece of values per thread; tokens in fours");
     constexpr int ROW = 3 * DIMC + BCOLS;                                    // a staged token: decay, key, query, values
     constexpr int ALL = GLA_CT + GLA_ST;
     extern __shared__ __align__(16) float gla_dyn[];                         // [ring][GROUP][ROW], outputs [ring][GROUP][BCOLS]
     const int vdim = vdim_in + ones;                                         // columns of the state and of the output
     const int b = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * BCOLS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (SINGLE) pdl_trigger();
     const int t0 = seq_start[b], t1 = seq_start[b + 1];
     const int slot = seq_slot[b];
     pdl_wait();
     if (t0 >= t1) return;                     // (a sequence without tokens keeps its state; the whole block leaves)
 
-    const int st_id = SINGLE ? threadIdx.x : threadIdx.x - GLA_CT;           // among the staging threads
-    GlaPiece<T, VEC> rk[PER], rq[PER], rz[SINGLE ? PER : 1], rv;
-    GlaPiece<float, VEC> ra[SINGLE ? 1 : PER];
+    const int st_id = threadIdx.x - GLA_CT;                                  // among the staging threads
+    GlaPiece<T, VEC> rk[PER], rq[PER], rv;
+    GlaPiece<float, VEC> ra[PER];
     float ga[PER], gb[PER];
     // Loads are never under a condition (a load that is gets waited for where it stands): past the group, the sequence or the
     // head something that exists is read and left out by `store`.
@@ -159,8 +156,6 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
             if (gates) {
                 ga[e] = gates[((size_t)t * H + h) * gate_pitch];
                 gb[e] = gates[((size_t)t * H + h) * gate_pitch + 1];
-            } else if (SINGLE) {
-                rz[e].load(z + ((size_t)t * H + h) * dim + d, dim - d);
             } else {
                 ra[e].load(decay + ((size_t)t * H + h) * dim + d, dim - d);
             }
@@ -184,7 +179,6 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
                     k[i] = !(live && own) ? 0.0f : gates ? ld_f(&rk[e].v[i]) * gb[e] : ld_f(&rk[e].v[i]);
                     q[i] = !(live && own) ? 0.0f : ld_f(&rq[e].v[i]) * qscale;
                     if (gates) a[i] = ga[e];
-                    else if (SINGLE) a[i] = gla_decay(ld_f(&rz[e].v[i]) + (own ? bias[h * dim + d + i] : 0.0f), inv_tau);
                     else a[i] = ra[e].v[i];
                     a[i] = !own ? 0.0f : live ? a[i] : 1.0f;
                 }
@@ -209,7 +203,7 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
         }
     };
     float* outs = gla_dyn + GLA_RING * GROUP * ROW;
-    if (!SINGLE && threadIdx.x >= GLA_CT) {
+    if (threadIdx.x >= GLA_CT) {
         // ---- the staging warps.  Barriers 1 + buf: the buffer is full; 1 + GLA_RING + buf: it was read, its outputs are there ----------
         // VEC: this thread's pieces of the groups on their way, [GLA_AHEAD][16 bytes of a piece][staging thread]
         constexpr int PT = sizeof(T) / 2;                                    // 16-byte pieces of eight elements
@@ -254,7 +248,7 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
                 if (gates) {
                     ga[e] = __uint_as_float(lo.x);
                     gb[e] = __uint_as_float(lo.y);
-                } else if (!SINGLE) {
+                } else {
                     reinterpret_cast<uint4*>(ra[e].v)[0] = lo;
                     reinterpret_cast<uint4*>(ra[e].v)[1] = piece16(slot_, e * EACH + 2 * PT + 1);
                 }
@@ -305,17 +299,6 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
     float* st = state + ((size_t)slot * H + h) * dim * vdim;
     f32x2 S[4][2];                            // [column][pair of channels]
     const bool whole = vdim % 4 == 0 && ((uintptr_t)state & 15) == 0;        // the state's rows start on 16 bytes, columns come in fours
-    // A single token is bound by its state's trip to memory: rows that do not start on 16 bytes go through shared memory, whole
-    // rows of the block's columns at a time.
-    float* tile = gla_dyn + ROW;              // [DIMC][BCOLS + 1]
-    if (SINGLE && !whole) {
-#pragma unroll 16
-        for (int i = threadIdx.x; i < DIMC * BCOLS; i += GLA_CT) {
-            const int d = i / BCOLS, c = i % BCOLS;
-            tile[d * (BCOLS + 1) + c] = d < dim && j0 + c < vdim ? st[(size_t)d * vdim + j0 + c] : 0.0f;
-        }
-        __syncthreads();
-    }
     float4 x4[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -324,9 +307,6 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
         if (d0 + i < dim) {
             if (whole) {
                 if (j < vdim) x4[i] = *reinterpret_cast<const float4*>(row);
-            } else if (SINGLE) {
-                const float* sr = tile + (d0 + i) * (BCOLS + 1) + col;
-                x4[i] = make_float4(sr[0], sr[1], sr[2], sr[3]);
             } else {
                 if (j < vdim) x4[i].x = row[0];
                 if (j + 1 < vdim) x4[i].y = row[1];
@@ -367,55 +347,38 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
             out[c] = lo + hi;
         }
     };
-    if (SINGLE) {
-        fetch(t0);
-        store(0, t0);
-        __syncthreads();
-        Token x;
-        load(x, gla_dyn);
-        float v[4];
-        token(x, v);
+    // the token of four and the column of four whose output this lane ends with (lanes 16 .. of 32 hold copies)
+    const int my_t = 2 * (part & 1) + ((part >> 1) & 1), my_c = 2 * ((part >> 2) & 1) + ((part >> 3) & 1);
+    int n = 0;
+    for (int base = t0; base < t1; base += GROUP, n++) {
+        const int buf = n % GLA_RING;
+        gla_bar_sync(1 + buf, ALL);
+        const float* rows = gla_dyn + buf * GROUP * ROW;
+        Token x[2];                       // the token at hand and the next one, on its way from shared memory
+        load(x[0], rows);
 #pragma unroll
-        for (int m = 1; m < LP; m <<= 1)
+        for (int g = 0; g < GROUP; g += 4) {
+            float v[16];
 #pragma unroll
-            for (int c = 0; c < 4; c++) v[c] += __shfl_xor_sync(0xffffffffu, v[c], m);
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (part == c && j + c < vdim) o[((size_t)t0 * H + h) * vdim + j + c] = v[c];
-    } else {
-        // the token of four and the column of four whose output this lane ends with (lanes 16 .. of 32 hold copies)
-        const int my_t = 2 * (part & 1) + ((part >> 1) & 1), my_c = 2 * ((part >> 2) & 1) + ((part >> 3) & 1);
-        int n = 0;
-        for (int base = t0; base < t1; base += GROUP, n++) {
-            const int buf = n % GLA_RING;
-            gla_bar_sync(1 + buf, ALL);
-            const float* rows = gla_dyn + buf * GROUP * ROW;
-            Token x[2];                       // the token at hand and the next one, on its way from shared memory
-            load(x[0], rows);
-#pragma unroll
-            for (int g = 0; g < GROUP; g += 4) {
-                float v[16];
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    if (g + t + 1 < GROUP) load(x[(t + 1) & 1], rows + (g + t + 1) * ROW);
-                    token(x[t & 1], v + 4 * t);
-                }
-#pragma unroll
-                for (int m = 1, k = 8; m < 16; m <<= 1, k >>= 1) {
-                    const bool upper = (lane & m) != 0;
-#pragma unroll
-                    for (int i = 0; i < k; i++) {
-                        const float give = upper ? v[i] : v[i + k], keep = upper ? v[i + k] : v[i];
-                        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
-                    }
-                }
-                if (LP == 32) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
-                if (part < 16) outs[(buf * GROUP + g + my_t) * BCOLS + col + my_c] = v[0];
+            for (int t = 0; t < 4; t++) {
+                if (g + t + 1 < GROUP) load(x[(t + 1) & 1], rows + (g + t + 1) * ROW);
+                token(x[t & 1], v + 4 * t);
             }
-            gla_bar_arrive(1 + GLA_RING + buf, ALL);
+#pragma unroll
+            for (int m = 1, k = 8; m < 16; m <<= 1, k >>= 1) {
+                const bool upper = (lane & m) != 0;
+#pragma unroll
+                for (int i = 0; i < k; i++) {
+                    const float give = upper ? v[i] : v[i + k], keep = upper ? v[i + k] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+                }
+            }
+            if (LP == 32) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+            if (part < 16) outs[(buf * GROUP + g + my_t) * BCOLS + col + my_c] = v[0];
         }
-        pdl_trigger();                        // the next kernel may come in once the walk is over
+        gla_bar_arrive(1 + GLA_RING + buf, ALL);
     }
+    pdl_trigger();                            // the next kernel may come in once the walk is over
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         float x[4], y[4];
@@ -426,9 +389,6 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
         if (d0 + i < dim) {
             if (whole) {
                 if (j < vdim) *reinterpret_cast<float4*>(row) = w;
-            } else if (SINGLE) {
-                float* sr = tile + (d0 + i) * (BCOLS + 1) + col;
-                sr[0] = w.x; sr[1] = w.y; sr[2] = w.z; sr[3] = w.w;
             } else {
                 if (j < vdim) row[0] = w.x;
                 if (j + 1 < vdim) row[1] = w.y;
@@ -437,13 +397,89 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
             }
         }
     }
-    if (SINGLE && !whole) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < DIMC * BCOLS; i += GLA_CT) {
-            const int d = i / BCOLS, c = i % BCOLS;
-            if (d < dim && j0 + c < vdim) st[(size_t)d * vdim + j0 + c] = tile[d * (BCOLS + 1) + c];
-        }
+}
+
+// The same for steps in which every sequence brings one token.  What bounds it: the state's trip to memory and back, and for
+// few sequences the chain of trips in front of it, so a token's own loads start first and the decays' exponentials run under
+// the state's loads.  A warp has eight key channels of 32 neighbouring columns (whole 128-byte lines of the state's rows,
+// whatever the columns' number), a lane one column; lanes 0..7 take the decays of its channels, 8..15 its keys, 16..23 its
+// queries, one each.  A block has all channels of its columns; its warps' sums are added down the walk's tree: the same bits.
+// A step of single tokens of 1 / 8 / 24 / 64 sequences, 32 heads of 64 x 128: 2.4 / 5.0 / 11.8 / 29 us, where 16 columns a block
+// with four channels a thread took 2.4 / 7.2 / 18 / 46; 32 heads of 128 x 128 2.9 / 8.8 / 23 / 79 (2.9 / 10.3 / 27 / 87).  With
+// four channels a warp, twice the threads: 2.4 / 6.7 / 17 / 42 and 2.9 / 16 / 47 / 151.
+template <typename T, int DIMC>
+__global__ void __launch_bounds__(4 * DIMC)
+gla_single_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, const T* z, const float* __restrict__ bias, float inv_tau,
+                  float qscale, float* state, float* __restrict__ o, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
+                  int H, int dim, int vdim_in, const float* gates, int gate_pitch, int ones) {
+    constexpr int WARPS = DIMC / 8;
+    __shared__ __align__(16) float s_x[WARPS][3][8];                         // decay, key, query of the warp's channels
+    __shared__ float s_sum[WARPS][32];
+    pdl_trigger();
+    const int vdim = vdim_in + ones;
+    const int b = blockIdx.z, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane, d0 = 8 * warp;
+    const int what = lane >> 3, d = d0 + (lane & 7);
+    const bool own = what < 3 && d < dim;
+    const int t0 = seq_start[b], t1 = seq_start[b + 1];
+    float* st = state + ((size_t)seq_slot[b] * H + h) * dim * vdim + (size_t)d0 * vdim + j;
+    const float add = own && what == 0 && !gates ? bias[h * dim + d] : 0.0f;
+    pdl_wait();
+    if (t0 >= t1) return;                     // (a sequence without tokens keeps its state; the whole block leaves)
+    const T* row = proj + (size_t)t0 * ld;
+    const T* src = (what == 0 && !gates ? z + (size_t)t0 * H * dim : row + (what == 2 ? q_col : k_col)) + h * dim + d;
+    const T raw = own ? *src : T(0.0f);
+    const float a = gates ? gates[((size_t)t0 * H + h) * gate_pitch] : 0.0f;
+    const float kb = gates ? gates[((size_t)t0 * H + h) * gate_pitch + 1] : 1.0f;
+    const float v = j < vdim_in ? ld_f(row + v_col + h * vdim_in + j) : j < vdim ? 1.0f : 0.0f;        // the column of ones
+    float S[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) S[i] = j < vdim && d0 + i < dim ? st[(size_t)i * vdim] : 0.0f;
+    if (what < 3) {
+        float x = ld_f(&raw);
+        if (what == 0) x = gates ? a : gla_decay(x + add, inv_tau);
+        else if (what == 1) x = gates ? x * kb : x;
+        else x *= qscale;
+        s_x[warp][what][lane & 7] = own ? x : 0.0f;
     }
+    __syncwarp();
+    float part[2];
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+        const float4 g = *reinterpret_cast<const float4*>(&s_x[warp][0][4 * p]), k = *reinterpret_cast<const float4*>(&s_x[warp][1][4 * p]),
+                     q = *reinterpret_cast<const float4*>(&s_x[warp][2][4 * p]);
+        float* x = S + 4 * p;
+        x[0] = fmaf(g.x, x[0], __fmul_rn(k.x, v));
+        x[1] = fmaf(g.y, x[1], __fmul_rn(k.y, v));
+        x[2] = fmaf(g.z, x[2], __fmul_rn(k.z, v));
+        x[3] = fmaf(g.w, x[3], __fmul_rn(k.w, v));
+        part[p] = fmaf(x[2], q.z, __fmul_rn(x[0], q.x)) + fmaf(x[3], q.w, __fmul_rn(x[1], q.y));
+    }
+    s_sum[warp][lane] = part[0] + part[1];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        if (j < vdim && d0 + i < dim) st[(size_t)i * vdim] = S[i];
+    __syncthreads();
+    if (warp == 0 && j < vdim) {
+        float x[WARPS];
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) x[w] = s_sum[w][lane];
+#pragma unroll
+        for (int m = 1; m < WARPS; m <<= 1)
+#pragma unroll
+            for (int w = 0; w < WARPS; w += 2 * m) x[w] += x[w + m];
+        o[((size_t)t0 * H + h) * vdim + j] = x[0];
+    }
+}
+
+template <typename T, int DIMC>
+static int gla_single_go(const void* proj, long long ld, int q_col, int k_col, int v_col, const void* z, const float* bias, float tau,
+                         float qscale, float* state, float* o, const int* seq_slot, const int* seq_start, int seqs, int H, int dim,
+                         int vdim_in, const float* gates, int gate_pitch, int ones, cudaStream_t stream) {
+    ri_launch_pdl(gla_single_kernel<T, DIMC>, dim3((vdim_in + ones + 31) / 32, H, seqs), dim3(4 * DIMC), 0, stream, (const T*)proj, ld, q_col,
+                  k_col, v_col, (const T*)z, bias, 1.0f / tau, qscale, state, o, seq_slot, seq_start, H, dim, vdim_in, gates, gate_pitch, ones);
+    RI_CHECK_LAUNCH("gla_recurrent");
+    return 0;
 }
 
 template <typename T, int DIMC, int GROUP, bool VEC>
@@ -451,8 +487,8 @@ static int gla_walk_go(const void* proj, long long ld, int q_col, int k_col, int
                        float qscale, const float* decay, float* state, float* o, const int* seq_slot, const int* seq_start, int seqs,
                        int H, int dim, int vdim_in, const float* gates, int gate_pitch, int ones, cudaStream_t stream) {
     constexpr int BCOLS = GLA_CT * 16 / DIMC, PER = (GROUP * (DIMC / 8) + GLA_ST - 1) / GLA_ST, PT = sizeof(T) / 2;
-    constexpr size_t RAW = GROUP > 1 && VEC ? (size_t)GLA_AHEAD * (PER * (2 * PT + 2) + PT) * GLA_ST * 16 : 0;      // the slots of pieces
-    constexpr size_t sm = (GROUP == 1 ? (size_t)(3 * DIMC + BCOLS + DIMC * (BCOLS + 1)) : (size_t)GLA_RING * GROUP * (3 * DIMC + 2 * BCOLS)) * sizeof(float) + RAW;
+    constexpr size_t RAW = VEC ? (size_t)GLA_AHEAD * (PER * (2 * PT + 2) + PT) * GLA_ST * 16 : 0;      // the slots of pieces
+    constexpr size_t sm = (size_t)GLA_RING * GROUP * (3 * DIMC + 2 * BCOLS) * sizeof(float) + RAW;
     const dim3 grid((vdim_in + ones + BCOLS - 1) / BCOLS, H, seqs);
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(gla_walk_kernel<T, DIMC, GROUP, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -460,12 +496,8 @@ static int gla_walk_go(const void* proj, long long ld, int q_col, int k_col, int
     }
     // A prompt's kernel is launched the ordinary way, not as a dependent launch: its long-lived blocks must spread over the
     // SMs, and blocks that come in while the kernel before still holds most SMs pile up on the first that get free.
-    if (GROUP == 1)
-        ri_launch_pdl(gla_walk_kernel<T, DIMC, GROUP, VEC>, grid, dim3(GLA_CT), sm, stream, (const T*)proj, ld, q_col, k_col, v_col,
-                      (const T*)z, bias, 1.0f / tau, qscale, decay, state, o, seq_slot, seq_start, H, dim, vdim_in, gates, gate_pitch, ones);
-    else
-        gla_walk_kernel<T, DIMC, GROUP, VEC><<<grid, dim3(GLA_CT + GLA_ST), sm, stream>>>((const T*)proj, ld, q_col, k_col, v_col, (const T*)z,
-                      bias, 1.0f / tau, qscale, decay, state, o, seq_slot, seq_start, H, dim, vdim_in, gates, gate_pitch, ones);
+    gla_walk_kernel<T, DIMC, GROUP, VEC><<<grid, dim3(GLA_CT + GLA_ST), sm, stream>>>((const T*)proj, ld, q_col, k_col, v_col, (const T*)z,
+                  bias, 1.0f / tau, qscale, decay, state, o, seq_slot, seq_start, H, dim, vdim_in, gates, gate_pitch, ones);
     RI_CHECK_LAUNCH("gla_recurrent");
     return 0;
 }
@@ -547,8 +579,9 @@ static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col
                                                 seq_start, seqs, H, dim, vdim_in, gates, gate_pitch, ones, stream)
 #define GLA_GO2(T, DIMC)                                                                                                       \
         do {                                                                                                                   \
-            if (single) { if (vec) GLA_GO3(T, DIMC, 1, true); else GLA_GO3(T, DIMC, 1, false); }                               \
-            else { if (vec) GLA_GO3(T, DIMC, 16, true); else GLA_GO3(T, DIMC, 16, false); }                                    \
+            if (single) return gla_single_go<T, DIMC>(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, state, o, seq_slot,  \
+                                                      seq_start, seqs, H, dim, vdim_in, gates, gate_pitch, ones, stream);      \
+            if (vec) GLA_GO3(T, DIMC, 16, true); else GLA_GO3(T, DIMC, 16, false);                                             \
         } while (0)
 #define GLA_GO1(T) do { if (dim <= 64) GLA_GO2(T, 64); else GLA_GO2(T, 128); } while (0)
         if (dtype == RI_DTYPE_F32) GLA_GO1(float);

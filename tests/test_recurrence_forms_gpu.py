@@ -63,6 +63,27 @@ class Gla:
             at = to
         return [torch.cat(o) for o in outs], state
 
+    def exact(self):
+        """Outputs and states in float64 (slots as above)."""
+        outs, state = [], self.state().double()
+        q_col, k_col, v_col = self.columns()
+        for b, n in enumerate(self.lens):
+            p = self.proj[b].double()
+            q, k = (p[:, c:c + self.H * self.dim].view(n, self.H, self.dim) for c in (q_col, k_col))
+            v = p[:, v_col:v_col + self.H * self.vdim].view(n, self.H, self.vdim)
+            if self.ones:
+                v = torch.cat([v, torch.ones_like(v[..., :1])], dim=-1)
+                a, k = self.gates[b][:, :, :1].double().expand_as(k), k * self.gates[b][:, :, 1:2].double()
+            else:
+                a = torch.sigmoid(self.z[b].double() + self.bias.double()).pow(1 / 16.0).view(n, self.H, self.dim)
+            S, o = torch.zeros_like(state[0]), []
+            for t in range(n):
+                S = a[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+                o.append((S * (q[t] * self.dim ** -0.5)[:, :, None]).sum(1))
+            outs.append(torch.stack(o))
+            state[int(self.slots[b])] = S
+        return outs, state
+
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("ones", [False, True])
@@ -75,3 +96,19 @@ def test_an_infinite_last_value_is_infinite_in_every_cutting(dim, vdim, ones, dt
     singly, state1 = gla.walk(list(range(1, 19)))
     assert all(_same(a, b) for a, b in zip(outs, singly)) and _same(state, state1)
     assert torch.isinf(state).any() and not torch.isnan(state).any()
+
+
+# 16-byte copies (everything a multiple of eight) and element by element; 3, 4, 13 groups of 16 tokens; a last column on its own
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("ones", [False, True])
+@pytest.mark.parametrize("dim, vdim, pad", [(64, 128, 0), (128, 64, 8), (48, 32, 0), (128, 128, 0), (96, 33, 0), (64, 64, 3), (20, 8, 0)])
+def test_gla_prompts_pieces_and_single_tokens(dim, vdim, pad, ones, dtype):
+    gla = Gla([47, 200, 1, 48, 65], 2, dim, vdim, dtype, ones, pad)
+    outs, state = gla.walk([])
+    want, want_state = gla.exact()
+    for got, exact in zip(outs + [state], want + [want_state]):
+        # float32 sums of up to 200 tokens and 128 channels, decays from float32 exponentials: some 1e-6 of the largest
+        assert (got.double() - exact).abs().max() <= 2e-5 * exact.abs().max()
+    for cuts in ([3, 19, 20, 51, 52, 130], list(range(1, 66)) + [80]):
+        pieces, state1 = gla.walk(cuts)
+        assert all(torch.equal(a, b) for a, b in zip(pieces, outs)) and torch.equal(state, state1)
