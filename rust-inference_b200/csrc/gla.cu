@@ -8,7 +8,7 @@
 // `gla_recurrent`: a block owns one (sequence, head, tile of value columns j) and walks the sequence's new
 // tokens in order with its part of the state in registers (heads of up to 128 key channels) or in shared memory, loaded
 // from / stored to the sequence's slot of the state tensor at the ends.  The decay is computed as
-// exp(log_sigmoid(z) / tau) with float32 functions (for prompts by `gla_decay`, once for all blocks of a head); q, k, v and z
+// exp(log_sigmoid(z) / tau) with float32 functions (for steps of many tokens by `gla_decay`, once for all blocks of a head); q, k, v and z
 // come from bfloat16 or float32 projections and are widened once.  A token's result depends on the tokens before it only through the state, so prompts,
 // pieces of prompts and single tokens give the same bits.
 //
@@ -110,6 +110,7 @@ __device__ __forceinline__ void gla_bar_arrive(int id, int threads) { asm volati
 // down a tree (neighbours first), for four tokens and columns side by side: every step halves the number of sums a lane still
 // holds, so that each lane ends with one.  Every token's sum thus has one order that depends on the head's size only: prompts,
 // pieces of prompts and single tokens (`gla_single`, below) give the same bits.
+// Steps of few tokens come without decays (`decay` null): the staging warps then take them from z, every block of a head its own.
 // 2,048 tokens of 32 heads of 64 x 128, with the decays' kernel: 608 -> 203 us (99 ns a token); three sequences of 2,302 tokens in
 // all 645 -> 207 us; 16 heads of 128 x 129 with one decay 445 -> 278 us.  (Before: one column and four channels a thread, the
 // tokens staged and the decays taken by the same warps of every block.)
@@ -140,9 +141,16 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
     if (t0 >= t1) return;                     // (a sequence without tokens keeps its state; the whole block leaves)
 
     const int st_id = threadIdx.x - GLA_CT;                                  // among the staging threads
-    GlaPiece<T, VEC> rk[PER], rq[PER], rv;
+    const bool own_decays = !decay && !gates;
+    GlaPiece<T, VEC> rk[PER], rq[PER], rz[PER], rv;
     GlaPiece<float, VEC> ra[PER];
-    float ga[PER], gb[PER];
+    float ga[PER], gb[PER], bs[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {             // (a thread's pieces are of the same channels in every token)
+        const int d = ((int)threadIdx.x % KP) * 8 + i;
+        bs[i] = own_decays && d < dim ? bias[h * dim + d] : 0.0f;
+    }
+    static_assert(GLA_ST % KP == 0 && GLA_CT % KP == 0, "a staging thread's channels");
     // Loads are never under a condition (a load that is gets waited for where it stands): past the group, the sequence or the
     // head something that exists is read and left out by `store`.
     auto fetch = [&](int base) {              // the raw values of tokens base .. base + GROUP - 1 into registers
@@ -156,12 +164,22 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
             if (gates) {
                 ga[e] = gates[((size_t)t * H + h) * gate_pitch];
                 gb[e] = gates[((size_t)t * H + h) * gate_pitch + 1];
+            } else if (own_decays) {
+                rz[e].load(z + ((size_t)t * H + h) * dim + d, dim - d);
             } else {
                 ra[e].load(decay + ((size_t)t * H + h) * dim + d, dim - d);
             }
         }
         const int t = min(base + st_id / VP, t1 - 1), jj = min(j0 + (st_id % VP) * 8, (vdim_in - 1) & ~7);
         rv.load(proj + (size_t)t * ld + v_col + h * vdim_in + jj, vdim_in - jj);
+    };
+    auto decays = [&](int base) {             // the decays from z, of the tokens that there are
+        if (!own_decays) return;
+#pragma unroll
+        for (int e = 0; e < PER; e++)
+            if (base + (st_id + e * GLA_ST) / KP < t1)
+#pragma unroll
+                for (int i = 0; i < 8; i++) ra[e].v[i] = gla_decay(ld_f(&rz[e].v[i]) + bs[i], inv_tau);
     };
     auto store = [&](int buf, int base) {     // ... and from there into a buffer
         float* to = gla_dyn + buf * GROUP * ROW;
@@ -221,7 +239,11 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
                     gla_copy<16>(&piece16(slot_, e * EACH + i), reinterpret_cast<const uint4*>(row + k_col) + i);
                     gla_copy<16>(&piece16(slot_, e * EACH + PT + i), reinterpret_cast<const uint4*>(row + q_col) + i);
                 }
-                if (!gates) {
+                if (own_decays) {
+                    const T* zz = z + ((size_t)t * H + h) * dim + d;
+#pragma unroll
+                    for (int i = 0; i < PT; i++) gla_copy<16>(&piece16(slot_, e * EACH + 2 * PT + i), reinterpret_cast<const uint4*>(zz) + i);
+                } else if (!gates) {
                     const float* dec = decay + ((size_t)t * H + h) * dim + d;
                     gla_copy<16>(&piece16(slot_, e * EACH + 2 * PT), dec);
                     gla_copy<16>(&piece16(slot_, e * EACH + 2 * PT + 1), dec + 4);
@@ -248,6 +270,9 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
                 if (gates) {
                     ga[e] = __uint_as_float(lo.x);
                     gb[e] = __uint_as_float(lo.y);
+                } else if (own_decays) {
+#pragma unroll
+                    for (int i = 0; i < PT; i++) reinterpret_cast<uint4*>(rz[e].v)[i] = piece16(slot_, e * EACH + 2 * PT + i);
                 } else {
                     reinterpret_cast<uint4*>(ra[e].v)[0] = lo;
                     reinterpret_cast<uint4*>(ra[e].v)[1] = piece16(slot_, e * EACH + 2 * PT + 1);
@@ -279,6 +304,7 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
                 if (base + GLA_AHEAD * GROUP < t1) issue(n % GLA_AHEAD, base + GLA_AHEAD * GROUP);
                 asm volatile("cp.async.commit_group;\n" ::: "memory");
             }
+            decays(base);
             if (n >= GLA_RING) {
                 gla_bar_sync(1 + GLA_RING + buf, ALL);
                 write_out(buf, base - GLA_RING * GROUP);
@@ -358,6 +384,7 @@ gla_walk_kernel(const T* proj, long long ld, int q_col, int k_col, int v_col, co
         load(x[0], rows);
 #pragma unroll
         for (int g = 0; g < GROUP; g += 4) {
+            if (g > 0 && base + g >= t1) break;
             float v[16];
 #pragma unroll
             for (int t = 0; t < 4; t++) {
@@ -558,8 +585,7 @@ static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col
     RI_REQUIRE(seqs <= 65535 && H <= 65535, "gla_recurrent: %d sequences, %d heads: too many for one launch", seqs, H);
     RI_REQUIRE(dtype == RI_DTYPE_F32 || dtype == RI_DTYPE_BF16, "gla_recurrent: unknown dtype %d", dtype);
     if (dim <= 128) {
-        if (!gates && !single) {
-            RI_REQUIRE(decay || tokens == 0, "gla_recurrent: a prompt needs room for its decays");
+        if (decay) {
             const int HD = H * dim;
             for (int t = 0; t < tokens; t += 65535) {        // (a grid's second dimension)
                 const dim3 g((HD + 511) / 512, tokens - t < 65535 ? tokens - t : 65535);
@@ -574,18 +600,39 @@ static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col
         }
         const bool vec = dim % 8 == 0 && vdim_in % 8 == 0 && ld % 8 == 0 && q_col % 8 == 0 && k_col % 8 == 0 && v_col % 8 == 0 &&
                          (((uintptr_t)proj | (uintptr_t)z | (uintptr_t)decay) & 15) == 0;
+        // Tokens staged at a time: 16, or eight for heads of more than 64 channels where there are more blocks than SMs (a block
+        // with 16 has an SM for itself, 135 KB; two fit with eight) or where sequences bring few tokens.  16 / 8 at a time, bfloat16: 32
+        // heads of 128 x 128 2,048 tokens 402 / 361 us, 64 sequences of 4 tokens 344 / 186; but 16 heads of 128 x 64 (64 blocks)
+        // 2,048 tokens 201 / 239, and for heads of 64 channels 172 / 255 (32 of 64 x 128).
+        static int sms = 0;
+        if (!sms) {
+            int dev = 0, n = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+            sms = n > 0 ? n : 148;
+        }
+        const bool eight = dim > 64 && ((long long)((vdim + 15) / 16) * H * seqs > sms || tokens <= 16 * (long long)seqs);
 #define GLA_GO3(T, DIMC, GROUP, VEC)                                                                                           \
         return gla_walk_go<T, DIMC, GROUP, VEC>(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, decay, state, o, seq_slot, \
                                                 seq_start, seqs, H, dim, vdim_in, gates, gate_pitch, ones, stream)
-#define GLA_GO2(T, DIMC)                                                                                                       \
+#define GLA_GO2(T, DIMC, GROUP)                                                                                                \
         do {                                                                                                                   \
-            if (single) return gla_single_go<T, DIMC>(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, state, o, seq_slot,  \
-                                                      seq_start, seqs, H, dim, vdim_in, gates, gate_pitch, ones, stream);      \
-            if (vec) GLA_GO3(T, DIMC, 16, true); else GLA_GO3(T, DIMC, 16, false);                                             \
+            if (vec) GLA_GO3(T, DIMC, GROUP, true);                                                                            \
+            else GLA_GO3(T, DIMC, GROUP, false);                                                                               \
         } while (0)
-#define GLA_GO1(T) do { if (dim <= 64) GLA_GO2(T, 64); else GLA_GO2(T, 128); } while (0)
+#define GLA_GO0(T, DIMC)                                                                                                       \
+        return gla_single_go<T, DIMC>(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, state, o, seq_slot, seq_start, seqs, H, \
+                                      dim, vdim_in, gates, gate_pitch, ones, stream)
+#define GLA_GO1(T)                                                                                                             \
+        do {                                                                                                                   \
+            if (single) { if (dim <= 64) GLA_GO0(T, 64); else GLA_GO0(T, 128); }                                               \
+            else if (dim <= 64) GLA_GO2(T, 64, 16);                                                                            \
+            else if (eight) GLA_GO2(T, 128, 8);                                                                                \
+            else GLA_GO2(T, 128, 16);                                                                                          \
+        } while (0)
         if (dtype == RI_DTYPE_F32) GLA_GO1(float);
         else GLA_GO1(__nv_bfloat16);
+#undef GLA_GO0
 #undef GLA_GO1
 #undef GLA_GO2
 #undef GLA_GO3
@@ -609,7 +656,8 @@ static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col
     return 0;
 }
 
-// decay: float32 scratch [tokens, H, dim] that a call for prompts (not `single`) with up to 128 key channels fills
+// decay: float32 scratch [tokens, H, dim] that a call for prompts (not `single`) with up to 128 key channels fills, or null: then
+// every block takes its tokens' decays itself
 extern "C" int ri_gla_recurrent(const void* proj, long long ld, int q_col, int k_col, int v_col, const void* z,
                                 const float* bias, float tau, float qscale, float* decay, float* state, float* o, const int* seq_slot,
                                 const int* seq_start, int tokens, int seqs, int H, int dim, int vdim, int single, int dtype,
@@ -622,10 +670,10 @@ extern "C" int ri_gla_recurrent(const void* proj, long long ld, int q_col, int k
 // state [slots, H, dim, vdim + 1] and the output [tokens, H, vdim + 1] carry the column of ones.
 extern "C" int ri_gla_recurrent_scalar(const void* proj, long long ld, int q_col, int k_col, int v_col, const float* gates,
                                        int gate_pitch, int ones, float qscale, float* state, float* o, const int* seq_slot,
-                                       const int* seq_start, int seqs, int H, int dim, int vdim, int single, int dtype,
+                                       const int* seq_start, int tokens, int seqs, int H, int dim, int vdim, int single, int dtype,
                                        cudaStream_t stream) {
     RI_REQUIRE(gates != nullptr && (ones == 0 || ones == 1), "gla_recurrent_scalar: gates are needed");
-    return gla_recurrent_go(proj, ld, q_col, k_col, v_col, nullptr, nullptr, 1.0f, qscale, nullptr, state, o, seq_slot, seq_start, 0,
+    return gla_recurrent_go(proj, ld, q_col, k_col, v_col, nullptr, nullptr, 1.0f, qscale, nullptr, state, o, seq_slot, seq_start, tokens,
                             seqs, H, dim, vdim, single, dtype, gates, gate_pitch, ones, stream);
 }
 

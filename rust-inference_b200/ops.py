@@ -32,7 +32,7 @@ _SIGNATURES = {
     ("norm_gains", "ri_norm_gains_post"): [_P] * 6 + [_P, _I, _F] + [_P] * 6 + [_I, _I, _F, _P, _F, _L, _I, _P, _I, _I, _P, _P],
     ("qkv_prep", "ri_qkv_prep_norm"): [_P, _L, _I, _I, _I] + [_P] * 9 + [_I, _I, _I, _I, _F, _P, _P, _I, _F, _P, _I, _I, _I] + [_I] * 11 + [_P, _P],
     ("moe", "ri_moe_route_rule"): [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _I, _P],
-    ("gla", "ri_gla_recurrent_scalar"): [_P, _L, _I, _I, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    ("gla", "ri_gla_recurrent_scalar"): [_P, _L, _I, _I, _I, _P, _I, _I, _F, _P, _P, _P, _P] + [_I] * 7 + [_P],
     ("mlstm", "ri_mlstm_gates"): [_P, _L, _I, _I, _P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     ("mlstm", "ri_mlstm_head_norm_gate"): [_P, _P, _P, _F, _P, _L, _P, _I, _I, _I, _I, _I, _P],
     ("elementwise", "ri_gate_heads"): [_P, _P, _L, _I, _I, _I, _I, _I, _I, _P],
@@ -90,6 +90,11 @@ MAX_FAST_HEAD_DIM = 256
 LATENT_TC_ROW, LATENT_TC_VALUES = 256, 192
 # ... which masks a score before it is scaled: -FLT_MAX times the scale has to lie far below every score that counts
 LATENT_TC_SCALE = 1e-30
+# gated linear attention: up to so many tokens a step the recurrence's blocks take the decays themselves; with more tokens a kernel
+# takes them once for all blocks of a head.  On the device the two meet at some 64 tokens (us, 32 heads of 64 x 128: 2 tokens 3.9 / 5.4
+# with that kernel, 64 9.1 / 9.5, 128 15.8 / 15.3, 256 27.1 / 25.4; 16 heads of 128 x 64: 4.2 / 5.4, 11.2 / 10.5, 19.9 / 17.2, 36.4 / 29.5),
+# but its scratch and launch cost the host 5 us (22.4 against 17.4 a call), and a prompt of so few tokens waits for the host
+GLA_OWN_DECAYS = 128
 TCGEN05_HEAD_DIMS = (64, 128)   # head sizes the tcgen05 prefill attention kernel is built for
 _NO_TCGEN05 = os.environ.get("RUST_INFERENCE_B200_NO_TCGEN05") == "1"   # for comparisons
 # the skinny linear applies the SiLU gate in its epilogue (one kernel less per layer: 2 % faster at batch 1 of
@@ -425,7 +430,7 @@ def gla_recurrent(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, z: tor
     o = torch.empty((tokens, heads, vdim), dtype=torch.float32, device=proj.device)
     alone = single and tokens == seqs
     # the decays of a prompt's tokens, which every block of a head reads
-    decay = None if alone or dim > 128 else torch.empty((tokens, heads * dim), dtype=torch.float32, device=proj.device)
+    decay = None if alone or dim > 128 or tokens <= GLA_OWN_DECAYS else torch.empty((tokens, heads * dim), dtype=torch.float32, device=proj.device)
     _call("gla", "ri_gla_recurrent", proj.data_ptr(), ld, int(q_col), int(k_col), int(v_col), z.data_ptr(), bias.data_ptr(),
           float(tau), float(qscale), _ptr(decay), state.data_ptr(), o.data_ptr(), seq_slot.data_ptr(), seq_start.data_ptr(), tokens,
           seqs, heads, dim, vdim, 1 if alone else 0, _code(proj.dtype), _stream())
@@ -503,7 +508,7 @@ def scalar_decay_recurrent(proj: torch.Tensor, q_col: int, k_col: int, v_col: in
     o = torch.empty((tokens, heads, wide), dtype=torch.float32, device=proj.device)
     _call("gla", "ri_gla_recurrent_scalar", proj.data_ptr(), ld, int(q_col), int(k_col), int(v_col), gates.data_ptr(),
           int(gates.shape[2]), 1 if ones else 0, float(qscale), state.data_ptr(), o.data_ptr(), seq_slot.data_ptr(),
-          seq_start.data_ptr(), seqs, heads, dim, vdim, 1 if single and tokens == seqs else 0, _code(proj.dtype), _stream())
+          seq_start.data_ptr(), tokens, seqs, heads, dim, vdim, 1 if single and tokens == seqs else 0, _code(proj.dtype), _stream())
     return o
 
 
