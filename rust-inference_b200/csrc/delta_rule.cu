@@ -17,10 +17,10 @@
 //          = sum_d (g[d] S_old[d, j]) qn[d] + u[j] (kn . qn)                   (the form the kernel computes)
 // all in float32; S [dim, vdim] lives in the sequence's slot of `state` [slots, H, dim, vdim].
 // What does not depend on the token before (unit vectors, decays, beta) is computed for all tokens at once by a kernel
-// of its own; the recurrence kernel only walks the tokens.  There a block owns 32 value columns of one (sequence, head);
-// a column is shared by four neighbouring lanes, each with a quarter of the key channels in registers.  Every sum over
-// d has one order that depends on the head's size only, so the result does not depend on how a sequence's tokens were
-// cut into steps.
+// of its own; the recurrence kernels only walk the tokens.  There a block owns some value columns of one (sequence, head), and
+// the key channels of a column are spread over 4 to 32 neighbouring lanes' registers (single tokens: over a block's warps).  Every
+// sum over d has one order that depends on the head's size only, so the result does not depend on how a sequence's tokens
+// were cut into steps.
 #include "common.cuh"
 
 __device__ __forceinline__ float dr_silu(float z) { return z / (1.0f + expf(-z)); }
@@ -205,9 +205,9 @@ delta_prep_kernel(float* __restrict__ qkv, int C, int q_col, int k_col, const T*
 
 // ---- the recurrence -------------------------------------------------------------------------------------------------
 #define DR_CT 128               // computing threads
-#define DR_ST 128               // staging threads
-#define DR_RING 6               // buffers of staged tokens
-#define DR_AHEAD 4              // of which so many are being filled
+// buffers of staged tokens and how many of them are being filled, for ST staging threads (128; 64 or 32 where many blocks wait)
+#define DR_RING(ST) ((ST) == 128 ? 6 : 4)
+#define DR_AHEAD(ST) ((ST) == 128 ? 4 : 3)
 
 // two float32 multiply-adds (products) per instruction, each rounded as fmaf (a product) rounds it
 typedef unsigned long long f32x2;
@@ -255,7 +255,7 @@ __device__ __forceinline__ void dr_bar_arrive(int id, int threads) { asm volatil
 // this token's sums are taken.  With two columns the first shuffle of a sum leaves the even lanes with the first column and the
 // odd ones with the second, and one more brings the other's u.  A sum over d is taken in four partial sums per lane (two pairs
 // of channels by turns), then over the lanes, neighbours first: the same bits with one column per lane as with two.
-// Four more warps of the block copy the tokens into a ring of DR_RING buffers, DR_AHEAD groups on their way together, and write
+// Four more warps of the block copy the tokens into a ring of buffers, several groups on their way together, and write
 // the outputs of the groups that have been computed, so that neither a group's trip to memory nor its outputs stand
 // between the tokens (with one group's loads in registers every group took a trip to memory, 2.5 us).
 // SCALAR (one decay per head): the sums run over the undecayed state and are multiplied by the decay afterwards,
@@ -264,40 +264,39 @@ __device__ __forceinline__ void dr_bar_arrive(int id, int threads) { asm volatil
 // 128 with one decay per head 586 -> 455 us; four sequences of 512 tokens and 16 heads 503 -> 314 us.  (Before: 16 lanes a column,
 // one multiply-add an instruction, the tokens staged by the warps that compute.)  What is left is some 370 cycles a token: the
 // chain of about 210 and the instructions that do not fit beside it, one warp to a scheduler.
-template <int R, int SPLIT, int COLS, int GROUP, bool SCALAR, bool VEC>
-__global__ void __launch_bounds__(GROUP == 1 ? DR_CT : DR_CT + DR_ST)
+template <int R, int SPLIT, int COLS, int GROUP, bool SCALAR, bool VEC, int ST>
+__global__ void __launch_bounds__(DR_CT + ST)
 delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, const float* decay, const float* beta, float* state,
                   float* __restrict__ o, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int H, int G, int dim,
                   int vdim) {
-    constexpr bool SINGLE = GROUP == 1;                                    // every sequence brings one token
     constexpr int DIMC = R * SPLIT;
     constexpr int BCOLS = COLS * DR_CT / SPLIT;
-    constexpr int RING = SINGLE ? 1 : DR_RING;
+    constexpr int RING = DR_RING(ST), FILL = DR_AHEAD(ST);
     constexpr int KP = DIMC / 4;                                           // staged pieces of four channels per token
-    constexpr int PER = (GROUP * KP + DR_ST - 1) / DR_ST;                  // ... and per thread
-    constexpr int VPER = (GROUP * BCOLS + DR_ST - 1) / DR_ST;
+    constexpr int PER = (GROUP * KP + ST - 1) / ST;                  // ... and per thread
+    constexpr int VPER = (GROUP * BCOLS + ST - 1) / ST;
     constexpr int VECS = SCALAR ? 2 : 3;                                   // k, q, and the decays g
-    constexpr bool AHEAD = !SINGLE && R <= 16;                             // the next token's vectors in registers
-    constexpr int ALL = DR_CT + DR_ST;
+    constexpr bool AHEAD = R <= 16;                                        // the next token's vectors in registers
+    constexpr int ALL = DR_CT + ST;
     extern __shared__ __align__(16) float dr_dyn[];
     float (*s_x)[GROUP][VECS][DIMC] = reinterpret_cast<float (*)[GROUP][VECS][DIMC]>(dr_dyn);                             // [RING]
     float (*s_c)[GROUP][4] = reinterpret_cast<float (*)[GROUP][4]>(dr_dyn + RING * GROUP * VECS * DIMC);                  // beta, k . q, the decay (SCALAR)
     float (*s_v)[GROUP][BCOLS] = reinterpret_cast<float (*)[GROUP][BCOLS]>(dr_dyn + RING * GROUP * (VECS * DIMC + 4));
     float (*s_o)[GROUP][BCOLS] = reinterpret_cast<float (*)[GROUP][BCOLS]>(dr_dyn + RING * GROUP * (VECS * DIMC + 4 + BCOLS));
-    static_assert(3 * GROUP <= DR_ST, "a thread per staged beta, product and decay");
+    static_assert(3 * GROUP <= ST, "a thread per staged beta, product and decay");
     // (the kernel after this one is let in only when the walk is over, see below)
     const int b = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * BCOLS;
     const int kvh = h / (H / G);
     pdl_wait();
     const int t0 = seq_start[b], t1 = seq_start[b + 1];
     if (t0 >= t1) return;                     // a sequence without tokens keeps its state (the whole block leaves)
-    const int st_id = SINGLE ? threadIdx.x : threadIdx.x - DR_CT;          // among the staging threads
+    const int st_id = threadIdx.x - DR_CT;                                 // among the staging threads
     // Copies of a group of tokens into its buffer (VEC: 16 bytes, else words): past the sequence's tokens and the columns
     // something that exists is copied and not used, past the head's channels zeros are written (the state is zero there).
     auto copy = [&](int buf, int base) {
 #pragma unroll
         for (int e = 0; e < PER; e++) {
-            const int idx = st_id + e * DR_ST;
+            const int idx = st_id + e * ST;
             const int g = idx / KP, d = (idx % KP) * 4, t = min(base + g, t1 - 1);
             if (g < GROUP) {
                 const float* src[3] = {qkv + (size_t)t * C + k_col + kvh * dim + d, qkv + (size_t)t * C + q_col + kvh * dim + d,
@@ -315,7 +314,7 @@ delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, cons
         }
 #pragma unroll
         for (int e = 0; e < VPER; e++) {
-            const int idx = st_id + e * DR_ST;
+            const int idx = st_id + e * ST;
             if (idx < GROUP * BCOLS)
                 dr_copy<4>(&(&s_v[buf][0][0])[idx], qkv + (size_t)min(base + idx / BCOLS, t1 - 1) * C + v_col + h * vdim + min(j0 + idx % BCOLS, vdim - 1), true);
         }
@@ -325,31 +324,31 @@ delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, cons
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    if (!SINGLE && threadIdx.x >= DR_CT) {
+    if (threadIdx.x >= DR_CT) {
         // ---- the staging warps.  Barriers 1 + buf: the buffer is full; 1 + RING + buf: it was read, its outputs are there ----------------
         auto write_out = [&](int buf, int base) {
-            for (int i = st_id; i < GROUP * BCOLS; i += DR_ST) {
+            for (int i = st_id; i < GROUP * BCOLS; i += ST) {
                 const int g = i / BCOLS, c = i % BCOLS;
                 if (base + g < t1 && j0 + c < vdim) o[((size_t)(base + g) * H + h) * vdim + j0 + c] = s_o[buf][g][c];
             }
         };
         const int groups = (t1 - t0 + GROUP - 1) / GROUP;
-        for (int i = 0; i < DR_AHEAD; i++) {
+        for (int i = 0; i < FILL; i++) {
             if (i < groups) copy(i, t0 + i * GROUP);
             else asm volatile("cp.async.commit_group;\n" ::: "memory");
         }
         for (int n = 0; n < groups; n++) {
-            asm volatile("cp.async.wait_group %0;\n" ::"n"(DR_AHEAD - 1) : "memory");
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(FILL - 1) : "memory");
             dr_bar_arrive(1 + n % RING, ALL);
-            const int m = n + DR_AHEAD, buf = m % RING;                    // the group whose copies start now
-            if (m >= RING) {                                               // (m - RING < groups: DR_AHEAD < RING)
+            const int m = n + FILL, buf = m % RING;                    // the group whose copies start now
+            if (m >= RING) {                                               // (m - RING < groups: FILL < RING)
                 dr_bar_sync(1 + RING + buf, ALL);
                 write_out(buf, t0 + (m - RING) * GROUP);
             }
             if (m < groups) copy(buf, t0 + m * GROUP);
             else asm volatile("cp.async.commit_group;\n" ::: "memory");
         }
-        for (int m = groups + DR_AHEAD > RING ? groups + DR_AHEAD - RING : 0; m < groups; m++) {      // the groups that the loop has not written
+        for (int m = groups + FILL > RING ? groups + FILL - RING : 0; m < groups; m++) {      // the groups that the loop has not written
             dr_bar_sync(1 + RING + m % RING, ALL);
             write_out(m % RING, t0 + m * GROUP);
         }
@@ -453,39 +452,29 @@ delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, cons
         acc = fmaf(u, t.kq, acc);
         if (part < COLS) s_o[buf][g][col] = acc;
     };
-    if (SINGLE) {
-        copy(0, t0);
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();
-        Token one;
-        load(one, 0, 0);
-        step(one, 0, 0);
-        if (part < COLS && j0 + col < vdim) o[((size_t)t0 * H + h) * vdim + j0 + col] = s_o[0][0][col];
-    } else {
-        int nth = 0;
-        for (int base = t0; base < t1; base += GROUP, nth++) {
-            const int buf = nth % RING, n = min(GROUP, t1 - base);
-            dr_bar_sync(1 + buf, ALL);
-            if (AHEAD) {
-                Token one, two;
-                load(one, buf, 0);
+    int nth = 0;
+    for (int base = t0; base < t1; base += GROUP, nth++) {
+        const int buf = nth % RING, n = min(GROUP, t1 - base);
+        dr_bar_sync(1 + buf, ALL);
+        if (AHEAD) {
+            Token one, two;
+            load(one, buf, 0);
 #pragma unroll 1
-                for (int g = 0; g < n; g += 2) {
-                    load(two, buf, g + 1);
-                    step(one, buf, g);
-                    if (g + 2 < GROUP) load(one, buf, g + 2);
-                    if (g + 1 < n) step(two, buf, g + 1);
-                }
-            } else {
-#pragma unroll 1
-                for (int g = 0; g < n; g++) {
-                    Token one;
-                    load(one, buf, g);
-                    step(one, buf, g);
-                }
+            for (int g = 0; g < n; g += 2) {
+                load(two, buf, g + 1);
+                step(one, buf, g);
+                if (g + 2 < GROUP) load(one, buf, g + 2);
+                if (g + 1 < n) step(two, buf, g + 1);
             }
-            dr_bar_arrive(1 + RING + buf, ALL);
+        } else {
+#pragma unroll 1
+            for (int g = 0; g < n; g++) {
+                Token one;
+                load(one, buf, g);
+                step(one, buf, g);
+            }
         }
+        dr_bar_arrive(1 + RING + buf, ALL);
     }
     pdl_trigger();               // the next kernel may come in once the walk is over
 #pragma unroll
@@ -504,6 +493,92 @@ delta_rule_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, cons
                 if (j + c < vdim && d + 1 < dim) st[(size_t)(d + 1) * vdim + j + c] = y[c];
             }
         }
+    }
+}
+
+// The same for steps in which every sequence brings one token.  What bounds it: the state's trip to memory and back, and for few
+// sequences the trips in front of it.  A lane has one value column, a warp 32 neighbouring ones (whole 128-byte lines of the
+// state's rows) with the key channels of PP neighbouring `parts` of the kernel above (R channels each); a block has all channels of its
+// columns.  The warps' sums meet in shared memory, and every warp adds them up in the order of that kernel: the same bits.
+// A step of 1 / 8 / 24 / 64 sequences with the preparation, us: 16 heads of 128 x 128 5.7 / 9.0 / 17 / 37, where the kernel above with
+// a token at a time took 6.5 / 13 / 31 / 75; 8 heads of 64 x 64 4.8 / 5.1 / 5.8 / 8.4 (5.7 / 5.7 / 6.7 / 9.3).
+template <int R, int SPLIT, int PP, bool SCALAR>
+__global__ void __launch_bounds__(32 * SPLIT / PP)
+delta_single_kernel(const float* qkv, int C, int q_col, int k_col, int v_col, const float* decay, const float* beta, float* state,
+                    float* __restrict__ o, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int H, int G, int dim,
+                    int vdim) {
+    constexpr int WARPS = SPLIT / PP, N = R * PP;                          // a lane's channels
+    static_assert(N <= 32 && (PP == 1 || PP == 2), "a lane per staged channel");
+    __shared__ __align__(16) float s_x[WARPS][3][N];                       // k, q and the decays of the warp's channels
+    __shared__ float s_sum[2][WARPS][32];
+    pdl_trigger();
+    const int b = blockIdx.z, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int kvh = h / (H / G), j = blockIdx.x * 32 + lane;
+    auto channel = [&](int n) { return 4 * SPLIT * ((n % R) / 4) + 4 * (PP * warp + n / R) + (n & 3); };
+    const int t0 = seq_start[b], t1 = seq_start[b + 1];
+    float* st = state + ((size_t)seq_slot[b] * H + h) * dim * vdim + j;
+    pdl_wait();
+    if (t0 >= t1) return;                     // a sequence without tokens keeps its state (the whole block leaves)
+    const float* row = qkv + (size_t)t0 * C;
+    const int mine = channel(lane % N);
+    const bool own = lane < N && mine < dim;
+    const float kx = own ? row[k_col + kvh * dim + mine] : 0.0f;
+    const float qx = own ? row[q_col + kvh * dim + mine] : 0.0f;
+    const float gx = own && !SCALAR ? decay[((size_t)t0 * H + h) * dim + mine] : 0.0f;
+    const float v = j < vdim ? row[v_col + h * vdim + j] : 0.0f;
+    const float bt = beta[(size_t)t0 * (H + G) + h], kq = beta[(size_t)t0 * (H + G) + H + kvh];
+    const float gs = SCALAR ? decay[(size_t)t0 * H + h] : 1.0f;
+    float S[N];
+#pragma unroll
+    for (int n = 0; n < N; n++) S[n] = j < vdim && channel(n) < dim ? st[(size_t)channel(n) * vdim] : 0.0f;
+    if (lane < N) {
+        s_x[warp][0][lane] = kx;
+        s_x[warp][1][lane] = qx;
+        s_x[warp][2][lane] = gx;
+    }
+    __syncwarp();
+    if (!SCALAR) {
+#pragma unroll
+        for (int n = 0; n < N; n++) S[n] = __fmul_rn(s_x[warp][2][n], S[n]);
+    }
+#pragma unroll
+    for (int w = 0; w < 2; w++) {                                          // S^T k, S^T q
+        float part[PP];
+#pragma unroll
+        for (int p = 0; p < PP; p++) {
+            float e[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                e[i] = __fmul_rn(S[p * R + i], s_x[warp][w][p * R + i]);
+#pragma unroll
+                for (int c = 4; c < R; c += 4) e[i] = fmaf(S[p * R + c + i], s_x[warp][w][p * R + c + i], e[i]);
+            }
+            part[p] = (e[0] + e[1]) + (e[2] + e[3]);
+        }
+        s_sum[w][warp][lane] = PP == 2 ? part[0] + part[PP - 1] : part[0];
+    }
+    __syncthreads();
+    auto total = [&](int w) {
+        float x[WARPS];
+#pragma unroll
+        for (int i = 0; i < WARPS; i++) x[i] = s_sum[w][i][lane];
+#pragma unroll
+        for (int m = 1; m < WARPS; m <<= 1)
+#pragma unroll
+            for (int i = 0; i < WARPS; i += 2 * m) x[i] += x[i + m];
+        return x[0];
+    };
+    const float pred = total(0);
+    const float u = bt * (SCALAR ? fmaf(-gs, pred, v) : v - pred);
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+        const float x = fmaf(s_x[warp][0][n], u, SCALAR ? __fmul_rn(gs, S[n]) : S[n]);
+        if (j < vdim && channel(n) < dim) st[(size_t)channel(n) * vdim] = x;
+    }
+    if (warp == 0 && j < vdim) {
+        float acc = total(1);
+        if (SCALAR) acc *= gs;
+        o[((size_t)t0 * H + h) * vdim + j] = fmaf(u, kq, acc);
     }
 }
 
@@ -534,10 +609,34 @@ extern "C" int ri_delta_rule_recurrent(float* qkv, int C, int q_col, int k_col, 
                       G, dim, ddim);
     else RI_FAIL(-1, "delta_rule_recurrent: unknown dtype %d", dtype);
     RI_CHECK_LAUNCH("delta_prep");
-    // The recurrence kernel is launched the ordinary way, not as a dependent launch: its few long-lived blocks (a chain of
+    // A prompt's recurrence kernel is launched the ordinary way, not as a dependent launch: its few long-lived blocks (a chain of
     // dependent instructions, one warp per scheduler) must spread one per SM, and blocks that come in while the kernel
     // before still holds most SMs pile up on the first SMs that get free and stay there (2,048 tokens of 8 heads of
     // 128 x 128: 0.97 ms as a dependent launch, 0.59 ms as an ordinary one).
+    // (Single tokens: a dependent launch as everything else.)
+#define DS_GO(R, SPLIT, PP, SC)                                                                                            \
+    ri_launch_pdl(delta_single_kernel<R, SPLIT, PP, SC>, dim3((vdim + 31) / 32, H, seqs), dim3(32 * SPLIT / PP), 0, stream, (const float*)qkv, \
+                  C, q_col, k_col, v_col, (const float*)decay, (const float*)beta, state, o, seq_slot, seq_start, H, G, dim, vdim)
+    if (single) {
+        if (ddim == 1 && dim > 1) {
+            if (dim <= 16) DS_GO(4, 4, 1, true);
+            else if (dim <= 32) DS_GO(4, 8, 1, true);
+            else if (dim <= 64) DS_GO(4, 16, 2, true);
+            else if (dim <= 128) DS_GO(4, 32, 2, true);
+            else if (dim <= 256) DS_GO(16, 16, 1, true);
+            else DS_GO(32, 16, 1, true);
+        } else {
+            if (dim <= 16) DS_GO(4, 4, 1, false);
+            else if (dim <= 32) DS_GO(4, 8, 1, false);
+            else if (dim <= 64) DS_GO(8, 8, 1, false);
+            else if (dim <= 128) DS_GO(8, 16, 1, false);
+            else if (dim <= 256) DS_GO(16, 16, 1, false);
+            else DS_GO(32, 16, 1, false);
+        }
+        RI_CHECK_LAUNCH("delta_rule_recurrent");
+        return 0;
+    }
+#undef DS_GO
     // 16-byte copies of four channels where every row of q, k and the decays starts on 16 bytes
     const bool vec = dim % 4 == 0 && C % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && (((uintptr_t)qkv | (uintptr_t)decay) & 15) == 0;
     static int sms = 0;
@@ -551,49 +650,54 @@ extern "C" int ri_delta_rule_recurrent(float* qkv, int C, int q_col, int k_col, 
     // 2,048 tokens: 8 heads of 128 x 128 395 / 418 us, 8 of 64 x 64 335 / 357, 16 of 128 x 128 516 / 435, four sequences
     // of 512 tokens and 16 heads 490 / 314).  With one decay per head half as many channels a lane (16 heads of 128 x 128: 455
     // us, with eight channels 516): there is a third less to read.
-#define DR_GO(R, SPLIT, COLS, GROUP, SC, VEC)                                                                              \
+#define DR_GO(R, SPLIT, COLS, GROUP, SC, VEC, ST)                                                                          \
     do {                                                                                                                 \
         constexpr int bcols = COLS * DR_CT / SPLIT;                                                                      \
-        constexpr size_t sm = (size_t)(GROUP == 1 ? 1 : DR_RING) * GROUP * ((SC ? 2 : 3) * R * SPLIT + 4 + 2 * bcols) * sizeof(float); \
+        constexpr size_t sm = (size_t)DR_RING(ST) * GROUP * ((SC ? 2 : 3) * R * SPLIT + 4 + 2 * bcols) * sizeof(float);   \
         const dim3 grid((vdim + bcols - 1) / bcols, H, seqs);                                                            \
-        cudaError_t e = sm > 48 * 1024 ? cudaFuncSetAttribute(delta_rule_kernel<R, SPLIT, COLS, GROUP, SC, VEC>,          \
+        cudaError_t e = sm > 48 * 1024 ? cudaFuncSetAttribute(delta_rule_kernel<R, SPLIT, COLS, GROUP, SC, VEC, ST>,      \
                                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) : cudaSuccess; \
         if (e != cudaSuccess) RI_FAIL((int)e, "delta_rule_recurrent: %s", cudaGetErrorString(e));                        \
-        delta_rule_kernel<R, SPLIT, COLS, GROUP, SC, VEC><<<grid, dim3(GROUP == 1 ? DR_CT : DR_CT + DR_ST), sm, stream>>>( \
+        delta_rule_kernel<R, SPLIT, COLS, GROUP, SC, VEC, ST><<<grid, dim3(DR_CT + ST), sm, stream>>>(                    \
             (const float*)qkv, C, q_col, k_col, v_col, (const float*)decay, (const float*)beta, state, o, seq_slot,      \
             seq_start, H, G, dim, vdim);                                                                                 \
     } while (0)
-#define DR_BY_VEC(R, SPLIT, COLS, GROUP, SC)                                                                             \
+#define DR_BY_VEC(R, SPLIT, COLS, GROUP, SC, ST)                                                                         \
     do {                                                                                                                 \
-        if (vec) DR_GO(R, SPLIT, COLS, GROUP, SC, true);                                                                 \
-        else DR_GO(R, SPLIT, COLS, GROUP, SC, false);                                                                    \
+        if (vec) DR_GO(R, SPLIT, COLS, GROUP, SC, true, ST);                                                             \
+        else DR_GO(R, SPLIT, COLS, GROUP, SC, false, ST);                                                                \
     } while (0)
-#define DR_CHANNEL(R, SPLIT, GROUP)                                                                                      \
+    auto blocks = [&](int columns) { return (long long)((vdim + columns - 1) / columns) * H * seqs; };
+    // With many blocks fewer staging threads, so that more blocks fit an SM (ST / 128 threads; 64 sequences of 4 tokens; 16 heads of 128 x 128
+    // with one decay per head 114 us, with 128 staging threads 130; 8 heads of 256 x 128 95 / 127 us).  Not for the eight channels a lane of per-channel
+    // decays: a long prompt beside many single tokens would have its blocks pile up on few SMs (500 tokens and 32 times one, 16
+    // heads of 128 x 128: 151 / 133 us).
+    auto many = [&](int columns) { return blocks(columns) > 4ll * sms; };
+#define DR_CHANNEL(R, SPLIT, GROUP, FEWER)                                                                               \
     do {                                                                                                                 \
-        const long long blocks = (long long)((vdim + DR_CT / SPLIT - 1) / (DR_CT / SPLIT)) * H * seqs;                   \
-        if (single) DR_BY_VEC(R, SPLIT, 2, 1, false);                                                                    \
-        else if (blocks <= sms) DR_BY_VEC(R, SPLIT, 1, GROUP, false);                                                    \
-        else DR_BY_VEC(R, SPLIT, 2, GROUP, false);                                                                       \
+        if (blocks(DR_CT / SPLIT) <= sms) DR_BY_VEC(R, SPLIT, 1, GROUP, false, 128);                                     \
+        else if (FEWER == 128 || !many(2 * DR_CT / SPLIT)) DR_BY_VEC(R, SPLIT, 2, GROUP, false, 128);                    \
+        else DR_BY_VEC(R, SPLIT, 2, GROUP, false, FEWER);                                                                \
     } while (0)
-#define DR_HEAD(R, SPLIT, GROUP)                                                                                         \
+#define DR_HEAD(R, SPLIT, GROUP, FEWER)                                                                                  \
     do {                                                                                                                 \
-        if (single) DR_BY_VEC(R, SPLIT, 2, 1, true);                                                                     \
-        else DR_BY_VEC(R, SPLIT, 2, GROUP, true);                                                                        \
+        if (!many(2 * DR_CT / SPLIT)) DR_BY_VEC(R, SPLIT, 2, GROUP, true, 128);                                          \
+        else DR_BY_VEC(R, SPLIT, 2, GROUP, true, FEWER);                                                                 \
     } while (0)
     if (ddim == 1 && dim > 1) {
-        if (dim <= 16) DR_HEAD(4, 4, 16);
-        else if (dim <= 32) DR_HEAD(4, 8, 16);
-        else if (dim <= 64) DR_HEAD(4, 16, 16);
-        else if (dim <= 128) DR_HEAD(4, 32, 8);
-        else if (dim <= 256) DR_HEAD(16, 16, 4);
-        else DR_HEAD(32, 16, 2);
+        if (dim <= 16) DR_HEAD(4, 4, 16, 64);
+        else if (dim <= 32) DR_HEAD(4, 8, 16, 64);
+        else if (dim <= 64) DR_HEAD(4, 16, 16, 64);
+        else if (dim <= 128) DR_HEAD(4, 32, 8, 32);
+        else if (dim <= 256) DR_HEAD(16, 16, 4, 64);
+        else DR_HEAD(32, 16, 2, 64);
     } else {
-        if (dim <= 16) DR_CHANNEL(4, 4, 16);
-        else if (dim <= 32) DR_CHANNEL(4, 8, 16);
-        else if (dim <= 64) DR_CHANNEL(8, 8, 16);
-        else if (dim <= 128) DR_CHANNEL(8, 16, 8);
-        else if (dim <= 256) DR_CHANNEL(16, 16, 4);
-        else DR_CHANNEL(32, 16, 2);
+        if (dim <= 16) DR_CHANNEL(4, 4, 16, 64);
+        else if (dim <= 32) DR_CHANNEL(4, 8, 16, 64);
+        else if (dim <= 64) DR_CHANNEL(8, 8, 16, 128);
+        else if (dim <= 128) DR_CHANNEL(8, 16, 8, 128);
+        else if (dim <= 256) DR_CHANNEL(16, 16, 4, 64);
+        else DR_CHANNEL(32, 16, 2, 64);
     }
 #undef DR_HEAD
 #undef DR_CHANNEL

@@ -112,3 +112,79 @@ def test_gla_prompts_pieces_and_single_tokens(dim, vdim, pad, ones, dtype):
     for cuts in ([3, 19, 20, 51, 52, 130], list(range(1, 66)) + [80]):
         pieces, state1 = gla.walk(cuts)
         assert all(torch.equal(a, b) for a, b in zip(pieces, outs)) and torch.equal(state, state1)
+
+
+class Delta(Gla):
+    """The gated delta rule, likewise; ``per_head``: one decay per head."""
+
+    def __init__(self, lens, H, Gq, dim, vdim, dtype, per_head=False, pad=0, seed=0):
+        g = torch.Generator(device=DEV).manual_seed(seed + 17 * sum(lens) + dim)
+        self.lens, self.H, self.Gq, self.dim, self.vdim, self.ones, self.per_head, self.pad = lens, H, Gq, dim, vdim, False, per_head, pad
+        wide = H if per_head else H * dim
+        self.qkv = [torch.randn((n, pad + 2 * Gq * dim + H * vdim), generator=g, device=DEV) for n in lens]
+        self.proj = [torch.randn((n, H + 3), generator=g, device=DEV).to(dtype) for n in lens]
+        self.z = [torch.randn((n, wide), generator=g, device=DEV).to(dtype) for n in lens]
+        self.dt_bias = torch.randn(wide, generator=g, device=DEV) - 3
+        self.a_log = torch.rand(H, generator=g, device=DEV)
+        self.slots = _i32([len(lens) - b for b in range(len(lens))])
+
+    def columns(self):
+        return self.pad, self.pad + self.Gq * self.dim, self.pad + 2 * self.Gq * self.dim
+
+    def step(self, state, pieces):
+        qkv, proj, z = (torch.cat([x[b][i:j] for b, i, j in pieces]) for x in (self.qkv, self.proj, self.z))
+        start = np.concatenate([[0], np.cumsum([j - i for _, i, j in pieces])])
+        slots, single = self.slots[[b for b, _, _ in pieces]].contiguous(), all(j - i == 1 for _, i, j in pieces)
+        o = ops.delta_rule_recurrent(qkv, *self.columns(), proj, 2, z, self.dt_bias, self.a_log, self.dim ** -0.5, state, slots,
+                                     _i32(start), self.H, self.Gq, self.dim, self.vdim, single=single)
+        return [o[start[k]:start[k + 1]] for k in range(len(pieces))]
+
+    def exact(self):
+        outs, state, H, per = [], self.state().double(), self.H, self.H // self.Gq
+        q_col, k_col, v_col = self.columns()
+        for b, n in enumerate(self.lens):
+            x = self.qkv[b].double()
+            q, k = (x[:, c:c + self.Gq * self.dim].view(n, self.Gq, self.dim) for c in (q_col, k_col))
+            q, k = (t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+            q, k = (q * self.dim ** -0.5).repeat_interleave(per, 1), k.repeat_interleave(per, 1)
+            v = x[:, v_col:v_col + H * self.vdim].view(n, H, self.vdim)
+            rate = torch.nn.functional.softplus(self.z[b].double() + self.dt_bias.double(), threshold=40).view(n, H, -1)
+            decay = torch.exp(-torch.exp(self.a_log.double())[None, :, None] * rate)
+            beta = torch.sigmoid(self.proj[b][:, 2:2 + H].double())
+            S, o = torch.zeros_like(state[0]), []
+            for t in range(n):
+                S = S * decay[t][:, :, None]
+                u = beta[t][:, None] * (v[t] - (S * k[t][:, :, None]).sum(1))
+                S = S + k[t][:, :, None] * u[:, None]
+                o.append((S * q[t][:, :, None]).sum(1))
+            outs.append(torch.stack(o))
+            state[int(self.slots[b])] = S
+        return outs, state
+
+
+# every size class of key channels, columns that do not fill a block or a pair, rings of six buffers that wrap
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("dim, vdim, pad", [(12, 20, 0), (16, 64, 0), (32, 33, 0), (48, 40, 1), (64, 64, 0), (96, 96, 0), (128, 128, 0),
+                                            (128, 31, 4), (200, 40, 0), (256, 64, 0), (300, 35, 0)])
+def test_delta_prompts_pieces_and_single_tokens(dim, vdim, pad, per_head, dtype):
+    delta = Delta([47, 130, 1, 48], 4, 2, dim, vdim, dtype, per_head, pad)
+    outs, state = delta.walk([])
+    want, want_state = delta.exact()
+    for got, exact in zip(outs + [state], want + [want_state]):
+        assert (got.double() - exact).abs().max() <= 2e-5 * exact.abs().max()       # as for gated linear attention
+    for cuts in ([3, 19, 20, 51, 52], list(range(1, 50)) + [80]):
+        pieces, state1 = delta.walk(cuts)
+        assert all(torch.equal(a, b) for a, b in zip(pieces, outs)) and torch.equal(state, state1)
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("dim, vdim, seqs", [(128, 128, 9), (64, 64, 40), (16, 32, 80), (96, 40, 64), (256, 64, 24)])
+def test_delta_in_a_large_step_and_alone(dim, vdim, seqs, per_head):
+    """Many sequences take two columns a lane (and other blocks), one alone may take one: the same bits."""
+    delta = Delta([70, 9, 1, 33] + [5] * (seqs - 4), 8, 4, dim, vdim, torch.bfloat16, per_head)
+    outs, state = delta.walk([])
+    for b in (0, 1, 2, 3, seqs - 1):
+        alone = delta.state()
+        o, = delta.step(alone, [(b, 0, delta.lens[b])])
+        assert torch.equal(o, outs[b]) and torch.equal(alone[delta.slots[b]], state[delta.slots[b]])
