@@ -635,7 +635,8 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
     const int lo = s * a.per_slice, hi = min(a.vocab, lo + a.per_slice);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned barriers = 0;                 // barriers of this row so far
-    int hp = 0, ti = 0;                    // histogram passes and total passes so far
+    // the copy of the histogram that the next pass adds to, and the step to the one after it (cleared meanwhile); total passes so far
+    int hp = 0, turn = 1, ti = 0;
 
     // this block's share of a copy of the row's histogram, cleared
     auto clear_share = [&](int copy) {
@@ -720,8 +721,8 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) bins[b] = 0;
         __syncthreads();
     };
-    // this slice's part of the top digit's histogram (sign, exponent, three bits of the mantissa: the tokens crowd into a few
-    // bins), collected in shared memory
+    // this slice's part of the top digit's histogram (the sign and seven bits of the exponent: the tokens crowd into a few
+    // bins, each of which spans a factor of four), collected in shared memory
     auto top_sweep = [&](int counting, u64* hist) {
         __syncthreads();
         clear_bins();
@@ -812,9 +813,9 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
     // the result of the last digit.
     auto select = [&](int pass, u64 prefix, u64 remaining, int counting, bool last, u64* K, int* found_out) -> bool {
         int found = 1;
-        for (; pass >= 0; pass--, hp++) {
+        for (; pass >= 0; pass--, hp = (hp + turn) % 3) {
             const int shift = pass * SP_DIGIT;
-            u64* hist = hist3 + (size_t)(hp % 3) * SP_BINS;
+            u64* hist = hist3 + (size_t)hp * SP_BINS;
             if (found && pass == SP_PASSES - 1) {
                 top_sweep(counting, hist);
             } else if (found) {
@@ -829,7 +830,7 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                     if (w) atomicAdd(&hist[(unsigned)(k >> shift) & (SP_BINS - 1)], w);
                 }
             }
-            clear_share((hp + 1) % 3);
+            clear_share((hp + turn) % 3);
             const bool waits = !(last && pass == 0) || s == 0;
             if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, waits, f.err)) return false;
             if (!waits) return true;                   // the last digit of the draw: slice 0 finishes alone
@@ -845,17 +846,25 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
 
     // ---- lists: the keys of a few bins, from which a block ends a search by itself ---------------------------------
     // the keys of this slice whose top digit lies in [first, last], into list `which` of the row (what does not fit is counted
-    // only); true when the wait ended
+    // only); true when the wait ended.  With `hist` their weights by the next digit as well, so that a list that does not fit has
+    // cost no sweep and no barrier more than the search without it (32 rows of 151,936 flat logits, a plain draw: without lists
+    // 115 us, with a sweep for a list that overflowed 121).
     u64* lists = f.lists + (size_t)row * 2 * SPF_LIST;
-    auto gather = [&](unsigned first, unsigned last, int which, bool wait) -> bool {
+    auto gather = [&](unsigned first, unsigned last, int which, bool wait, u64* hist) -> bool {
         int mine = 0, j = 0;
         unsigned hits = 0;                                // which of this thread's first 32 tokens
 #pragma unroll 4
         for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS, j++) {
-            const unsigned top = (unsigned)(r.key(i, r.z(i)) >> SPF_TOP);
+            const float zi = r.z(i);
+            const u64 k = r.key(i, zi);
+            const unsigned top = (unsigned)(k >> SPF_TOP);
             const bool in = top >= first && top <= last;
             mine += in;
             if (in && j < 32) hits |= 1u << j;
+            if (in && hist && k >= floor_key) {
+                const u64 w = weight_of(zi, zmax, 0);
+                if (w) atomicAdd(&hist[(unsigned)(k >> (SPF_TOP - SP_DIGIT)) & (SP_BINS - 1)], w);
+            }
         }
         int upto = mine;
 #pragma unroll
@@ -875,8 +884,8 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             s_base = all ? atomicAdd(&shared_row->listed[which], (unsigned)all) : 0u;
         }
         __syncthreads();
-        if (mine) {
-            unsigned at = s_base + (unsigned)(ired[warp] + upto - mine);
+        unsigned at = s_base + (unsigned)(ired[warp] + upto - mine);
+        if (mine && at < SPF_LIST) {
             j = 0;
             for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS, j++) {
                 if (j < 32 && !(hits >> j & 1)) continue;
@@ -898,10 +907,16 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         return i < listed ? list[i] : ~0ull;
     };
     // exp(z - zmax) of a key, with z from the key: the same bits as from the logit
-    auto key_weight = [&](u64 k) {
+    auto key_value = [](u64 k) {
         const unsigned u = (unsigned)(k >> SP_IDX_BITS);
-        const float zi = u == 0u ? __uint_as_float(0x7fffffffu) : __uint_as_float((u & 0x80000000u) ? u ^ 0x80000000u : ~u);
-        return weight_of(zi, zmax, 0);
+        return u == 0u ? __uint_as_float(0x7fffffffu) : __uint_as_float((u & 0x80000000u) ? u ^ 0x80000000u : ~u);
+    };
+    auto key_weight = [&](u64 k) { return weight_of(key_value(k), zmax, 0); };
+    // A bin of the top digit that certainly holds more tokens than a list takes: none of them weighs more than the bin's upper
+    // edge, or the row's maximum
+    auto too_many = [&](unsigned bin) {
+        const u64 edge = (((u64)bin + 1) << SPF_TOP) - 1;
+        return bins[bin] > (u64)SPF_LIST * weight_of(fminf(key_value(edge), zmax), zmax, 0);
     };
     auto list_sum = [&](u64 from) {
         u64 part = 0;
@@ -1020,6 +1035,7 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
     // the top digit of the first search: the count for a top-k, else the weight
     top_sweep(top_k, hist3);
     clear_share(1);
+    if (!top_k && tp < 1.0f) clear_share(2);
     if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, true, f.err)) return;
     read_hist(hist3);
     hp = 1;
@@ -1031,7 +1047,7 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         const u64 n = (u64)k - remaining + bins[first];   // tokens in that bin and above
         if (found && n <= SPF_LIST) {
             // all that the rest can choose from fits a list: slice 0 ends the work alone
-            if (!gather(first, SP_BINS - 1, 0, s == 0) || s != 0) return;
+            if (!gather(first, SP_BINS - 1, 0, s == 0, nullptr) || s != 0) return;
             listed = (unsigned)n;
             if (select_list(SP_PASSES - 2, prefix, remaining, 1, &K)) {
                 floor_key = K;                            // k keys are left
@@ -1068,8 +1084,14 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             if (found) {
                 const u64 above = target - remaining;
                 floor_bin = (unsigned)(prefix >> SPF_TOP);
-                if (!gather(floor_bin, floor_bin, 0, true)) return;
-                const unsigned n = __ldcg(&shared_row->listed[0]);
+                // the copies' turns: the list's weights go into copy 2, the draw's into 1 (2 is cleared meanwhile); after a list
+                // that overflows 1, 0, 2, .., so that nobody clears the copy that a late block still reads
+                const bool listing = !too_many(floor_bin);
+                unsigned n = SPF_LIST + 1;
+                if (listing) {
+                    if (!gather(floor_bin, floor_bin, 0, true, hist3 + 2 * SP_BINS)) return;
+                    n = __ldcg(&shared_row->listed[0]);
+                }
                 if (n <= SPF_LIST) {
                     listed = n;
                     floor_listed = select_list(SP_PASSES - 2, prefix, remaining, 0, &K) != 0;
@@ -1085,7 +1107,12 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                         __syncthreads();
                     }
                 } else {
-                    if (!select(SP_PASSES - 2, prefix, remaining, 0, false, &K, &found)) return;
+                    if (listing) {
+                        read_hist(hist3 + 2 * SP_BINS);
+                        pick(SPF_TOP - SP_DIGIT, prefix, remaining, found);
+                        turn = 2;
+                    }
+                    if (found && !select(listing ? SP_PASSES - 3 : SP_PASSES - 2, prefix, remaining, 0, false, &K, &found)) return;
                     if (found) floor_key = K;
                     if (!sum_total()) return;
                     narrowed = true;
@@ -1101,10 +1128,20 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             }
             const unsigned bin = (unsigned)(prefix >> SPF_TOP);
             if (!(floor_listed && bin == floor_bin)) {
-                if (!gather(bin, bin, 1, true)) return;
-                const unsigned n = __ldcg(&shared_row->listed[1]);
+                const bool listing = !too_many(bin);
+                unsigned n = SPF_LIST + 1;
+                if (listing) {
+                    clear_share(2);
+                    if (!gather(bin, bin, 1, true, hist3 + SP_BINS)) return;
+                    n = __ldcg(&shared_row->listed[1]);
+                }
                 if (n > SPF_LIST) {
-                    if (!select(SP_PASSES - 2, prefix, remaining, 0, true, &K, &found)) return;
+                    if (listing) {
+                        read_hist(hist3 + SP_BINS);
+                        pick(SPF_TOP - SP_DIGIT, prefix, remaining, found);
+                        hp = 2;
+                    }
+                    if (found && !select(listing ? SP_PASSES - 3 : SP_PASSES - 2, prefix, remaining, 0, true, &K, &found)) return;
                     finish(found, K);
                     return;
                 }
