@@ -96,7 +96,7 @@ class MixtureOfExperts(FeedForward):
         with section("moe router"):
             # many pairs per expert (a prompt): tiles of 256 rows, where the tcgen05 kernel for them takes the sizes
             wide = (x.dtype == torch.bfloat16 and T * s.top >= 48 * s.experts and s.hidden_size % 8 == 0
-                    and ex.intermediate_size % 8 == 0)
+                    and ex.intermediate_size % 8 == 0 and not ops._NO_TCGEN05)
             if self.by_table:
                 weight = None                              # every choice weighs 1 / top
                 idx, plan = ops.moe_plan_table(ctx.ids, self.table, s.experts, wide)

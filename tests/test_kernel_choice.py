@@ -63,3 +63,20 @@ def test_forms_of_latent_prompts(launches, monkeypatch, form, want):
     assert fn == want
     if want == TCGEN05:
         assert sent[7] == 5 and sent[9] == 5                        # tokens; the most of one sequence is no more than that
+
+
+@pytest.mark.parametrize("switch", [False, True])
+def test_the_switch_leaves_the_routed_products_to_mma_sync(launches, monkeypatch, switch):
+    from rust_inference_b200.config.specs import GatedFFSpec, MoESpec
+    from rust_inference_b200.parts import BuildEnv, build_part, part_class
+    monkeypatch.setattr(ops, "_NO_TCGEN05", switch)
+    spec = MoESpec(hidden_size=16, experts=2, top=1, expert=GatedFFSpec(16, 24, gate="silu"))
+    part = build_part("ffn", spec, BuildEnv(torch.bfloat16, torch.device("cpu")))
+    infos = part_class("ffn", spec).param_infos(spec)
+    part.load({n: torch.zeros(i.shape, dtype=torch.bfloat16 if i.role == "matrix" else torch.float32) for n, i in infos.items()})
+    asked = []
+    monkeypatch.setattr(ops, "moe_plan", lambda idx, experts, wide=False: asked.append(wide) or _plan(200, 2, 256 if wide else 32))
+    part(torch.zeros((200, 16), dtype=torch.bfloat16), None)
+    assert asked == [not switch]
+    assert [fn for _, fn, _ in launches if fn.startswith(("ri_moe_tc", "ri_moe_grouped"))] == (
+        ["ri_moe_grouped_gated", "ri_moe_grouped_linear"] if switch else ["ri_moe_tc", "ri_moe_tc"])
