@@ -26,9 +26,10 @@
 // hand-over to the tensor core waits for the copies under way (fence.proxy.async; 1.5 us per 64 k).
 // 2,048 tokens of width 4,096, 16 experts of 1,376 channels, 4 choices (7,300 rows, 246 GFLOP in both products): 179 us with the
 // gather and 89 us, 0.92 PFLOP/s, where mma.sync tiles of 64 rows x 64 outputs took 687 and 401 us and the gate's own kernel 38.
-// The plan has wide tiles from 48 pairs per expert on (gather and both products, wide / tiles of 32 rows: width 4,096, 16 experts
-// of 1,376: 25 pairs per expert 177 / 180 us, 48 pairs 169 / 237; width 2,048, 32 experts of 704: 12 pairs 116 / 100, 50 pairs
-// 114 / 138).
+// The plan has wide tiles from 48 pairs per expert on, where they also lay for the tiles before these.  Gather and both products, wide / tiles
+// of 32 rows: width 4,096, 16 experts of 1,376: 25 pairs per expert 177 / 180 us, 48 pairs 169 / 237; width 2,048, 32 experts of
+// 704: 12 pairs 116 / 100, 50 pairs 114 / 138.  So the two forms meet at some 25 pairs, and from there to 47 the plan takes the
+// slower one by up to 40 %; a wide step costs the host a launch more, which is what bounds small ones.
 //
 // Waits are bounded (error 5): whoever gives up says so in shared memory, no further copy or product is started, the copies
 // under way are waited for once more, and the block ends as usual with a wrong result.
@@ -348,22 +349,11 @@ static int mt_tensor_map(CUtensorMap* map, const void* p, long long rows, int K,
     return 0;
 }
 
-// x [tokens, ldx] bfloat16; xg [pairs, K]: rows of the plan, those past its count are left alone
-extern "C" int ri_moe_gather(const void* x, long long ldx, void* xg, const int* perm, const int* meta, int pairs, int div, int K,
-                             cudaStream_t stream) {
-    if (pairs == 0) return 0;
-    RI_REQUIRE(pairs > 0 && div > 0 && K > 0 && K % 8 == 0 && ldx % 8 == 0 && (((uintptr_t)x | (uintptr_t)xg) & 15) == 0,
-               "moe_gather: rows of whole 16-byte pieces are needed");
-    ri_launch_pdl(moe_gather_kernel, dim3(pairs < 8192 ? pairs : 8192), dim3(256), 0, stream, (const uint4*)x, ldx / 8, (uint4*)xg, perm,
-                  meta, div, K / 8);
-    RI_CHECK_LAUNCH("moe_gather");
-    return 0;
-}
-
 // a [a_rows, lda] bfloat16, w [E, N, K] (gate 0) or [E, 2 N, K] (gate rows, then up rows; gate 1 silu, 2 gelu_tanh, 3 clamped
-// swish); y [.., ldy] bfloat16 or float32 (out_f32; without a gate only).  The plan's tiles have MT_ROWS rows.
-extern "C" int ri_moe_tc(const void* a, long long a_rows, long long lda, const void* w, void* y, long long ldy, const int* perm,
-                         const int* tiles, const int* meta, int max_tiles, int E, int N, int K, int scatter, int out_f32, int gate,
+// swish); y [.., ldy] bfloat16 or float32 (out_f32; without a gate only).  The plan's tiles have MT_ROWS rows.  x not null: row r
+// of a is scratch that becomes x[perm[r] / div] first, for the plan's rows (x [.., ldx] bfloat16).
+extern "C" int ri_moe_tc(const void* x, long long ldx, int div, void* a, long long a_rows, long long lda, const void* w, void* y,
+                         long long ldy, const int* perm, const int* tiles, const int* meta, int max_tiles, int E, int N, int K, int scatter, int out_f32, int gate,
                          float limit, float alpha, int* err_flag, cudaStream_t stream) {
     if (max_tiles == 0 || a_rows == 0) return 0;
     RI_REQUIRE(max_tiles > 0 && a_rows > 0 && E > 0 && N > 0 && K > 0, "moe_tc: bad sizes");
@@ -371,6 +361,12 @@ extern "C" int ri_moe_tc(const void* a, long long a_rows, long long lda, const v
     RI_REQUIRE(gate >= 0 && gate <= 3 && !(gate && out_f32), "moe_tc: gate function %d", gate);
     const long long w_rows = (long long)E * N * (gate ? 2 : 1);
     RI_REQUIRE(w_rows < (1ll << 31) && a_rows < (1ll << 31), "moe_tc: too many rows");
+    if (x) {
+        RI_REQUIRE(div > 0 && lda == K && ldx % 8 == 0 && ldx >= K && ((uintptr_t)x & 15) == 0, "moe_tc: rows of whole 16-byte pieces are needed");
+        ri_launch_pdl(moe_gather_kernel, dim3((unsigned)(a_rows < 8192 ? a_rows : 8192)), dim3(256), 0, stream, (const uint4*)x, ldx / 8, (uint4*)a,
+                      perm, meta, div, K / 8);
+        RI_CHECK_LAUNCH("moe_gather");
+    }
     static int sms = 0;
     if (!sms) {
         int dev = 0, n = 0;

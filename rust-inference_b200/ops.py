@@ -47,8 +47,7 @@ _SIGNATURES = {
     ("moe", "ri_moe_plan"): [_P, _P, _P, _P, _I, _I, _I, _I, _P],
     ("moe", "ri_moe_grouped_linear"): [_P, _L, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     ("moe", "ri_moe_grouped_gated"): [_P, _L, _P, _P, _L, _P, _P, _P] + [_I] * 6 + [_F, _F, _P],
-    ("moe_tc", "ri_moe_tc"): [_P, _L, _L, _P, _P, _L, _P, _P, _P] + [_I] * 7 + [_F, _F, _P, _P],
-    ("moe_tc", "ri_moe_gather"): [_P, _L, _P, _P, _P, _I, _I, _I, _P],
+    ("moe_tc", "ri_moe_tc"): [_P, _L, _I, _P, _L, _L, _P, _P, _L, _P, _P, _P] + [_I] * 7 + [_F, _F, _P, _P],
     ("moe", "ri_moe_combine"): [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     ("rope_kv", "ri_qk_norm_rope_append_pairs"): [_P] * 10 + [_F, _P, _I, _I] + [_I] * 10 + [_P, _P],
     ("latent_attention", "ri_latent_prep"): [_P, _L, _I, _I] + [_P] * 8 + [_F, _P] + [_I] * 12 + [_P, _P],
@@ -1516,11 +1515,7 @@ def moe_grouped_linear(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, ga
         raise KernelError(f"moe_grouped_linear: a plan with tiles of {bm} rows is for bfloat16 products, not {a.dtype}")
     y = torch.empty((rows_out, N), dtype=out_dtype, device=a.device)
     if bm == MOE_TILE_ROWS_WIDE:
-        if gather_div > 0:
-            a = _moe_gather(a, plan, rows_out, gather_div)
-        _call("moe_tc", "ri_moe_tc", a.data_ptr(), a.shape[0], a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
-              tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], E, N, K, 1 if scatter else 0,
-              1 if out_dtype == torch.float32 else 0, 0, 0.0, 0.0, error_flag(a.device).data_ptr(), _stream())
+        _moe_tc(a, w, y, plan, N, gather_div, 1 if scatter else 0, 1 if out_dtype == torch.float32 else 0, 0, 0.0, 0.0)
         return y
     _call("moe", "ri_moe_grouped_linear", a.data_ptr(), a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
           tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], int(bm), N, K, int(gather_div), 1 if scatter else 0,
@@ -1528,14 +1523,19 @@ def moe_grouped_linear(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, ga
     return y
 
 
-def _moe_gather(x: torch.Tensor, plan, pairs: int, div: int) -> torch.Tensor:
-    """[pairs, K]: row r is x[perm[r] // div] for the plan's rows (bfloat16 rows of whole 16-byte pieces)."""
-    perm, _, meta, _ = plan
-    _need(x, "x", torch.bfloat16)
-    out = torch.empty((pairs, x.shape[1]), dtype=x.dtype, device=x.device)
-    _call("moe_tc", "ri_moe_gather", x.data_ptr(), x.stride(0), out.data_ptr(), perm.data_ptr(), meta.data_ptr(), perm.numel(), int(div),
-          x.shape[1], _stream())
-    return out
+def _moe_tc(a: torch.Tensor, w: torch.Tensor, y: torch.Tensor, plan, N: int, gather_div: int, scatter: int, out_f32: int, gate: int,
+            limit: float, alpha: float) -> None:
+    """The tcgen05 products of a plan of wide tiles into ``y`` (a row per row of the plan); ``gather_div`` > 0: the rows a[perm[r] //
+    gather_div] are brought into the plan's order first."""
+    perm, tiles, meta, _ = plan
+    x, ldx, K = None, 0, a.shape[1]
+    if gather_div > 0:
+        x, ldx = a.data_ptr(), a.stride(0)
+        a = torch.empty((y.shape[0], K), dtype=a.dtype, device=a.device)
+        add_launches(1)
+    _call("moe_tc", "ri_moe_tc", x, ldx, int(gather_div), a.data_ptr(), a.shape[0], a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
+          tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], w.shape[0], N, K, scatter, out_f32, gate, float(limit), float(alpha),
+          error_flag(y.device).data_ptr(), _stream())
 
 
 def moe_grouped_gated(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, kind: str, limit: float = 0.0, alpha: float = 1.0,
@@ -1561,12 +1561,8 @@ def moe_grouped_gated(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, kin
               tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], int(bm), N, K, int(gather_div), GATES[kind] + 1, float(limit),
               float(alpha), _stream())
         return y
-    if gather_div > 0:
-        a = _moe_gather(a, plan, rows_out, gather_div)
     y = torch.empty((rows_out, N), dtype=a.dtype, device=a.device)
-    _call("moe_tc", "ri_moe_tc", a.data_ptr(), a.shape[0], a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
-          tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], E, N, K, 0, 0, GATES[kind] + 1, float(limit),
-          float(alpha), error_flag(a.device).data_ptr(), _stream())
+    _moe_tc(a, w, y, plan, N, gather_div, 0, 0, GATES[kind] + 1, limit, alpha)
     return y
 
 

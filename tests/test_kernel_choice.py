@@ -39,7 +39,8 @@ def test_plans_of_wide_tiles_are_for_bfloat16(launches, dtype, gather):
     a, w = a.bfloat16(), w.bfloat16()
     ops.moe_grouped_linear(a, w, plan, 8, gather_div=gather)
     ops.moe_grouped_gated(a, w, plan, 8, "silu", gather_div=gather)
-    assert [fn for _, fn, _ in launches] == (["ri_moe_gather"] if gather else []) + ["ri_moe_tc"] + (["ri_moe_gather"] if gather else []) + ["ri_moe_tc"]
+    assert [fn for _, fn, _ in launches] == ["ri_moe_tc", "ri_moe_tc"]
+    assert all((sent[0] is not None) == (gather > 0) and sent[2] == gather for _, _, sent in launches)
 
 
 # latent rows (keys of 256 elements whose first ones are the values): what the tcgen05 kernel does not do stays with the mma.sync kernel
