@@ -381,7 +381,8 @@ extern "C" int ri_moe_route_rule(const void* x, const float* router, const float
     RI_REQUIRE(N <= 4096, "moe_route: %d router outputs (up to 4096 are built)", N);
     const size_t smem = (size_t)MOE_ROUTE_WARPS * (2 * N + groups) * sizeof(float);
     const dim3 grid((tokens + MOE_ROUTE_WARPS - 1) / MOE_ROUTE_WARPS);
-    // (which form runs depends on the sizes and addresses only, never on the batch)
+    // (which form runs depends on sizes, the number of tokens among them, and addresses; the forms for rows of whole 16-byte
+    // pieces give the same bits)
     const int vec = (D % 4 == 0 && (((uintptr_t)router | (uintptr_t)x) & 15) == 0) ? 1 : 0;
     cudaError_t e = cudaSuccess;
     const long long items = (long long)N * ((D + 127) / 128);
@@ -617,14 +618,15 @@ moe_grouped_f32_kernel(const float* __restrict__ a, long long lda, const float* 
 }
 
 // bfloat16: 4 warps; warp w owns columns 16 w .. 16 w + 15 of the tile and all 32 rows (2 x 2 mma tiles per k16).
-// VEC (K a multiple of 8, 16-byte aligned rows): the tiles of A and W come by cp.async through a ring of MOE_STAGES
-// stages of 64 k each, so that two stages are on their way while one is multiplied; otherwise element by element.
-// Four stages: a few tokens are bound by reading the experts' matrices, and four blocks an SM have 96 KB of them on their way
-// (8 tokens of 4 choices, 16 experts of 1,376 channels and width 4,096, 338 + 172 MB: with three stages 77 and 45 us
-// and 5 us for the gate's own kernel; the layer's decode step 150.7 -> 138.7 us).
+// VEC (K a multiple of 8, 16-byte aligned rows): the tiles of A and W come by cp.async through a ring of STAGES
+// stages of 64 k each, so that all others are on their way while one is multiplied; otherwise element by element.
+// STAGES: four where all blocks find a place at once with four on an SM (56 KB each: 96 KB of the experts' matrices on their way),
+// three where five on an SM save a round of blocks (`moe_stages`).  A few tokens are bound by reading those matrices.  First product with
+// the gate, four / three stages: 24 tokens of one choice, 8 experts of 1,376 channels and width 4,096 (344 blocks) 53 / 56 us; 24 tokens of four
+// choices, 16 experts (688 blocks, two rounds of four an SM, one of five) 92 / 76 us, 32 experts of 704 and width 2,048 alike; second
+// product (1,024 blocks, two rounds either way) 41.4 / 44.4 us.
 // GATED: W [E, 2 N, K] holds an expert's gate rows, then its up rows; a tile takes 32 channels, the gate rows as its columns
 // 0 .. 31 and the up rows as 32 .. 63, and the epilogue puts the two float32 sums of a channel together.
-#define MOE_STAGES 4
 #define MOE_BK 64
 #define MOE_PITCH (MOE_BK + 8)
 #define MOE_SMEM(stages) ((stages) * (MOE_BM + MOE_BN) * MOE_PITCH * 2)
@@ -641,12 +643,12 @@ __device__ __forceinline__ float moe_gate(float g, float u, const MoeGate& c) {
     if (c.kind == 2) return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
     return g / (1.0f + expf(-g)) * u;
 }
-template <typename TO, bool VEC, bool GATED>
+template <typename TO, bool VEC, bool GATED, int STAGES>
 __global__ void __launch_bounds__(128)
 moe_grouped_bf16_kernel(const bf16* __restrict__ a, long long lda, const bf16* __restrict__ w, TO* __restrict__ y,
                         long long ldy, const int* __restrict__ perm, const int* __restrict__ tiles,
                         const int* __restrict__ meta, int N, int K, int gather_div, int scatter, MoeGate gate) {
-    constexpr int ST = VEC ? MOE_STAGES : 1;
+    constexpr int ST = VEC ? STAGES : 1;
     extern __shared__ __align__(16) unsigned char moe_grouped_sm[];
     bf16 (*As)[MOE_BM][MOE_PITCH] = reinterpret_cast<bf16 (*)[MOE_BM][MOE_PITCH]>(moe_grouped_sm);
     bf16 (*Ws)[MOE_BN][MOE_PITCH] = reinterpret_cast<bf16 (*)[MOE_BN][MOE_PITCH]>(moe_grouped_sm + ST * MOE_BM * MOE_PITCH * 2);
@@ -712,17 +714,17 @@ moe_grouped_bf16_kernel(const bf16* __restrict__ a, long long lda, const bf16* _
     };
     const int nk = (K + MOE_BK - 1) / MOE_BK;
     if (VEC) {
-        for (int st = 0; st < MOE_STAGES - 1; st++) {
+        for (int st = 0; st < STAGES - 1; st++) {
             if (st < nk) copy_stage(st, st * MOE_BK);
             cp_async_commit();
         }
         for (int it = 0; it < nk; it++) {
-            cp_async_wait<MOE_STAGES - 2>();
+            cp_async_wait<STAGES - 2>();
             __syncthreads();                         // stage `it` has landed for everyone; the stage of it - 1 is free
-            const int ahead = it + MOE_STAGES - 1;
-            if (ahead < nk) copy_stage(ahead % MOE_STAGES, ahead * MOE_BK);
+            const int ahead = it + STAGES - 1;
+            if (ahead < nk) copy_stage(ahead % STAGES, ahead * MOE_BK);
             cp_async_commit();
-            multiply(it % MOE_STAGES);
+            multiply(it % STAGES);
         }
         cp_async_wait<0>();
     } else {
@@ -771,23 +773,43 @@ moe_grouped_bf16_kernel(const bf16* __restrict__ a, long long lda, const bf16* _
             }
 }
 
-template <typename TO, bool VEC, bool GATED>
-static int moe_grouped_go(dim3 grid, cudaStream_t stream, const void* a, long long lda, const void* w, void* y, long long ldy,
-                          const int* perm, const int* tiles, const int* meta, int N, int K, int gather_div, int scatter, MoeGate gate) {
-    constexpr int sm = MOE_SMEM(VEC ? MOE_STAGES : 1);
+// rounds of blocks that the SMs take with four (four stages) and five (three stages) on each
+static int moe_stages(long long blocks) {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        sms = n > 0 ? n : 148;
+    }
+    return (blocks + 5 * sms - 1) / (5 * sms) < (blocks + 4 * sms - 1) / (4 * sms) ? 3 : 4;
+}
+template <typename TO, bool VEC, bool GATED, int STAGES>
+static int moe_grouped_launch(dim3 grid, cudaStream_t stream, const void* a, long long lda, const void* w, void* y, long long ldy,
+                              const int* perm, const int* tiles, const int* meta, int N, int K, int gather_div, int scatter, MoeGate gate) {
+    constexpr int sm = MOE_SMEM(VEC ? STAGES : 1);
     if (sm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(moe_grouped_bf16_kernel<TO, VEC, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        cudaError_t e = cudaFuncSetAttribute(moe_grouped_bf16_kernel<TO, VEC, GATED, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
         if (e != cudaSuccess) RI_FAIL((int)e, "moe_grouped: %s", cudaGetErrorString(e));
     }
-    ri_launch_pdl(moe_grouped_bf16_kernel<TO, VEC, GATED>, grid, dim3(128), (size_t)sm, stream, (const bf16*)a, lda, (const bf16*)w,
+    ri_launch_pdl(moe_grouped_bf16_kernel<TO, VEC, GATED, STAGES>, grid, dim3(128), (size_t)sm, stream, (const bf16*)a, lda, (const bf16*)w,
                   (TO*)y, ldy, perm, tiles, meta, N, K, gather_div, scatter, gate);
     return 0;
 }
+// likely: the tiles that a step of so many pairs has as a rule (the grid covers the most it can have)
+template <typename TO, bool VEC, bool GATED>
+static int moe_grouped_go(dim3 grid, int likely, cudaStream_t stream, const void* a, long long lda, const void* w, void* y, long long ldy,
+                          const int* perm, const int* tiles, const int* meta, int N, int K, int gather_div, int scatter, MoeGate gate) {
+    if (VEC && moe_stages((long long)likely * grid.y) == 3)
+        return moe_grouped_launch<TO, VEC, GATED, 3>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, gate);
+    return moe_grouped_launch<TO, VEC, GATED, 4>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, gate);
+}
 
 // a [rows, lda] and w [E, N, K] in the compute type; y [.., ldy] float32 (out_f32) or the compute type
-// bm: the tile height that the plan was made with (plans with tiles of MOE_BM_WIDE rows are for moe_tc.cu)
+// bm: the tile height that the plan was made with (plans with tiles of MOE_BM_WIDE rows are for moe_tc.cu); likely: how many of the
+// max_tiles tiles the step has as a rule (it chooses between forms with the same results)
 extern "C" int ri_moe_grouped_linear(const void* a, long long lda, const void* w, void* y, long long ldy, const int* perm,
-                                     const int* tiles, const int* meta, int max_tiles, int bm, int N, int K, int gather_div,
+                                     const int* tiles, const int* meta, int max_tiles, int likely, int bm, int N, int K, int gather_div,
                                      int scatter, int out_f32, int dtype, cudaStream_t stream) {
     if (max_tiles == 0) return 0;
     RI_REQUIRE(bm == MOE_BM, "moe_grouped_linear: tiles of %d rows", bm);
@@ -801,10 +823,10 @@ extern "C" int ri_moe_grouped_linear(const void* a, long long lda, const void* w
     } else if (dtype == RI_DTYPE_BF16) {
         const bool vec = K % 8 == 0 && lda % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
         const MoeGate none{0, 0.0f, 0.0f};
-        int rc = out_f32 ? (vec ? moe_grouped_go<float, true, false>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none)
-                                : moe_grouped_go<float, false, false>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none))
-                         : (vec ? moe_grouped_go<bf16, true, false>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none)
-                                : moe_grouped_go<bf16, false, false>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none));
+        int rc = out_f32 ? (vec ? moe_grouped_go<float, true, false>(grid, likely, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none)
+                                : moe_grouped_go<float, false, false>(grid, likely, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none))
+                         : (vec ? moe_grouped_go<bf16, true, false>(grid, likely, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none)
+                                : moe_grouped_go<bf16, false, false>(grid, likely, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, scatter, none));
         if (rc) return rc;
     } else RI_FAIL(-1, "moe_grouped_linear: unknown dtype %d", dtype);
     RI_CHECK_LAUNCH("moe_grouped_linear");
@@ -814,7 +836,7 @@ extern "C" int ri_moe_grouped_linear(const void* a, long long lda, const void* w
 // bfloat16: w [E, 2 N, K] (an expert's gate rows, then its up rows), y [.., ldy] = f(gate) * up' with gate function 1 silu, 2
 // gelu_tanh, 3 the clamped swish with `limit` and `alpha`
 extern "C" int ri_moe_grouped_gated(const void* a, long long lda, const void* w, void* y, long long ldy, const int* perm,
-                                    const int* tiles, const int* meta, int max_tiles, int bm, int N, int K, int gather_div,
+                                    const int* tiles, const int* meta, int max_tiles, int likely, int bm, int N, int K, int gather_div,
                                     int gate, float limit, float alpha, cudaStream_t stream) {
     if (max_tiles == 0) return 0;
     RI_REQUIRE(bm == MOE_BM, "moe_grouped_gated: tiles of %d rows", bm);
@@ -823,8 +845,8 @@ extern "C" int ri_moe_grouped_gated(const void* a, long long lda, const void* w,
     RI_REQUIRE(grid.y <= 65535, "moe_grouped_gated: %d channels are too many for one launch", N);
     const bool vec = K % 8 == 0 && lda % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
     const MoeGate g{gate, limit, alpha};
-    int rc = vec ? moe_grouped_go<bf16, true, true>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, 0, g)
-                 : moe_grouped_go<bf16, false, true>(grid, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, 0, g);
+    int rc = vec ? moe_grouped_go<bf16, true, true>(grid, likely, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, 0, g)
+                 : moe_grouped_go<bf16, false, true>(grid, likely, stream, a, lda, w, y, ldy, perm, tiles, meta, N, K, gather_div, 0, g);
     if (rc) return rc;
     RI_CHECK_LAUNCH("moe_grouped_gated");
     return 0;

@@ -45,8 +45,8 @@ _SIGNATURES = {
     ("elementwise", "ri_scale_f32"): [_P, _L, _F, _P],
     ("moe", "ri_moe_route"): [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     ("moe", "ri_moe_plan"): [_P, _P, _P, _P, _I, _I, _I, _I, _P],
-    ("moe", "ri_moe_grouped_linear"): [_P, _L, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
-    ("moe", "ri_moe_grouped_gated"): [_P, _L, _P, _P, _L, _P, _P, _P] + [_I] * 6 + [_F, _F, _P],
+    ("moe", "ri_moe_grouped_linear"): [_P, _L, _P, _P, _L, _P, _P, _P] + [_I] * 9 + [_P],
+    ("moe", "ri_moe_grouped_gated"): [_P, _L, _P, _P, _L, _P, _P, _P] + [_I] * 7 + [_F, _F, _P],
     ("moe_tc", "ri_moe_tc"): [_P, _L, _I, _P, _L, _L, _P, _P, _L, _P, _P, _P] + [_I] * 7 + [_F, _F, _P, _P],
     ("moe", "ri_moe_combine"): [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     ("rope_kv", "ri_qk_norm_rope_append_pairs"): [_P] * 10 + [_F, _P, _I, _I] + [_I] * 10 + [_P, _P],
@@ -1518,9 +1518,14 @@ def moe_grouped_linear(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, ga
         _moe_tc(a, w, y, plan, N, gather_div, 1 if scatter else 0, 1 if out_dtype == torch.float32 else 0, 0, 0.0, 0.0)
         return y
     _call("moe", "ri_moe_grouped_linear", a.data_ptr(), a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
-          tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], int(bm), N, K, int(gather_div), 1 if scatter else 0,
+          tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], _likely_tiles(perm.numel(), E, bm), int(bm), N, K, int(gather_div), 1 if scatter else 0,
           1 if out_dtype == torch.float32 else 0, _code(a.dtype), _stream())
     return y
+
+
+def _likely_tiles(pairs: int, experts: int, bm: int) -> int:
+    """The tiles of a plan whose pairs are spread evenly over the experts."""
+    return min(pairs, experts * -(-pairs // (experts * bm)))
 
 
 def _moe_tc(a: torch.Tensor, w: torch.Tensor, y: torch.Tensor, plan, N: int, gather_div: int, scatter: int, out_f32: int, gate: int,
@@ -1558,7 +1563,7 @@ def moe_grouped_gated(a: torch.Tensor, w: torch.Tensor, plan, rows_out: int, kin
     if bm != MOE_TILE_ROWS_WIDE:
         y = torch.empty((rows_out, N), dtype=a.dtype, device=a.device)
         _call("moe", "ri_moe_grouped_gated", a.data_ptr(), a.stride(0), w.data_ptr(), y.data_ptr(), N, perm.data_ptr(),
-              tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], int(bm), N, K, int(gather_div), GATES[kind] + 1, float(limit),
+              tiles.data_ptr(), meta.data_ptr(), tiles.shape[0], _likely_tiles(perm.numel(), E, bm), int(bm), N, K, int(gather_div), GATES[kind] + 1, float(limit),
               float(alpha), _stream())
         return y
     y = torch.empty((rows_out, N), dtype=a.dtype, device=a.device)
