@@ -550,17 +550,19 @@ __global__ void sp_select_end_kernel(SpArgs a, int mode, int rows) {
 // them hold the same floor, prefix and remaining weight in registers and nobody waits for a leader.  The row's
 // histogram has three copies that take turns: while a pass adds to one, the blocks clear the next, and the one
 // before may still be read by a block that is late.  Sums are the same integers as in the other forms, so the
-// token is the same bit for bit.  Every wait is bounded by time (error 5, and the block returns).
+// token is the same; only in rows with three or more NaN, or three or more +inf, whose weights of 2^63 make the sums wrap
+// around, the forms may choose differently.  Every wait is bounded by time (error 5, and the block returns).
 //
 // A pass over the vocabulary costs about five trips to the L2 cache and a barrier, 6 to 8 us, and a search over five digits
 // has five of them; so only the top digit is searched that way.  What it leaves, the tokens of one bin (a top-k: of that bin
 // and those above it, all that the rest of the work can choose from), goes into a list of 2,048 keys in memory, from which a
 // block ends the search by itself, the same digits and sums over eight keys a thread (the L1 cache has them).  Three barriers with a top-k or a plain
-// draw, four with a top-p, where each search had five and each total one.  A list that does not fit (flat rows, a top-k of
-// thousands) leaves the lower digits to passes over the vocabulary as before.  8 rows of 151,936 logits, top-k 50 and top-p
-// 0.9: 37 us, where a barrier for every digit took 145.
+// draw, four with a top-p, where each search had five and each total one.  A list that does not fit leaves the lower digits to
+// passes over the vocabulary as before: flat rows, a top-k of thousands, and what falls into a crowded bin, since the first
+// digit has no more than the sign and seven bits of the exponent.  8 rows of 151,936 logits, top-k 50 and top-p 0.9,
+// temperature 0.7: spread 2.5 (1,916 keys) 37 us, where a barrier for every digit took 145; spread 3 (4,646 keys) 146.
 //
-// Scratch memory per row (SpFusedRow): zero at the start for `arrive` and `totals`: the launcher clears them.
+// Scratch memory per row (SpFusedRow): all zero at the start, the launcher clears it.
 // ---------------------------------------------------------------------------
 #define SPF_TOTALS 4
 #define SPF_TOP ((SP_PASSES - 1) * SP_DIGIT)     // the shift of a key's top digit

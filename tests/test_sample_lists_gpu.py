@@ -1,5 +1,5 @@
 """The one-kernel sampler ends a search over a list of at most 2,048 keys: the same tokens, bit for bit, as the form that passes
-over the vocabulary for every digit (whole-number sums, so there is nothing to tolerate).  Rows without NaN and +inf: their
+over the vocabulary for every digit (whole-number sums, so there is nothing to tolerate).  Rows with three or more NaN or +inf are left out: their
 weights make the sums wrap around, which the two forms do not do alike."""
 import pytest
 import torch
@@ -47,3 +47,23 @@ def test_lists_choose_what_the_passes_choose(kind, rows, vocab, monkeypatch):
             monkeypatch.setattr(ops, "SAMPLE_ONE_KERNEL", False)
             want = ops.sample(logits, temperature, u, top_k=k, top_p=p)
             assert torch.equal(got, want), (shift, k is not None, p is not None)
+
+
+@pytest.mark.parametrize("nans, infs", [(1, 0), (2, 0), (0, 1), (0, 2), (2, 1)])
+def test_one_or_two_values_that_are_not_finite(nans, infs, monkeypatch):
+    """Their weights are 2^63: sums of up to two of them are the same in both forms (from three on they are not)."""
+    rows, vocab = 16, 50257
+    g = torch.Generator(device="cuda").manual_seed(10 * nans + infs)
+    logits = torch.randn((rows, vocab), generator=g, device="cuda") * 2.5
+    for row in logits:
+        at = torch.randperm(vocab, generator=g, device="cuda")
+        row[at[:nans]] = float("nan")
+        row[at[nans:nans + infs]] = float("inf")
+    temperature, u = torch.full((rows,), 0.7, device="cuda"), torch.rand(rows, generator=g, device="cuda")
+    for k, p in ((0, 1.0), (50, 1.0), (0, 0.9), (50, 0.9), (3000, 0.9)):
+        top_k, top_p = torch.full((rows,), k, dtype=torch.int32, device="cuda"), torch.full((rows,), p, device="cuda")
+        got = []
+        for one in (True, False):
+            monkeypatch.setattr(ops, "SAMPLE_ONE_KERNEL", one)
+            got.append(ops.sample(logits, temperature, u, top_k=top_k, top_p=top_p, uses_top_k=k > 0, uses_top_p=p < 1.0))
+        assert torch.equal(*got), (k, p)
