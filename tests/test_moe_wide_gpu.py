@@ -139,3 +139,27 @@ def test_combination_in_groups_of_four(tokens, D, top, extra, dtype):
         want = want + more.double() if extra else want
         tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6
         assert ((got.double() - want).abs() <= tol * want.abs() + (top + 1) * 2.0 ** -22).all()
+
+
+# tiles of 32 rows whose blocks need fewer rounds with three stages of the ring (16 x 43 blocks on 148 SMs), and one that has four; k in
+# whole stages, with a rest, less than the ring
+@pytest.mark.parametrize("E, N", [(16, 1376), (4, 64)])
+@pytest.mark.parametrize("K", [256, 200, 72])
+def test_few_tokens_in_rings_of_three_and_four_stages(E, N, K):
+    ops = _ops()
+    g = _gen(N + K)
+    tokens, top = 24, 2
+    x = torch.randn((tokens, K), generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn((E, 2 * N, K), generator=g, device=DEV) * 0.1).to(torch.bfloat16)
+    idx = torch.randint(0, E, (tokens, top), generator=g, device=DEV, dtype=torch.int32)
+    plan = ops.moe_plan(idx, E)
+    e, rows = idx.flatten().long(), tokens * top
+    want = torch.einsum("rk,rnk->rn", x.double().repeat_interleave(top, 0), w.double()[e])
+    got = ops.moe_grouped_linear(x, w, plan, rows, gather_div=top, scatter=True, out_dtype=torch.float32)
+    # float32 sums of K products, in any order: K 2^-24 of the magnitudes' sum
+    most = torch.einsum("rk,rnk->rn", x.double().abs().repeat_interleave(top, 0), w.double().abs()[e])
+    assert ((got.double() - want).abs() <= K * 2.0 ** -24 * most).all()
+    gated = ops.moe_grouped_gated(x, w, plan, rows, "silu", gather_div=top)
+    gate, up = want[plan[0].long()].chunk(2, dim=1)
+    want = gate * torch.sigmoid(gate) * up
+    assert ((gated.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
