@@ -512,15 +512,18 @@ static int gla_single_go(const void* proj, long long ld, int q_col, int k_col, i
 template <typename T, int DIMC, int GROUP, bool VEC>
 static int gla_walk_go(const void* proj, long long ld, int q_col, int k_col, int v_col, const void* z, const float* bias, float tau,
                        float qscale, const float* decay, float* state, float* o, const int* seq_slot, const int* seq_start, int seqs,
-                       int H, int dim, int vdim_in, const float* gates, int gate_pitch, int ones, cudaStream_t stream) {
+                       int H, int dim, int vdim_in, const float* gates, int gate_pitch, int ones, int sms, cudaStream_t stream) {
     constexpr int BCOLS = GLA_CT * 16 / DIMC, PER = (GROUP * (DIMC / 8) + GLA_ST - 1) / GLA_ST, PT = sizeof(T) / 2;
     constexpr size_t RAW = VEC ? (size_t)GLA_AHEAD * (PER * (2 * PT + 2) + PT) * GLA_ST * 16 : 0;      // the slots of pieces
-    constexpr size_t sm = (size_t)GLA_RING * GROUP * (3 * DIMC + 2 * BCOLS) * sizeof(float) + RAW;
+    constexpr size_t need = (size_t)GLA_RING * GROUP * (3 * DIMC + 2 * BCOLS) * sizeof(float) + RAW;
     const dim3 grid((vdim_in + ones + BCOLS - 1) / BCOLS, H, seqs);
-    if (sm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(gla_walk_kernel<T, DIMC, GROUP, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) RI_FAIL((int)e, "gla_recurrent: %s", cudaGetErrorString(e));
-    }
+    // No more blocks than SMs: more than half of an SM's shared memory for each, so that no two share one (behind a small product
+    // two had: 300 tokens of 32 heads of 64 x 128, the layer 151 -> 111 us)
+    constexpr size_t alone = 116 * 1024;
+    const size_t sm = need < alone && (long long)grid.x * H * seqs <= sms ? alone : need;
+    // (the same bound from every thread)
+    cudaError_t e = cudaFuncSetAttribute(gla_walk_kernel<T, DIMC, GROUP, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(need < alone ? alone : need));
+    if (e != cudaSuccess) RI_FAIL((int)e, "gla_recurrent: %s", cudaGetErrorString(e));
     // A prompt's kernel is launched the ordinary way, not as a dependent launch: its long-lived blocks must spread over the
     // SMs, and blocks that come in while the kernel before still holds most SMs pile up on the first that get free.
     gla_walk_kernel<T, DIMC, GROUP, VEC><<<grid, dim3(GLA_CT + GLA_ST), sm, stream>>>((const T*)proj, ld, q_col, k_col, v_col, (const T*)z,
@@ -614,7 +617,7 @@ static int gla_recurrent_go(const void* proj, long long ld, int q_col, int k_col
         const bool eight = dim > 64 && ((long long)((vdim + 15) / 16) * H * seqs > sms || tokens <= 16 * (long long)seqs);
 #define GLA_GO3(T, DIMC, GROUP, VEC)                                                                                           \
         return gla_walk_go<T, DIMC, GROUP, VEC>(proj, ld, q_col, k_col, v_col, z, bias, tau, qscale, decay, state, o, seq_slot, \
-                                                seq_start, seqs, H, dim, vdim_in, gates, gate_pitch, ones, stream)
+                                                seq_start, seqs, H, dim, vdim_in, gates, gate_pitch, ones, sms, stream)
 #define GLA_GO2(T, DIMC, GROUP)                                                                                                \
         do {                                                                                                                   \
             if (vec) GLA_GO3(T, DIMC, GROUP, true);                                                                            \
