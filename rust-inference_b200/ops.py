@@ -89,11 +89,12 @@ MAX_FAST_HEAD_DIM = 256
 LATENT_TC_ROW, LATENT_TC_VALUES = 256, 192
 # ... which masks a score before it is scaled: -FLT_MAX times the scale has to lie far below every score that counts
 LATENT_TC_SCALE = 1e-30
-# gated linear attention: up to so many tokens a step the recurrence's blocks take the decays themselves; with more tokens a kernel
-# takes them once for all blocks of a head.  On the device the two meet at some 64 tokens (us, 32 heads of 64 x 128: 2 tokens 3.9 / 5.4
-# with that kernel, 64 9.1 / 9.5, 128 15.8 / 15.3, 256 27.1 / 25.4; 16 heads of 128 x 64: 4.2 / 5.4, 11.2 / 10.5, 19.9 / 17.2, 36.4 / 29.5),
-# but its scratch and launch cost the host 5 us (22.4 against 17.4 a call), and a prompt of so few tokens waits for the host
-GLA_OWN_DECAYS = 128
+# gated linear attention: up to so many decays a step (tokens x key channels of all heads) the recurrence's blocks take them themselves;
+# with more a kernel takes them once for all blocks of a head.  On the device the two meet earlier (us, 32 heads of 64 x 128: 64 tokens 9.1 / 9.5
+# with that kernel, 256 27.0 / 25.5; 16 heads of 128 x 64 11.2 / 10.5, 35.7 / 29.5), but its scratch and launch cost the host 5 us, and a
+# prompt of so few tokens waits for the host (the layer: 32 heads of 64 x 128, 350 tokens 112 / 117, 512 136 / 133; 32 of 128 x 128, 150
+# tokens 110 / 115, 200 120 / 115.5)
+GLA_OWN_DECAYS = 5 << 17
 TCGEN05_HEAD_DIMS = (64, 128)   # head sizes the tcgen05 prefill attention kernel is built for
 _NO_TCGEN05 = os.environ.get("RUST_INFERENCE_B200_NO_TCGEN05") == "1"   # for comparisons
 # the skinny linear applies the SiLU gate in its epilogue (one kernel less per layer: 2 % faster at batch 1 of
@@ -429,7 +430,8 @@ def gla_recurrent(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, z: tor
     o = torch.empty((tokens, heads, vdim), dtype=torch.float32, device=proj.device)
     alone = single and tokens == seqs
     # the decays of a prompt's tokens, which every block of a head reads
-    decay = None if alone or dim > 128 or tokens <= GLA_OWN_DECAYS else torch.empty((tokens, heads * dim), dtype=torch.float32, device=proj.device)
+    own = alone or dim > 128 or tokens * heads * dim <= GLA_OWN_DECAYS
+    decay = None if own else torch.empty((tokens, heads * dim), dtype=torch.float32, device=proj.device)
     _call("gla", "ri_gla_recurrent", proj.data_ptr(), ld, int(q_col), int(k_col), int(v_col), z.data_ptr(), bias.data_ptr(),
           float(tau), float(qscale), _ptr(decay), state.data_ptr(), o.data_ptr(), seq_slot.data_ptr(), seq_start.data_ptr(), tokens,
           seqs, heads, dim, vdim, 1 if alone else 0, _code(proj.dtype), _stream())

@@ -102,15 +102,18 @@ def test_an_infinite_last_value_is_infinite_in_every_cutting(dim, vdim, ones, dt
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("ones", [False, True])
 @pytest.mark.parametrize("dim, vdim, pad", [(64, 128, 0), (128, 64, 8), (48, 32, 0), (128, 128, 0), (96, 33, 0), (64, 64, 3), (20, 8, 0)])
-def test_gla_prompts_pieces_and_single_tokens(dim, vdim, pad, ones, dtype):
+def test_gla_prompts_pieces_and_single_tokens(dim, vdim, pad, ones, dtype, monkeypatch):
     gla = Gla([47, 200, 1, 48, 65], 2, dim, vdim, dtype, ones, pad)
     outs, state = gla.walk([])
     want, want_state = gla.exact()
     for got, exact in zip(outs + [state], want + [want_state]):
         # float32 sums of up to 200 tokens and 128 channels, decays from float32 exponentials: some 1e-6 of the largest
         assert (got.double() - exact).abs().max() <= 2e-5 * exact.abs().max()
-    for cuts in ([3, 19, 20, 51, 52, 130], list(range(1, 66)) + [80]):
+    for cuts in ([], [3, 19, 20, 51, 52, 130], list(range(1, 66)) + [80]):
+        if not cuts:                                        # the decays by a kernel of their own
+            monkeypatch.setattr(ops, "GLA_OWN_DECAYS", 0)
         pieces, state1 = gla.walk(cuts)
+        monkeypatch.undo()
         assert all(torch.equal(a, b) for a, b in zip(pieces, outs)) and torch.equal(state, state1)
 
 
