@@ -32,7 +32,7 @@ SOURCES: Dict[str, Tuple[str, ...]] = {
     "elementwise": ("elementwise.cu", "common.cuh", "linear_skinny_geometry.cuh"),
     "rope_kv": ("rope_kv.cu", "common.cuh"),
     "attention_rows": ("attention_rows.cu", "common.cuh", "distance_bias.cuh"),
-    "linear_f32": ("linear_f32.cu", "common.cuh"),
+    "linear_f32": ("linear_f32.cu", "linear_f32_tc.cuh", "common.cuh", "mma_helpers.cuh", "tcgen05_helpers.cuh"),
     "streams": ("streams.cu", "common.cuh"),
     "norm_gains": ("norm_gains.cu", "common.cuh", "linear_skinny_geometry.cuh"),
     "dyn_tanh": ("dyn_tanh.cu", "common.cuh", "linear_skinny_geometry.cuh"),

@@ -1,9 +1,13 @@
-// y[M, N] = x[M, K] . W[N, K]^T in true float32 (FMA on the CUDA cores, no tensor
-// cores, no reduced-precision mode).  Every output element is the sum over
-// k = 0..K-1 in that order with one accumulator, whatever M, N and the tile a
-// row falls into: a token's result does not depend on what it is batched with.
+// y[M, N] = x[M, K] . W[N, K]^T in true float32, in two forms that K and W alone decide between.
+// `ri_linear_f32`, `ri_linear_heads_f32`: multiply-adds on the CUDA cores.  Every output element is the sum over
+// k = 0..K-1 in that order with one accumulator, whatever M, N and the tile a row falls into: a token's result does not
+// depend on what it is batched with.
+// `ri_linear_f32_tc`: exact cuts of the float32 values into bfloat16 on the tensor cores (linear_f32_tc.cuh), likewise one chain per
+// output whatever M, N and the tile.
 // Formula: thanhauco/rust-inference src/ops/linear.rs:7-20.
 #include "common.cuh"
+#include "linear_f32_tc.cuh"
+#include <cuda.h>
 
 #define LF_BK 16
 #define LF_THREADS 256
@@ -172,4 +176,110 @@ extern "C" int ri_linear_heads_f32(const float* x, const float* w, float* y, int
     RI_REQUIRE((M + 63) / 64 <= 65535 && heads <= 65535, "linear_heads_f32: too many rows or heads (%d, %d)", M, heads);
     int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && (x_head % 4 == 0) && (((uintptr_t)x | (uintptr_t)w) % 16 == 0);
     return lf_launch(x, w, y, M, N, K, heads, vec_ok, ldx, ldy, x_head, (long long)N * K, y_head, stream);
+}
+
+// ---- the tensor cores' form ------------------------------------------------------------------------------------------------
+typedef CUresult (*lt_encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                       const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                       CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+template <int CH, int GROUPS, int BUFS>
+static int lt_launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const float* x, const float* w, float* y, int M, int N, int K,
+                     int tn, int* err, cudaStream_t stream) {
+    auto kernel = linear_f32_tc_kernel<CH, GROUPS, BUFS>;
+    const int stage = LT_W_BYTES + 3 * 64 * tn;
+    int stages = LT_SMEM_MAX / stage, wstages = (512 - BUFS * tn) / LT_W_COLS;
+    if (stages > LT_MAX_STAGES) stages = LT_MAX_STAGES;
+    if (wstages > LT_MAX_WSTAGES) wstages = LT_MAX_WSTAGES;
+    // A wait knows a barrier's phases by their parity only, so that whoever waits must know the phase before to be over.  A place of the
+    // first ring is always the same group's, which has waited for it there; copies into the place of stage s start when the
+    // products up to s - stages are done, so that the second ring's phase before last is over if it has half as many places.
+    stages -= stages % GROUPS;
+    RI_REQUIRE(tn <= 32 * CH && stages >= GROUPS && wstages >= GROUPS && 2 * wstages >= stages, "linear_f32_tc: %d tokens a block", tn);
+    if (CH == 6) {                                 // its warps hand registers over: the sum has to be what they are launched with
+        static int regs = 0;
+        if (!regs) {
+            cudaFuncAttributes attr;
+            cudaError_t e = cudaFuncGetAttributes(&attr, (const void*)kernel);
+            if (e != cudaSuccess) RI_FAIL((int)e, "linear_f32_tc: %s", cudaGetErrorString(e));
+            regs = attr.numRegs;
+        }
+        RI_REQUIRE(regs == 128, "linear_f32_tc: built with %d registers a thread", regs);
+    }
+    cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM_MAX);
+    if (e != cudaSuccess) RI_FAIL((int)e, "linear_f32_tc: %s", cudaGetErrorString(e));
+    ri_launch_pdl(kernel, dim3((N + LT_ROWS - 1) / LT_ROWS, (M + tn - 1) / tn), dim3(128 * GROUPS + LT_SUMS), (size_t)stages * stage, stream,
+                  map_w, map_x, x, w, y, M, N, K, tn, stages, wstages, (long long)K, (long long)N, err);
+    RI_CHECK_LAUNCH("linear_f32_tc");
+    return 0;
+}
+
+// `parts`: scratch for the cut rows of x, 6 bytes for each of K rounded up to 32 and each of `part_rows` rows; more rows than that are
+// taken in several launches.  K a multiple of 4, x and w on 16 bytes.
+//
+// Tokens a block: the multiple of 16 with the least time, rounds of blocks (one an SM) times what a round takes.  Measured in us at K =
+// 4,096 with the cut of x: 16 tokens 60, 48 70, 96 85, 128 91, 176 107, that is some 57 + 0.285 a token; two rounds of 128 tokens 165, four of
+// 176 445.  At that K, the tensor cores' form / multiply-adds: 512 tokens and 6,144 outputs 114 / 640, 512 and 4,096 93 / 454, 300 and 6,144 90
+// / 454, 128 and 6,144 73 / 269, 16 and 6,144 61 / 190, 1 and 4,096 60 / 190; K = 2,048, 300 and 4,096 48 / 184.  2-norm of the error against float64
+// over that of the result: 2.3e-7 / 1.15e-6 at K = 4,096, 1.3e-7 / 4.0e-7 at 512, 1.2e-7 / 2.5e-7 at 200.
+extern "C" int ri_linear_f32_tc(const float* x, const float* w, float* y, void* parts, int part_rows, int M, int N, int K, int* err_flag,
+                                cudaStream_t stream) {
+    if (M == 0 || N == 0) return 0;
+    RI_REQUIRE(M > 0 && N > 0 && K > 0 && part_rows > 0, "linear_f32_tc: bad sizes M=%d N=%d K=%d", M, N, K);
+    RI_REQUIRE(K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)parts) & 15) == 0, "linear_f32_tc: rows of whole 16-byte pieces are needed");
+    static lt_encode_tiled_fn encode = nullptr;
+    static int sms = 0;
+    if (!sms) {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult res;
+        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &res);
+        if (e != cudaSuccess || res != cudaDriverEntryPointSuccess || !fn) RI_FAIL(-1, "linear_f32_tc: the driver has no cuTensorMapEncodeTiled");
+        encode = (lt_encode_tiled_fn)fn;
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        sms = n > 0 ? n : 148;
+    }
+    const int Kp = (K + LT_K - 1) / LT_K * LT_K;
+    const cuuint32_t one[3] = {1, 1, 1};
+    CUtensorMap map_w;
+    {
+        cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N}, strides[1] = {(cuuint64_t)K * 4};
+        cuuint32_t box[2] = {LT_K, LT_ROWS};
+        CUresult r = encode(&map_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(w), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) RI_FAIL(-1, "linear_f32_tc: cuTensorMapEncodeTiled failed with %d (N=%d, K=%d)", (int)r, N, K);
+    }
+    for (int at = 0; at < M; at += part_rows) {
+        const int rows = M - at < part_rows ? M - at : part_rows;
+        int tn = 16;
+        double least = 0;
+        for (int t = 16; t <= LT_MAX_TOKENS; t += 16) {
+            const long long blocks = (long long)((N + LT_ROWS - 1) / LT_ROWS) * ((rows + t - 1) / t);
+            const double time = (double)((blocks + sms - 1) / sms) * (57 + 0.285 * t);
+            if (t == 16 || time < least) {
+                tn = t;
+                least = time;
+            }
+        }
+        RI_REQUIRE((rows + tn - 1) / tn <= 65535, "linear_f32_tc: too many rows (%d)", M);
+        CUtensorMap map_x;
+        cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, 3}, strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * 2 * rows};
+        cuuint32_t box[3] = {LT_K, (cuuint32_t)tn, 3};
+        CUresult r = encode(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, parts, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) RI_FAIL(-1, "linear_f32_tc: cuTensorMapEncodeTiled failed with %d (M=%d, K=%d)", (int)r, rows, K);
+        const float* xs = x + (size_t)at * K;
+        float* ys = y + (size_t)at * N;
+        const long long pieces = (long long)rows * (Kp / 8);
+        RI_REQUIRE((pieces + 255) / 256 < (1ll << 31), "linear_f32_tc: too many rows (%d)", M);
+        ri_launch_pdl(linear_f32_cut_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, stream, xs, (uint4*)parts, rows, K, Kp / 8);
+        RI_CHECK_LAUNCH("linear_f32_cut");
+        int rc;
+        if (tn <= 64) rc = lt_launch<2, 4, 4>(map_w, map_x, xs, w, ys, rows, N, K, tn, err_flag, stream);
+        else if (tn <= 128) rc = lt_launch<4, 2, 2>(map_w, map_x, xs, w, ys, rows, N, K, tn, err_flag, stream);
+        else rc = lt_launch<6, 2, 2>(map_w, map_x, xs, w, ys, rows, N, K, tn, err_flag, stream);
+        if (rc) return rc;
+    }
+    return 0;
 }

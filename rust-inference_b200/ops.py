@@ -65,6 +65,7 @@ _SIGNATURES = {
     ("dyn_tanh", "ri_embed_dyn_tanh"): [_P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P],
     ("pair_heads", "ri_pair_heads"): [_P, _P, _F, _F, _F, _I, _I, _I, _I, _I, _I, _I, _P],
     ("linear_f32", "ri_linear_f32"): [_P, _P, _P, _I, _I, _I, _P],
+    ("linear_f32", "ri_linear_f32_tc"): [_P] * 4 + [_I] * 4 + [_P, _P],
     ("sampling", "ri_sample"): [_P, _L, _I, _I, _P, _P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _I, _I, _P, _I, _P],
     ("sampling", "ri_sample_work_bytes"): [_I, _I],
     ("sampling", "ri_argmax"): [_P, _L, _I, _I, _P, _P, _P, _P],
@@ -689,10 +690,25 @@ def linear_act_rows(x: torch.Tensor, w: torch.Tensor, act: str, ids: torch.Tenso
     return out
 
 
+# The float32 product takes the tensor cores from here on.  The line depends on the sum's length and on how the weights lie, never on the
+# tokens: a row's bits are the same in every batch.  One of ten in a graph, tensor cores / multiply-adds, us at 300 tokens and 4,096
+# outputs; 1 and 4,096; 1 and 256: K = 64 9.0 / 8.6, 4.5 / 4.1, 5.3 / 4.5; 128 10.0 / 14.1, 5.5 / 7.0, 5.3 / 7.0; 256 12.1 / 25.4, 7.0 / 11.7,
+# 6.8 / 11.7.  From a program that launches them alone 128 is the first where neither is slower (11.3 / 12.4), and its error is the smaller one
+# from some 64 on.
+F32_TC_MIN_K = 128
+# bytes for the cut rows of x; larger steps take several launches
+F32_TC_SCRATCH = 128 << 20
+
+
+def _takes_f32_tc(K: int, w_ptr: int) -> bool:
+    return K >= F32_TC_MIN_K and K % 4 == 0 and w_ptr % 16 == 0 and not _NO_TCGEN05
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """y = x w^T for x [M, K], w [N, K].
 
-    float32: this package's own FMA kernel (no tensor cores, no TF32).
+    float32: this package's own kernels in full 32-bit precision (no TF32): exact cuts of the values into bfloat16 on the
+    tensor cores (tcgen05), or multiply-adds for short sums and odd rows; which of the two, K and ``w`` alone decide.
     bfloat16, up to 12 tokens (up to 16 for matrices of one wave of blocks): this package's weight-streaming
     tensor-core kernel (mma.sync).
     bfloat16, from there to 32 tokens (and up to 128 for wide matrices such as the output head): this package's
@@ -710,6 +726,13 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         x = x.clone()            # a one-row slice of a wider matrix: the kernels read 16-byte pieces
     if x.dtype == torch.float32:
         y = torch.empty((M, N), dtype=torch.float32, device=x.device)
+        if _takes_f32_tc(K, w.data_ptr()):
+            row = 6 * (-(-K // 32) * 32)                  # bytes of a row's three parts
+            rows = min(M, max(F32_TC_SCRATCH // row, 1024))
+            parts = torch.empty(rows * row, dtype=torch.uint8, device=x.device)
+            _call("linear_f32", "ri_linear_f32_tc", x.data_ptr(), w.data_ptr(), y.data_ptr(), parts.data_ptr(), rows, M, N, K,
+                  error_flag(x.device).data_ptr(), _stream())
+            return y
         _call("linear_f32", "ri_linear_f32", x.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, K, _stream())
         return y
     if x.dtype != torch.bfloat16:

@@ -1,0 +1,94 @@
+"""The float32 product on the tensor cores: sizes at the edges of its tiles, stages and launches against float64, a row of a large
+product bit for bit as the row alone, and values that are not finite."""
+import pytest
+import torch
+
+from rust_inference_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _inputs(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    return torch.randn((M, K), generator=g, device=DEV), torch.randn((N, K), generator=g, device=DEV)
+
+
+def _close(got, x, w):
+    """The parts' products that are left out are below 3 x 2^-23 of a product; a sum of 32 k is cut off twelve times by at most
+    2^-23 of its magnitudes, and the K / 32 sums' additions round by 2^-24 each."""
+    want, most = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((got.double() - want).abs() <= (x.shape[1] / 32 + 32) * 2.0 ** -24 * most).all()
+
+
+def _multiply_adds(x, w):
+    y = torch.empty((x.shape[0], w.shape[0]), device=DEV)
+    ops._call("linear_f32", "ri_linear_f32", x.data_ptr(), w.data_ptr(), y.data_ptr(), x.shape[0], w.shape[0], x.shape[1], ops._stream())
+    return y
+
+
+# one to three rounds of the rings, a last stage of 4 and of 28 k
+@pytest.mark.parametrize("K", [128, 132, 412, 1056])
+@pytest.mark.parametrize("M, N", [
+    (1, 1), (16, 128), (17, 129), (64, 4096), (65, 700),        # up to 64 tokens a block
+    (80, 9500), (128, 9473), (250, 4000),                       # up to 128
+    (176, 9473), (512, 6144), (353, 6100)])                     # up to 176
+def test_sizes(M, N, K):
+    x, w = _inputs(M, N, K)
+    assert ops._takes_f32_tc(K, w.data_ptr())
+    got = ops.linear(x, w)
+    _close(got, x, w)
+    for row in (0, M // 2, M - 1):
+        assert torch.equal(ops.linear(x[row:row + 1].contiguous(), w)[0], got[row])
+    assert torch.equal(ops.linear(x, w), got)
+
+
+def test_no_larger_error_than_multiply_adds():
+    for M, N, K in ((40, 300, 128), (300, 4000, 128), (100, 500, 1000), (300, 1000, 4096)):
+        x, w = _inputs(M, N, K)
+        want = x.double() @ w.double().T
+        errors = [((y.double() - want).norm() / want.norm()).item() for y in (ops.linear(x, w), _multiply_adds(x, w))]
+        assert errors[0] <= errors[1], (K, errors)
+
+
+def test_rows_in_several_launches(monkeypatch):
+    x, w = _inputs(2500, 200, 288)
+    whole = ops.linear(x, w)
+    monkeypatch.setattr(ops, "F32_TC_SCRATCH", 1)                # 1,024 rows a launch
+    assert torch.equal(ops.linear(x, w), whole)
+
+
+def test_rows_that_are_not_whole_pieces_take_multiply_adds():
+    for K in (257, 258):
+        x, w = _inputs(5, 70, K)
+        assert not ops._takes_f32_tc(K, w.data_ptr()) and torch.equal(ops.linear(x, w), _multiply_adds(x, w))
+    buffer = torch.randn(70 * 256 + 1, device=DEV)
+    w = buffer[1:].view(70, 256)                                 # rows that do not start on 16 bytes
+    x = torch.randn((5, 256), device=DEV)
+    assert torch.equal(ops.linear(x, w), _multiply_adds(x, w))
+
+
+def test_values_that_are_not_finite():
+    x, w = _inputs(40, 200, 512)
+    x[3, 7], x[5, 9], w[10, 100], x[21, 0] = float("inf"), float("nan"), float("-inf"), float("-inf")
+    x[8, 20], w[20, 20] = 3.4e38, 3e38                           # a product that overflows
+    # sums near the end of the range that stay inside it (512 products of 1e36: some 2e37, at most 2e38 on their way; a sum that
+    # leaves the range for less than 32 k and returns is finite here and infinite as a chain)
+    x[30] *= 1e36
+    got, want = ops.linear(x, w), _multiply_adds(x, w)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    endless = torch.isinf(want)
+    assert torch.equal(torch.isinf(got), endless) and torch.equal(got[endless], want[endless])
+    near = torch.isfinite(want)
+    assert ((got - want)[near].abs() <= 512 * 2.0 ** -23 * (x.abs().nan_to_num(posinf=0) @ w.abs().nan_to_num(posinf=0).T)[near]).all()
+
+
+def test_replayed_from_a_graph():
+    x, w = _inputs(7, 300, 512)
+    want = ops.linear(x, w)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = ops.linear(x, w)
+    x.copy_(x.flip(0))
+    graph.replay()
+    assert torch.equal(got, want.flip(0))
