@@ -8,13 +8,13 @@
 // keeps 128 rows of a and 128 rows of W (32 KB for 64 k) and accumulates its 128 rows x 256 outputs.  Per 64 k that is 32 KB
 // written and 32 KB read in 512 cycles of the tensor core.  A block alone with 128 x 256 has 48 KB written and 48 KB read
 // for the same products: it took 0.48 us per 64 k where the products need 0.27.
-// The pair stays on its SMs (six stages of 32 KB) and takes tiles one after the other, all row tiles of the plan for one
-// range of outputs before the next, so that the row tiles of an expert, which lie next to each other, read the
+// The pair stays on its SMs (six stages of 32 KB) and takes tiles one after the other, some row tiles of the plan for one
+// range of outputs before the next (`mt_place`), so that the row tiles of an expert, which lie next to each other, read the
 // expert's matrix at the same time (one trip to memory); two accumulators of 256 columns fill the tensor memory, so that a tile's
 // epilogue runs beside the next tile's products.  In each block:
-//   warp 0      one lane starts the copies: 128 rows of W as one TMA box of 64 k (with the gate the first block the gate rows and
-//               the second the up rows of the same channels, so that a channel's two sums meet in one thread) and 128
-//               rows of a as another; they signal the first block's barrier
+//   warps 0, 6  one lane of each starts copies: 128 rows of a as one TMA box of 64 k, and 128 rows of W as another (with the gate the
+//               first block the gate rows and the second the up rows of the same channels, so that a channel's two sums meet
+//               in one thread); they signal the first block's barrier
 //   warp 1      of the first block: one lane issues tcgen05.mma (256 x 256 x 16, kind::f16), four a stage, and the commits that
 //               hand back the stage and hand over the accumulator, to both blocks
 //   warps 2..5  the epilogue of the block's own 128 rows: a thread reads a row of the accumulator (a lane of the tensor memory)
@@ -24,8 +24,12 @@
 // The rows are gathered by a kernel of their own (60 MB, 12 us for the step below) because gathering in this one costs more: TMA's
 // gather4 brings four rows an instruction but takes some 40 cycles for each (0.78 us per 64 k), and with cp.async every
 // hand-over to the tensor core waits for the copies under way (fence.proxy.async; 1.5 us per 64 k).
-// 2,048 tokens of width 4,096, 16 experts of 1,376 channels, 4 choices (7,300 rows, 246 GFLOP in both products): 179 us with the
-// gather and 89 us, 0.92 PFLOP/s, where mma.sync tiles of 64 rows x 64 outputs took 687 and 401 us and the gate's own kernel 38.
+// The warps that issue walk their loops whole and one lane of them issues, and a wait that is over costs one instruction: with one lane
+// in the loop every product took some 60 cycles to issue and every wait 200, more than the 512 that a stage's products take
+// (now some 550 a stage).  Layer below: 556 us with one lane and all row tiles for one range of outputs, 534 without, 519 with the row
+// tiles in groups of 12 (520 in groups of 6 and of 18: what a group reads of a stays in L2).
+// 2,048 tokens of width 4,096, 16 experts of 1,376 channels, 4 choices (7,300 rows, 246 GFLOP in both products): 165 us and 95 us
+// in a cold pass, 0.95 PFLOP/s, where mma.sync tiles of 64 rows x 64 outputs took 687 and 401 us and the gate's own kernel 38.
 // The plan has wide tiles from 48 pairs per expert on, where they also lay for the tiles before these.  Gather and both products, wide / tiles
 // of 32 rows: width 4,096, 16 experts of 1,376: 25 pairs per expert 177 / 180 us, 48 pairs 169 / 237; width 2,048, 32 experts of
 // 704: 12 pairs 116 / 100, 50 pairs 114 / 138.  So the two forms meet at some 25 pairs, and from there to 47 the plan takes the
@@ -45,7 +49,7 @@
 #define MT_W_BYTES (MT_COLS / 2 * 128)
 #define MT_STAGE_BYTES (MT_A_BYTES + MT_W_BYTES)
 #define MT_STAGES 6
-#define MT_THREADS 192
+#define MT_THREADS 224
 #define MT_PITCH 36                        // floats between rows of an epilogue warp's 32 x 32 block
 #define MT_EPI_BYTES (4 * 32 * MT_PITCH * 4)
 #define MT_SMEM (MT_STAGES * MT_STAGE_BYTES + MT_EPI_BYTES + 256)
@@ -61,12 +65,13 @@ __device__ __forceinline__ unsigned long long mt_desc(unsigned addr) {
     d |= 2ull << 61;
     return d;
 }
-__device__ __forceinline__ void mt_mma(unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned acc) {
+template <int ACC>
+__device__ __forceinline__ void mt_mma(unsigned tmem_d, unsigned long long a, unsigned long long b) {
     constexpr unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((MT_COLS >> 3) << 17) | ((MT_ROWS >> 4) << 24);
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}\n"
-        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0u) : "memory");
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "n"(ACC), "r"(0u) : "memory");
 }
 // arrives on the barrier at this place in both blocks when the products issued so far are done
 __device__ __forceinline__ void mt_commit(unsigned long long* bar) {
@@ -152,6 +157,15 @@ __device__ __forceinline__ float mt_gate(float g, float u, const MtGate& c) {
     return g / (1.0f + expf(-g)) * u;
 }
 
+// The order of the tiles: MT_GROUP row tiles for one range of outputs after the other, then the next MT_GROUP.  What a group reads
+// of a (MT_GROUP x 256 rows of 8 KB at width 4,096: 25 MB) stays in L2 over all ranges, and its experts' matrices are read once.
+#define MT_GROUP 12
+__device__ __forceinline__ void mt_place(int t, int row_tiles, int col_tiles, int& m, int& c) {
+    const int g = t / (MT_GROUP * col_tiles), rest = t - g * MT_GROUP * col_tiles, here = min(MT_GROUP, row_tiles - g * MT_GROUP);
+    c = rest / here;
+    m = g * MT_GROUP + rest - c * here;
+}
+
 struct MtTail {
     unsigned long long full[MT_STAGES], empty[MT_STAGES], acc_full[2], acc_empty[2], drained;
     unsigned tmem_base;
@@ -159,14 +173,26 @@ struct MtTail {
 };
 static_assert(sizeof(MtTail) <= 256, "the tail fits behind the stages");
 
-// A wait of a role: false when it ran out, or when somebody else has given up (nothing further is started then).
+__device__ __forceinline__ bool mt_test(unsigned long long* bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return __all_sync(0xffffffffu, ok);
+}
+// A warp's wait: false when it ran out, or when somebody else has given up (nothing further is started then).
 __device__ __forceinline__ bool mt_wait(unsigned long long* bar, unsigned parity, MtTail& tail, int* err) {
-    if (!ri_mbar_wait(bar, parity)) {
+    if (mt_test(bar, parity)) return true;
+    if (!__all_sync(0xffffffffu, ri_mbar_wait(bar, parity))) {
         atomicExch(err, 5);
         *(volatile int*)&tail.dead = 1;
         return false;
     }
-    return *(volatile int*)&tail.dead == 0;
+    return __all_sync(0xffffffffu, *(volatile int*)&tail.dead == 0);
+}
+__device__ __forceinline__ bool mt_elect() {
+    unsigned one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(one));
+    return one != 0;
 }
 
 // N: outputs per row (with a gate: channels, W has 2 N rows per expert); y rows start ldy elements apart
@@ -215,55 +241,75 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     const int steps = (K + MT_STAGE_K - 1) / MT_STAGE_K;
     const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;    // the pair's tiles
 
-    if (warp == 0) {
-        // ---- copies ------------------------------------------------------------------------------------------------------
-        if (lane == 0) {
-            long long it = 0;                                      // stages so far, over all tiles
-            bool ok = true;
-            for (int t = first; t < total && ok; t += stride) {
-                const int m = t % row_tiles, n0 = (t / row_tiles) * cols;
-                const int e = tiles[3 * m], r0 = tiles[3 * m + 1] + (int)rank * MT_HALF;
-                const int w0 = GATED ? e * 2 * N + (int)rank * N + n0 : e * N + n0 + (int)rank * (MT_COLS / 2);
-                for (int k = 0; k < steps; k++, it++) {
-                    const int s = (int)(it % MT_STAGES);
-                    if (it >= MT_STAGES && !mt_wait(&tail.empty[s], (unsigned)((it / MT_STAGES - 1) & 1), tail, err)) { ok = false; break; }
-                    const unsigned st = smem_u32(mt_smem + s * MT_STAGE_BYTES), bar = mt_in_block(&tail.full[s], 0);
-                    if (rank == 0)                                 // what both blocks copy
-                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
-                                     ::"r"(smem_u32(&tail.full[s])), "r"(2 * MT_STAGE_BYTES) : "memory");
-                    mt_box(st + MT_A_BYTES, &map_w, k * MT_STAGE_K, w0, bar);
-                    mt_box(st, &map_a, k * MT_STAGE_K, r0, bar);
+    if (warp == 0 || warp == 6) {
+        // ---- copies: the first warp a, the last one W ----------------------------------------------------------------------
+        const bool one = mt_elect();
+        const unsigned ring = smem_u32(mt_smem) + (warp == 0 ? 0 : MT_A_BYTES), bars = mt_in_block(&tail.full[0], 0);
+        int s = 0, laps = 0;                                       // the ring's place, and how often it has been filled
+        bool ok = true;
+        for (int t = first; t < total && ok; t += stride) {
+            int m, c;
+            mt_place(t, row_tiles, col_tiles, m, c);
+            const int e = tiles[3 * m], r0 = tiles[3 * m + 1] + (int)rank * MT_HALF, n0 = c * cols;
+            const int w0 = GATED ? e * 2 * N + (int)rank * N + n0 : e * N + n0 + (int)rank * (MT_COLS / 2);
+            for (int k = 0; k < steps; k++) {
+                if (laps > 0 && !mt_wait(&tail.empty[s], (unsigned)((laps - 1) & 1), tail, err)) { ok = false; break; }
+                if (one) {
+                    if (warp == 6) {
+                        mt_box(ring + s * MT_STAGE_BYTES, &map_w, k * MT_STAGE_K, w0, bars + s * 8);
+                    } else {
+                        if (rank == 0)                             // what both blocks copy
+                            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+                                         ::"r"(smem_u32(&tail.full[s])), "r"(2 * MT_STAGE_BYTES) : "memory");
+                        mt_box(ring + s * MT_STAGE_BYTES, &map_a, k * MT_STAGE_K, r0, bars + s * 8);
+                    }
+                }
+                if (++s == MT_STAGES) {
+                    s = 0;
+                    laps++;
                 }
             }
-            if (rank == 0 && *(volatile int*)&tail.dead)           // somebody gave up: what was started lands first
-                for (long long i = it > MT_STAGES ? it - MT_STAGES : 0; i < it; i++)
-                    ri_mbar_wait(&tail.full[i % MT_STAGES], (unsigned)((i / MT_STAGES) & 1));
         }
+        if (rank == 0 && warp == 0 && one && *(volatile int*)&tail.dead)       // somebody gave up: what was started lands first
+            for (int i = 0; i < MT_STAGES; i++)
+                if (i < s || laps > 0) ri_mbar_wait(&tail.full[i], (unsigned)((i < s ? laps : laps - 1) & 1));
+        __syncwarp();
     } else if (warp == 1) {
         // ---- products ----------------------------------------------------------------------------------------------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            // (the whole warp walks the loop and one lane issues: what the products take is the same for all lanes, and stays so)
+            const bool one = mt_elect();
             const unsigned long long a0 = mt_desc(smem_u32(mt_smem)), w0 = mt_desc(smem_u32(mt_smem + MT_A_BYTES));
-            long long it = 0;
-            int nth = 0;
+            int nth = 0, s = 0;
+            unsigned lap = 0;
             bool ok = true;
             for (int t = first; t < total && ok; t += stride, nth++) {
                 const int buf = nth & 1;
                 if (nth >= 2 && !mt_wait(&tail.acc_empty[buf], (unsigned)((nth / 2 - 1) & 1), tail, err)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                for (int k = 0; k < steps; k++, it++) {
-                    const int s = (int)(it % MT_STAGES);
-                    if (!mt_wait(&tail.full[s], (unsigned)((it / MT_STAGES) & 1), tail, err)) { ok = false; break; }
+                for (int k = 0; k < steps; k++) {
+                    if (!mt_wait(&tail.full[s], lap & 1, tail, err)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const unsigned long long off = (unsigned long long)(s * (MT_STAGE_BYTES >> 4));
+                    if (one) {
+                        const unsigned long long off = (unsigned long long)(s * (MT_STAGE_BYTES >> 4));
+                        const unsigned d = tmem + buf * MT_COLS;
+                        if (k == 0) mt_mma<0>(d, a0 + off, w0 + off);
+                        else mt_mma<1>(d, a0 + off, w0 + off);
 #pragma unroll
-                    for (int j = 0; j < MT_STAGE_K / 16; j++)
-                        mt_mma(tmem + buf * MT_COLS, a0 + off + j * 2, w0 + off + j * 2, (k > 0 || j > 0) ? 1u : 0u);
-                    mt_commit(&tail.empty[s]);
+                        for (int j = 1; j < MT_STAGE_K / 16; j++) mt_mma<1>(d, a0 + off + j * 2, w0 + off + j * 2);
+                        mt_commit(&tail.empty[s]);
+                    }
+                    if (++s == MT_STAGES) {
+                        s = 0;
+                        lap++;
+                    }
                 }
-                if (ok) mt_commit(&tail.acc_full[buf]);
+                if (ok && one) mt_commit(&tail.acc_full[buf]);
             }
-            mt_commit(&tail.drained);                              // no product is under way when the tensor memory goes back
-            ri_mbar_wait(&tail.drained, 0);
+            if (one) {
+                mt_commit(&tail.drained);                          // no product is under way when the tensor memory goes back
+                ri_mbar_wait(&tail.drained, 0);
+            }
+            __syncwarp();
         }
     } else {
         // ---- epilogue: warp w reads the lanes 32 (w % 4) .. + 31 of the tensor memory -----------------------------------------
@@ -273,7 +319,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         int nth = 0;
         for (int t = first; t < total; t += stride, nth++) {
             const int buf = nth & 1;
-            const int m = t % row_tiles, n0 = (t / row_tiles) * cols;
+            int m, c;
+            mt_place(t, row_tiles, col_tiles, m, c);
+            const int n0 = c * cols;
             const int r0 = tiles[3 * m + 1], rows = tiles[3 * m + 2];
             const int base = (int)rank * MT_HALF + quad * 32;      // the warp's first row of the tile
             int out[8];
@@ -282,7 +330,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                 const int r = base + 4 * i + sub;
                 out[i] = r < rows ? (scatter ? perm[r0 + r] : r0 + r) : -1;
             }
-            if (!__all_sync(0xffffffffu, mt_wait(&tail.acc_full[buf], (unsigned)((nth / 2) & 1), tail, err))) break;
+            if (!mt_wait(&tail.acc_full[buf], (unsigned)((nth / 2) & 1), tail, err)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned taddr = tmem + buf * MT_COLS + ((unsigned)(quad * 32) << 16);
             if (base < rows) {
