@@ -129,7 +129,7 @@ __device__ __forceinline__ void moe_choose(float* s, float* c, float* gs, const 
             if (gs[n / size] != INFINITY) c[n] = -INFINITY;
         __syncwarp();
     }
-    float picked_sum = 0.0f;
+    float picked_sum = 0.0f, mine = 0.0f;                 // mine: lane j's is the j-th choice's score (of up to 32)
     for (int j = 0; j < top; j++) {
         float best = -INFINITY;
         int at = 0x7fffffff;
@@ -148,15 +148,26 @@ __device__ __forceinline__ void moe_choose(float* s, float* c, float* gs, const 
             }
         }
         if (at >= N) at = 0;                           // no finite score left (NaN inputs): still a valid index
+        const float picked = s[at];
         if (lane == 0) {
             idx[(size_t)t * top + j] = at;
-            weight[(size_t)t * top + j] = s[at];
+            if (top > 32) weight[(size_t)t * top + j] = picked;
             c[at] = -INFINITY;
         }
-        picked_sum += s[at];
+        if (lane == j) mine = picked;
+        picked_sum += picked;
         __syncwarp();
     }
-    if (lane == 0 && rule.mode == 2) {
+    if (top <= 32) {                                      // (more choices than lanes: from memory, below)
+        float div = rule.renorm ? picked_sum + 1e-20f : 1.0f;
+        if (rule.mode == 2) {
+            // the first choice has the largest logit
+            mine = expf(mine - __shfl_sync(0xffffffffu, mine, 0));
+            div = 0.0f;
+            for (int j = 0; j < top; j++) div += __shfl_sync(0xffffffffu, mine, j);
+        }
+        if (lane < top) weight[(size_t)t * top + lane] = mine / div * rule.scale;
+    } else if (lane == 0 && rule.mode == 2) {
         // the first choice has the largest logit
         float* w = weight + (size_t)t * top;
         const float mx = w[0];
@@ -232,12 +243,13 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router, cons
 }
 
 // The same with a block of 1,024 threads per token, for routers small enough that all their partial sums fit in shared
-// memory: a warp takes (output, segment of 128 k) items, so the whole router is asked for at once instead of row after
-// row (one trip to memory instead of dozens: the warp-per-token form took 75 us whatever the number of tokens); a
-// segment's sum is the warp's tree, an output's logit the sum of its segments in ascending order.
+// memory: a warp takes (output, run of MOE_ROUTE_RUN segments of 128 k) items, so the whole router is asked for at once instead of row after
+// row (one trip to memory instead of dozens: the warp-per-token form took 75 us whatever the number of tokens); a lane adds up
+// its four k of every segment of a run, the run's sum is the warp's tree, an output's logit the sum of its runs in ascending order.
+#define MOE_ROUTE_RUN 4
 #define MOE_ROUTE_WIDE_THREADS 1024
 #define MOE_ROUTE_WIDE_ITEMS 8192
-#define MOE_ROUTE_AHEAD 6
+#define MOE_ROUTE_AHEAD 2
 template <typename T>
 __global__ void __launch_bounds__(MOE_ROUTE_WIDE_THREADS)
 moe_route_wide_kernel(const T* __restrict__ x, const float* __restrict__ router, const float* __restrict__ correction,
@@ -247,39 +259,45 @@ moe_route_wide_kernel(const T* __restrict__ x, const float* __restrict__ router,
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x;
-    const int segs = (D + 127) / 128;
+    const int runs = (D + 128 * MOE_ROUTE_RUN - 1) / (128 * MOE_ROUTE_RUN);
     float* part = moe_sm;
-    float* s = part + (size_t)N * segs;
+    float* s = part + (size_t)N * runs;
     float* c = s + N;
     const T* xr = x + (size_t)t * D;
     const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    // MOE_ROUTE_AHEAD items' loads are on their way together (one at a time: a trip to L2 per item; 18 outputs of width 4,096, cold:
-    // 22.5 -> 18.4 us)
+    // MOE_ROUTE_AHEAD items' loads are on their way together
     constexpr int WARPS = MOE_ROUTE_WIDE_THREADS / 32;
-    for (int item0 = warp; item0 < N * segs; item0 += WARPS * MOE_ROUTE_AHEAD) {
-        float4 xv[MOE_ROUTE_AHEAD], wv[MOE_ROUTE_AHEAD];
+    for (int item0 = warp; item0 < N * runs; item0 += WARPS * MOE_ROUTE_AHEAD) {
+        float4 xv[MOE_ROUTE_AHEAD][MOE_ROUTE_RUN], wv[MOE_ROUTE_AHEAD][MOE_ROUTE_RUN];
 #pragma unroll
         for (int u = 0; u < MOE_ROUTE_AHEAD; u++) {
-            const int item = item0 + u * WARPS, n = item / segs, k = (item - n * segs) * 128 + 4 * lane;
-            const bool ok = item < N * segs && k < D;
-            xv[u] = ok ? moe_ld4(xr + k) : zero4;
-            wv[u] = ok ? *reinterpret_cast<const float4*>(router + (size_t)n * D + k) : zero4;
+            const int item = min(item0 + u * WARPS, N * runs - 1), n = item / runs, k0 = (item - n * runs) * 128 * MOE_ROUTE_RUN + 4 * lane;
+#pragma unroll
+            for (int i = 0; i < MOE_ROUTE_RUN; i++) {
+                const int k = k0 + 128 * i;
+                xv[u][i] = k < D ? moe_ld4(xr + k) : zero4;
+                wv[u][i] = k < D ? *reinterpret_cast<const float4*>(router + (size_t)n * D + k) : zero4;
+            }
         }
 #pragma unroll
         for (int u = 0; u < MOE_ROUTE_AHEAD; u++) {
             const int item = item0 + u * WARPS;
-            float a = xv[u].x * wv[u].x;
-            a = fmaf(xv[u].y, wv[u].y, a);
-            a = fmaf(xv[u].z, wv[u].z, a);
-            a = fmaf(xv[u].w, wv[u].w, a);
+            float a = 0.0f;
+#pragma unroll
+            for (int i = 0; i < MOE_ROUTE_RUN; i++) {
+                a = fmaf(xv[u][i].x, wv[u][i].x, a);
+                a = fmaf(xv[u][i].y, wv[u][i].y, a);
+                a = fmaf(xv[u][i].z, wv[u][i].z, a);
+                a = fmaf(xv[u][i].w, wv[u][i].w, a);
+            }
             a = warp_sum(a);
-            if (lane == 0 && item < N * segs) part[item] = a;
+            if (lane == 0 && item < N * runs) part[item] = a;
         }
     }
     __syncthreads();
     for (int n = threadIdx.x; n < N; n += MOE_ROUTE_WIDE_THREADS) {
         float a = 0.0f;
-        for (int g = 0; g < segs; g++) a += part[n * segs + g];
+        for (int g = 0; g < runs; g++) a += part[n * runs + g];
         s[n] = a;
     }
     __syncthreads();
@@ -288,67 +306,91 @@ moe_route_wide_kernel(const T* __restrict__ x, const float* __restrict__ router,
 }
 
 // The same for many tokens: a block takes MOE_ROUTE_TILE tokens, so that a piece of the router that a warp has loaded serves
-// all of them (a block per token reads the whole router from L2 for every token: 2,048 tokens of width 4,096 and 18 outputs
-// are 600 MB of L2 traffic: 123 us, 53 us here, cold).  A warp takes segments of 128 k, four outputs at a time; the 16 sums of
-// four tokens and four outputs go down the warp's tree side by side, every step halving the number of values a lane still
-// holds, so that lanes 2 i and 2 i + 1 end with the sum of token i / 4 and output i % 4.  The additions of a sum and their order are those of the
-// kernel above: the same bits.
+// all of them (a block per token reads the whole router from L2 for every token).  What bounds it: the router's way from L2, the
+// multiply-adds and the trees, and for few blocks the trips to memory, one for each item of a warp.  A warp takes a run for four outputs, its
+// loads on their way together, and keeps the 16 sums of four tokens and four outputs in registers; they go down the warp's tree side by side,
+// every step halving the number of values a lane still holds, so that lanes 2 i and 2 i + 1 end with the sum of token i / 4 and output i % 4.  The
+// additions of a sum and their order are those of the kernel above: the same bits.
+// Cold, width 4,096 and 18 outputs, 256 / 512 / 2,048 tokens: 16.6 / 18.4 / 35 us; with a tree for every segment of 128 k 23.5 / 23.6 / 53.
+// (Eight tokens and eight outputs a warp's item, a segment at a time: 26.7 / 28.6 / 35.5.)
 #define MOE_ROUTE_TILE 4
-#define MOE_ROUTE_TILE_THREADS 512
-#define MOE_ROUTE_TILE_TOKENS 256
+#define MOE_ROUTE_TILE_THREADS 256
+#define MOE_ROUTE_TILE_TOKENS 149
+template <typename T> struct MoePiece;                // four neighbouring elements as they come from memory
+template <> struct MoePiece<float> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p) { v = moe_ld4(p); }
+    __device__ __forceinline__ float4 value() const { return v; }
+};
+template <> struct MoePiece<bf16> {
+    uint2 v;
+    __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ float4 value() const {
+        return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+    }
+};
 template <typename T>
 __global__ void __launch_bounds__(MOE_ROUTE_TILE_THREADS, 2)
 moe_route_tile_kernel(const T* x, const float* __restrict__ router, const float* __restrict__ correction, int* __restrict__ idx,
                       float* __restrict__ weight, int tokens, int D, int N, int top, MoeRule rule) {
-    extern __shared__ float moe_sm[];                 // partial sums [segs][TILE][N4], per token: scores, choice scores, runs' scores
+    extern __shared__ float moe_sm[];                 // partial sums [runs][TILE][N4], per token: scores, choice scores, groups' scores
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t0 = blockIdx.x * MOE_ROUTE_TILE;
-    const int segs = (D + 127) / 128, quads = (N + 3) / 4, N4 = 4 * quads;
+    const int runs = (D + 128 * MOE_ROUTE_RUN - 1) / (128 * MOE_ROUTE_RUN), quads = (N + 3) / 4, N4 = 4 * quads;
     float* part = moe_sm;
-    float* scores = part + (size_t)segs * MOE_ROUTE_TILE * N4;
-    const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    // a warp takes whole segments, so that its eight pieces of x are loaded once for all outputs
-    for (int seg = warp; seg < segs; seg += MOE_ROUTE_TILE_THREADS / 32) {
-        const int k = seg * 128 + 4 * lane;
-        const bool ok = k < D;
-        float4 xv[MOE_ROUTE_TILE];
+    float* scores = part + (size_t)runs * MOE_ROUTE_TILE * N4;
+    constexpr int AHEAD = sizeof(T) == 2 ? MOE_ROUTE_RUN : MOE_ROUTE_RUN / 2;      // segments whose loads are on their way together
+    for (int item = warp; item < runs * quads; item += MOE_ROUTE_TILE_THREADS / 32) {
+        const int run = item / quads, q = item - run * quads;
+        float v[4 * MOE_ROUTE_TILE];
 #pragma unroll
-        for (int j = 0; j < MOE_ROUTE_TILE; j++) xv[j] = ok ? moe_ld4(x + (size_t)min(t0 + j, tokens - 1) * D + k) : zero4;
-        float4 wv[4];
+        for (int i = 0; i < 4 * MOE_ROUTE_TILE; i++) v[i] = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4; i++) wv[i] = ok ? *reinterpret_cast<const float4*>(router + (size_t)min(i, N - 1) * D + k) : zero4;
-        for (int q = 0; q < quads; q++) {
-            float v[4 * MOE_ROUTE_TILE];
+        for (int i0 = 0; i0 < MOE_ROUTE_RUN; i0 += AHEAD) {
+            MoePiece<T> xv[AHEAD][MOE_ROUTE_TILE];
+            float4 wv[AHEAD][4];
 #pragma unroll
-            for (int j = 0; j < MOE_ROUTE_TILE; j++) {
+            for (int i = 0; i < AHEAD; i++) {
+                const int k = (run * MOE_ROUTE_RUN + i0 + i) * 128 + 4 * lane, at = k < D ? k : 0;      // past the row: zeros in place of x
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float a = xv[j].x * wv[i].x;
-                    a = fmaf(xv[j].y, wv[i].y, a);
-                    a = fmaf(xv[j].z, wv[i].z, a);
-                    v[4 * j + i] = fmaf(xv[j].w, wv[i].w, a);
+                for (int n = 0; n < 4; n++) wv[i][n] = *reinterpret_cast<const float4*>(router + (size_t)min(4 * q + n, N - 1) * D + at);
+#pragma unroll
+                for (int j = 0; j < MOE_ROUTE_TILE; j++) xv[i][j].load(x + (size_t)min(t0 + j, tokens - 1) * D + at);
+            }
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++) {
+                const bool ok = (run * MOE_ROUTE_RUN + i0 + i) * 128 + 4 * lane < D;
+                if (!ok)
+#pragma unroll
+                    for (int n = 0; n < 4; n++) wv[i][n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (int j = 0; j < MOE_ROUTE_TILE; j++) {
+                    const float4 a = ok ? xv[i][j].value() : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                    for (int n = 0; n < 4; n++) {
+                        float c = v[4 * j + n];
+                        c = fmaf(a.x, wv[i][n].x, c);
+                        c = fmaf(a.y, wv[i][n].y, c);
+                        c = fmaf(a.z, wv[i][n].z, c);
+                        v[4 * j + n] = fmaf(a.w, wv[i][n].w, c);
+                    }
                 }
             }
-            if (q + 1 < quads) {                      // the next four outputs' rows, under the additions
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    wv[i] = ok ? *reinterpret_cast<const float4*>(router + (size_t)min(4 * (q + 1) + i, N - 1) * D + k) : zero4;
-            }
-#pragma unroll
-            for (int o = 16; o > 1; o >>= 1) {
-                const bool upper = (lane & o) != 0;
-#pragma unroll
-                for (int i = 0; i < o / 2; i++) {
-                    const float give = upper ? v[i] : v[i + o / 2];
-                    const float keep = upper ? v[i + o / 2] : v[i];
-                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-                }
-            }
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-            if ((lane & 1) == 0) part[((size_t)seg * MOE_ROUTE_TILE + (lane >> 3)) * N4 + 4 * q + ((lane >> 1) & 3)] = v[0];
         }
+#pragma unroll
+        for (int o = 16; o > 1; o >>= 1) {
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < o / 2; i++) {
+                const float give = upper ? v[i] : v[i + o / 2];
+                const float keep = upper ? v[i + o / 2] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+        if ((lane & 1) == 0) part[((size_t)run * MOE_ROUTE_TILE + (lane >> 3)) * N4 + 4 * q + ((lane >> 1) & 3)] = v[0];
     }
     __syncthreads();
     const int pitch = 2 * N + rule.groups;
@@ -356,10 +398,11 @@ moe_route_tile_kernel(const T* x, const float* __restrict__ router, const float*
         const int j = i / N, n = i - j * N;
         float a = 0.0f;
 #pragma unroll 8
-        for (int g = 0; g < segs; g++) a += part[((size_t)g * MOE_ROUTE_TILE + j) * N4 + n];
+        for (int g = 0; g < runs; g++) a += part[((size_t)g * MOE_ROUTE_TILE + j) * N4 + n];
         scores[j * pitch + n] = a;
     }
     __syncthreads();
+    static_assert(MOE_ROUTE_TILE <= MOE_ROUTE_TILE_THREADS / 32, "a warp per token");
     if (warp >= MOE_ROUTE_TILE || t0 + warp >= tokens) return;
     float* s = scores + (size_t)warp * pitch;
     moe_choose(s, s + N, s + 2 * N, correction, idx, weight, t0 + warp, N, top, lane, rule);
@@ -386,9 +429,10 @@ extern "C" int ri_moe_route_rule(const void* x, const float* router, const float
     const int vec = (D % 4 == 0 && (((uintptr_t)router | (uintptr_t)x) & 15) == 0) ? 1 : 0;
     cudaError_t e = cudaSuccess;
     const long long items = (long long)N * ((D + 127) / 128);
-    // From 256 tokens on, blocks of four tokens.  Cold, width 4,096 and 18 outputs, four tokens / one token a block: 128 tokens
-    // 22.5 / 18.4 us, 256 tokens 24.6 / 28.7, 512 tokens 22.5 / 51.
-    const size_t tile_sm = ((size_t)((D + 127) / 128) * MOE_ROUTE_TILE * ((N + 3) / 4 * 4) + (size_t)MOE_ROUTE_TILE * (2 * N + groups)) * sizeof(float);
+    // Blocks of four tokens from where blocks of one token, which have an SM each, need a second round of the 148 SMs.  Cold, width 4,096 and
+    // 18 outputs: one token a block 14.4 us up to 148 tokens and 22.5 for 200, four 16.6 for 256; width 2,048 and 34 outputs 14.4, 22.5, 16.4.
+    const long long runs = (D + 128 * MOE_ROUTE_RUN - 1) / (128 * MOE_ROUTE_RUN);
+    const size_t tile_sm = ((size_t)runs * MOE_ROUTE_TILE * ((N + 3) / 4 * 4) + (size_t)MOE_ROUTE_TILE * (2 * N + groups)) * sizeof(float);
     if (vec && items <= MOE_ROUTE_WIDE_ITEMS && tokens >= MOE_ROUTE_TILE_TOKENS && tile_sm <= 96 * 1024) {
         const dim3 tiles((tokens + MOE_ROUTE_TILE - 1) / MOE_ROUTE_TILE);
         if (dtype == RI_DTYPE_F32) {
@@ -406,7 +450,7 @@ extern "C" int ri_moe_route_rule(const void* x, const float* router, const float
         return 0;
     }
     if (vec && items <= MOE_ROUTE_WIDE_ITEMS && tokens <= 65535 * 32) {
-        const size_t sm = (size_t)(items + 2 * N + groups) * sizeof(float);
+        const size_t sm = (size_t)(N * runs + 2 * N + groups) * sizeof(float);
         if (dtype == RI_DTYPE_F32)
             ri_launch_pdl(moe_route_wide_kernel<float>, dim3(tokens), dim3(MOE_ROUTE_WIDE_THREADS), sm, stream, (const float*)x,
                           router, correction, idx, weight, D, N, top, rule);
