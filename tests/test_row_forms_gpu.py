@@ -1,0 +1,83 @@
+"""The forms of the kernels between the products that take whole pieces of rows, at the edges of their pieces and tokens, against
+float64 and against the forms that take an element at a time (rows that do not start on whole pieces)."""
+import numpy as np
+import pytest
+import torch
+
+from rust_inference_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+DT = {"float32": torch.float32, "bfloat16": torch.bfloat16}
+TOL = {"float32": 2e-6, "bfloat16": 5e-3}      # float32 functions; one rounding to 8 bits
+
+
+def _i32(v):
+    return torch.tensor(np.asarray(v, dtype=np.int32), device=DEV)
+
+
+def _rand(seed, *shape):
+    return torch.randn(shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+
+
+def _close(got, want, tol):
+    assert ((got.double() - want.double()).norm() / want.double().norm()).item() <= tol
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("tokens, heads, vdim", [(1, 1, 4), (3, 5, 96), (700, 16, 128), (7, 3, 132), (2, 2, 256), (5, 2, 260), (9, 4, 66)])
+@pytest.mark.parametrize("fn", ["silu", "sigmoid"])
+def test_head_norm_gate(tokens, heads, vdim, fn, dtype):
+    o, gain = _rand(1, tokens, heads, vdim), 1 + 0.1 * _rand(2, vdim)
+    wide = _rand(3, tokens, heads * vdim + 8).to(DT[dtype])
+    for g in (wide[:, 8:], wide[:, 4:4 + heads * vdim], wide[:, 1:1 + heads * vdim]):       # the last: element by element
+        z = g.double().view(tokens, heads, vdim)
+        want = o.double() / torch.sqrt((o.double() ** 2).mean(-1, keepdim=True) + 1e-6) * gain.double() * torch.sigmoid(z) * (z if fn == "silu" else 1)
+        _close(ops.head_norm_gate(o, gain, 1e-6, g, DT[dtype], fn).view(tokens, heads, vdim), want, TOL[dtype])
+
+
+# from 256 tokens on four tokens a thread; sequences that begin and end anywhere in a thread's four, of one and two tokens too
+@pytest.mark.parametrize("lens", [[256], [259], [1, 2, 3, 250, 1, 1, 4], [64] * 5, [255, 2]])
+def test_short_conv_over_many_tokens(lens):
+    T, C, slots = sum(lens), 72, len(lens) + 2
+    x = _rand(4, T, C + 8).bfloat16()[:, :]
+    w = 0.5 * _rand(5, C, 4)
+    wt = w.t().contiguous()
+    state = _rand(6, slots, 3, C)
+    order = list(range(len(lens)))[::-1]
+    args = (_i32(np.repeat(np.arange(len(lens)), lens)), _i32(order), _i32(np.concatenate([[0], np.cumsum(lens)])))
+    a, b = state.clone(), state.clone()
+    got = ops.short_conv(x, 8, w, a, *args, weight_t=wt)
+    assert torch.equal(got, ops.short_conv(x, 8, w, b, *args)) and torch.equal(a, b)             # an element at a time
+    start = np.concatenate([[0], np.cumsum(lens)])
+    for i, n in enumerate(lens):
+        seq = torch.cat([state[order[i]].double(), x[start[i]:start[i + 1], 8:].double()])
+        z = sum(w[:, j].double() * seq[j:j + n] for j in range(4))
+        _close(got[start[i]:start[i + 1]], z * torch.sigmoid(z), 1e-6)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("tokens, H, dim, rot, rank, row", [(1, 1, 8, 8, 8, 16), (3, 5, 16, 24, 40, 64), (300, 7, 128, 64, 192, 256), (260, 32, 8, 8, 248, 272),
+                                                            (5, 3, 12, 4, 20, 32)])
+def test_latent_rows(tokens, H, dim, rot, rank, row, dtype):
+    dt, page = DT[dtype], 32
+    pages = -(-tokens // page)
+    cols = H * (dim + rot) + rank + rot
+    table = _rand(7, tokens, rot // 2, 2)
+    gain = 1 + 0.1 * _rand(8, rank)
+    base = _rand(9, tokens, cols + 9).to(dt)
+    qa = _rand(10, tokens, H, rank).to(dt)
+    meta = (_i32([range(pages)]), _i32([0] * tokens), _i32(range(tokens)), _i32([0]))
+    results = []
+    for first in (8, 1):                                      # the second: element by element
+        proj = torch.zeros((tokens, cols + 16), dtype=dt, device=DEV)
+        proj[:, first:first + cols] = base[:, :cols]
+        pool = torch.zeros((pages, 1, page, row), dtype=dt, device=DEV)
+        qf = ops.latent_prep(proj, first, first + H * (dim + rot), qa, H, dim, rot, rank, gain, 1e-6, table, pool, *meta, row=row)
+        results.append((qf, pool))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    q = base[:, :H * (dim + rot)].double().view(tokens, H, dim + rot)[:, :, dim:]
+    c, s = table[..., 0].double()[:, None], table[..., 1].double()[:, None]
+    u, v = q[..., 0::2], q[..., 1::2]
+    want = torch.cat([qa.double(), torch.stack([u * c - v * s, v * c + u * s], -1).flatten(-2), torch.zeros((tokens, H, row - rank - rot), device=DEV)], -1)
+    _close(results[0][0], want, TOL[dtype])
