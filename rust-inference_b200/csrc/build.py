@@ -48,6 +48,7 @@ SOURCES: Dict[str, Tuple[str, ...]] = {
     "sampling": ("sampling.cu", "common.cuh"),
     "attention_decode": ("attention_decode.cu", "common.cuh", "mma_helpers.cuh", "softcap.cuh", "distance_bias.cuh", "pair_heads.cuh"),
     "attention_prefill": ("attention_prefill.cu", "common.cuh", "mma_helpers.cuh", "softcap.cuh", "distance_bias.cuh"),
+    "low_rank": ("low_rank.cu", "common.cuh", "mma_helpers.cuh"),
     "linear_skinny": ("linear_skinny.cu", "common.cuh", "mma_helpers.cuh", "linear_skinny_geometry.cuh"),
     "linear_stream_tc": ("linear_stream_tc.cu", "common.cuh", "mma_helpers.cuh"),
     "attention_latent_tc": ("attention_latent_tc.cu", "common.cuh", "mma_helpers.cuh", "tcgen05_helpers.cuh"),

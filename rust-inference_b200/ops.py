@@ -72,6 +72,7 @@ _SIGNATURES = {
     ("sampling", "ri_mark_seen"): [_P, _L, _P, _P, _I, _I, _P],
     ("attention_decode", "ri_attention_decode_sink"): [_P] * 9 + [_I] * 8 + [_F, _I, _P, _P, _P],
     ("attention_decode", "ri_attention_decode_cap"): [_P] * 9 + [_I] * 8 + [_F, _I, _P, _F, _P, _I] + [_I, _I, _I, _F, _F, _F] + [_P, _P],
+    ("low_rank", "ri_low_rank"): [_P, _L, _I, _I, _I, _P, _P, _I, _I, _I, _P, _P, _I, _P],
     ("linear_skinny", "ri_linear_skinny"): [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     ("linear_skinny", "ri_linear_skinny_act"): [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     ("linear_skinny", "ri_linear_skinny_gated"): [_P, _P, _P, _I, _I, _I, _I, _P, _P],
@@ -748,6 +749,31 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     if out_dtype == torch.float32:
         return torch.mm(x, w.t(), out_dtype=torch.float32)
     return torch.mm(x, w.t())
+
+
+LOW_RANK_MAX_K = 128
+
+
+def low_rank(x: torch.Tensor, *sets) -> list:
+    """The outer products of low-rank projections: for every (col, w) of ``sets``, w [N, K], the product
+    x[:, col:col + K] w^T [tokens, N].  ``x`` [tokens, columns] holds the inner parts side by side.
+    bfloat16, up to two products of K up to 128 over columns in multiples of 8: one kernel of this package (mma.sync) that
+    reads the columns where they lie; anything else a copy of the columns and ``linear`` each."""
+    tokens, ld = x.shape
+    for col, w in sets:
+        if w.dim() != 2 or w.dtype != x.dtype or col < 0 or col + w.shape[1] > ld:
+            raise KernelError(f"low_rank: columns {col} .. of x {tuple(x.shape)} and w {tuple(w.shape)} do not fit")
+    if (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and 1 <= len(sets) <= 2 and ld % 8 == 0
+            and x.data_ptr() % 16 == 0 and tokens <= 64 * 65535
+            and all(col % 8 == 0 and w.shape[0] % 8 == 0 and w.shape[0] > 0 and w.shape[1] % 8 == 0 and 0 < w.shape[1] <= LOW_RANK_MAX_K
+                    and w.is_cuda and w.is_contiguous() and w.data_ptr() % 16 == 0 for col, w in sets)):
+        out = [torch.empty((tokens, w.shape[0]), dtype=x.dtype, device=x.device) for _, w in sets]
+        (c0, w0), (c1, w1) = sets[0], sets[-1]
+        two = len(sets) == 2
+        _call("low_rank", "ri_low_rank", x.data_ptr(), ld, tokens, c0, w0.shape[1], w0.data_ptr(), out[0].data_ptr(), w0.shape[0],
+              c1, w1.shape[1], w1.data_ptr(), out[-1].data_ptr(), w1.shape[0] if two else 0, _stream())
+        return out
+    return [linear(x[:, col:col + w.shape[1]].contiguous(), w) for col, w in sets]
 
 
 _STREAM_TC_GATES = {"silu": 1, "gelu_tanh": 2, "clamped_swish": 3}

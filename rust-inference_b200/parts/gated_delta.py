@@ -14,7 +14,7 @@ Everything after the projections' and the convolution's rounding is float32.  Pe
 tokens in order from what the steps before left, so a prompt, its pieces and single tokens give the same result.
 
 Order of work: q, k, v, beta and the inner parts of the two low-rank projections (or the decay's and the gate's own
-projections) are one product with the stacked matrix; the small outer products of what is low-rank; convolution and silu (``ops.short_conv``); the recurrence
+projections) are one product with the stacked matrix; the small outer products of what is low-rank (``ops.low_rank``); convolution and silu (``ops.short_conv``); the recurrence
 (``ops.delta_rule_recurrent``: unit vectors, decays, beta and the state); norm and gate in one kernel; the output
 projection.
 """
@@ -115,14 +115,10 @@ class GatedDeltaRule(Mixer):
         with section("delta q/k/v/beta/low-rank proj"):
             proj = ops.linear(x, self.proj)
         with section("delta decay and gate proj"):
-            if self.per_head:
-                za = proj[:, self.a_col:self.a_col + H]
-            else:
-                za = ops.linear(proj[:, self.a_col:self.a_col + self.a_rank].contiguous(), self.a2)
-            if self.g2 is None:
-                zg = proj[:, self.g_col:self.g_col + H * s.vdim]
-            else:
-                zg = ops.linear(proj[:, self.g_col:self.g_col + self.g_rank].contiguous(), self.g2)
+            outer = [(col, w) for col, w in ((self.a_col, self.a2), (self.g_col, self.g2)) if w is not None]
+            outer = ops.low_rank(proj, *outer) if outer else []
+            za = proj[:, self.a_col:self.a_col + H] if self.per_head else outer[0]
+            zg = proj[:, self.g_col:self.g_col + H * s.vdim] if self.g2 is None else outer[-1]
         with section("delta conv"):
             qkv = ops.short_conv(proj, 0, self.conv, cache.more_state[0], ctx.tok_seq, ctx.seq_slot, ctx.seq_start, single=single,
                                  weight_t=self.conv_t)

@@ -9,8 +9,8 @@ With h the mixer's input, per token t and head:
 The state lives in the cache's per-sequence state ([slots, H, dim, vdim]); a step walks its new tokens in
 order from the state the steps before left, so a prompt, its pieces and single tokens give the same result.
 
-Order of work: q, k, v and the gate are one product with the stacked matrix; the decay's two small products; the
-recurrence (``ops.gla_recurrent``, which also turns the decay's projection into the decay); norm and gate in one
+Order of work: q, k, v, the gate and the decay's inner product are one product with the stacked matrix; the decay's outer
+product; the recurrence (``ops.gla_recurrent``, which also turns the decay's projection into the decay); norm and gate in one
 kernel; the output projection.
 """
 from __future__ import annotations
@@ -36,15 +36,20 @@ class GatedLinearAttention(Mixer):
 
     def load(self, tensors):
         s = self.spec
-        self.proj = torch.cat([tensors["q"], tensors["k"], tensors["v"], tensors["g"]], dim=0).contiguous()
+        # the decay's inner matrix with zero rows up to a multiple of 8, so that its columns of the product come in whole pieces, and
+        # a2 with zero columns for them
+        pad = -s.decay_rank % 8
+        a1 = torch.nn.functional.pad(tensors["a1"], (0, 0, 0, pad))
+        self.proj = torch.cat([tensors["q"], tensors["k"], tensors["v"], tensors["g"], a1], dim=0).contiguous()
         self.q_col, self.k_col = 0, s.num_heads * s.dim
         self.v_col = 2 * s.num_heads * s.dim
         self.g_col = self.v_col + s.num_heads * s.vdim
-        self.a1, self.a2, self.bias = tensors["a1"].contiguous(), tensors["a2"].contiguous(), tensors["a2.b"]
+        self.a_col = self.g_col + s.num_heads * s.vdim
+        self.a2, self.bias = torch.nn.functional.pad(tensors["a2"], (0, pad)).contiguous(), tensors["a2.b"]
         self.gain, self.o = tensors["norm"], tensors["o"].contiguous()
 
     def weight_bytes(self):
-        return (self.proj.numel() + self.a1.numel() + self.a2.numel() + self.o.numel()) * self.proj.element_size()
+        return (self.proj.numel() + self.a2.numel() + self.o.numel()) * self.proj.element_size()
 
     def reads_first(self):
         return self.proj
@@ -56,10 +61,10 @@ class GatedLinearAttention(Mixer):
     def __call__(self, x, ctx, cache):
         s = self.spec
         H = s.num_heads
-        with section("gla q/k/v/gate proj"):
+        with section("gla q/k/v/gate/decay proj"):
             proj = ops.linear(x, self.proj)
         with section("gla decay proj"):
-            z = ops.linear(ops.linear(x, self.a1), self.a2)
+            z = ops.low_rank(proj, (self.a_col, self.a2))[0]
         with section("gla recurrence"):
             o = ops.gla_recurrent(proj, self.q_col, self.k_col, self.v_col, z, self.bias, s.tau, s.dim ** -0.5, cache.state,
                                   ctx.seq_slot, ctx.seq_start, H, s.dim, s.vdim, single=ctx.decode_only)

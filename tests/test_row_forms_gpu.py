@@ -81,3 +81,19 @@ def test_latent_rows(tokens, H, dim, rot, rank, row, dtype):
     u, v = q[..., 0::2], q[..., 1::2]
     want = torch.cat([qa.double(), torch.stack([u * c - v * s, v * c + u * s], -1).flatten(-2), torch.zeros((tokens, H, row - rank - rot), device=DEV)], -1)
     _close(results[0][0], want, TOL[dtype])
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17, 64, 65, 300])
+@pytest.mark.parametrize("sets", [[(8, 64, 64)], [(0, 64, 2048), (64, 64, 2048)], [(16, 8, 72), (24, 128, 8)], [(8, 16, 136), (32, 24, 1000)]])
+def test_low_rank_products(tokens, sets):
+    x = _rand(11, tokens, 160).bfloat16()
+    given = [(col, _rand(12 + i, N, K).bfloat16()) for i, (col, K, N) in enumerate(sets)]
+    for (col, w), y in zip(given, ops.low_rank(x, *given)):
+        want = x[:, col:col + w.shape[1]].double() @ w.double().T
+        _close(y, want, 3e-3)                                # one rounding to 8 bits: 2^-9 at most, uniform 2^-9 / sqrt(3)
+        assert torch.equal(y, ops.low_rank(x.clone(), (col, w))[0])
+
+
+def test_low_rank_columns_that_are_not_whole_pieces():
+    x, w = _rand(13, 9, 83).bfloat16(), _rand(14, 50, 20).bfloat16()
+    _close(ops.low_rank(x, (3, w))[0], x[:, 3:23].double() @ w.double().T, 3e-3)
