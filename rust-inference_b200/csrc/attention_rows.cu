@@ -275,6 +275,244 @@ attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, con
     }
 }
 
+// The same rows, the same arithmetic and order of every row, for float32 steps of more than a few rows: a block takes AT_ROWS rows of one kv head
+// (tile_q tokens of all its query heads) and walks the strips with the scores and the outputs in registers, four rows of two keys and four
+// rows of DH / 16 elements a thread.  What bounds it: the words that come from shared memory, 32 a cycle for an SM whether the lanes of a warp want
+// the same ones or not: 0.75 words a multiply-add of the scores and 0.375 of the outputs, where a lane with one key and four rows takes 1.25 for
+// either; for few blocks the chain of a strip.  The next strip's keys are copied under the softmax and the outputs, its values under the scores.
+// Cold, us, this / a row at a time, heads over kv heads of size: 32 / 8 of 128, 512 tokens 141 / 283, 32 behind 300 64 / 160, 8 sequences of one token
+// behind 300 57 / 60; 16 / 2 of 64, 300 tokens 45 / 176; 16 / 1 of 256, 300 tokens 92 / 256.  Tiles of 64 rows (0.5 and 0.25 words) leave two blocks
+// to an SM and take 172, 96, 84; 62; 141.
+#define AT_ROWS 32
+#define AT_MIN_ROWS 8
+#define AT_THREADS 128
+#define AT_P_PITCH 36
+template <bool V> struct AtFlag { static constexpr bool value = V; };
+template <int DH>
+constexpr int at_smem_floats() { return AT_ROWS * (DH + 4) + AR_STRIP * (DH + 4) + AR_STRIP * DH + AT_ROWS * AT_P_PITCH + 2 * AT_ROWS; }
+
+__device__ __forceinline__ void at_copy16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void at_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void at_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+template <int DH>
+__global__ void __launch_bounds__(AT_THREADS, DH <= 128 ? 4 : 2)
+attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool, float* __restrict__ out,
+                      const int* __restrict__ page_table, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
+                      const int* __restrict__ seq_len, int H, int KV, int mpps, int page_size, int num_pages, int tile_q, float scale, int window,
+                      int keep, const float* __restrict__ sink, float softcap, DistBias bias, int* __restrict__ err) {
+    constexpr int PITCH = DH + 4, DC = DH / 64;                   // DC pieces of four elements a thread
+    constexpr int LANES = 16, KEYS = 2, PR = 4;                   // lanes that share four rows, keys of each; rows of outputs
+    static_assert(AT_ROWS * LANES == 4 * AT_THREADS && LANES * KEYS == AR_STRIP && 8 * PR == AT_ROWS, "the threads cover the tile");
+    extern __shared__ __align__(16) float ar_smem[];
+    const int b = blockIdx.z, kvh = blockIdx.y;
+    const int t_begin = seq_start[b], n_new = seq_start[b + 1] - t_begin;
+    const int r_base = (gridDim.x - 1 - blockIdx.x) * tile_q;     // the longest walks first
+    if (r_base >= n_new) return;
+    const int nq = min(tile_q, n_new - r_base), G = H / KV, rows = nq * G;
+    float* qs = ar_smem;                                          // [AT_ROWS][PITCH]
+    float* ks = qs + AT_ROWS * PITCH;                             // [32][PITCH]
+    float* vs = ks + AR_STRIP * PITCH;                            // [32][DH]
+    float* ps = vs + AR_STRIP * DH;                               // [AT_ROWS][AT_P_PITCH]
+    float* s_corr = ps + AT_ROWS * AT_P_PITCH;                    // [AT_ROWS], at the end the rows' factors
+    unsigned* s_mask = reinterpret_cast<unsigned*>(s_corr + AT_ROWS);
+    const int tid = threadIdx.x;
+    const int len = seq_len[b];
+    const int pos0 = len - n_new + r_base, pos_last = pos0 + nq - 1;       // positions of the tile's queries
+    const int key_lo = ri_first_visible(pos0, window);
+    const int* table = page_table + (size_t)seq_slot[b] * mpps;
+    for (int i = tid; i < AT_ROWS * (DH / 4); i += AT_THREADS) {
+        const int row = i / (DH / 4), c = (i % (DH / 4)) * 4, tok = row / G;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (row < rows) v = *reinterpret_cast<const float4*>(q + ((size_t)(t_begin + r_base + tok) * H + kvh * G + row - tok * G) * DH + c);
+        *reinterpret_cast<float4*>(qs + row * PITCH + c) = v;
+    }
+    // strips of 32 keys, whole ones: pages hold a multiple of 32
+    const int window_strip = key_lo - (key_lo % page_size) % AR_STRIP;      // start of the strip that holds key_lo
+    auto next = [&](int& key0) -> long long {                     // the first strip from key0 on that has a page: its elements' place, or -1
+        while (key0 <= pos_last) {
+            if (key0 >= keep && key0 < window_strip) {            // past the strips of the kept keys
+                key0 = window_strip;
+                continue;
+            }
+            const int page_idx = key0 / page_size;
+            const int page = page_idx < mpps ? table[page_idx] : -1;
+            if (page >= 0 && page < num_pages) return (((long long)page * KV + kvh) * page_size + key0 - page_idx * page_size) * DH;
+            if (tid == 0) atomicExch(err, 4);
+            key0 += AR_STRIP;
+        }
+        return -1;
+    };
+    auto copy_k = [&](long long at) {
+        if (at >= 0)
+            for (int i = tid; i < AR_STRIP * (DH / 4); i += AT_THREADS) at_copy16(ks + i / (DH / 4) * PITCH + (i % (DH / 4)) * 4, k_pool + at + (size_t)i * 4);
+        at_commit();
+    };
+    auto copy_v = [&](long long at) {
+        if (at >= 0)
+            for (int i = tid; i < AR_STRIP * (DH / 4); i += AT_THREADS) at_copy16(vs + i * 4, v_pool + at + (size_t)i * 4);
+        at_commit();
+    };
+    // scores: rows 4 ty .., keys tx, tx + LANES, ..;  outputs: rows PR ry .., elements 4 rx + 64 c ..
+    const int ty = tid / LANES, tx = tid % LANES, ry = tid >> 4, rx = tid & 15;
+    float m[4], l[4];
+    int pos[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        m[i] = -INFINITY;
+        l[i] = 0.0f;
+        pos[i] = 4 * ty + i < rows ? pos0 + (4 * ty + i) / G : -1;      // -1: no such row, it sees nothing
+    }
+    float o[PR][DC][4];
+#pragma unroll
+    for (int r = 0; r < PR; r++)
+#pragma unroll
+        for (int c = 0; c < DC; c++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) o[r][c][e] = 0.0f;
+    int key0 = keep > 0 ? 0 : window_strip;
+    long long at = next(key0);
+    copy_k(at);
+    copy_v(at);
+    while (at >= 0) {
+        int key1 = key0 + AR_STRIP;
+        const long long at1 = next(key1);
+        at_wait<1>();                                             // the keys
+        __syncthreads();
+        float s[4][KEYS];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < KEYS; j++) s[i][j] = 0.0f;
+#pragma unroll 4
+        for (int d = 0; d < DH; d += 4) {
+            float4 a[4], k[KEYS];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = *reinterpret_cast<const float4*>(qs + (4 * ty + i) * PITCH + d);
+#pragma unroll
+            for (int j = 0; j < KEYS; j++) k[j] = *reinterpret_cast<const float4*>(ks + (tx + LANES * j) * PITCH + d);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < KEYS; j++) {
+                    s[i][j] = fmaf(a[i].x, k[j].x, s[i][j]);
+                    s[i][j] = fmaf(a[i].y, k[j].y, s[i][j]);
+                    s[i][j] = fmaf(a[i].z, k[j].z, s[i][j]);
+                    s[i][j] = fmaf(a[i].w, k[j].w, s[i][j]);
+                }
+        }
+        __syncthreads();                                          // the keys were read, the weights of the strip before too
+        copy_k(at1);
+        const bool all = key0 + AR_STRIP - 1 <= pos0 && key0 >= ri_first_visible(pos_last, window);      // every row sees every key
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int row = 4 * ty + i;
+            const int first = ri_first_visible(max(pos[i], 0), window);
+            // the row's keys in this strip, as for a row alone
+            const int hole_lo = max(keep - key0, 0), hole_hi = first - key0;
+            const int j_lo = hole_lo > 0 ? 0 : max(hole_hi, 0);
+            int j_hi = min(pos[i] - key0, AR_STRIP - 1);
+            if (hole_hi > j_hi) j_hi = min(j_hi, hole_lo - 1);
+            const bool any = pos[i] >= 0 && j_lo <= j_hi;
+            const float* bias_row = bias.table && any ? ri_bias_row(bias, kvh * G + row % G) : nullptr;
+            bool mine[KEYS];
+            float most = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < KEYS; j++) {
+                const int key = tx + LANES * j;
+                mine[j] = any && key >= j_lo && key <= j_hi && !(key >= hole_lo && key < hole_hi);
+                float v = s[i][j] * scale;
+                if (softcap > 0.0f) v = softcap * tanhf(v / softcap);
+                if (bias_row && mine[j]) v += ri_bias_at(bias_row, bias.len, pos[i] - key0 - key);
+                s[i][j] = mine[j] ? v : -INFINITY;
+                most = fmaxf(most, s[i][j]);
+            }
+#pragma unroll
+            for (int w = LANES / 2; w > 0; w >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, w));
+            const float m_new = fmaxf(m[i], most);
+            const float corr = any ? expf(m[i] - m_new) : 1.0f;
+            float p[KEYS];
+#pragma unroll
+            for (int j = 0; j < KEYS; j++) p[j] = mine[j] ? expf(s[i][j] - m_new) : 0.0f;
+            float sum = p[0] + p[1];                              // the tree of a warp with a key a lane: sixteen apart, eight, four ..
+#pragma unroll
+            for (int w = LANES / 2; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+            if (any) {
+                l[i] = l[i] * corr + sum;
+                m[i] = m_new;
+            }
+#pragma unroll
+            for (int j = 0; j < KEYS; j++) ps[row * AT_P_PITCH + tx + LANES * j] = p[j];
+            if (tx == 0) {
+                s_corr[row] = corr;
+                s_mask[row] = any ? (0xffffffffu >> (31 - j_hi)) & (0xffffffffu << j_lo) : 0u;
+            }
+        }
+        at_wait<1>();                                             // the values
+        __syncthreads();
+        unsigned mask[PR];
+#pragma unroll
+        for (int r = 0; r < PR; r++) {
+            const float corr = s_corr[PR * ry + r];
+            mask[r] = s_mask[PR * ry + r];
+#pragma unroll
+            for (int c = 0; c < DC; c++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) o[r][c][e] *= corr;
+        }
+        auto outputs = [&](auto every) {                          // every: all rows see all keys (a key that a row does not see may hold anything)
+#pragma unroll 2
+            for (int j0 = 0; j0 < AR_STRIP; j0 += 4) {
+                float p[PR][4];
+#pragma unroll
+                for (int r = 0; r < PR; r++) *reinterpret_cast<float4*>(p[r]) = *reinterpret_cast<const float4*>(ps + (PR * ry + r) * AT_P_PITCH + j0);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    float v[DC][4];
+#pragma unroll
+                    for (int c = 0; c < DC; c++) *reinterpret_cast<float4*>(v[c]) = *reinterpret_cast<const float4*>(vs + (j0 + j) * DH + 64 * c + 4 * rx);
+#pragma unroll
+                    for (int r = 0; r < PR; r++) {
+                        if (!decltype(every)::value && !((mask[r] >> (j0 + j)) & 1u)) continue;
+#pragma unroll
+                        for (int c = 0; c < DC; c++)
+#pragma unroll
+                            for (int e = 0; e < 4; e++) o[r][c][e] = fmaf(p[r][j], v[c][e], o[r][c][e]);
+                    }
+                }
+            }
+        };
+        if (all) outputs(AtFlag<true>());
+        else outputs(AtFlag<false>());
+        __syncthreads();                                          // the values were read
+        copy_v(at1);
+        key0 = key1;
+        at = at1;
+    }
+    at_wait<0>();
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = 4 * ty + i;
+        // a sink: one more term exp(sink[head]) in the denominator, with no key and no value (not scaled)
+        if (sink && l[i] > 0.0f) l[i] += expf(sink[kvh * G + row % G] - m[i]);
+        if (tx == 0) s_corr[row] = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;      // no key at all: only after error 4
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < PR; r++) {
+        const int row = PR * ry + r, tok = row / G;
+        if (row >= rows) break;
+        const float inv = s_corr[row];
+        float* dst = out + ((size_t)(t_begin + r_base + tok) * H + kvh * G + row - tok * G) * DH + 4 * rx;
+#pragma unroll
+        for (int c = 0; c < DC; c++)
+            *reinterpret_cast<float4*>(dst + 64 * c) = make_float4(o[r][c][0] * inv, o[r][c][1] * inv, o[r][c][2] * inv, o[r][c][3] * inv);
+    }
+}
+
 // how a launch is cut: rows per block from the shared memory that the staged strip leaves
 static void ar_geometry(int G, int Dh, int max_new, bool vec4, int* tile_q, int* group_chunk, size_t* smem) {
     const size_t strip = (size_t)AR_STRIP * (ar_key_pitch(Dh, vec4) + Dh) * sizeof(float);
@@ -316,6 +554,21 @@ static int ar_launch(const void* q, const void* k_pool, const void* v_pool, void
     return 0;
 }
 
+template <int DH>
+static int at_launch(const void* q, const void* k_pool, const void* v_pool, void* out, const int* page_table, const int* seq_slot,
+                     const int* seq_start, const int* seq_len, int seqs, int max_new, int H, int KV, int mpps, int page_size, int num_pages,
+                     float scale, int window, int keep, const float* sink, float softcap, DistBias bias, int* err_flag, cudaStream_t stream) {
+    constexpr int smem = at_smem_floats<DH>() * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(attention_tile_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) RI_FAIL((int)e, "attention_rows: shared memory limit: %s", cudaGetErrorString(e));
+    const int tile_q = AT_ROWS / (H / KV);
+    attention_tile_kernel<DH><<<dim3((max_new + tile_q - 1) / tile_q, KV, seqs), AT_THREADS, smem, stream>>>(
+        (const float*)q, (const float*)k_pool, (const float*)v_pool, (float*)out, page_table, seq_slot, seq_start, seq_len, H, KV, mpps, page_size,
+        num_pages, tile_q, scale, window, keep, sink, softcap, bias, err_flag);
+    RI_CHECK_LAUNCH("attention_tile");
+    return 0;
+}
+
 // q, out [tokens, H, Dh]; max_new = the most tokens one sequence brings in this step
 // sink [H] float32 or null: a learned term per head that joins the softmax's denominator only
 // softcap > 0: score <- softcap * tanh(score / softcap) after the scale (0: none)
@@ -338,6 +591,18 @@ extern "C" int ri_attention_rows(const void* q, const void* k_pool, const void* 
     // vector loads need rows of the pools and of q that start on 16 bytes (float32) or 8 bytes (bfloat16)
     const uintptr_t align = f32 ? 15 : 7;
     const bool vec4 = Dh % 4 == 0 && (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & align) == 0;
+    // Tiles of rows (the same bits) from AT_MIN_ROWS rows a kv head on.  Cold, behind 300 keys, tiles / a row at a time, us: 32 heads over 8 kv heads of 128,
+    // one token 55 / 60 but one of 24 sequences 74 / 68, two tokens 55 / 63, four 55 / 74; 32 over 32, four tokens 57 / 57, eight 55 / 64; 16 over 2
+    // of 64, one token of 24 sequences 43 / 47.
+    if (f32 && vec4 && ((uintptr_t)out & 15) == 0 && page_size % AR_STRIP == 0 && H / KV <= AT_ROWS && (long long)max_new * (H / KV) >= AT_MIN_ROWS &&
+        KV <= 65535 && seqs <= 65535) {
+#define AT_GO(D) at_launch<D>(q, k_pool, v_pool, out, page_table, seq_slot, seq_start, seq_len, seqs, max_new, H, KV, mpps, page_size, num_pages, \
+                              scale, window, keep, sink, softcap, bias, err_flag, stream)
+        if (Dh == 64) return AT_GO(64);
+        if (Dh == 128) return AT_GO(128);
+        if (Dh == 256) return AT_GO(256);
+#undef AT_GO
+    }
 #define AR_GO(T, V) ar_launch<T, V>(q, k_pool, v_pool, out, page_table, seq_slot, seq_start, seq_len, seqs, max_new, H, KV, \
                                     Dh, mpps, page_size, num_pages, scale, window, keep, sink, softcap, bias, err_flag, stream)
     if (f32) return vec4 ? AR_GO(float, true) : AR_GO(float, false);
