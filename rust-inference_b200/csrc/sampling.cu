@@ -556,17 +556,22 @@ __global__ void sp_select_end_kernel(SpArgs a, int mode, int rows) {
 // A pass over the vocabulary costs about five trips to the L2 cache and a barrier, 6 to 8 us, and a search over five digits
 // has five of them; so only the top digit is searched that way.  What it leaves, the tokens of one bin (a top-k: of that bin
 // and those above it, all that the rest of the work can choose from), goes into a list of 2,048 keys in memory, from which a
-// block ends the search by itself, the same digits and sums over eight keys a thread (the L1 cache has them).  Three barriers with a top-k or a plain
-// draw, four with a top-p, where each search had five and each total one.  A list that does not fit leaves the lower digits to
+// block ends the search by itself, the same digits and sums over eight keys a thread (the L1 cache has them).  The keys' numbers by the
+// top digit, which a top-k searches first, need no maximum: the sweep for the maximum counts them as well.  Two barriers with a top-k, three with
+// a plain draw, four with a top-p, where each search had five and each total one.  A list that does not fit leaves the lower digits to
 // passes over the vocabulary as before: flat rows, a top-k of thousands, and what falls into a crowded bin, since the first
 // digit has no more than the sign and seven bits of the exponent.  8 rows of 151,936 logits, top-k 50 and top-p 0.9,
-// temperature 0.7: spread 2.5 (1,916 keys) 37 us, where a barrier for every digit took 145; spread 3 (4,646 keys) 146.
+// temperature 0.7: spread 2.5 (1,916 keys) 29.6 us, 33.2 with all 4,096 bins of a digit in the top digit's steps, where 256 can be met, 38 with a sweep and a
+// barrier of their own for the top digit's count, and 145 with a barrier for every digit; spread 3 (4,646 keys) 146.
 //
 // Scratch memory per row (SpFusedRow): all zero at the start, the launcher clears it.
 // ---------------------------------------------------------------------------
 #define SPF_TOTALS 4
 #define SPF_TOP ((SP_PASSES - 1) * SP_DIGIT)     // the shift of a key's top digit
+// ... and the bins that it can fall into: the top digit has the key's last eight bits only
+#define SPF_TOP_BINS (1 << (SP_IDX_BITS + 32 - SPF_TOP))
 #define SPF_LIST 2048                       // keys of a list: eight per thread
+static_assert(SPF_TOP_BINS % (SP_BINS / 32) == 0, "whole groups of bins");
 static_assert(2 * SPF_LIST <= SP_BINS, "the lists lie in the histogram that the kernels of one pass each use");
 struct __align__(16) SpFusedRow {
     unsigned arrive;
@@ -578,7 +583,7 @@ struct __align__(16) SpFusedRow {
 struct SpFusedArgs {
     SpArgs a;
     SpFusedRow* rows;        // [rows]
-    u64* hist3;              // [rows][3][SP_BINS]
+    u64* hist3;              // [3][rows][SP_BINS]
     u64* lists;              // [rows][2][SPF_LIST]
     int* err;
 };
@@ -632,7 +637,6 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
     const SpArgs& a = f.a;
     const int row = blockIdx.y, s = blockIdx.x, slices = a.slices;
     SpFusedRow* shared_row = f.rows + row;
-    u64* hist3 = f.hist3 + (size_t)row * 3 * SP_BINS;
     const RowView r = spw_row(a, row);
     const int lo = s * a.per_slice, hi = min(a.vocab, lo + a.per_slice);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -640,21 +644,40 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
     // the copy of the histogram that the next pass adds to, and the step to the one after it (cleared meanwhile); total passes so far
     int hp = 0, turn = 1, ti = 0;
 
+    auto hist_copy = [&](int copy) { return f.hist3 + ((size_t)copy * gridDim.y + row) * SP_BINS; };
     // this block's share of a copy of the row's histogram, cleared
     auto clear_share = [&](int copy) {
-        u64* h = hist3 + (size_t)copy * SP_BINS;
+        u64* h = hist_copy(copy);
         const int per = (SP_BINS + slices - 1) / slices;
         for (int b = s * per + threadIdx.x; b < min(SP_BINS, (s + 1) * per); b += SPW_THREADS) h[b] = 0;
     };
 
-    // ---- the slice's maximum of x and its first index ----------------------------------------------------------
+    unsigned* bins32 = reinterpret_cast<unsigned*>(bins);
+    auto clear_bins = [&](int n) {
+        for (int b = threadIdx.x; b < n; b += SPW_THREADS) bins[b] = 0;
+        __syncthreads();
+    };
+    auto add_top_to = [&](u64* hist) {
+        __syncthreads();
+        for (int b = threadIdx.x; b < SPF_TOP_BINS; b += SPW_THREADS) {
+            const u64 v = bins[b];
+            if (v) atomicAdd(&hist[b], v);
+        }
+    };
+
+    // ---- the slice's maximum of x and its first index; for a top-k the keys' numbers by their top digit on the same way --------------
+    const int k = (use_top_k && a.top_k) ? a.top_k[row] : 0;
+    const bool top_k = k > 0 && k < a.vocab && r.temperature > 0.0f;
     float best = -FLT_MAX;
     int bi = 0x7fffffff;
+    if (top_k) clear_bins(SPF_TOP_BINS);
 #pragma unroll 4
     for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
         float v = r.x(i);
         if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+        if (top_k) atomicAdd(&bins32[2 * ((unsigned)(r.key(i, v / r.temperature) >> SPF_TOP) & (SP_BINS - 1))], 1u);      // a vocabulary's count fits the low word
     }
+    if (top_k) add_top_to(hist_copy(0));                       // (cleared by the launcher)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -669,20 +692,28 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         a.part_val[(size_t)row * slices + s] = best;
         a.part_idx[(size_t)row * slices + s] = bi;
     }
-    clear_share(0);
+    clear_share(top_k ? 1 : 0);
     if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, true, f.err)) return;
-    // the row's maximum from the slices' (every block the same walk, in slice order)
-    if (threadIdx.x == 0) {
+    // the row's maximum from the slices': every block the same
+    if (warp == 0) {
         float rb = -FLT_MAX;
         int ri = 0x7fffffff;
-        for (int q = 0; q < slices; q++) {
+        for (int q = lane; q < slices; q += 32) {
             const float v = __ldcg(a.part_val + (size_t)row * slices + q);
             const int i = __ldcg(a.part_idx + (size_t)row * slices + q);
             if (v > rb || (v == rb && i < ri)) { rb = v; ri = i; }
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float v = __shfl_xor_sync(0xffffffffu, rb, o);
+            const int i = __shfl_xor_sync(0xffffffffu, ri, o);
+            if (v > rb || (v == rb && i < ri)) { rb = v; ri = i; }
+        }
         if (ri == 0x7fffffff) ri = 0;      // a row of NaN: the reference's loop also ends at index 0
-        fred[0] = rb;
-        ired[0] = ri;
+        if (lane == 0) {
+            fred[0] = rb;
+            ired[0] = ri;
+        }
     }
     __syncthreads();
     best = fred[0];
@@ -712,47 +743,37 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
     // w added to a bin: a 64-bit addition to shared memory is a compare-and-swap loop that crawls when many threads want
     // one address, so the low word is added with the old value coming back (which tells whether this addition carried) and
     // the high word takes the carry along.
-    unsigned* bins32 = reinterpret_cast<unsigned*>(bins);
     auto add_bin = [&](unsigned bin, u64 w) {
         const unsigned w_lo = (unsigned)w, w_hi = (unsigned)(w >> 32);
         const unsigned old = atomicAdd(&bins32[2 * bin], w_lo);
         const unsigned carry = old + w_lo < old ? 1u : 0u;
         if (w_hi + carry) atomicAdd(&bins32[2 * bin + 1], w_hi + carry);
     };
-    auto clear_bins = [&]() {
-        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) bins[b] = 0;
-        __syncthreads();
-    };
-    // this slice's part of the top digit's histogram (the sign and seven bits of the exponent: the tokens crowd into a few
+    // this slice's part of the top digit's histogram of weights (the sign and seven bits of the exponent: the tokens crowd into a few
     // bins, each of which spans a factor of four), collected in shared memory
-    auto top_sweep = [&](int counting, u64* hist) {
+    auto top_sweep = [&](u64* hist) {
         __syncthreads();
-        clear_bins();
+        clear_bins(SPF_TOP_BINS);
 #pragma unroll 4
         for (int i = lo + threadIdx.x; i < hi; i += SPW_THREADS) {
             float zi = r.z(i);
             u64 k = r.key(i, zi);
             if (k < floor_key) continue;
-            const u64 w = weight_of(zi, zmax, counting);
-            const unsigned bin = (unsigned)(k >> SPF_TOP) & (SP_BINS - 1);
-            if (counting) atomicAdd(&bins32[2 * bin], 1u);        // a vocabulary's count fits the low word
-            else if (w) add_bin(bin, w);
+            const u64 w = weight_of(zi, zmax, 0);
+            if (w) add_bin((unsigned)(k >> SPF_TOP) & (SP_BINS - 1), w);
         }
-        __syncthreads();
-        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) {
-            const u64 v = bins[b];
-            if (v) atomicAdd(&hist[b], v);
-        }
+        add_top_to(hist);
     };
-    auto read_hist = [&](const u64* hist) {
+    auto read_hist = [&](const u64* hist, int n) {
         __syncthreads();
 #pragma unroll 8
-        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) bins[b] = __ldcg(hist + b);
+        for (int b = threadIdx.x; b < n; b += SPW_THREADS) bins[b] = __ldcg(hist + b);
         __syncthreads();
     };
     // The bin, from the top one down, at which the bins' running sum reaches `remaining`: its digit goes into prefix, what is
     // above it comes off remaining; found 0 when all bins together stay below.
     auto pick = [&](int shift, u64& prefix, u64& remaining, int& found) {
+        const int n = shift == SPF_TOP ? SPF_TOP_BINS : SP_BINS;
         // sums of the 32 groups of 128 bins: a warp takes four groups, its lanes stride through a group
         // (neighbouring lanes, neighbouring bins: no two lanes on one bank)
         {
@@ -762,7 +783,8 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                 const int g = warp * (32 / (SPW_THREADS / 32)) + q;
                 u64 t = 0;
 #pragma unroll
-                for (int j = 0; j < per / 32; j++) t += bins[g * per + j * 32 + lane];
+                for (int j = 0; j < per / 32; j++)
+                    if (g * per < n) t += bins[g * per + j * 32 + lane];
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
                 if (lane == 0) s_group[g] = t;
@@ -817,9 +839,9 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         int found = 1;
         for (; pass >= 0; pass--, hp = (hp + turn) % 3) {
             const int shift = pass * SP_DIGIT;
-            u64* hist = hist3 + (size_t)hp * SP_BINS;
+            u64* hist = hist_copy(hp);
             if (found && pass == SP_PASSES - 1) {
-                top_sweep(counting, hist);
+                top_sweep(hist);                           // (a count's top digit is known from the first sweep)
             } else if (found) {
                 // a lower digit: only the tokens that share the digits found so far count; they are added to the row's
                 // histogram directly
@@ -837,7 +859,7 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
             if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, waits, f.err)) return false;
             if (!waits) return true;                   // the last digit of the draw: slice 0 finishes alone
             if (found) {
-                read_hist(hist);
+                read_hist(hist, pass == SP_PASSES - 1 ? SPF_TOP_BINS : SP_BINS);
                 pick(shift, prefix, remaining, found);
             }
         }
@@ -952,7 +974,7 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                 __syncthreads();
                 break;
             }
-            clear_bins();
+            clear_bins(shift == SPF_TOP ? SPF_TOP_BINS : SP_BINS);
 #pragma unroll
             for (int q = 0; q < SPF_LIST / SPW_THREADS; q++)
                 if (alive >> q & 1) {
@@ -1032,14 +1054,14 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
 
     u64 K;
     int found;
-    const int k = (use_top_k && a.top_k) ? a.top_k[row] : 0;
-    const bool top_k = k > 0 && k < a.vocab;
-    // the top digit of the first search: the count for a top-k, else the weight
-    top_sweep(top_k, hist3);
-    clear_share(1);
-    if (!top_k && tp < 1.0f) clear_share(2);
-    if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, true, f.err)) return;
-    read_hist(hist3);
+    // the top digit of the first search: the count for a top-k, which is there, else the weight
+    if (!top_k) {
+        top_sweep(hist_copy(0));
+        clear_share(1);
+        if (tp < 1.0f) clear_share(2);
+        if (!spf_barrier(&shared_row->arrive, ++barriers * (unsigned)slices, true, f.err)) return;
+    }
+    read_hist(hist_copy(0), SPF_TOP_BINS);
     hp = 1;
     bool narrowed = false;                                // the vocabulary is down to floor_key and `total` is its weight
     if (top_k) {
@@ -1075,7 +1097,7 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
         narrowed = true;
     } else {
         u64 part = 0;
-        for (int b = threadIdx.x; b < SP_BINS; b += SPW_THREADS) part += bins[b];
+        for (int b = threadIdx.x; b < SPF_TOP_BINS; b += SPW_THREADS) part += bins[b];
         total = block_sum_u64(part, red);
         unsigned floor_bin = 0;                           // bins below it are out; list 0 has its keys when floor_listed
         bool floor_listed = false;
@@ -1091,7 +1113,7 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                 const bool listing = !too_many(floor_bin);
                 unsigned n = SPF_LIST + 1;
                 if (listing) {
-                    if (!gather(floor_bin, floor_bin, 0, true, hist3 + 2 * SP_BINS)) return;
+                    if (!gather(floor_bin, floor_bin, 0, true, hist_copy(2))) return;
                     n = __ldcg(&shared_row->listed[0]);
                 }
                 if (n <= SPF_LIST) {
@@ -1103,14 +1125,14 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                         inside = list_sum(K);
                         total = above + inside;
                     }
-                    read_hist(hist3);
+                    read_hist(hist_copy(0), SPF_TOP_BINS);
                     if (floor_listed) {
                         for (int b = threadIdx.x; b <= (int)floor_bin; b += SPW_THREADS) bins[b] = b == (int)floor_bin ? inside : 0;
                         __syncthreads();
                     }
                 } else {
                     if (listing) {
-                        read_hist(hist3 + 2 * SP_BINS);
+                        read_hist(hist_copy(2), SP_BINS);
                         pick(SPF_TOP - SP_DIGIT, prefix, remaining, found);
                         turn = 2;
                     }
@@ -1134,12 +1156,12 @@ __global__ void __launch_bounds__(SPW_THREADS) sp_fused_kernel(SpFusedArgs f, in
                 unsigned n = SPF_LIST + 1;
                 if (listing) {
                     clear_share(2);
-                    if (!gather(bin, bin, 1, true, hist3 + SP_BINS)) return;
+                    if (!gather(bin, bin, 1, true, hist_copy(1))) return;
                     n = __ldcg(&shared_row->listed[1]);
                 }
                 if (n > SPF_LIST) {
                     if (listing) {
-                        read_hist(hist3 + SP_BINS);
+                        read_hist(hist_copy(1), SP_BINS);
                         pick(SPF_TOP - SP_DIGIT, prefix, remaining, found);
                         hp = 2;
                     }
@@ -1212,7 +1234,9 @@ static int launch_sample_wide(SpArgs a, int rows, void* work, int use_top_k, int
         const int fit = spw_fused_capacity() / rows;
         if (a.slices > fit) a.slices = fit;
         a.per_slice = (a.vocab + a.slices - 1) / a.slices;
-        cudaError_t e = cudaMemsetAsync(fused_rows, 0, (size_t)rows * sizeof(SpFusedRow), stream);
+        // the rows' words, and with a top-k the first copies of their histograms, which lie behind them
+        const size_t words = use_top_k ? spw_align((size_t)rows * sizeof(SpFusedRow)) + (size_t)rows * SP_BINS * sizeof(u64) : (size_t)rows * sizeof(SpFusedRow);
+        cudaError_t e = cudaMemsetAsync(fused_rows, 0, words, stream);
         if (e != cudaSuccess) RI_FAIL((int)e, "sample: %s", cudaGetErrorString(e));
         SpFusedArgs f;
         f.a = a;
