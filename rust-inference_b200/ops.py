@@ -155,7 +155,7 @@ class KernelError(RuntimeError):
 
 
 def _fn(lib_name: str, fn_name: str, defines=None):
-    key = (lib_name, fn_name, tuple(sorted((defines or {}).items())))
+    key = (lib_name, fn_name) if defines is None else (lib_name, fn_name, tuple(sorted(defines.items())))
     f = _fn_cache.get(key)
     if f is None:
         lib = _build.library(lib_name, defines)
@@ -186,8 +186,15 @@ def _call(lib_name: str, fn_name: str, *args, defines=None):
         raise KernelError(f"{fn_name}: {lib.ri_last_error().decode(errors='replace')} (code {rc})")
 
 
+# The current stream's handle without the object around it: 0.2 us in place of 3.2, at every launch
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None or _raw_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_raw_device())
 
 
 def _code(dtype: torch.dtype) -> int:
@@ -220,8 +227,11 @@ def error_flag(device) -> torch.Tensor:
     """One int32 per device that kernels set when they meet an index they must
     not follow (an unmapped page, a token id or position out of range).  The
     engine reads it whenever it synchronises anyway."""
+    f = _err_flags.get(device)                  # (a tensor's device: it has an index)
+    if f is not None:
+        return f
     dev = torch.device(device)
-    key = (dev.type, dev.index if dev.index is not None else torch.cuda.current_device())
+    key = dev if dev.index is not None else torch.device(dev.type, torch.cuda.current_device())
     f = _err_flags.get(key)
     if f is None:
         f = torch.zeros(1, dtype=torch.int32, device=dev)
