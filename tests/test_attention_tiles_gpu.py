@@ -1,4 +1,4 @@
-"""The float32 attention over many rows (tiles of 64 rows and strips of 32 keys in registers): bit for bit what the form with a row per
+"""The float32 attention over many rows (tiles of 32 rows and strips of 32 keys in registers): bit for bit what the form with a row per
 warp gives, which rows of queries that do not start on 16 bytes take, over all kinds of masks, and against float64."""
 import numpy as np
 import pytest
