@@ -262,8 +262,8 @@ delta_prep_kernel(float* __restrict__ qkv, int C, int q_col, int k_col, const T*
         beta[(size_t)t * (H + G) + h] = 1.0f / (1.0f + expf(-ld_f(proj + (size_t)t * ld + b_col + h)));
 }
 
-// The same for heads of whole groups of four channels (up to 128 PIECES of them): a lane has four neighbouring channels of q and k, a
-// thread four neighbouring decays, whose rate is taken once.  What bounds it: memory and, beside it, the functions of the decays.  2,048
+// The same, bit for bit, for heads of whole groups of four channels (up to 128 PIECES of them): a lane's channels of q and k are asked for
+// together, a thread has four neighbouring decays, whose rate is taken once.  What bounds it: memory and, beside it, the functions of the decays.  2,048
 // tokens, 8 q/k heads and 16 heads of 128 (73 MB), behind the convolution: 14 us, 28 a channel at a time.
 __device__ __forceinline__ float4 dr_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 dr_ld4(const __nv_bfloat16* p) {
@@ -283,22 +283,19 @@ delta_prep_vec_kernel(float* __restrict__ qkv, int C, int q_col, int k_col, cons
     for (int g = blockIdx.y * 8 + warp; g < G; g += 8 * gridDim.y) {      // a warp per q/k head: both unit vectors and their product
         float* q = row + q_col + g * dim;
         float* k = row + k_col + g * dim;
-        float4 a[PIECES], b[PIECES];
+        float a[4 * PIECES], b[4 * PIECES];                     // channels lane, lane + 32, ..: a lane's sums go over them in that order
 #pragma unroll
-        for (int p = 0; p < PIECES; p++) {
-            const int d = p * 128 + 4 * lane;
-            a[p] = b[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (d < dim) {
-                a[p] = dr_ld4(q + d);
-                b[p] = dr_ld4(k + d);
-            }
+        for (int p = 0; p < 4 * PIECES; p++) {
+            const int d = p * 32 + lane;
+            a[p] = d < dim ? q[d] : 0.0f;
+            b[p] = d < dim ? k[d] : 0.0f;
         }
         float sq = 0.0f, sk = 0.0f, qk = 0.0f;
 #pragma unroll
-        for (int p = 0; p < PIECES; p++) {
-            sq = fmaf(a[p].x, a[p].x, fmaf(a[p].y, a[p].y, fmaf(a[p].z, a[p].z, fmaf(a[p].w, a[p].w, sq))));
-            sk = fmaf(b[p].x, b[p].x, fmaf(b[p].y, b[p].y, fmaf(b[p].z, b[p].z, fmaf(b[p].w, b[p].w, sk))));
-            qk = fmaf(a[p].x, b[p].x, fmaf(a[p].y, b[p].y, fmaf(a[p].z, b[p].z, fmaf(a[p].w, b[p].w, qk))));
+        for (int p = 0; p < 4 * PIECES; p++) {
+            sq = fmaf(a[p], a[p], sq);
+            sk = fmaf(b[p], b[p], sk);
+            qk = fmaf(a[p], b[p], qk);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -308,11 +305,11 @@ delta_prep_vec_kernel(float* __restrict__ qkv, int C, int q_col, int k_col, cons
         }
         const float iq = qscale / sqrtf(sq + 1e-6f), ik = 1.0f / sqrtf(sk + 1e-6f);
 #pragma unroll
-        for (int p = 0; p < PIECES; p++) {
-            const int d = p * 128 + 4 * lane;
+        for (int p = 0; p < 4 * PIECES; p++) {
+            const int d = p * 32 + lane;
             if (d < dim) {
-                *reinterpret_cast<float4*>(q + d) = make_float4(a[p].x * iq, a[p].y * iq, a[p].z * iq, a[p].w * iq);
-                *reinterpret_cast<float4*>(k + d) = make_float4(b[p].x * ik, b[p].y * ik, b[p].z * ik, b[p].w * ik);
+                q[d] = a[p] * iq;
+                k[d] = b[p] * ik;
             }
         }
         if (lane == 0) beta[(size_t)t * (H + G) + H + g] = qk * iq * ik;

@@ -36,6 +36,30 @@ def test_head_norm_gate(tokens, heads, vdim, fn, dtype):
         _close(ops.head_norm_gate(o, gain, 1e-6, g, DT[dtype], fn).view(tokens, heads, vdim), want, TOL[dtype])
 
 
+def _at_odd_place(t):
+    """The same values as a block of columns that starts one element behind a whole piece."""
+    wide = torch.empty((t.shape[0], t.shape[1] + 5), dtype=t.dtype, device=DEV)
+    wide[:, 1:1 + t.shape[1]] = t
+    return wide[:, 1:1 + t.shape[1]]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("tokens, H, G, dim", [(1, 2, 1, 4), (3, 4, 2, 36), (300, 4, 4, 128), (65, 2, 1, 132), (257, 2, 2, 260), (7, 2, 1, 512)])
+def test_unit_vectors_and_decays_give_the_bits_of_a_channel_at_a_time(tokens, H, G, dim, dtype):
+    vdim = 8
+    qkv = _rand(18, tokens, 2 * G * dim + H * vdim)
+    proj, z = _rand(19, tokens, H).to(DT[dtype]), _rand(20, tokens, H * dim).to(DT[dtype])
+    dt_bias, a_log = _rand(21, H * dim), 0.3 * _rand(22, H)
+    results = []
+    for decays in (z, _at_odd_place(z)):                      # the second: a channel at a time
+        q, state = qkv.clone(), _rand(23, 1, H, dim, vdim)
+        o = ops.delta_rule_recurrent(q, 0, G * dim, 2 * G * dim, proj, 0, decays, dt_bias, a_log, dim ** -0.5, state, _i32([0]), _i32([0, tokens]),
+                                     H, G, dim, vdim)
+        results.append((q, o, state))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 # from 256 tokens on four tokens a thread; sequences that begin and end anywhere in a thread's four, of one and two tokens too
 @pytest.mark.parametrize("lens", [[256], [259], [1, 2, 3, 250, 1, 1, 4], [64] * 5, [255, 2]])
 def test_short_conv_over_many_tokens(lens):
