@@ -724,7 +724,8 @@ __global__ void gla_head_norm_gate_kernel(const float* __restrict__ o, const flo
     }
 }
 
-// The same for rows of whole groups of four columns, up to 128 PIECES: a lane has four neighbouring columns (PIECES times).  What bounds it:
+// The same, bit for bit, for rows of whole groups of four columns, up to 128 PIECES: a lane has four neighbouring columns (PIECES times).  Its
+// part of the sum goes over the columns lane, lane + 32, .. all the same, which it reads beside them from the same lines.  What bounds it:
 // memory, and the gate's functions beside it.  2,302 tokens of 32 heads of 128 columns (75 MB): 21 us, 31 with a column a lane and
 // trip; two or four rows a warp with their loads on their way together take 21 and 23.
 template <typename T, int PIECES>
@@ -739,7 +740,10 @@ gla_head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restri
     const size_t t = unit / H;
     const int h = (int)(unit - t * H);
     float4 v[PIECES], gn[PIECES];
+    float part[4 * PIECES];
     GlaFour<T> z[PIECES];
+#pragma unroll
+    for (int p = 0; p < 4 * PIECES; p++) part[p] = p * 32 + lane < vdim ? o[unit * vdim + p * 32 + lane] : 0.0f;
 #pragma unroll
     for (int p = 0; p < PIECES; p++) {
         const int j = p * 128 + 4 * lane, at = j < vdim ? j : 0;
@@ -749,8 +753,7 @@ gla_head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restri
     }
     float ss = 0.0f;
 #pragma unroll
-    for (int p = 0; p < PIECES; p++)
-        if (p * 128 + 4 * lane < vdim) ss += (v[p].x * v[p].x + v[p].y * v[p].y) + (v[p].z * v[p].z + v[p].w * v[p].w);
+    for (int p = 0; p < 4 * PIECES; p++) ss = fmaf(part[p], part[p], ss);
     const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)vdim + eps);
 #pragma unroll
     for (int p = 0; p < PIECES; p++) {

@@ -44,6 +44,14 @@ def _at_odd_place(t):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("tokens, heads, vdim", [(1, 1, 4), (3, 5, 96), (700, 16, 128), (70, 3, 132), (40, 2, 256)])
+def test_head_norm_gate_gives_the_bits_of_a_column_at_a_time(tokens, heads, vdim, dtype):
+    o, gain, g = _rand(15, tokens, heads, vdim), 1 + 0.1 * _rand(16, vdim), _rand(17, tokens, heads * vdim).to(DT[dtype])
+    for fn in ("silu", "sigmoid"):
+        assert torch.equal(ops.head_norm_gate(o, gain, 1e-6, g, DT[dtype], fn), ops.head_norm_gate(o, gain, 1e-6, _at_odd_place(g), DT[dtype], fn))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("tokens, H, G, dim", [(1, 2, 1, 4), (3, 4, 2, 36), (300, 4, 4, 128), (65, 2, 1, 132), (257, 2, 2, 260), (7, 2, 1, 512)])
 def test_unit_vectors_and_decays_give_the_bits_of_a_channel_at_a_time(tokens, H, G, dim, dtype):
     vdim = 8
