@@ -72,7 +72,7 @@ _SIGNATURES = {
     ("sampling", "ri_mark_seen"): [_P, _L, _P, _P, _I, _I, _P],
     ("attention_decode", "ri_attention_decode_sink"): [_P] * 9 + [_I] * 8 + [_F, _I, _P, _P, _P],
     ("attention_decode", "ri_attention_decode_cap"): [_P] * 9 + [_I] * 8 + [_F, _I, _P, _F, _P, _I] + [_I, _I, _I, _F, _F, _F] + [_P, _P],
-    ("low_rank", "ri_low_rank"): [_P, _L, _I, _I, _I, _P, _P, _I, _I, _I, _P, _P, _I, _P],
+    ("low_rank", "ri_low_rank"): [_P, _L] + [_I, _I, _I, _P, _P, _I, _I] + [_I, _I, _P, _P, _I, _I] + [_P],
     ("linear_skinny", "ri_linear_skinny"): [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     ("linear_skinny", "ri_linear_skinny_act"): [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     ("linear_skinny", "ri_linear_skinny_gated"): [_P, _P, _P, _I, _I, _I, _I, _P, _P],
@@ -768,7 +768,7 @@ def low_rank(x: torch.Tensor, *sets) -> list:
     """The outer products of low-rank projections: for every (col, w) of ``sets``, w [N, K], the product
     x[:, col:col + K] w^T [tokens, N].  ``x`` [tokens, columns] holds the inner parts side by side.
     bfloat16, up to two products of K up to 128 over columns in multiples of 8: one kernel of this package (mma.sync) that
-    reads the columns where they lie; anything else a copy of the columns and ``linear`` each."""
+    reads the columns where they lie; anything else a copy of the columns and ``linear`` each.  The same bits either way."""
     tokens, ld = x.shape
     for col, w in sets:
         if w.dim() != 2 or w.dtype != x.dtype or col < 0 or col + w.shape[1] > ld:
@@ -780,8 +780,9 @@ def low_rank(x: torch.Tensor, *sets) -> list:
         out = [torch.empty((tokens, w.shape[0]), dtype=x.dtype, device=x.device) for _, w in sets]
         (c0, w0), (c1, w1) = sets[0], sets[-1]
         two = len(sets) == 2
-        _call("low_rank", "ri_low_rank", x.data_ptr(), ld, tokens, c0, w0.shape[1], w0.data_ptr(), out[0].data_ptr(), w0.shape[0],
-              c1, w1.shape[1], w1.data_ptr(), out[-1].data_ptr(), w1.shape[0] if two else 0, _stream())
+        s0, s1 = (int(_takes_skinny(tokens, w.shape[0], w.shape[1], x.device)) for w in (w0, w1))
+        _call("low_rank", "ri_low_rank", x.data_ptr(), ld, tokens, c0, w0.shape[1], w0.data_ptr(), out[0].data_ptr(), w0.shape[0], s0,
+              c1, w1.shape[1], w1.data_ptr(), out[-1].data_ptr(), w1.shape[0] if two else 0, s1, _stream())
         return out
     return [linear(x[:, col:col + w.shape[1]].contiguous(), w) for col, w in sets]
 

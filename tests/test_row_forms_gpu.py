@@ -126,6 +126,15 @@ def test_low_rank_products(tokens, sets):
         assert torch.equal(y, ops.low_rank(x.clone(), (col, w))[0])
 
 
+# the product's order of sums changes with its kernel: the weight-streaming one up to 12 tokens and for few outputs up to 16, then the
+# tcgen05 one, then the library's
+@pytest.mark.parametrize("tokens", [1, 8, 12, 13, 16, 17, 32, 33, 65, 1000])
+@pytest.mark.parametrize("K, N", [(8, 1024), (24, 2048), (64, 2048), (72, 5000), (128, 1024), (128, 5632)])
+def test_low_rank_products_give_the_bits_of_the_product_of_a_copy(tokens, K, N):
+    x, w = _rand(24, tokens, 256).bfloat16(), _rand(25, N, K).bfloat16()
+    assert torch.equal(ops.low_rank(x, (16, w))[0], ops.linear(x[:, 16:16 + K].contiguous(), w))
+
+
 def test_low_rank_columns_that_are_not_whole_pieces():
     x, w = _rand(13, 9, 83).bfloat16(), _rand(14, 50, 20).bfloat16()
     _close(ops.low_rank(x, (3, w))[0], x[:, 3:23].double() @ w.double().T, 3e-3)
