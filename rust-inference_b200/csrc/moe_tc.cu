@@ -35,8 +35,10 @@
 // 704: 12 pairs 116 / 100, 50 pairs 114 / 138.  So the two forms meet at some 25 pairs, and from there to 47 the plan takes the
 // slower one by up to 40 %; a wide step costs the host a launch more, which is what bounds small ones.
 //
-// Waits are bounded (error 5): whoever gives up says so in shared memory, no further copy or product is started, the copies
-// under way are waited for once more, and the block ends as usual with a wrong result.
+// Waits are bounded (error 5): whoever gives up says so in shared memory, the other roles end when they next have to wait, the copies
+// under way land (`mt_land`), and the blocks end as usual with a wrong result.  -DMT_TEST_STOP_COPY_K=<k> (tests only; nothing in
+// an ordinary build) makes one copying warp of each block of the first pair give up before the fourth stage in launches with K == k, a's
+// in the first block and W's in the second, so that this path can be run with copies that nobody else completes.
 #include "common.cuh"
 #include "mma_helpers.cuh"
 #include <cuda.h>
@@ -170,6 +172,7 @@ struct MtTail {
     unsigned long long full[MT_STAGES], empty[MT_STAGES], acc_full[2], acc_empty[2], drained;
     unsigned tmem_base;
     int dead;
+    int fills[2];                          // how often the block's copying warps have filled a stage: a, W
 };
 static_assert(sizeof(MtTail) <= 256, "the tail fits behind the stages");
 
@@ -179,7 +182,8 @@ __device__ __forceinline__ bool mt_test(unsigned long long* bar, unsigned parity
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return __all_sync(0xffffffffu, ok);
 }
-// A warp's wait: false when it ran out, or when somebody else has given up (nothing further is started then).
+// A warp's wait: false when it ran out, or when it took long and somebody in the block has given up meanwhile.  Whoever finds the
+// barrier over goes on, so that the copying warps may stop at different stages: `mt_land` sees to what is then under way.
 __device__ __forceinline__ bool mt_wait(unsigned long long* bar, unsigned parity, MtTail& tail, int* err) {
     if (mt_test(bar, parity)) return true;
     if (!__all_sync(0xffffffffu, ri_mbar_wait(bar, parity))) {
@@ -193,6 +197,31 @@ __device__ __forceinline__ bool mt_elect() {
     unsigned one;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(one));
     return one != 0;
+}
+
+// After somebody has given up: the copies that were started land before either block leaves.  One thread of both blocks calls this, behind
+// a barrier of the cluster, when no product is under way.  A stage is full when all four copies into it (a and W of both blocks) are, but
+// the four warps may have stopped at different stages; so each block makes up what its own warps have not started of the stages
+// that somebody has (any rows do), after which every such barrier completes, and the first block, whose barriers they are, waits for
+// the last round of them.  No two warps are a whole round apart: a stage is filled again only when its products, which need all four
+// copies, are done.
+__device__ __forceinline__ void mt_land(const CUtensorMap* map_a, const CUtensorMap* map_w, MtTail& tail, unsigned ring, unsigned rank) {
+    int most = 0;
+    for (unsigned r = 0; r < 2; r++)
+        for (int i = 0; i < 2; i++) {
+            int f;
+            asm volatile("ld.shared::cluster.s32 %0, [%1];\n" : "=r"(f) : "r"(mt_in_block(&tail.fills[i], r)) : "memory");
+            most = max(most, f);
+        }
+    for (int i = 0; i < 2; i++)
+        for (int f = tail.fills[i]; f < most; f++) {
+            const int s = f % MT_STAGES;
+            if (i == 0 && rank == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&tail.full[s])), "r"(2 * MT_STAGE_BYTES) : "memory");
+            mt_box(ring + s * MT_STAGE_BYTES + (i ? MT_A_BYTES : 0), i ? map_w : map_a, 0, 0, mt_in_block(&tail.full[s], 0));
+        }
+    if (rank == 0)
+        for (int f = max(0, most - MT_STAGES); f < most; f++) ri_mbar_wait(&tail.full[f % MT_STAGES], (unsigned)((f / MT_STAGES) & 1));
 }
 
 // N: outputs per row (with a gate: channels, W has 2 N rows per expert); y rows start ldy elements apart
@@ -254,6 +283,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             const int w0 = GATED ? e * 2 * N + (int)rank * N + n0 : e * N + n0 + (int)rank * (MT_COLS / 2);
             for (int k = 0; k < steps; k++) {
                 if (laps > 0 && !mt_wait(&tail.empty[s], (unsigned)((laps - 1) & 1), tail, err)) { ok = false; break; }
+#ifdef MT_TEST_STOP_COPY_K
+                if (K == MT_TEST_STOP_COPY_K && blockIdx.x < 2 && warp == 6 * rank && laps * MT_STAGES + s == 3) {      // tests only: see the top
+                    atomicExch(err, 5);
+                    *(volatile int*)&tail.dead = 1;
+                    ok = false;
+                    break;
+                }
+#endif
                 if (one) {
                     if (warp == 6) {
                         mt_box(ring + s * MT_STAGE_BYTES, &map_w, k * MT_STAGE_K, w0, bars + s * 8);
@@ -270,9 +307,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                 }
             }
         }
-        if (rank == 0 && warp == 0 && one && *(volatile int*)&tail.dead)       // somebody gave up: what was started lands first
-            for (int i = 0; i < MT_STAGES; i++)
-                if (i < s || laps > 0) ri_mbar_wait(&tail.full[i], (unsigned)((i < s ? laps : laps - 1) & 1));
+        if (one) tail.fills[warp == 0 ? 0 : 1] = laps * MT_STAGES + s;
         __syncwarp();
     } else if (warp == 1) {
         // ---- products ----------------------------------------------------------------------------------------------------
@@ -367,6 +402,13 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     __syncthreads();
     if (rank == 1 && tid == 0) ri_mbar_wait(&tail.drained, 0);     // the last commit has reached this block as well
     mt_cluster_sync();                             // nobody leaves while the other block may still signal its barriers
+    int gave_up;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];\n" : "=r"(gave_up) : "r"(mt_in_block(&tail.dead, rank ^ 1)) : "memory");
+    if (gave_up | *(volatile int*)&tail.dead) {    // (the same in both blocks, whose roles are all over)
+        if (tid == 0) mt_land(&map_a, &map_w, tail, smem_u32(mt_smem), rank);
+        __syncthreads();
+        mt_cluster_sync();
+    }
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
 }

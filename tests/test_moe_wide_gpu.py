@@ -163,3 +163,47 @@ def test_few_tokens_in_rings_of_three_and_four_stages(E, N, K):
     gate, up = want[plan[0].long()].chunk(2, dim=1)
     want = gate * torch.sigmoid(gate) * up
     assert ((gated.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+
+
+def test_copying_warps_that_stop_at_different_stages():
+    """The way out of a wait that has run out, with one copying warp of each block of the first pair of blocks stopped (by a test-only
+    define, for K = 1536) before its fourth stage while the other copies go on to the end of the ring.  Error 5 is reported, what was
+    started lands, the kernel returns, the other tiles are right, and so is the next launch.  Nothing hangs or faults: the waits are the
+    bounded ones."""
+    import os
+    import subprocess
+    import sys
+    code = r'''
+import time, torch
+from rust_inference_b200 import ops
+torch.manual_seed(0)
+flag = ops.error_flag("cuda")
+def run(K):
+    x = torch.randn(700, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2, 520, K, device="cuda") * 0.1).to(torch.bfloat16)
+    idx = torch.randint(0, 2, (700, 1), device="cuda", dtype=torch.int32)
+    plan = ops.moe_plan(idx, 2, True)
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    y = ops.moe_grouped_linear(x, w, plan, 700, gather_div=1, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    ms = (time.perf_counter() - t0) * 1e3
+    perm = plan[0].long()
+    want = torch.stack([x[perm].float() @ w[e].float().t() for e in range(2)])[idx.flatten().long()[perm], torch.arange(700, device="cuda")]
+    near = (y - want).abs() <= 1e-3 * want.abs().max()
+    return near, ms
+assert run(1024)[0].all() and int(flag.item()) == 0               # builds and loads the library (another K: nothing stops)
+near, ms = run(1536)
+assert int(flag.item()) == 5, int(flag.item())
+flag.zero_()
+assert near[256:].all() and near[:, 256:].all(), "the other tiles"
+assert not near[:256, :256].all(), "nothing was stopped"
+assert run(1536 + 64)[0].all() and int(flag.item()) == 0
+print("gave up after %.1f ms" % ms)
+'''
+    env = dict(os.environ, RUST_INFERENCE_B200_DEFINES="MT_TEST_STOP_COPY_K=1536", PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600, env=env)
+    assert r.returncode == 0, r.stdout + r.stderr
+    # the products' wait and those of the epilogues (4 ms each, side by side); a copy that never landed would add one for each stage
+    ms = float(r.stdout.split("after")[1].split()[0])
+    assert 3.0 <= ms <= 2000.0, r.stdout
