@@ -2,8 +2,8 @@
 // `ri_linear_f32`, `ri_linear_heads_f32`: multiply-adds on the CUDA cores.  Every output element is the sum over
 // k = 0..K-1 in that order with one accumulator, whatever M, N and the tile a row falls into: a token's result does not
 // depend on what it is batched with.
-// `ri_linear_f32_tc`: exact cuts of the float32 values into bfloat16 on the tensor cores (linear_f32_tc.cuh), likewise one chain per
-// output whatever M, N and the tile.
+// `ri_linear_f32_tc`: exact cuts of the float32 values into bfloat16 on the tensor cores (linear_f32_tc.cuh), likewise the same chains for
+// every output whatever M, N and the tile.
 // Formula: thanhauco/rust-inference src/ops/linear.rs:7-20.
 #include "common.cuh"
 #include "linear_f32_tc.cuh"
@@ -188,7 +188,7 @@ static int lt_launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const f
                      int tn, int* err, cudaStream_t stream) {
     auto kernel = linear_f32_tc_kernel<CH, GROUPS, BUFS>;
     const int stage = LT_W_BYTES + 3 * 64 * tn;
-    int stages = LT_SMEM_MAX / stage, wstages = (512 - BUFS * tn) / LT_W_COLS;
+    int stages = LT_SMEM_MAX / stage, wstages = (512 - (BUFS + 1) * tn) / LT_W_COLS;
     if (stages > LT_MAX_STAGES) stages = LT_MAX_STAGES;
     if (wstages > LT_MAX_WSTAGES) wstages = LT_MAX_WSTAGES;
     // A wait knows a barrier's phases by their parity only, so that whoever waits must know the phase before to be over.  A place of the
@@ -214,14 +214,31 @@ static int lt_launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const f
     return 0;
 }
 
+// Tokens a block: the multiple of 16 with the least time, rounds of blocks (one an SM) times what a round takes, some 57 us +
+// 0.285 a token at K = 4,096 where the blocks fill the device (16 tokens 55, 128 and 48 blocks 68, 176 and 48 blocks 69, 176 and 144 blocks 112).
+static int lt_tokens(int rows, int N, int sms) {
+    int tn = 16;
+    double least = 0;
+    for (int t = 16; t <= LT_MAX_TOKENS; t += 16) {
+        const long long blocks = (long long)((N + LT_ROWS - 1) / LT_ROWS) * ((rows + t - 1) / t);
+        const double time = (double)((blocks + sms - 1) / sms) * (57 + 0.285 * t);
+        if (t == 16 || time < least) {
+            tn = t;
+            least = time;
+        }
+    }
+    return tn;
+}
+
 // `parts`: scratch for the cut rows of x, 6 bytes for each of K rounded up to 32 and each of `part_rows` rows; more rows than that are
 // taken in several launches.  K a multiple of 4, x and w on 16 bytes.
 //
-// Tokens a block: the multiple of 16 with the least time, rounds of blocks (one an SM) times what a round takes.  Measured in us at K =
-// 4,096 with the cut of x: 16 tokens 60, 48 70, 96 85, 128 91, 176 107, that is some 57 + 0.285 a token; two rounds of 128 tokens 165, four of
-// 176 445.  At that K, the tensor cores' form / multiply-adds: 512 tokens and 6,144 outputs 114 / 640, 512 and 4,096 93 / 454, 300 and 6,144 90
-// / 454, 128 and 6,144 73 / 269, 16 and 6,144 61 / 190, 1 and 4,096 60 / 190; K = 2,048, 300 and 4,096 48 / 184.  2-norm of the error against float64
-// over that of the result: 2.3e-7 / 1.15e-6 at K = 4,096, 1.3e-7 / 4.0e-7 at 512, 1.2e-7 / 2.5e-7 at 200.
+// Cold, with the cut of x, in us at K = 4,096, tensor cores / multiply-adds: 512 tokens and 6,144 outputs 112 / 639,
+// 512 and 4,096 87 / 449, 300 and 6,144 85 / 450, 128 and 6,144 68 / 265, 16 and 6,144 55 / 184, 1 and 4,096 53 / 184; K = 2,048, 300 and 4,096 42 / 180;
+// K = 512, 300 and 4,096 16 / 47, 1 and 4,096 9.6 / 24.
+// 2-norm of the error against float64 over that of the result, normal values: 2.2e-7 / 1.15e-6 at K = 4,096, 9.0e-8 / 4.1e-7 at 512,
+// 6.2e-8 / 2.0e-7 at 128; with one entry that is not zero 2.60e-8 / 2.53e-8, two 2.6e-8 / 3.1e-8, four 2.7e-8 / 4.0e-8, 32 4.4e-8 / 1.0e-7; all of
+// one sign and size, K = 4,096, 1.2e-7 / 8.6e-7.  With all terms in one sum of 32 k, parts cut towards zero: 1.0e-7 for one entry, 1.1e-7 for four.
 extern "C" int ri_linear_f32_tc(const float* x, const float* w, float* y, void* parts, int part_rows, int M, int N, int K, int* err_flag,
                                 cudaStream_t stream) {
     if (M == 0 || N == 0) return 0;
@@ -252,16 +269,7 @@ extern "C" int ri_linear_f32_tc(const float* x, const float* w, float* y, void* 
     }
     for (int at = 0; at < M; at += part_rows) {
         const int rows = M - at < part_rows ? M - at : part_rows;
-        int tn = 16;
-        double least = 0;
-        for (int t = 16; t <= LT_MAX_TOKENS; t += 16) {
-            const long long blocks = (long long)((N + LT_ROWS - 1) / LT_ROWS) * ((rows + t - 1) / t);
-            const double time = (double)((blocks + sms - 1) / sms) * (57 + 0.285 * t);
-            if (t == 16 || time < least) {
-                tn = t;
-                least = time;
-            }
-        }
+        const int tn = lt_tokens(rows, N, sms);
         RI_REQUIRE((rows + tn - 1) / tn <= 65535, "linear_f32_tc: too many rows (%d)", M);
         CUtensorMap map_x;
         cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, 3}, strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * 2 * rows};
@@ -278,7 +286,7 @@ extern "C" int ri_linear_f32_tc(const float* x, const float* w, float* y, void* 
         int rc;
         if (tn <= 64) rc = lt_launch<2, 4, 4>(map_w, map_x, xs, w, ys, rows, N, K, tn, err_flag, stream);
         else if (tn <= 128) rc = lt_launch<4, 2, 2>(map_w, map_x, xs, w, ys, rows, N, K, tn, err_flag, stream);
-        else rc = lt_launch<6, 2, 2>(map_w, map_x, xs, w, ys, rows, N, K, tn, err_flag, stream);
+        else rc = lt_launch<6, 2, 1>(map_w, map_x, xs, w, ys, rows, N, K, tn, err_flag, stream);
         if (rc) return rc;
     }
     return 0;

@@ -1,12 +1,16 @@
 // The float32 product y[M, N] = x[M, K] . W[N, K]^T on the 5th-generation tensor cores (tcgen05), in full 32-bit precision.
 //
-// Every float32 is the sum of three bfloat16 (8 significant bits each, cut off one after the other: the sum is exact), and a
-// product of two such sums is taken as the six of its nine terms that reach above 2^-23 of it:
+// Every float32 is the sum of three bfloat16, each the rest's nearest (8 significant bits and a sign: the sum is exact), and a product of
+// two such sums is taken as six of its nine terms:
 //     x w = hi hi + (hi mid + mid hi) + (mid mid + hi lo + lo hi)
-// The tensor cores multiply bfloat16 exactly and add in float32, but they cut the sum off instead of rounding it.  So only
-// LT_K = 32 k are added up there: first the small terms, then the two instructions of hi hi, into an accumulator that starts
-// at zero; then the sum is read back and added to a float32 register, rounded to nearest, over ascending k.  Every output is that one chain whatever
-// M, N and the tile a row falls into: a token's result does not depend on what it is batched with.
+// What is left out is 2^-24.2 of a product at most, of either sign (mid is 2^-8 of the value's power of two at most, lo 2^-17).
+//
+// The tensor cores multiply bfloat16 exactly and add in float32, but they cut a sum off instead of rounding it.  So the terms go two ways.
+// hi hi, whose products have 16 bits, is added up there for LT_K = 32 k only, into an accumulator that starts at zero; a few products of
+// like size fit its 24 bits as they are.  Then the sum is read back and added to a float32 register, rounded to nearest, over ascending k.  The
+// others, some 2^-8 of the product, are added up there over all k: what is cut off is 2^-31 of a product.  Their sum joins the register at
+// the end.  Every output is these two chains whatever M, N and the tile a row falls into: a
+// token's result does not depend on what it is batched with.
 #pragma once
 #include "common.cuh"
 #include "mma_helpers.cuh"
@@ -61,18 +65,31 @@ __device__ __forceinline__ bool lt_elect() {
     return one != 0;
 }
 
-// eight neighbouring k of a row as three times eight bfloat16
+__device__ __forceinline__ unsigned lt_nearest2(float a, float b) {          // a in the low half
+    unsigned r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
+// a pair of values without the pair of parts that `h` holds (exact)
+__device__ __forceinline__ unsigned long long lt_rest2(unsigned long long v, unsigned h) {
+    return ffma2(pack2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), pack2(-1.0f, -1.0f), v);
+}
+// eight neighbouring k of a row as three times eight bfloat16.  A value that leaves the range on the way is no number in one
+// of its parts, and so are the outputs that it is part of (see the end of the kernel).
 __device__ __forceinline__ void lt_cut(const float (&v)[8], uint4& hi, uint4& mid, uint4& lo) {
     unsigned h[4], m[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const unsigned a = __float_as_uint(v[2 * i]), b = __float_as_uint(v[2 * i + 1]);
-        const float ra = v[2 * i] - __uint_as_float(a & 0xffff0000u), rb = v[2 * i + 1] - __uint_as_float(b & 0xffff0000u);
-        const unsigned c = __float_as_uint(ra), d = __float_as_uint(rb);
-        const float la = ra - __uint_as_float(c & 0xffff0000u), lb = rb - __uint_as_float(d & 0xffff0000u);
-        h[i] = __byte_perm(a, b, 0x7632);
-        m[i] = __byte_perm(c, d, 0x7632);
-        l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+        unsigned long long rest = pack2(v[2 * i], v[2 * i + 1]);
+        float a, b;
+        unpack2(rest, a, b);
+        h[i] = lt_nearest2(a, b);
+        rest = lt_rest2(rest, h[i]);
+        unpack2(rest, a, b);
+        m[i] = lt_nearest2(a, b);
+        rest = lt_rest2(rest, m[i]);
+        unpack2(rest, a, b);
+        l[i] = lt_nearest2(a, b);
     }
     hi = make_uint4(h[0], h[1], h[2], h[3]);
     mid = make_uint4(m[0], m[1], m[2], m[3]);
@@ -100,7 +117,8 @@ linear_f32_cut_kernel(const float* x, uint4* __restrict__ parts, int M, int K, i
 }
 
 struct LtTail {
-    unsigned long long full[LT_MAX_STAGES], w_full[LT_MAX_WSTAGES], w_empty[LT_MAX_WSTAGES], acc_full[4], acc_empty[4], drained[LT_MAX_GROUPS];
+    unsigned long long full[LT_MAX_STAGES], w_full[LT_MAX_WSTAGES], w_empty[LT_MAX_WSTAGES], acc_full[LT_MAX_GROUPS], acc_empty[LT_MAX_GROUPS], turn[LT_MAX_GROUPS],
+        drained[LT_MAX_GROUPS];
     unsigned tmem_base;
     int dead;
 };
@@ -112,7 +130,6 @@ __device__ __forceinline__ bool lt_test(unsigned long long* bar, unsigned parity
     return __all_sync(0xffffffffu, ok);
 }
 // A warp's wait: false when it ran out (after some milliseconds), or when somebody else has given up
-
 __device__ __forceinline__ bool lt_wait_on(unsigned long long* bar, unsigned parity, int* dead, int* err) {
     unsigned start;
     asm volatile("mov.u32 %0, %globaltimer_lo;\n" : "=r"(start));
@@ -143,23 +160,24 @@ __device__ __forceinline__ void lt_tma_3d(void* dst, const CUtensorMap* map, int
 
 // A block: 128 rows of W as the product's M side, from the tensor memory; `tn` tokens (a multiple of 16, up to 32 CH) as its N side, from
 // shared memory.  A ring of `stages` holds LT_K k of W as they are (128-byte swizzle) and of the three parts of x (64-byte swizzle), copied
-// by TMA; another of `wstages` the parts of W in the tensor memory, and BUFS buffers there the sums.
+// by TMA; another of `wstages` the parts of W in the tensor memory, and there BUFS buffers hold hi hi's sums and one more the small terms'.
 //   4 GROUPS warps  take the stages by turns, four a stage: a lane reads its row of W from shared memory, cuts it and puts the parts
-//                   into the tensor memory; one of the four then issues the twelve tcgen05.mma of the stage
+//                   into the tensor memory; one of the four then issues the twelve tcgen05.mma of the stage, in its turn: the small
+//                   terms' sum is one chain over the stages of all groups
 //   8 warps         read a stage's sums back and add them to their registers: a lane has a row of W, two warps share its tokens; two of
 //                   them then start the copies into the place that the stage has left
 // x is cut once, by a kernel of its own: cut in here by every block, with loads into registers, the loads' trips and the words
-// written to shared memory took more time than the products (233 us and 197 where this takes 114 and 93, see linear_f32.cu).
-// What bounds it: with many tokens a block the tensor cores (twelve products of 128 x tn x 16 a stage, 1,060 cycles at 176 tokens) and the way
-// of a sum back to the next product into its buffer (some 1,450 cycles for two stages beside the product itself); with few tokens the
-// hand-overs alone, some 750 cycles a stage, where the copies of W would take 300.
+// written to shared memory took more time than the products (233 us and 197 where this took 114 and 93, see linear_f32.cu).
+// What bounds it: with many tokens a block the tensor cores (twelve products of 128 x tn x 16 a stage, 1,060 cycles at 176 tokens, where one
+// buffer for hi hi's sums is enough: they are read back under the next stage's small terms); with few tokens the hand-overs alone, some 700
+// cycles a stage, where the copies of W would take 300.
 template <int CH, int GROUPS, int BUFS>
 __global__ void __launch_bounds__(128 * GROUPS + LT_SUMS, 1)
 linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const float* x,
                      const float* __restrict__ w, float* __restrict__ y, int M, int N, int K, int tn, int stages, int wstages,
                      long long ldx, long long ldy, int* __restrict__ err) {
     constexpr bool SPLIT = CH == 6;                                // registers: 88 and 168 instead of 128 each
-    static_assert(BUFS == GROUPS, "a buffer of sums is always the same group's");
+    static_assert(BUFS == GROUPS || BUFS == 1, "a buffer of sums is always the same group's, or each stage's issuer has waited for the one before");
     static_assert(!SPLIT || GROUPS == 2, "256 threads of 88 and 256 of 168 registers are what 512 of 128 have");
     extern __shared__ __align__(1024) unsigned char lt_smem[];
     __shared__ LtTail tail;
@@ -186,14 +204,17 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tail.acc_full[b])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;\n" ::"r"(smem_u32(&tail.acc_empty[b])));
         }
-        for (int g = 0; g < GROUPS; g++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tail.drained[g])));
+        for (int g = 0; g < GROUPS; g++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tail.turn[g])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tail.drained[g])));
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         tail.dead = 0;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = tail.tmem_base, w_cols = tmem + BUFS * tn;      // the sums, then the stages' rows of W
+    const unsigned tmem = tail.tmem_base, small = tmem + BUFS * tn, w_cols = small + tn;      // the sums, then the stages' rows of W
     pdl_wait();
 
     if (warp < 4 * GROUPS) {
@@ -230,28 +251,36 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             __syncwarp();
             if (lane == 0) lt_arrive(&tail.w_full[wslot]);
             if (quad == group) {                                   // (the issuing warps on different schedulers)
-                const int buf = s % BUFS;
-                if (s >= BUFS && !lt_wait(&tail.acc_empty[buf], (unsigned)((s / BUFS - 1) & 1), tail, err)) break;
+                const int buf = s % BUFS, before = (group + GROUPS - 1) % GROUPS;
                 if (!lt_wait(&tail.w_full[wslot], wparity, tail, err)) break;
+                if (s > 0 && !lt_wait(&tail.turn[before], (unsigned)(((s - 1) / GROUPS) & 1), tail, err)) break;
+                tc_fence_after();
+                const unsigned wm = wh + 16, wl = wh + 32;
+                const unsigned long long xh = x0 + (unsigned long long)(slot * (x_bytes >> 4)), xm = xh + (x_part >> 4), xl = xm + (x_part >> 4);
+                if (one) {
+                    if (s == 0) lt_mma<0>(small, wl, xh, idesc);
+                    else lt_mma<1>(small, wl, xh, idesc);
+                    lt_mma<1>(small, wl + 8, xh + 2, idesc);
+                    lt_mma<1>(small, wh, xl, idesc);
+                    lt_mma<1>(small, wh + 8, xl + 2, idesc);
+                    lt_mma<1>(small, wm, xm, idesc);
+                    lt_mma<1>(small, wm + 8, xm + 2, idesc);
+                    lt_mma<1>(small, wm, xh, idesc);
+                    lt_mma<1>(small, wm + 8, xh + 2, idesc);
+                    lt_mma<1>(small, wh, xm, idesc);
+                    lt_mma<1>(small, wh + 8, xm + 2, idesc);
+                }
+                __syncwarp();
+                // hi hi, when the sums of the stage that had the buffer have been read (beside the small terms' products)
+                if (s >= BUFS && !lt_wait(&tail.acc_empty[buf], (unsigned)((s / BUFS - 1) & 1), tail, err)) break;
                 tc_fence_after();
                 if (one) {
-                    const unsigned d = tmem + buf * tn, wm = wh + 16, wl = wh + 32;
-                    const unsigned long long xh = x0 + (unsigned long long)(slot * (x_bytes >> 4)), xm = xh + (x_part >> 4), xl = xm + (x_part >> 4);
-                    // the terms of a product, small ones first, hi hi last
-                    lt_mma<0>(d, wl, xh, idesc);
-                    lt_mma<1>(d, wl + 8, xh + 2, idesc);
-                    lt_mma<1>(d, wh, xl, idesc);
-                    lt_mma<1>(d, wh + 8, xl + 2, idesc);
-                    lt_mma<1>(d, wm, xm, idesc);
-                    lt_mma<1>(d, wm + 8, xm + 2, idesc);
-                    lt_mma<1>(d, wm, xh, idesc);
-                    lt_mma<1>(d, wm + 8, xh + 2, idesc);
-                    lt_mma<1>(d, wh, xm, idesc);
-                    lt_mma<1>(d, wh + 8, xm + 2, idesc);
-                    lt_mma<1>(d, wh, xh, idesc);
-                    lt_mma<1>(d, wh + 8, xh + 2, idesc);
+                    lt_mma<0>(tmem + buf * tn, wh, xh, idesc);
+                    lt_mma<1>(tmem + buf * tn, wh + 8, xh + 2, idesc);
                     umma_commit(&tail.w_empty[wslot]);
                     umma_commit(&tail.acc_full[buf]);
+                    tc_fence_before();
+                    lt_arrive(&tail.turn[group]);
                 }
                 __syncwarp();
             }
@@ -295,12 +324,8 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         for (int c = 0; c < CH; c++)
 #pragma unroll
             for (int i = 0; i < 8; i++) acc[c][i] = 0ull;
-        int slot = 0, s = 0;
-        for (; s < steps; s++) {
-            const int buf = s % BUFS;
-            if (!lt_wait(&tail.acc_full[buf], (unsigned)((s / BUFS) & 1), tail, err)) break;
-            tc_fence_after();
-            const unsigned taddr = tmem + buf * tn + from + ((unsigned)(quad * 32) << 16);
+        // adds the sums in the tensor memory's columns from `taddr` on to the registers
+        auto add = [&](unsigned taddr) {
 #pragma unroll
             for (int c = 0; c < CH; c += 2) {
                 if (from + 16 * c >= to) break;
@@ -313,6 +338,14 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
                     for (int i = 0; i < 8; i++) acc[c + e][i] = fadd2(acc[c + e][i], pack2(__uint_as_float(r[e][2 * i]), __uint_as_float(r[e][2 * i + 1])));
             }
+        };
+        const unsigned mine = from + ((unsigned)(quad * 32) << 16);
+        int slot = 0, s = 0;
+        for (; s < steps; s++) {
+            const int buf = s % BUFS;
+            if (!lt_wait(&tail.acc_full[buf], (unsigned)((s / BUFS) & 1), tail, err)) break;
+            tc_fence_after();
+            add(tmem + buf * tn + mine);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) lt_arrive(&tail.acc_empty[buf]);
@@ -320,6 +353,7 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             __syncwarp();
             if (++slot == stages) slot = 0;
         }
+        add(small + mine);                                         // (the last stage's products were issued behind all others)
         if (copier && s < steps)                                   // somebody gave up: what was started lands first
             for (int i = s; i < s + stages && i < steps; i++) ri_mbar_wait(&tail.full[i % stages], (unsigned)((i / stages) & 1));
         __syncwarp();
@@ -335,8 +369,8 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     float lo, hi;
                     unpack2(acc[c][i / 2], lo, hi);
                     float v = i & 1 ? hi : lo;
-                    // An infinity's parts are no numbers, so its products are none either: what is not finite is taken again, as
-                    // the chain of multiply-adds over ascending k (until it is no number, which it then stays)
+                    // An infinity's parts are no numbers, so its products are none either: what is not finite is taken again, as the chain of
+                    // multiply-adds over ascending k (until it is no number, which it then stays)
                     if (!(fabsf(v) <= 3.402823466e38f)) {
                         const float *a = x + (size_t)(m0 + t) * ldx, *b = w + (size_t)n * K;
                         v = 0.0f;

@@ -703,9 +703,9 @@ def linear_act_rows(x: torch.Tensor, w: torch.Tensor, act: str, ids: torch.Tenso
 
 # The float32 product takes the tensor cores from here on.  The line depends on the sum's length and on how the weights lie, never on the
 # tokens: a row's bits are the same in every batch.  One of ten in a graph, tensor cores / multiply-adds, us at 300 tokens and 4,096
-# outputs; 1 and 4,096; 1 and 256: K = 64 9.0 / 8.6, 4.5 / 4.1, 5.3 / 4.5; 128 10.0 / 14.1, 5.5 / 7.0, 5.3 / 7.0; 256 12.1 / 25.4, 7.0 / 11.7,
-# 6.8 / 11.7.  From a program that launches them alone 128 is the first where neither is slower (11.3 / 12.4), and its error is the smaller one
-# from some 64 on.
+# outputs; 1 and 4,096; 1 and 256: K = 128 9.8 / 13.9, 4.9 / 6.4, 4.7 / 6.2; 256 12.0 / 25.1, 6.3 / 11.1, 6.0 / 10.9; at K = 64 multiply-adds were the
+# faster ones.  (Below 256 they still are for thousands of tokens and a few dozen outputs, 9.0 / 6.5 at 4,096 and 16, and a program that
+# launches products one by one pays the host for a second kernel, 6.4 / 4.0 us a call.)  The error against float64 is no larger at any length.
 F32_TC_MIN_K = 128
 # bytes for the cut rows of x; larger steps take several launches
 F32_TC_SCRATCH = 128 << 20

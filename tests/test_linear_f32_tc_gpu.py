@@ -15,8 +15,9 @@ def _inputs(M, N, K):
 
 
 def _close(got, x, w):
-    """The parts' products that are left out are below 3 x 2^-23 of a product; a sum of 32 k is cut off twelve times by at most
-    2^-23 of its magnitudes, and the K / 32 sums' additions round by 2^-24 each."""
+    """What is left out of a product is below 2^-24 of it, the two additions of 16 products of 16 bits cut a sum of 32 k off by 2^-23 of its
+    magnitudes each, the small terms' sum (2^-7 of the magnitudes at most) is cut off ten times a stage by 2^-23, and the
+    K / 32 + 1 additions of sums round by 2^-24 each."""
     want, most = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
     assert ((got.double() - want).abs() <= (x.shape[1] / 32 + 32) * 2.0 ** -24 * most).all()
 
@@ -49,6 +50,26 @@ def test_no_larger_error_than_multiply_adds():
         want = x.double() @ w.double().T
         errors = [((y.double() - want).norm() / want.norm()).item() for y in (ops.linear(x, w), _multiply_adds(x, w))]
         assert errors[0] <= errors[1], (K, errors)
+
+
+def _sparse(M, K, entries):
+    x, g = torch.randn((M, K), device=DEV), torch.Generator(device=DEV).manual_seed(entries)
+    return x * torch.zeros_like(x).scatter_(1, torch.rand((M, K), generator=g, device=DEV).topk(entries, 1).indices, 1.0)
+
+
+@pytest.mark.parametrize("K", [128, 4096])
+@pytest.mark.parametrize("M", [60, 120, 700])                     # the three variants of the kernel
+def test_sums_with_few_terms_and_of_one_sign(M, K):
+    w = torch.randn((9473, K), generator=torch.Generator(device=DEV).manual_seed(K), device=DEV)
+    # one product: its rounding to float32, 2^-24, and what is left out of it, below 2^-24.1
+    x = _sparse(M, K, 1)
+    want = x.double() @ w.double().T
+    assert ((ops.linear(x, w).double() - want).abs() <= 1.95 * 2.0 ** -24 * want.abs()).all()
+    near = 1 + 2.0 ** -7 + 1e-3 * torch.rand((M, K), device=DEV)       # values whose middle parts are large
+    for x, w in [(_sparse(M, K, n), w) for n in (2, 4, 8, 32)] + [(near, 1 + 2.0 ** -7 - 2.0 ** -23 + 1e-4 * w.abs())]:
+        want = x.double() @ w.double().T
+        errors = [(y.double() - want).norm().item() for y in (ops.linear(x, w), _multiply_adds(x, w))]
+        assert errors[0] <= errors[1], errors
 
 
 def test_rows_in_several_launches(monkeypatch):
