@@ -3,13 +3,14 @@
 // Every float32 is the sum of three bfloat16, each the rest's nearest (8 significant bits and a sign: the sum is exact), and a product of
 // two such sums is taken as six of its nine terms:
 //     x w = hi hi + (hi mid + mid hi) + (mid mid + hi lo + lo hi)
-// What is left out is 2^-24.2 of a product at most, of either sign (mid is 2^-8 of the value's power of two at most, lo 2^-17).
+// What is left out is 2^-24.2 of a product at most, of either sign (mid is 2^-8 of the value's power of two at most, lo 2^-17).  Both values are
+// taken times 2^16, exactly, so that a part's last bit, 2^-149 at the least, is one that bfloat16 has (2^-133).
 //
 // The tensor cores multiply bfloat16 exactly and add in float32, but they cut a sum off instead of rounding it.  So the terms go two ways.
 // hi hi, whose products have 16 bits, is added up there for LT_K = 32 k only, into an accumulator that starts at zero; a few products of
 // like size fit its 24 bits as they are.  Then the sum is read back and added to a float32 register, rounded to nearest, over ascending k.  The
 // others, some 2^-8 of the product, are added up there over all k: what is cut off is 2^-31 of a product.  Their sum joins the register at
-// the end.  Every output is these two chains whatever M, N and the tile a row falls into: a
+// the end, then 2^-32 takes the powers of two back.  Every output is these two chains whatever M, N and the tile a row falls into: a
 // token's result does not depend on what it is batched with.
 #pragma once
 #include "common.cuh"
@@ -74,13 +75,13 @@ __device__ __forceinline__ unsigned lt_nearest2(float a, float b) {          // 
 __device__ __forceinline__ unsigned long long lt_rest2(unsigned long long v, unsigned h) {
     return ffma2(pack2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), pack2(-1.0f, -1.0f), v);
 }
-// eight neighbouring k of a row as three times eight bfloat16.  A value that leaves the range on the way is no number in one
+// eight neighbouring k of a row, times 2^16, as three times eight bfloat16.  A value that leaves the range on the way is no number in one
 // of its parts, and so are the outputs that it is part of (see the end of the kernel).
 __device__ __forceinline__ void lt_cut(const float (&v)[8], uint4& hi, uint4& mid, uint4& lo) {
     unsigned h[4], m[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        unsigned long long rest = pack2(v[2 * i], v[2 * i + 1]);
+        unsigned long long rest = fmul2(pack2(v[2 * i], v[2 * i + 1]), pack2(65536.0f, 65536.0f));
         float a, b;
         unpack2(rest, a, b);
         h[i] = lt_nearest2(a, b);
@@ -368,9 +369,10 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     if (t >= to || m0 + t >= M) break;
                     float lo, hi;
                     unpack2(acc[c][i / 2], lo, hi);
-                    float v = i & 1 ? hi : lo;
-                    // An infinity's parts are no numbers, so its products are none either: what is not finite is taken again, as the chain of
-                    // multiply-adds over ascending k (until it is no number, which it then stays)
+                    float v = (i & 1 ? hi : lo) * 2.3283064365386963e-10f;      // 2^-32
+                    // An infinity's parts are no numbers, so its products are none either, and with the powers of two values from 2^112 and
+                    // sums from 2^96 on leave the range: what is not finite is taken again, as the chain of multiply-adds over ascending k (until
+                    // it is no number, which it then stays)
                     if (!(fabsf(v) <= 3.402823466e38f)) {
                         const float *a = x + (size_t)(m0 + t) * ldx, *b = w + (size_t)n * K;
                         v = 0.0f;

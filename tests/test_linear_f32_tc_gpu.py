@@ -72,6 +72,26 @@ def test_sums_with_few_terms_and_of_one_sign(M, K):
         assert errors[0] <= errors[1], errors
 
 
+# float32 numbers whose third parts are below bfloat16's smallest, in either operand; sums that are below float32's smallest normal number
+@pytest.mark.parametrize("scale_x, scale_w", [(1e-34, 1.0), (1e-37, 1.0), (1.0, 1e-36), (1e5, 1e-40), (1e-42, 1e5), (1e-20, 1e-16)])
+def test_small_values(scale_x, scale_w):
+    x, w = _inputs(70, 300, 256)
+    x, w = x * scale_x, w * scale_w
+    want, most = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    got, multiply_adds = ops.linear(x, w), _multiply_adds(x, w)
+    assert ((got.double() - want).abs() <= 8 * 2.0 ** -24 * most + 2.0 ** -150).all()
+    assert (got.double() - want).norm() <= (multiply_adds.double() - want).norm()
+
+
+def test_values_beyond_the_scaled_range_are_taken_by_multiply_adds():
+    x, w = _inputs(70, 300, 256)
+    for a, b in ((x * 1e35, w * 1e-3), (x * 1e-3, w * 1e35), (x * 1e15, w * 1e15)):          # 2^112 for a value, 2^96 for a sum
+        got, want = ops.linear(a, b), _multiply_adds(a, b)
+        far = want.abs() > 2.0 ** 97
+        assert torch.isfinite(want).all() and far.any() and torch.equal(got[far], want[far])
+        _close(got, a, b)
+
+
 def test_rows_in_several_launches(monkeypatch):
     x, w = _inputs(2500, 200, 288)
     whole = ops.linear(x, w)
