@@ -196,16 +196,6 @@ static int lt_launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const f
     // products up to s - stages are done, so that the second ring's phase before last is over if it has half as many places.
     stages -= stages % GROUPS;
     RI_REQUIRE(tn <= 32 * CH && stages >= GROUPS && wstages >= GROUPS && 2 * wstages >= stages, "linear_f32_tc: %d tokens a block", tn);
-    if (CH == 6) {                                 // its warps hand registers over: the sum has to be what they are launched with
-        static int regs = 0;
-        if (!regs) {
-            cudaFuncAttributes attr;
-            cudaError_t e = cudaFuncGetAttributes(&attr, (const void*)kernel);
-            if (e != cudaSuccess) RI_FAIL((int)e, "linear_f32_tc: %s", cudaGetErrorString(e));
-            regs = attr.numRegs;
-        }
-        RI_REQUIRE(regs == 128, "linear_f32_tc: built with %d registers a thread", regs);
-    }
     cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM_MAX);
     if (e != cudaSuccess) RI_FAIL((int)e, "linear_f32_tc: %s", cudaGetErrorString(e));
     ri_launch_pdl(kernel, dim3((N + LT_ROWS - 1) / LT_ROWS, (M + tn - 1) / tn), dim3(128 * GROUPS + LT_SUMS), (size_t)stages * stage, stream,
@@ -214,12 +204,25 @@ static int lt_launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const f
     return 0;
 }
 
-// Tokens a block: the multiple of 16 with the least time, rounds of blocks (one an SM) times what a round takes, some 57 us +
+// The most tokens a block takes: the largest variant's warps hand registers over, whose sum has to be what they are launched with, so that it
+// is left out where the compiler gave it another number.
+static int lt_most_tokens() {
+    static int most = 0;
+    if (!most) {
+        cudaFuncAttributes attr;
+        cudaError_t e = cudaFuncGetAttributes(&attr, (const void*)linear_f32_tc_kernel<6, 2, 1>);
+        if (e != cudaSuccess) RI_FAIL(0, "linear_f32_tc: %s", cudaGetErrorString(e));
+        most = attr.numRegs == 128 ? LT_MAX_TOKENS : 128;
+    }
+    return most;
+}
+
+// Tokens a block: the multiple of 16, up to `most`, with the least time, rounds of blocks (one an SM) times what a round takes, some 57 us +
 // 0.285 a token at K = 4,096 where the blocks fill the device (16 tokens 55, 128 and 48 blocks 68, 176 and 48 blocks 69, 176 and 144 blocks 112).
-static int lt_tokens(int rows, int N, int sms) {
+extern "C" int ri_linear_f32_tc_tokens(int rows, int N, int sms, int most) {
     int tn = 16;
     double least = 0;
-    for (int t = 16; t <= LT_MAX_TOKENS; t += 16) {
+    for (int t = 16; t <= most; t += 16) {
         const long long blocks = (long long)((N + LT_ROWS - 1) / LT_ROWS) * ((rows + t - 1) / t);
         const double time = (double)((blocks + sms - 1) / sms) * (57 + 0.285 * t);
         if (t == 16 || time < least) {
@@ -257,6 +260,8 @@ extern "C" int ri_linear_f32_tc(const float* x, const float* w, float* y, void* 
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         sms = n > 0 ? n : 148;
     }
+    const int most = lt_most_tokens();
+    if (!most) return -1;
     const int Kp = (K + LT_K - 1) / LT_K * LT_K;
     const cuuint32_t one[3] = {1, 1, 1};
     CUtensorMap map_w;
@@ -269,7 +274,7 @@ extern "C" int ri_linear_f32_tc(const float* x, const float* w, float* y, void* 
     }
     for (int at = 0; at < M; at += part_rows) {
         const int rows = M - at < part_rows ? M - at : part_rows;
-        const int tn = lt_tokens(rows, N, sms);
+        const int tn = ri_linear_f32_tc_tokens(rows, N, sms, most);
         RI_REQUIRE((rows + tn - 1) / tn <= 65535, "linear_f32_tc: too many rows (%d)", M);
         CUtensorMap map_x;
         cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, 3}, strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * 2 * rows};

@@ -66,6 +66,7 @@ _SIGNATURES = {
     ("pair_heads", "ri_pair_heads"): [_P, _P, _F, _F, _F, _I, _I, _I, _I, _I, _I, _I, _P],
     ("linear_f32", "ri_linear_f32"): [_P, _P, _P, _I, _I, _I, _P],
     ("linear_f32", "ri_linear_f32_tc"): [_P] * 4 + [_I] * 4 + [_P, _P],
+    ("linear_f32", "ri_linear_f32_tc_tokens"): [_I] * 4,
     ("sampling", "ri_sample"): [_P, _L, _I, _I, _P, _P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _I, _I, _P, _I, _P],
     ("sampling", "ri_sample_work_bytes"): [_I, _I],
     ("sampling", "ri_argmax"): [_P, _L, _I, _I, _P, _P, _P, _P],

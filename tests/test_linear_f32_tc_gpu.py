@@ -92,6 +92,14 @@ def test_values_beyond_the_scaled_range_are_taken_by_multiply_adds():
         _close(got, a, b)
 
 
+def test_tokens_a_block_stay_below_the_largest_variant():
+    """Where the largest variant cannot be taken (its warps hand registers over, which the compiler has to have given them) the rule stays
+    at 128 tokens a block."""
+    tokens = lambda rows, N, most: ops._fn("linear_f32", "ri_linear_f32_tc_tokens")[0](rows, N, 148, most)
+    assert tokens(512, 6144, 176) == 176
+    assert all(tokens(rows, N, 128) <= 128 for rows in (1, 100, 176, 512, 3000) for N in (1, 6144, 9473))
+
+
 def test_rows_in_several_launches(monkeypatch):
     x, w = _inputs(2500, 200, 288)
     whole = ops.linear(x, w)
