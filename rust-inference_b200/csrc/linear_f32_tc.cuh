@@ -12,6 +12,10 @@
 // others, some 2^-8 of the product, are added up there over all k: what is cut off is 2^-31 of a product.  Their sum joins the register at
 // the end, then 2^-32 takes the powers of two back.  Every output is these two chains whatever M, N and the tile a row falls into: a
 // token's result does not depend on what it is batched with.
+//
+// Waits are bounded (error 5): whoever gives up says so in shared memory, the others end when they next have to wait, the copies that were
+// started are waited for once more, and the block ends as usual with a wrong result.  -DLF_TEST_DROP_COPY_K=<k> (tests only; nothing
+// in an ordinary build) makes the first block leave out the copy of W of its first stage in launches with K == k, so that this path can be run.
 #pragma once
 #include "common.cuh"
 #include "mma_helpers.cuh"
@@ -309,6 +313,9 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         auto copy = [&](int s, int slot) {
             if (copier == 1) {
                 tc_expect_tx(&tail.full[slot], (unsigned)LT_W_BYTES);
+#ifdef LF_TEST_DROP_COPY_K
+                if (K == LF_TEST_DROP_COPY_K && blockIdx.x == 0 && blockIdx.y == 0 && s == 0) return;      // tests only: see the top
+#endif
                 tc_tma_2d(lt_smem + slot * LT_W_BYTES, &map_w, s * LT_K, n0, &tail.full[slot]);
             } else if (copier == 2) {
                 tc_expect_tx(&tail.full[slot], (unsigned)x_bytes);

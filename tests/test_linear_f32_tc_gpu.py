@@ -100,6 +100,42 @@ def test_tokens_a_block_stay_below_the_largest_variant():
     assert all(tokens(rows, N, 128) <= 128 for rows in (1, 100, 176, 512, 3000) for N in (1, 6144, 9473))
 
 
+def test_a_wait_that_runs_out():
+    """Built with a test-only define, the first block of a launch with K = 1536 leaves out a copy of W.  Error 5 is reported, the kernel
+    returns, the other blocks' outputs are right, and so is the next launch.  Nothing hangs or faults: the waits are the bounded ones."""
+    import os
+    import subprocess
+    import sys
+    code = r'''
+import time, torch
+from rust_inference_b200 import ops
+torch.manual_seed(0)
+flag = ops.error_flag("cuda")
+def run(M, K, N=9473):
+    x, w = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda")
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    y = ops.linear(x, w)
+    torch.cuda.synchronize()
+    ms = (time.perf_counter() - t0) * 1e3
+    want = x.double() @ w.double().t()
+    return (y.double() - want).abs() <= 1e-3, ms
+for M in (40, 120, 176):                                          # the three variants
+    assert run(M, 1024)[0].all() and int(flag.item()) == 0        # (another K: nothing is left out)
+    near, ms = run(M, 1536)
+    assert int(flag.item()) == 5, int(flag.item())
+    flag.zero_()
+    assert near[:, 128:].all() and not near.all(), "the other blocks"
+    assert run(M, 2048)[0].all() and int(flag.item()) == 0
+    print("gave up after %.1f ms" % ms)
+'''
+    env = dict(os.environ, RUST_INFERENCE_B200_DEFINES="LF_TEST_DROP_COPY_K=1536", PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600, env=env)
+    assert r.returncode == 0, r.stdout + r.stderr
+    for line in r.stdout.strip().splitlines():
+        assert 3.0 <= float(line.split("after")[1].split()[0]) <= 2000.0, r.stdout
+
+
 def test_rows_in_several_launches(monkeypatch):
     x, w = _inputs(2500, 200, 288)
     whole = ops.linear(x, w)
