@@ -315,7 +315,6 @@ moe_route_wide_kernel(const T* __restrict__ x, const float* __restrict__ router,
 // (Eight tokens and eight outputs a warp's item, a segment at a time: 26.7 / 28.6 / 35.5.)
 #define MOE_ROUTE_TILE 4
 #define MOE_ROUTE_TILE_THREADS 256
-#define MOE_ROUTE_TILE_TOKENS 149
 template <typename T> struct MoePiece;                // four neighbouring elements as they come from memory
 template <> struct MoePiece<float> {
     float4 v;
@@ -408,6 +407,17 @@ moe_route_tile_kernel(const T* x, const float* __restrict__ router, const float*
     moe_choose(s, s + N, s + 2 * N, correction, idx, weight, t0 + warp, N, top, lane, rule);
 }
 
+static int moe_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        sms = n > 0 ? n : 148;
+    }
+    return sms;
+}
+
 extern "C" int ri_moe_route_rule(const void* x, const float* router, const float* correction, int* idx, float* weight,
                                  int tokens, int D, int N, int top, int mode, int groups, int keep, int gtop, float scale,
                                  int renorm, const float* bias, int dtype, cudaStream_t stream) {
@@ -424,16 +434,16 @@ extern "C" int ri_moe_route_rule(const void* x, const float* router, const float
     RI_REQUIRE(N <= 4096, "moe_route: %d router outputs (up to 4096 are built)", N);
     const size_t smem = (size_t)MOE_ROUTE_WARPS * (2 * N + groups) * sizeof(float);
     const dim3 grid((tokens + MOE_ROUTE_WARPS - 1) / MOE_ROUTE_WARPS);
-    // (which form runs depends on sizes, the number of tokens among them, and addresses; the forms for rows of whole 16-byte
-    // pieces give the same bits)
+    // (which form runs depends on sizes, the number of tokens among them, and addresses; the two forms that the tokens decide between give
+    // the same bits)
     const int vec = (D % 4 == 0 && (((uintptr_t)router | (uintptr_t)x) & 15) == 0) ? 1 : 0;
     cudaError_t e = cudaSuccess;
     const long long items = (long long)N * ((D + 127) / 128);
-    // Blocks of four tokens from where blocks of one token, which have an SM each, need a second round of the 148 SMs.  Cold, width 4,096 and
+    // Blocks of four tokens from where blocks of one token, which have an SM each, need a second round of the SMs.  Cold, 148 SMs, width 4,096 and
     // 18 outputs: one token a block 14.4 us up to 148 tokens and 22.5 for 200, four 16.6 for 256; width 2,048 and 34 outputs 14.4, 22.5, 16.4.
     const long long runs = (D + 128 * MOE_ROUTE_RUN - 1) / (128 * MOE_ROUTE_RUN);
     const size_t tile_sm = ((size_t)runs * MOE_ROUTE_TILE * ((N + 3) / 4 * 4) + (size_t)MOE_ROUTE_TILE * (2 * N + groups)) * sizeof(float);
-    if (vec && items <= MOE_ROUTE_WIDE_ITEMS && tokens >= MOE_ROUTE_TILE_TOKENS && tile_sm <= 96 * 1024) {
+    if (vec && items <= MOE_ROUTE_WIDE_ITEMS && tokens > moe_sms() && tile_sm <= 96 * 1024) {
         const dim3 tiles((tokens + MOE_ROUTE_TILE - 1) / MOE_ROUTE_TILE);
         if (dtype == RI_DTYPE_F32) {
             if (tile_sm > 48 * 1024) e = cudaFuncSetAttribute(moe_route_tile_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_sm);
@@ -819,13 +829,7 @@ moe_grouped_bf16_kernel(const bf16* __restrict__ a, long long lda, const bf16* _
 
 // rounds of blocks that the SMs take with four (four stages) and five (three stages) on each
 static int moe_stages(long long blocks) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        sms = n > 0 ? n : 148;
-    }
+    const int sms = moe_sms();
     return (blocks + 5 * sms - 1) / (5 * sms) < (blocks + 4 * sms - 1) / (4 * sms) ? 3 : 4;
 }
 template <typename TO, bool VEC, bool GATED, int STAGES>

@@ -104,7 +104,8 @@ def test_gate_in_the_epilogue(kind, limit, alpha, tokens, top, E, N, K):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("tokens, D, N, top, rule", [(256, 128, 4, 2, {}), (257, 132, 18, 4, {}), (300, 4096, 18, 4, {}), (512, 260, 33, 3, {}),
+# (the number of SMs, 148, is where the forms meet; widths whose last run of 512 k is four k and a whole one)
+@pytest.mark.parametrize("tokens, D, N, top, rule", [(149, 516, 18, 4, {}), (150, 1028, 34, 3, {}), (200, 1024, 7, 2, {}), (256, 128, 4, 2, {}), (257, 132, 18, 4, {}), (300, 4096, 18, 4, {}), (512, 260, 33, 3, {}),
                                                      (391, 512, 16, 4, dict(score="sigmoid", groups=4, keep=2, scale=2.0, renormalize=False)),
                                                      (259, 640, 9, 3, dict(score="logits"))])
 def test_router_by_tiles_gives_the_bits_of_a_block_per_token(tokens, D, N, top, rule, dtype):
@@ -115,9 +116,35 @@ def test_router_by_tiles_gives_the_bits_of_a_block_per_token(tokens, D, N, top, 
     correction = None if rule.get("score") == "logits" else torch.randn((N,), generator=g, device=DEV) * 0.1
     bias = torch.randn((N,), generator=g, device=DEV) if rule.get("score") == "logits" else None
     idx, weight = ops.moe_route(x, router, correction, top, bias=bias, **rule)
-    for lo, hi in ((0, 100), (100, 255), (255, tokens)):         # few tokens: a block per token
+    for lo in range(0, tokens, 100):                             # few tokens: a block per token
+        hi = min(lo + 100, tokens)
         i1, w1 = ops.moe_route(x[lo:hi].clone(), router, correction, top, bias=bias, **rule)
         assert torch.equal(idx[lo:hi], i1) and torch.equal(weight[lo:hi], w1)
+
+
+# up to 32 choices a lane keeps each; with more they go through memory
+@pytest.mark.parametrize("top", [31, 32, 33, 70])
+@pytest.mark.parametrize("tokens", [3, 300])
+@pytest.mark.parametrize("score, renormalize", [("softmax", True), ("sigmoid", False), ("logits", True)])
+def test_router_with_more_choices_than_lanes(tokens, top, score, renormalize):
+    ops = _ops()
+    g = _gen(top)
+    D, N = 64, 100
+    x = torch.randn((tokens, D), generator=g, device=DEV)
+    router = torch.randn((N, D), generator=g, device=DEV) * 0.2
+    correction = None if score == "logits" else torch.randn((N,), generator=g, device=DEV) * 0.1
+    idx, weight = ops.moe_route(x, router, correction, top, score=score, scale=1.5, renormalize=renormalize)
+    logits = x.double() @ router.double().t()
+    scores = {"softmax": logits.softmax(-1), "sigmoid": logits.sigmoid(), "logits": logits}[score]
+    choice = scores if correction is None else scores + correction.double()
+    # the chosen are distinct, in descending order, and nothing that was left out is better (float32 sums of 64 products: 1e-5)
+    assert (idx.sort(1).values.diff(dim=1) > 0).all()
+    at = choice.gather(1, idx.long())
+    left = choice.scatter(1, idx.long(), float("-inf")).max(1).values
+    assert (at.diff(dim=1) <= 1e-5).all() and (left <= at[:, -1] + 1e-5).all()
+    want = scores.gather(1, idx.long())
+    want = want.softmax(-1) if score == "logits" else want / want.sum(-1, keepdim=True) if renormalize else want
+    assert ((weight.double() - 1.5 * want).abs() <= 1e-5 * (1 + want.abs())).all()
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
