@@ -763,19 +763,25 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
 
 
 LOW_RANK_MAX_K = 128
+# ... and the most work, outputs times (K + 64), of the own kernel for one product and for two: beyond it the library's larger tiles save more
+# than the copies of the columns cost.  Own kernel / copies and library products, us, at 2,048 tokens: one of K = 16 and 2,048 outputs 4.6 / 6.8,
+# 8,192 12.7 / 11.9, of K = 64 5.6 / 6.7 and 16.5 / 11.7, of K = 128 1,024 5.8 / 5.9, 2,048 8.3 / 7.3; two of K = 64 and 2,048 outputs 9.0 / 13.1, 8,192
+# 31.8 / 25.3, of K = 128 2,048 13.6 / 14.4.
+LOW_RANK_MOST_WORK = (0, 550_000_000, 1_650_000_000)
 
 
 def low_rank(x: torch.Tensor, *sets) -> list:
     """The outer products of low-rank projections: for every (col, w) of ``sets``, w [N, K], the product
     x[:, col:col + K] w^T [tokens, N].  ``x`` [tokens, columns] holds the inner parts side by side.
-    bfloat16, up to two products of K up to 128 over columns in multiples of 8: one kernel of this package (mma.sync) that
-    reads the columns where they lie; anything else a copy of the columns and ``linear`` each.  The same bits either way."""
+    bfloat16, up to two products of K up to 128 over columns in multiples of 8, of some size: one kernel of this package (mma.sync)
+    that reads the columns where they lie; anything else a copy of the columns and ``linear`` each.  The same bits either way."""
     tokens, ld = x.shape
     for col, w in sets:
         if w.dim() != 2 or w.dtype != x.dtype or col < 0 or col + w.shape[1] > ld:
             raise KernelError(f"low_rank: columns {col} .. of x {tuple(x.shape)} and w {tuple(w.shape)} do not fit")
     if (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and 1 <= len(sets) <= 2 and ld % 8 == 0
             and x.data_ptr() % 16 == 0 and tokens <= 64 * 65535
+            and sum(tokens * w.shape[0] * (w.shape[1] + 64) for _, w in sets) <= LOW_RANK_MOST_WORK[len(sets)]
             and all(col % 8 == 0 and w.shape[0] % 8 == 0 and w.shape[0] > 0 and w.shape[1] % 8 == 0 and 0 < w.shape[1] <= LOW_RANK_MAX_K
                     and w.is_cuda and w.is_contiguous() and w.data_ptr() % 16 == 0 for col, w in sets)):
         out = [torch.empty((tokens, w.shape[0]), dtype=x.dtype, device=x.device) for _, w in sets]

@@ -130,7 +130,8 @@ def test_low_rank_products(tokens, sets):
 # tcgen05 one, then the library's
 @pytest.mark.parametrize("tokens", [1, 8, 12, 13, 16, 17, 32, 33, 65, 1000])
 @pytest.mark.parametrize("K, N", [(8, 1024), (24, 2048), (64, 2048), (72, 5000), (128, 1024), (128, 5632)])
-def test_low_rank_products_give_the_bits_of_the_product_of_a_copy(tokens, K, N):
+def test_low_rank_products_give_the_bits_of_the_product_of_a_copy(tokens, K, N, monkeypatch):
+    monkeypatch.setattr(ops, "LOW_RANK_MOST_WORK", (0, 1 << 60, 1 << 60))
     x, w = _rand(24, tokens, 256).bfloat16(), _rand(25, N, K).bfloat16()
     assert torch.equal(ops.low_rank(x, (16, w))[0], ops.linear(x[:, 16:16 + K].contiguous(), w))
 
