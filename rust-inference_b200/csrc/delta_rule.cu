@@ -112,7 +112,10 @@ short_conv_x8_kernel(const __nv_bfloat16* __restrict__ x, long long ld, int col0
 
 // The same with CONV_TOKENS neighbouring tokens per thread, for prompts with four taps: the weights and the tokens before are read once for
 // all of them, and the tokens' loads are on their way together.  What bounds it: the functions of silu, and memory.  2,048 tokens of 4,096 channels (50 MB): 19 us,
-// 22 with a token per thread, whose weights come from L2 again for every token (134 MB), and with eight.  An element's arithmetic and its order are the same.
+// 20 to 22 with a token per thread, whose weights come from L2 again for every token (134 MB), and with eight.  An element's arithmetic and its order are the same.
+// From CONV_MANY elements on: below it the blocks are too few (us, this / a token per thread: 1,000 tokens of 256 channels 5.4 / 4.6, 320 of 4,096 7.2 / 6.3)
+// or take a second round for a few (2.5 million elements 9.6 / 8.9); 3.3 million 10.5 / 11.0, 6.1 million 15.2 / 16.3, 24 million 53 / 62.
+#define CONV_MANY (3 << 20)
 #define CONV_TOKENS 4
 __global__ void __launch_bounds__(128)
 short_conv_x8_many_kernel(const __nv_bfloat16* __restrict__ x, long long ld, int col0, const float* __restrict__ wt, float* __restrict__ y,
@@ -195,7 +198,7 @@ extern "C" int ri_short_conv(const void* x, long long ld, int col0, const float*
     const dim3 grid(tokens, (C + 255) / 256);
     const bool x8 = dtype == RI_DTYPE_BF16 && wt && C % 8 == 0 && ld % 8 == 0 && col0 % 8 == 0 &&
                     (((uintptr_t)x | (uintptr_t)wt | (uintptr_t)y | (uintptr_t)state) & 15) == 0;
-    if (x8 && taps == 4 && !upd && tokens >= 256)
+    if (x8 && taps == 4 && !upd && (long long)tokens * C >= CONV_MANY)
         ri_launch_pdl(short_conv_x8_many_kernel, dim3((tokens + CONV_TOKENS - 1) / CONV_TOKENS, (C / 8 + 127) / 128), dim3(128), 0, stream,
                       (const __nv_bfloat16*)x, ld, col0, wt, y, (const float*)state, tok_seq, seq_slot, seq_start, tokens, C);
     else if (x8)

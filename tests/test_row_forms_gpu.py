@@ -68,10 +68,11 @@ def test_unit_vectors_and_decays_give_the_bits_of_a_channel_at_a_time(tokens, H,
         assert torch.equal(a, b)
 
 
-# from 256 tokens on four tokens a thread; sequences that begin and end anywhere in a thread's four, of one and two tokens too
+# steps of many elements take four tokens a thread; sequences that begin and end anywhere in a thread's four, of one and two tokens too
+@pytest.mark.parametrize("C", [72, 12296])
 @pytest.mark.parametrize("lens", [[256], [259], [1, 2, 3, 250, 1, 1, 4], [64] * 5, [255, 2]])
-def test_short_conv_over_many_tokens(lens):
-    T, C, slots = sum(lens), 72, len(lens) + 2
+def test_short_conv_over_many_tokens(lens, C):
+    T, slots = sum(lens), len(lens) + 2
     x = _rand(4, T, C + 8).bfloat16()[:, :]
     w = 0.5 * _rand(5, C, 4)
     wt = w.t().contiguous()
