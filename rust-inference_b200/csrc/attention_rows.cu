@@ -284,7 +284,8 @@ attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, con
 // behind 300 57 / 60; 16 / 2 of 64, 300 tokens 45 / 176; 16 / 1 of 256, 300 tokens 92 / 256.  Tiles of 64 rows (0.5 and 0.25 words) leave two blocks
 // to an SM and take 172, 96, 84; 62; 141.
 #define AT_ROWS 32
-#define AT_MIN_ROWS 8
+#define AT_MIN_ROWS 10             // ... and with fewer rows, down to eight, from AT_MIN_WORK elements of queries on
+#define AT_MIN_WORK 65536
 #define AT_THREADS 128
 #define AT_P_PITCH 36
 template <bool V> struct AtFlag { static constexpr bool value = V; };
@@ -591,11 +592,14 @@ extern "C" int ri_attention_rows(const void* q, const void* k_pool, const void* 
     // vector loads need rows of the pools and of q that start on 16 bytes (float32) or 8 bytes (bfloat16)
     const uintptr_t align = f32 ? 15 : 7;
     const bool vec4 = Dh % 4 == 0 && (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & align) == 0;
-    // Tiles of rows (the same bits) from AT_MIN_ROWS rows a kv head on.  Cold, behind 300 keys, tiles / a row at a time, us: 32 heads over 8 kv heads of 128,
-    // one token 55 / 60 but one of 24 sequences 74 / 68, two tokens 55 / 63, four 55 / 74; 32 over 32, four tokens 57 / 57, eight 55 / 64; 16 over 2
-    // of 64, one token of 24 sequences 43 / 47.
-    if (f32 && vec4 && ((uintptr_t)out & 15) == 0 && page_size % AR_STRIP == 0 && H / KV <= AT_ROWS && (long long)max_new * (H / KV) >= AT_MIN_ROWS &&
-        KV <= 65535 && seqs <= 65535) {
+    // Tiles of rows (the same bits) from ten rows a kv head on, from eight where the blocks are many: a row at a time is the shorter chain, but takes
+    // more words from shared memory a row.  Pools from memory, behind 300 keys, tiles / a row at a time, us: eight rows of 8 kv heads of 128 50 / 42, of 64
+    // 50 / 46, of 192 68 / 66, of 768 166 / 205, of 48 of 256 elements 78 / 99; ten rows of 8 kv heads of 64 38 / 49, of 128 (five query heads each)
+    // 50 / 47, of 192 68 / 74; 16 rows of 8 kv heads of 128 50 / 51, of 192 70 / 84.  Behind a few keys only the chain counts: 12 rows behind none 9.7 / 7.9,
+    // 16 9.7 / 8.9, 24 10.2 / 12.1.
+    const long long rows = (long long)max_new * (H / KV);
+    const bool many = rows >= AT_MIN_ROWS || (rows >= 8 && rows * KV * seqs * Dh >= AT_MIN_WORK);
+    if (f32 && vec4 && ((uintptr_t)out & 15) == 0 && page_size % AR_STRIP == 0 && H / KV <= AT_ROWS && many && KV <= 65535 && seqs <= 65535) {
 #define AT_GO(D) at_launch<D>(q, k_pool, v_pool, out, page_table, seq_slot, seq_start, seq_len, seqs, max_new, H, KV, mpps, page_size, num_pages, \
                               scale, window, keep, sink, softcap, bias, err_flag, stream)
         if (Dh == 64) return AT_GO(64);
