@@ -171,7 +171,7 @@ __device__ __forceinline__ void mt_place(int t, int row_tiles, int col_tiles, in
 struct MtTail {
     unsigned long long full[MT_STAGES], empty[MT_STAGES], acc_full[2], acc_empty[2], drained;
     unsigned tmem_base;
-    int dead;
+    int dead, peer_dead;                   // somebody has given up in this block; in the other one (written by it when its roles are over)
     int fills[2];                          // how often the block's copying warps have filled a stage: a, W
 };
 static_assert(sizeof(MtTail) <= 256, "the tail fits behind the stages");
@@ -254,7 +254,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tail.drained)));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        tail.dead = 0;
+        tail.dead = tail.peer_dead = 0;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -401,10 +401,11 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (rank == 1 && tid == 0) ri_mbar_wait(&tail.drained, 0);     // the last commit has reached this block as well
+    if (tid == 0) asm volatile("st.shared::cluster.s32 [%0], %1;\n" ::"r"(mt_in_block(&tail.peer_dead, rank ^ 1)), "r"(*(volatile int*)&tail.dead) : "memory");
+    __syncwarp();
     mt_cluster_sync();                             // nobody leaves while the other block may still signal its barriers
-    int gave_up;
-    asm volatile("ld.shared::cluster.s32 %0, [%1];\n" : "=r"(gave_up) : "r"(mt_in_block(&tail.dead, rank ^ 1)) : "memory");
-    if (gave_up | *(volatile int*)&tail.dead) {    // (the same in both blocks, whose roles are all over)
+    // (from here on a block may be gone, unless both know that somebody gave up: nothing of the other one's is read before that is known)
+    if (*(volatile int*)&tail.dead | *(volatile int*)&tail.peer_dead) {
         if (tid == 0) mt_land(&map_a, &map_w, tail, smem_u32(mt_smem), rank);
         __syncthreads();
         mt_cluster_sync();
